@@ -833,12 +833,6 @@ constexpr int kOuterNb = 4 * kLuNb;   // 256: width of the big exact trailing up
 constexpr int kSwapMapInts = kSwapMapStride;  // one panel's swap map (257 ints used): 2 KB per slot
 constexpr int kLookaheadMinN = 1024;  // smaller factorisations run their steps in order on one stream
 constexpr int kLookaheadCtas = kMaxPanelCtas;  // SMs kept for the look-ahead block beside the trailing update
-// Below this many trailing rows the next block's factorisation (linear in the rows) outlasts the trailing
-// update (quadratic): the side stream then forks as soon as the next block's own columns are ready, and the
-// rest of the step's interchanges and U row follow beside it.  Above it they stay before the fork, on all
-// SMs, where they shorten the update stream that bounds the step.
-constexpr int kEarlyForkRows = 12288;
-
 size_t lu_df_workspace_bytes(int n) {
   // panel scratch (rounded up to 256 B), the swap maps of two 256-column blocks' panels, the digit scratch of
   // the trailing update and that of the look-ahead block's own updates (the two run at the same time)
@@ -997,7 +991,10 @@ int lu_factor_df(int n, float* Whi, float* Wlo, int64_t ld, int32_t* piv, void* 
     for (int k = K0, p = 0; k < KE; k += nb, ++p) {
       const int w = std::min(nb, KE - k);
       int32_t* map = block_maps(K0) + p * kSwapMapInts;
-      e = launch_panel_f32(Whi, ld, n, k, w, piv, recs, map, st, us);
+      // on a cluster while its registers hold the rows (up to 12,288), else on up to 32 CTAs that meet in L2: at
+      // 12,000 rows 121 us against 176 for 64 columns, at 4,000 80 against 146, at 600 72 against 130
+      e = panel_cluster(Whi, ld, n, k, w, piv, map, st, us);
+      if (e == UPDES_ERR_UNSUPPORTED) e = launch_panel_f32(Whi, ld, n, k, w, piv, recs, map, st, us);
       if (e == UPDES_ERR_UNSUPPORTED)
         e = launch_panel<float, true>(Whi, Wlo, ld, Whi, ld, n, k, w, piv, bar, cand, cand_row, diag_row, map, st,
                                       us);
@@ -1033,13 +1030,13 @@ int lu_factor_df(int n, float* Whi, float* Wlo, int64_t ld, int32_t* piv, void* 
     UPDES_LAUNCH_CHECK();
     return UPDES_OK;
   };
-  // Block row of U for block [K0, KE) on trailing columns [c0, c1), the updates on at most ctas CTAs.
-  auto block_row = [&](int K0, int KE, int c0, int c1, int ctas) -> int {
+  // Block row of U for block [K0, KE) on trailing columns [c0, c1).
+  auto block_row = [&](int K0, int KE, int c0, int c1) -> int {
     for (int b = K0; b < KE; b += nb) {
       const int w = std::min(nb, KE - b);
       if (int e = trsm(b, w, c0, c1, s)) return e;
       if (b + w < KE)
-        if (int e = upd(b + w, KE, c0, c1, b, b + w, s, digits, digits_bytes, ctas)) return e;
+        if (int e = upd(b + w, KE, c0, c1, b, b + w, s, digits, digits_bytes, 0)) return e;
     }
     return UPDES_OK;
   };
@@ -1048,31 +1045,23 @@ int lu_factor_df(int n, float* Whi, float* Wlo, int64_t ld, int32_t* piv, void* 
   int e;
   if (lookahead && (e = side.create(s))) return e;
   const int rest_ctas = std::max(num_sms() - kLookaheadCtas, num_sms() / 2);
-  // UPDES_EARLY_FORK_ROWS overrides kEarlyForkRows (same factors either way)
-  static const int early_rows = [] {
-    const char* v = std::getenv("UPDES_EARLY_FORK_ROWS");
-    return v ? std::atoi(v) : kEarlyForkRows;
-  }();
   int K0 = 0, KE = std::min(kOuter, n);
   if ((e = factor_block(K0, KE, false, s, 0))) return e;
   bool pending = false;  // block [K0, KE) was factored beside the update: its outside interchanges are due
   while (KE < n) {
     const int KE2 = std::min(KE + kOuter, n);
-    const bool early_fork = lookahead && KE2 < n && n - KE <= early_rows;
-    // what the next block [KE, KE2) needs before it can be factored: this block's interchanges, U row and
-    // update on its columns (with an early fork), or on all trailing columns
-    const int c1 = early_fork ? KE2 : n;
-    if (pending && (e = swaps_deferred(K0, KE, KE, c1, !early_fork))) return e;
-    if ((e = block_row(K0, KE, KE, c1, 0))) return e;
+    // What the next block [KE, KE2) needs before it can be factored is this block's interchanges, U row and update
+    // on its own columns.  The interchanges and the U row of all trailing columns go first all the same, on all SMs:
+    // with panels of 1.2 to 1.9 us a column the next block is done before the rest of the update in any case (a
+    // fork ahead of them below 6,144 trailing rows: 27.48 ms against 27.55 at n = 10,006, 130.9 against 129.4 at
+    // 22,506).
+    if (pending && (e = swaps_deferred(K0, KE, KE, n, true))) return e;
+    if ((e = block_row(K0, KE, KE, n))) return e;
     if ((e = upd(KE, n, KE, KE2, K0, KE, s, digits, digits_bytes, 0))) return e;
     if (lookahead && KE2 < n) {
       // the next block on the side stream; the rest of this step on this stream, on the SMs it leaves
       if ((e = side.start())) return e;
       if ((e = factor_block(KE, KE2, true, side.side, kLookaheadCtas))) return e;
-      if (early_fork) {
-        if (pending && (e = swaps_deferred(K0, KE, KE2, n, true))) return e;
-        if ((e = block_row(K0, KE, KE2, n, rest_ctas))) return e;
-      }
       if ((e = upd(KE, n, KE2, n, K0, KE, s, digits, digits_bytes, rest_ctas))) return e;
       if ((e = side.finish())) return e;
       pending = true;
