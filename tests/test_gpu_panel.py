@@ -35,6 +35,38 @@ def test_mixed_panel_backward_error(n):
     assert np.max(np.abs(L)) <= 1 + 2.0 ** -22  # the multipliers of a partial pivoting, rounded in FP32
 
 
+@pytest.mark.parametrize("n", SIZES + [1100, 1281, 2400])
+def test_fp64_lu(n):
+    from scipy.linalg import lapack
+    A, F, _, piv, _, _ = lu_factor_random(n, 0, n)
+    PA, L, U, p = _reconstruct(A, F, piv)
+    _, want, _ = lapack.dgetrf(A)
+    assert np.array_equal(p, want)
+    # the trailing updates (at most n / 256 + 12 of an entry) cut each operand at 2^-56 of a power of two up to twice
+    # its row's (column's) largest entry and leave out products that sum to at most 2^-43 of the two largest ones in
+    # the worst case; the panels and triangular solves round like FP64 arithmetic
+    worst = np.max(np.abs(L), axis=1)[:, None] * np.max(np.abs(U), axis=0)[None, :]
+    assert np.all(np.abs(PA - L @ U) <= (n / 256 + 12) * 2.0 ** -43 * worst + n * 2.0 ** -53 * (np.abs(L) @ np.abs(U)))
+    # and on random data it is as good as LAPACK's own factors
+    lu, _, _ = lapack.dgetrf(A)
+    ref = np.linalg.norm(PA - (np.tril(lu, -1) + np.eye(n)) @ np.triu(lu))
+    assert np.linalg.norm(PA - L @ U) <= 4 * ref + 1e-300
+
+
+def test_fp64_update_scales():
+    # rows and columns of very different size, exact zeros and a zero row, against LAPACK column by column
+    from scipy.linalg import lapack
+    rng = np.random.default_rng(3)
+    n = 700
+    A = rng.standard_normal((n, n)) * 2.0 ** rng.integers(-300, 300, n)[None, :]
+    A[rng.random((n, n)) < 0.3] = 0.0
+    st, info, F, piv = _factor(A, 0)
+    assert st == 0 and info == 0
+    PA, L, U, p = _reconstruct(A, F, piv)
+    scale = np.max(np.abs(A), axis=0)
+    assert np.max(np.abs((PA - L @ U) / scale)) <= 1e-12
+
+
 def _factor(A, precision):
     import torch
     from updes_gb300 import _lib

@@ -17,3 +17,10 @@ size_t ozaki3_scratch_bytes(int mmax, int ncmax, int Kmax);
 int ozaki3_update(float* Chi, float* Clo, int64_t ldc, const float* A, int64_t lda, const float* B, int64_t ldb,
                   int m, int nc, int K, void* scratch, size_t scratch_bytes, DeviceStatus* st, cudaStream_t s,
                   int max_ctas = 0, bool a_digits_ready = false);
+
+// C (FP64, ldc) -= A (m x K FP64, lda) * B (K x nc FP64, ldb), K <= 256, from exact products of 7 digits of each
+// operand (gemm_tc64.cu); scratch, max_ctas and a_digits_ready as for ozaki3_update.
+size_t ozaki64_scratch_bytes(int mmax, int ncmax, int Kmax);
+int ozaki64_update(double* C, int64_t ldc, const double* A, int64_t lda, const double* B, int64_t ldb, int m, int nc,
+                   int K, void* scratch, size_t scratch_bytes, DeviceStatus* st, cudaStream_t s, int max_ctas = 0,
+                   bool a_digits_ready = false);

@@ -29,11 +29,11 @@
 // word and an abort flag that every role checks, and tensor memory is freed on every path.
 #include <atomic>
 
-#include <cuda.h>
 #include <cuda_bf16.h>
 
 #include "gemm_tc.cuh"
 #include "stats.cuh"
+#include "tc.cuh"
 
 namespace {
 
@@ -55,10 +55,6 @@ static_assert(kSmemBytes <= 227 * 1024, "shared memory");
 
 // instruction descriptor: D = F32, A = B = BF16, both K-major, N = 64, M = 128
 constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(TN >> 3) << 17) | (uint32_t(TM >> 4) << 24);
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
 
 // tcgen05 shared-memory matrix descriptor: K-major, 128B swizzle, 8-row groups 1024 B apart.
 __device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
@@ -93,52 +89,6 @@ __device__ __forceinline__ void fast_two_sum2(float2 a, float2 b, float2& s, flo
   e = sub2(b, sub2(s, a));
 }
 
-// ---- mbarrier / tcgen05 / TMA primitives -------------------------------------------------------------
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t phase) {
-  uint32_t ok;
-  asm volatile(
-      "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(phase)
-      : "memory");
-  return ok != 0;
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-
-// Bounded wait; gives up when the abort flag is raised by another role.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase, volatile int* abort_flag) {
-  for (long long it = 0; it < kTcSpinLimit; ++it) {
-    if (mbar_try_wait(bar, phase)) return true;
-    if ((it & 63) == 63 && *abort_flag) return false;
-    if (it > 256) __nanosleep(32);
-  }
-  return false;
-}
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-// D (+)= A * B with both operands from shared-memory descriptors; ACC = false overwrites D.
-template <bool ACC>
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(kIdesc), "n"(ACC ? 1 : 0)
-      : "memory");
-}
-
 // The 32 MMAs of one k block: digit products (a, b) with a + b <= 3 (d2 * e2 is below the digit cut), four
 // k-steps of 16 each, into accumulator group a + b.  Descriptors are built once; every operand offset is a
 // compile-time constant added to them (descriptor address units are 16 bytes: a digit plane of A is 1024
@@ -151,69 +101,9 @@ __device__ __forceinline__ void mma_product(uint32_t tset, uint64_t a0, uint64_t
 #pragma unroll
   for (int kk = 0; kk < TK / 16; ++kk) {
     const uint64_t ad = a0 + uint64_t(A * (kATile >> 4) + kk * 2), bd = b0 + uint64_t(B * (kBTile >> 4) + kk * 2);
-    if (first && kk == 0) mma_bf16<false>(d, ad, bd);
-    else mma_bf16<true>(d, ad, bd);
+    if (first && kk == 0) mma_bf16<false>(d, ad, bd, kIdesc);
+    else mma_bf16<true>(d, ad, bd, kIdesc);
   }
-}
-
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
-}
-
-__device__ __forceinline__ void tmem_ld4(uint32_t taddr, float* v) {
-  uint32_t r[4];
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
-               : "r"(taddr)
-               : "memory");
-#pragma unroll
-  for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-
-// L2 eviction policies for the copies below: the digit tiles of L and U are reused by every tile of their
-// row band / column across the whole launch, while each C tile is read and written once; marking C
-// evict-first and the digits evict-last keeps the streamed C planes (gigabytes per launch at n = 22,506) from
-// pushing the digit tiles out of L2 between their uses.
-__device__ __forceinline__ uint64_t l2_policy_evict_last() {
-  uint64_t p;
-  asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
-__device__ __forceinline__ uint64_t l2_policy_evict_first() {
-  uint64_t p;
-  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-  return p;
-}
-
-// 3-D tiled TMA load (x = k offset, y = row, z = digit plane) completing on an mbarrier, with an L2 policy.
-__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar,
-                                            uint64_t policy) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
-      " [%0], [%1, {%2, %3, %4}], [%5], %6;" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar)), "l"(policy)
-      : "memory");
-}
-
-// 2-D tiled TMA load (x = column, y = row) completing on an mbarrier, and the matching bulk-group store, with
-// an L2 policy.
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint64_t* bar,
-                                            uint64_t policy) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint"
-      " [%0], [%1, {%2, %3}], [%4], %5;" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar)), "l"(policy)
-      : "memory");
-}
-
-__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int y, uint32_t src, uint64_t policy) {
-  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group.L2::cache_hint [%0, {%1, %2}], [%3], %4;" ::"l"(
-                   reinterpret_cast<uint64_t>(map)),
-               "r"(x), "r"(y), "r"(src), "l"(policy)
-               : "memory");
 }
 
 // ---- digit pre-pass ------------------------------------------------------------------------------------
@@ -593,24 +483,6 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
-// cuTensorMapEncodeTiled, resolved at run time through the runtime's entry-point query, so the library
-// does not link against the driver library and still loads on hosts without a GPU driver.
-using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiledFn encode_tiled() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
-    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-  }
-  return fn;
-}
-
 // 3-D map over digit planes [3][rows][Kp] bf16, box 64 (k) x box_rows x 1, 128B swizzle
 int make_map(CUtensorMap* map, void* base, int rows, int Kp, int box_rows) {
   cuuint64_t dims[3] = {cuuint64_t(Kp), cuuint64_t(rows), cuuint64_t(kDigits)};
@@ -637,17 +509,6 @@ int make_map_c(CUtensorMap* map, float* base, int rows, int cols, int64_t ld) {
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? UPDES_OK : UPDES_ERR_CUDA;
-}
-
-int num_sms_cached() {
-  static std::atomic<int> sms{0};
-  if (!sms.load()) {
-    int dev = 0, v = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    sms.store(v > 0 ? v : 1);
-  }
-  return sms.load();
 }
 
 }  // namespace

@@ -1,11 +1,9 @@
 // Blocked right-looking LU with partial pivoting and triangular solves.
 //
-// Two storage schemes share the kernels:
-//   * FP64 LU: the working matrix W (FP64) is factored in place (F == W).
-//   * mixed LU: W (FP64) holds the not-yet-factored trailing matrix; the
-//     factors are stored in FP32 in F.  Every product of factor entries is
-//     formed from the FP32 values and accumulated in FP64 into W, so the
-//     Schur complements keep FP64 accuracy while L and U are FP32.
+// Two storage schemes:
+//   * FP64 LU: the working matrix W (FP64) is factored in place.
+//   * mixed LU: two FP32 planes hold the not-yet-factored trailing matrix in
+//     double-float; the factors are stored in FP32 over the hi plane.
 // Replaces the LAPACK getrf behind jnp.linalg.inv (updes/assembly.py:87-90)
 // and the lineax QR factorisation (updes/operators.py:612-613).
 #include <cooperative_groups.h>
@@ -378,84 +376,90 @@ __global__ void __launch_bounds__(256) trsm_df64_kernel(float* Whi, const float*
   }
 }
 
-// Apply the row interchanges piv[k0, k0+cnt) to columns [c0, c1) of M.
-template <typename T>
-__global__ void laswp_kernel(T* __restrict__ M, int64_t ld, const int32_t* __restrict__ piv, int k0, int cnt,
-                             int64_t c0, int64_t c1) {
-  const int64_t c = c0 + int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (c >= c1) return;
-  for (int i = k0; i < k0 + cnt; ++i) {
-    const int p = piv[i];
-    if (p != i) {
-      T a = M[int64_t(i) * ld + c];
-      M[int64_t(i) * ld + c] = M[int64_t(p) * ld + c];
-      M[int64_t(p) * ld + c] = a;
-    }
-  }
-}
+// ---- FP64 interchanges and triangular solve ---------------------------------------------------------------
+// W[k:k+NBK, c0:c1] <- L11^-1 W[k:k+NBK, c0:c1], L11 unit lower in W[k:k+w, k:k+w] (w <= NBK), 32 columns a CTA,
+// four lanes a column: lane s keeps rows s, s + 4, ... in registers, row j goes round by shuffle.  With a swap map
+// (a panel's, w <= 32) the panel's interchanges are applied to the columns on the way in; the first left_ctas CTAs
+// take 32 columns from `left` on and only interchange.  Bound by the FP64 pipe: NBK^2 / 2 multiply-adds a column
+// (64 rows of 10,000 columns: 33 us at two a cycle and SM).
+template <int NBK>
+struct Trsm64Smem {
+  double L[NBK][NBK + 1];
+  double X[NBK][33];
+  double moved[2 * 32][33];
+};
 
-// U12 = L11^-1 W12 (L11 unit lower from F), one thread per column, FP64 arithmetic.
-template <typename TF>
-__global__ void __launch_bounds__(64) trsm_kernel(double* W, int64_t ldw, TF* F,
-                                                  int64_t ldf, int n, int k, int nb) {
-  extern __shared__ double sL[];  // nb x nb
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-    const int i = e / nb, j = e % nb;
-    sL[e] = (j < i) ? double(F[int64_t(k + i) * ldf + k + j]) : 0.0;
+template <int NBK>
+__global__ void __launch_bounds__(128) trsm64_kernel(double* W, int64_t ld, int k, int w, int64_t c0, int64_t c1,
+                                                     const int32_t* __restrict__ map, int64_t left, int64_t left_end,
+                                                     int left_ctas) {
+  extern __shared__ double trsm64_smem[];
+  Trsm64Smem<NBK>& sm = *reinterpret_cast<Trsm64Smem<NBK>*>(trsm64_smem);
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  const bool only_swap = int(blockIdx.x) < left_ctas;
+  const int64_t cb = only_swap ? left + int64_t(blockIdx.x) * 32 : c0 + (int64_t(blockIdx.x) - left_ctas) * 32;
+  const int64_t ce = only_swap ? left_end : c1;
+  const bool in = cb + lane < ce;
+  if (!only_swap)
+    for (int i = wid; i < NBK; i += 4)
+      for (int j = lane; j < NBK; j += 32) sm.L[i][j] = (j < i && i < w) ? W[int64_t(k + i) * ld + k + j] : 0.0;
+  if (map) {
+    const int cnt = map[0];
+    for (int q = wid; q < cnt; q += 4) sm.moved[q][lane] = in ? W[int64_t(map[129 + q]) * ld + cb + lane] : 0.0;
+    __syncthreads();
+    for (int q = wid; q < cnt; q += 4) {
+      const int r = map[1 + q];
+      const double v = sm.moved[q][lane];
+      if (!only_swap && r < k + w) sm.X[r - k][lane] = v;  // destinations below k + w are the panel's own rows
+      else if (in) W[int64_t(r) * ld + cb + lane] = v;
+    }
+    for (int i = w + wid; i < NBK; i += 4) sm.X[i][lane] = 0.0;
+  } else {
+    for (int i = wid; i < NBK; i += 4) sm.X[i][lane] = (in && i < w) ? W[int64_t(k + i) * ld + cb + lane] : 0.0;
   }
+  if (only_swap) return;
   __syncthreads();
-  const int64_t c = int64_t(k) + nb + int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (c >= n) return;
-  double x[128];
-  for (int i = 0; i < nb; ++i) {
-    double s = W[int64_t(k + i) * ldw + c];
-    for (int j = 0; j < i; ++j) s -= sL[i * nb + j] * x[j];
-    x[i] = s;
+  const int col = tid >> 2, s = tid & 3, gbase = lane & ~3;
+  double x[NBK / 4];
+#pragma unroll
+  for (int q = 0; q < NBK / 4; ++q) x[q] = sm.X[s + 4 * q][col];
+#pragma unroll
+  for (int j = 0; j < NBK; ++j) {
+    const double xj = __shfl_sync(0xffffffffu, x[j >> 2], gbase | (j & 3));
+#pragma unroll
+    for (int q = j >> 2; q < NBK / 4; ++q) {
+      const int i = s + 4 * q;
+      const double t = fma(-sm.L[i][j], xj, x[q]);
+      if (4 * q > j || i > j) x[q] = t;
+    }
   }
-  for (int i = 0; i < nb; ++i) F[int64_t(k + i) * ldf + c] = TF(x[i]);
+#pragma unroll
+  for (int q = 0; q < NBK / 4; ++q) sm.X[s + 4 * q][col] = x[q];
+  __syncthreads();
+  for (int i = wid; i < w; i += 4)
+    if (in) W[int64_t(k + i) * ld + cb + lane] = sm.X[i][lane];
 }
 
-// W[r0:n, c0:n] -= F[r0:n, k:k+nb] * F[k:k+nb, c0:n], FP64 accumulation (SIMT reference path).
-template <typename TF>
-__global__ void __launch_bounds__(256) gemm_update_kernel(double* W, int64_t ldw,
-                                                          const TF* F, int64_t ldf, int n, int k,
-                                                          int nb) {
-  __shared__ double As[32][65];
-  __shared__ double Bs[32][65];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int r0 = k + nb + blockIdx.y * 64, c0 = k + nb + blockIdx.x * 64;
-  double acc[4][4] = {};
-  for (int kb = 0; kb < nb; kb += 32) {
-    for (int e = threadIdx.x; e < 64 * 32; e += 256) {
-      const int i = e >> 5, j = e & 31;           // A: row i, k-column j
-      const int ra = r0 + i;
-      As[j][i] = (ra < n && kb + j < nb) ? double(F[int64_t(ra) * ldf + k + kb + j]) : 0.0;
-      const int kr = e >> 6, cj = e & 63;         // B: k-row kr, column cj
-      const int cb = c0 + cj;
-      Bs[kr][cj] = (kb + kr < nb && cb < n) ? double(F[int64_t(k + kb + kr) * ldf + cb]) : 0.0;
-    }
+// The interchanges of nmaps consecutive 32-wide panels on columns [a0, a1) and [b0, b1), 32 columns a CTA, each CTA
+// applying the maps in panel order.
+__global__ void __launch_bounds__(256) swap_rows64_maps_kernel(double* W, int64_t ld, const int32_t* __restrict__ maps,
+                                                               int nmaps, int64_t a0, int64_t a1, int64_t b0,
+                                                               int64_t b1) {
+  __shared__ double buf[64][32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int na = int(ceil_div(a1 - a0, 32));
+  const bool first = int(blockIdx.x) < na;
+  const int64_t c = (first ? a0 + int64_t(blockIdx.x) * 32 : b0 + (int64_t(blockIdx.x) - na) * 32) + lane;
+  const bool in = c < (first ? a1 : b1);
+  for (int m = 0; m < nmaps; ++m) {
+    const int32_t* map = maps + m * kSwapMapStride;
+    const int cnt = map[0];
+    for (int q = wid; q < cnt; q += 8)
+      if (in) buf[q][lane] = W[int64_t(map[129 + q]) * ld + c];
     __syncthreads();
-#pragma unroll 8
-    for (int kk = 0; kk < 32; ++kk) {
-      double a[4], b[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) { a[u] = As[kk][ty + 16 * u]; b[u] = Bs[kk][tx + 16 * u]; }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) acc[u][v] = fma(a[u], b[v], acc[u][v]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int r = r0 + ty + 16 * u;
-    if (r >= n) continue;
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int c = c0 + tx + 16 * v;
-      if (c < n) W[int64_t(r) * ldw + c] -= acc[u][v];
-    }
+    for (int q = wid; q < cnt; q += 8)
+      if (in) W[int64_t(map[1 + q]) * ld + c] = buf[q][lane];
+    __syncthreads();  // this map's rows are in place (and buf free) before the next map reads them
   }
 }
 
@@ -1076,60 +1080,132 @@ int lu_factor_df(int n, float* Whi, float* Wlo, int64_t ld, int32_t* piv, void* 
   return UPDES_OK;
 }
 
-template <typename TF>
-int lu_factor_impl(int n, double* W, int64_t ldw, TF* F, int64_t ldf, int32_t* piv, void* ws, size_t ws_bytes,
-                   DeviceStatus* st, cudaStream_t s, const LuHooks* hooks) {
-  const int nb = kLuNb;
-  if (ws_bytes < lu_panel_workspace_bytes(nb)) return UPDES_ERR_WORKSPACE;
+// FP64 LU with LAPACK's pivots, in place.  Blocks of 256 columns of 32-wide panels; every update of the block's own
+// columns (K = 32), of the block row of U (K = 64) and of the trailing matrix (K = 256) runs on the tensor cores
+// (gemm_tc64.cu).  Panels are 32 wide because the FP64 pipe of the cluster's SMs bounds them (half the multiply-adds
+// of 64).  The look-ahead is that of lu_factor_df: the next block on a second stream beside the update of the rest.
+namespace {
+constexpr int kNb64 = 32;
+constexpr int kMaps64 = kOuterNb / kNb64;
+}  // namespace
+
+size_t lu_64_workspace_bytes(int n) {
+  return ((lu_panel_workspace_bytes(kLuNb) + 255) & ~size_t(255)) + 2 * size_t(kMaps64) * kSwapMapInts * 4 +
+         ozaki64_scratch_bytes(n, n, kOuterNb) + ozaki64_scratch_bytes(n, kOuterNb, kNb64);
+}
+
+int lu_factor_64(int n, double* W, int64_t ld, int32_t* piv, void* ws, size_t ws_bytes, DeviceStatus* st,
+                 cudaStream_t s) {
+  if (ws_bytes < lu_64_workspace_bytes(n)) return UPDES_ERR_WORKSPACE;
   char* base = static_cast<char*>(ws);
   unsigned int* bar = reinterpret_cast<unsigned int*>(base);
   Cand* cand = reinterpret_cast<Cand*>(base + 256);
   double* cand_row = reinterpret_cast<double*>(base + 256 + 2 * 1024 * sizeof(Cand));
-  double* diag_row = cand_row + 2ll * 1024 * nb;
+  double* diag_row = cand_row + 2ll * 1024 * kLuNb;
+  char* after = base + ((lu_panel_workspace_bytes(kLuNb) + 255) & ~size_t(255));
+  int32_t* swap_maps = reinterpret_cast<int32_t*>(after);
+  char* digits = after + 2 * size_t(kMaps64) * kSwapMapInts * 4;
+  const size_t digits_bytes = ozaki64_scratch_bytes(n, n, kOuterNb);
+  char* digits_la = digits + digits_bytes;
+  const size_t digits_la_bytes = ozaki64_scratch_bytes(n, kOuterNb, kNb64);
+  auto block_maps = [&](int K0) { return swap_maps + ((K0 / kOuterNb) & 1) * kMaps64 * kSwapMapInts; };
+  static const bool lookahead_on = [] {
+    const char* v = std::getenv("UPDES_LOOKAHEAD");
+    return !(v && v[0] == '0');
+  }();
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  UPDES_CUDA_TRY(cudaStreamIsCapturing(s, &cs));
+  const bool lookahead = lookahead_on && n >= kLookaheadMinN && cs == cudaStreamCaptureStatusNone;
   UPDES_CUDA_TRY(cudaMemsetAsync(bar, 0, 256 + 2 * 1024 * sizeof(Cand), s));  // barrier words and candidate tags
-  // the single-exchange panel's records live in the candidate-row area (tags must start at zero)
-  PanelRec* recs = reinterpret_cast<PanelRec*>(cand_row);
-  static_assert(2 * (kMaxPanelCtas + 1) * sizeof(PanelRec) <= 2 * 1024 * kLuNb * sizeof(double), "panel records");
-  UPDES_CUDA_TRY(cudaMemsetAsync(recs, 0, 2 * (kMaxPanelCtas + 1) * sizeof(PanelRec), s));
-  for (int k = 0; k < n; k += nb) {
-    const int w = std::min(nb, n - k);
-    {
-      int e = launch_panel<TF, false>(W, nullptr, ldw, F, ldf, n, k, w, piv, bar, cand, cand_row, diag_row,
-                                      nullptr, st, s);
+
+  auto trsm = [&](int k, int w, int64_t c0, int64_t c1, const int32_t* map, int64_t left, int64_t left_end,
+                  cudaStream_t us) -> int {
+    const int lc = map ? int(ceil_div(left_end - left, 32)) : 0, tc = c1 > c0 ? int(ceil_div(c1 - c0, 32)) : 0;
+    if (lc + tc == 0) return UPDES_OK;
+    StatScope sc(kStatTrsm, us, double(w) * w * (c1 - c0), double(w) * (c1 - c0) * 16.0);
+    static std::atomic<unsigned long long> attr32{0}, attr64{0};
+    if (w <= 32) {
+      if (int e = smem_opt_in((const void*)trsm64_kernel<32>, int(sizeof(Trsm64Smem<32>)), attr32)) return e;
+      trsm64_kernel<32><<<unsigned(lc + tc), 128, sizeof(Trsm64Smem<32>), us>>>(W, ld, k, w, c0, c1, map, left,
+                                                                               left_end, lc);
+    } else {
+      if (int e = smem_opt_in((const void*)trsm64_kernel<64>, int(sizeof(Trsm64Smem<64>)), attr64)) return e;
+      trsm64_kernel<64><<<unsigned(lc + tc), 128, sizeof(Trsm64Smem<64>), us>>>(W, ld, k, w, c0, c1, map, left,
+                                                                               left_end, lc);
+    }
+    UPDES_LAUNCH_CHECK();
+    return UPDES_OK;
+  };
+  // W[r0:r1, c0:c1] -= W[r0:r1, k0:k1] * W[k0:k1, c0:c1]; the digits of A of the last update on `digits` are reused
+  // when the rows and k range are the same (the rest of the trailing matrix after the next block's columns)
+  struct {
+    int r0 = -1, r1 = -1, k0 = -1, k1 = -1;
+  } last;
+  auto upd = [&](int r0, int r1, int c0, int c1, int k0, int k1, cudaStream_t us, bool la, int ctas) -> int {
+    const bool ready = !la && last.r0 == r0 && last.r1 == r1 && last.k0 == k0 && last.k1 == k1;
+    const int e = ozaki64_update(W + int64_t(r0) * ld + c0, ld, W + int64_t(r0) * ld + k0, ld,
+                                 W + int64_t(k0) * ld + c0, ld, r1 - r0, c1 - c0, k1 - k0, la ? digits_la : digits,
+                                 la ? digits_la_bytes : digits_bytes, st, us, ctas, ready);
+    if (!la) last = {r0, r1, k0, k1};
+    return e;
+  };
+  // Columns [K0, KE): panels, their interchanges inside the block (panel p's swap map stays in slot p for the columns
+  // outside) and the block's own updates.
+  auto factor_block = [&](int K0, int KE, cudaStream_t us, bool la, int ctas) -> int {
+    for (int k = K0, p = 0; k < KE; k += kNb64, ++p) {
+      const int w = std::min(kNb64, KE - k);
+      int32_t* map = block_maps(K0) + p * kSwapMapInts;
+      int e = panel_cluster(W, ld, n, k, w, piv, map, st, us);
+      if (e == UPDES_ERR_UNSUPPORTED)
+        e = launch_panel<double, false>(W, nullptr, ld, W, ld, n, k, w, piv, bar, cand, cand_row, diag_row, map, st,
+                                        us);
       if (e) return e;
+      if ((e = trsm(k, w, k + w, KE, map, K0, k, us))) return e;
+      if (k + w < KE && (e = upd(k + w, n, k + w, KE, k, k + w, us, la, ctas))) return e;
     }
-    // row interchanges: factored columns [0, k) of F, trailing columns [k+w, n) of W
-    if (k > 0) {
-      laswp_kernel<TF><<<unsigned(ceil_div(k, 256)), 256, 0, s>>>(F, ldf, piv, k, w, 0, k);
-      UPDES_LAUNCH_CHECK();
+    return UPDES_OK;
+  };
+  // The interchanges of block [K0, KE) on the columns outside it.
+  auto swaps_outside = [&](int K0, int KE) -> int {
+    const int64_t chunks = ceil_div(K0, 32) + ceil_div(n - KE, 32);
+    if (chunks == 0) return UPDES_OK;
+    const int nmaps = int(ceil_div(KE - K0, kNb64));
+    StatScope sc(kStatOther, s, 0.0, 2.0 * 2 * kNb64 * nmaps * double(n - (KE - K0)) * 8.0);
+    swap_rows64_maps_kernel<<<unsigned(chunks), 256, 0, s>>>(W, ld, block_maps(K0), nmaps, 0, K0, KE, n);
+    UPDES_LAUNCH_CHECK();
+    return UPDES_OK;
+  };
+
+  SideStream side;
+  int e;
+  if (lookahead && (e = side.create(s))) return e;
+  const int rest_ctas = std::max(num_sms() - kLookaheadCtas, num_sms() / 2);
+  int K0 = 0, KE = std::min(kOuterNb, n);
+  if ((e = factor_block(K0, KE, s, false, 0))) return e;
+  for (;;) {
+    if ((e = swaps_outside(K0, KE))) return e;
+    if (KE >= n) break;
+    const int KE2 = std::min(KE + kOuterNb, n);
+    for (int b = K0; b < KE; b += kLuNb) {  // block row of U
+      const int w = std::min(kLuNb, KE - b);
+      if ((e = trsm(b, w, KE, n, nullptr, 0, 0, s))) return e;
+      if (b + w < KE && (e = upd(b + w, KE, KE, n, b, b + w, s, false, 0))) return e;
     }
-    if (k + w < n) {
-      laswp_kernel<double><<<unsigned(ceil_div(n - k - w, 256)), 256, 0, s>>>(W, ldw, piv, k, w, k + w, n);
-      UPDES_LAUNCH_CHECK();
-      {
-        StatScope sc(kStatTrsm, s, double(w) * w * (n - k - w), double(w) * (n - k - w) * (8.0 + sizeof(TF)));
-        trsm_kernel<TF><<<unsigned(ceil_div(n - k - w, 64)), 64, size_t(w) * w * sizeof(double), s>>>(W, ldw, F, ldf, n, k, w);
-        UPDES_LAUNCH_CHECK();
-      }
-      const double mm = double(n - k - w);
-      StatScope sc(kStatGemm, s, 2.0 * mm * mm * w, mm * mm * 16.0 + 2.0 * mm * w * sizeof(TF));
-      if (hooks && hooks->gemm) {
-        int e = hooks->gemm(hooks->ctx, n, k, w, W, ldw, F, ldf, s);
-        if (e) return e;
-      } else {
-        dim3 grid(unsigned(ceil_div(n - k - w, 64)), unsigned(ceil_div(n - k - w, 64)));
-        gemm_update_kernel<TF><<<grid, 256, 0, s>>>(W, ldw, F, ldf, n, k, w);
-        UPDES_LAUNCH_CHECK();
-      }
+    if ((e = upd(KE, n, KE, KE2, K0, KE, s, false, 0))) return e;
+    if (lookahead && KE2 < n) {
+      if ((e = side.start())) return e;
+      if ((e = factor_block(KE, KE2, side.side, true, kLookaheadCtas))) return e;
+      if ((e = upd(KE, n, KE2, n, K0, KE, s, false, rest_ctas))) return e;
+      if ((e = side.finish())) return e;
+    } else {
+      if (KE2 < n && (e = upd(KE, n, KE2, n, K0, KE, s, false, 0))) return e;
+      if ((e = factor_block(KE, KE2, s, false, 0))) return e;
     }
+    K0 = KE;
+    KE = KE2;
   }
   return UPDES_OK;
 }
-
-template int lu_factor_impl<double>(int, double*, int64_t, double*, int64_t, int32_t*, void*, size_t, DeviceStatus*,
-                                    cudaStream_t, const LuHooks*);
-template int lu_factor_impl<float>(int, double*, int64_t, float*, int64_t, int32_t*, void*, size_t, DeviceStatus*,
-                                   cudaStream_t, const LuHooks*);
 
 // ---------------------------------------------------------------------------
 // Triangular solves (single right-hand side, FP64 arithmetic on TF factors).

@@ -5,17 +5,10 @@
 
 constexpr int kLuNb = 64;  // panel width
 
-// Optional replacement of the trailing update W[k+nb:, k+nb:] -= F21 * F12.
-struct LuHooks {
-  void* ctx;
-  int (*gemm)(void* ctx, int n, int k, int nb, double* W, int64_t ldw, const void* F, int64_t ldf, cudaStream_t s);
-};
-
-size_t lu_panel_workspace_bytes(int nb);
-
-template <typename TF>
-int lu_factor_impl(int n, double* W, int64_t ldw, TF* F, int64_t ldf, int32_t* piv, void* ws, size_t ws_bytes,
-                   DeviceStatus* st, cudaStream_t s, const LuHooks* hooks);
+// FP64 LU in place, LAPACK's pivot choices (interchanges to piv[0, n)).
+size_t lu_64_workspace_bytes(int n);
+int lu_factor_64(int n, double* W, int64_t ld, int32_t* piv, void* ws, size_t ws_bytes, DeviceStatus* st,
+                 cudaStream_t s);
 
 // The panel W[k:n, k:k+w] (w <= 64) factored in place on one thread-block cluster (panel.cu): interchanges to
 // piv[k..k+w) and their net permutation to swap_map (257 ints, may be null).  UPDES_ERR_UNSUPPORTED when its rows do

@@ -480,7 +480,9 @@ size_t lu_ws_layout(int n, int precision, char* base, LuWs* out, bool lo_plane =
   Carve c{base};
   LuWs w;
   w.st = c.take<DeviceStatus>(1);
-  w.panel_bytes = precision == UPDES_PREC_FP32 ? lu_df_workspace_bytes(n) : lu_panel_workspace_bytes(kLuNb);
+  // a mixed solve may fall back to the FP64 factorisation in the same workspace
+  const size_t df = precision == UPDES_PREC_FP32 ? lu_df_workspace_bytes(n) : 0;
+  w.panel_bytes = (precision == UPDES_PREC_FP32 && lo_plane) ? df : std::max(df, lu_64_workspace_bytes(n));
   w.panel = c.take<char>(w.panel_bytes);
   w.sync = c.take<int>(ceil_div(n, 64) + 2);
   w.tmp = c.take<double>(n);
@@ -553,7 +555,7 @@ int factor_core(int n, double* A, int64_t lda, int precision, void* F, int64_t l
       A = Fd;
       lda = ldf;
     }
-    e = lu_factor_impl<double>(n, A, lda, A, lda, piv, w.panel, w.panel_bytes, w.st, s, nullptr);
+    e = lu_factor_64(n, A, lda, piv, w.panel, w.panel_bytes, w.st, s);
   }
   if (e) return e;
   return perm_core(n, piv, s);
