@@ -286,7 +286,7 @@ UPDES_API int updes_solve_factored(const updes_problem* p, int32_t nrhs, const d
  * sweep reaches FP64 quality; FP32 factors converge only as fast as classical
  * refinement on them allows.
  * updes_batch_prepare (once per factorisation; synchronises) derives the
- * batch's copy of the factors.  updes_solve_batch then only launches kernels on
+ * batch's copy of the factors, and the digits of K and of the value matrix.  updes_solve_batch then only launches kernels on
  * `stream`: no synchronisation and no host reads, so a time step built from it
  * can be captured in a CUDA graph.  A stale or missing preparation, and any
  * timed-out wait, land in the workspace's status word, which
@@ -308,6 +308,15 @@ UPDES_API int updes_workspace_status(const updes_problem* p, void* workspace, si
  * counterpart of updes_eval_values (kernel values regenerated once per pair, shared by the columns). */
 UPDES_API int updes_eval_values_batch(const updes_problem* p, int32_t R, const double* C, int64_t ldc, double* vals,
                                       int64_t ldv, void* stream);
+
+/*
+ * The same values from what updes_batch_prepare derived (the value matrix [Phi P] as digits, multiplied on the
+ * tensor cores): for callers that evaluate many blocks of one system, such as a time step after updes_solve_batch.
+ * workspace and batch_ws as there; a missing preparation gives NaN values.  UPDES_ERR_UNSUPPORTED on local supports.
+ */
+UPDES_API int updes_eval_values_prepared(const updes_problem* p, int32_t R, const double* C, int64_t ldc, double* vals,
+                                         int64_t ldv, void* workspace, size_t workspace_bytes, void* batch_ws,
+                                         size_t batch_ws_bytes, void* stream);
 
 /*
  * Many independent systems in one call: problems[i] (its own cloud, kernel and

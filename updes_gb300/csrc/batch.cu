@@ -4,17 +4,20 @@
 // (demos/Advection/00_advection_with_rbf.py:83-93); here the factors of updes_factor are reused and R
 // right-hand sides (R <= 64) advance together:
 //   X = M^-1 Bs;  repeat `sweeps` times:  X += M^-1 (Bs - Ks X)
-// with Ks the equilibrated K (double-float planes of the solve workspace) and M^-1 the LU factors
-// applied in double-float arithmetic.  FP64 factors are split once (updes_batch_prepare) into hi/lo FP32
-// planes, so M^-1 is as accurate as an FP64 triangular solve while running on the FP32 pipes; FP32
-// factors are used as they are (lo = 0).
+// with Ks the equilibrated K (the exact sum of the solve workspace's double-float planes) and M^-1 the LU factors
+// applied in double-float arithmetic.  updes_batch_prepare derives once per factorisation what the calls read:
+//   * the inverses of the factors' 64 x 64 diagonal blocks and each block row times its inverse, as hi/lo FP32
+//     planes (about as accurate as an FP64 triangular solve, on the FP32 pipes);
+//   * the digits of Ks and of the value matrix [Phi P] for the tensor-core products (gemm_tc64.cu).
 //
 // Every double-float accumulation renormalises after each term (fast two-sum), so its error stays at
 // about 2^-48 of the running sum however many terms a thread adds.
+#include <algorithm>
 #include <atomic>
 #include <cstring>
 
 #include "common.cuh"
+#include "gemm_tc.cuh"
 #include "lu.cuh"
 #include "stats.cuh"
 
@@ -22,31 +25,34 @@ namespace {
 
 constexpr int kB = 64;       // block rows
 constexpr int kMaxR = 64;    // right-hand sides per call
-constexpr int kRG = 16;      // right-hand sides per triangular-solve CTA
-constexpr int kGroups = kMaxR / kRG;
-constexpr int kParts = 4;    // split of the residual's inner dimension
+constexpr int kCG = 8;       // right-hand sides per triangular-solve CTA
+constexpr int kLdt = kB + 8; // row stride of a staged tile: the 4 rows x 8 columns a warp reads at once fall in 32 banks
+constexpr int kChunk = 256;  // value rows staged at a time
 
-// (sh, sl) += (a + al) * (b + bl), dropping al * bl; renormalised
-__device__ __forceinline__ void df_mac(float a, float al, float b, float bl, float& sh, float& sl) {
-  const float p = __fmul_rn(a, b);
-  const float e = __fmaf_rn(a, b, -p);
-  const float s = __fadd_rn(sh, p);
-  const float bb = __fsub_rn(s, sh);
-  float t = __fadd_rn(__fsub_rn(sh, __fsub_rn(s, bb)), __fsub_rn(p, bb));
-  t = __fadd_rn(t, __fadd_rn(sl, __fmaf_rn(a, bl, __fmaf_rn(al, b, e))));
-  sh = __fadd_rn(s, t);
-  sl = __fsub_rn(t, __fsub_rn(sh, s));
+__device__ __forceinline__ float2 sub2(float2 y, float2 x) { return __ffma2_rn(x, make_float2(-1.f, -1.f), y); }
+
+// Double-float accumulators of a pair of columns: (sh, sl) += (a + al) * (b + bl), dropping al * bl; renormalised.
+// Packed FP32x2 instructions, one issue slot a pair.
+__device__ __forceinline__ void df_mac2(float a, float al, float2 b, float2 bl, float2& sh, float2& sl) {
+  const float2 a2 = make_float2(a, a), al2 = make_float2(al, al);
+  const float2 p = __fmul2_rn(a2, b);
+  const float2 e = __ffma2_rn(a2, b, make_float2(-p.x, -p.y));
+  const float2 s = __fadd2_rn(sh, p);
+  const float2 bb = sub2(s, sh);
+  float2 t = __fadd2_rn(sub2(sh, sub2(s, bb)), sub2(p, bb));
+  t = __fadd2_rn(t, __fadd2_rn(sl, __ffma2_rn(a2, bl, __ffma2_rn(al2, b, e))));
+  sh = __fadd2_rn(s, t);
+  sl = sub2(t, sub2(sh, s));
 }
 
-// (qh, ql) = (bh + bl) / (dh + dl)
-__device__ __forceinline__ void df_div(float bh, float bl, float dh, float dl, float& qh, float& ql) {
-  const float q1 = __fdiv_rn(bh, dh);
-  const float p = __fmul_rn(q1, dh);
-  const float pe = __fmaf_rn(q1, dh, -p);
-  const float r = __fadd_rn(__fsub_rn(__fsub_rn(bh, p), pe), __fsub_rn(bl, __fmul_rn(q1, dl)));
-  const float q2 = __fdiv_rn(r, dh);
-  qh = __fadd_rn(q1, q2);
-  ql = __fsub_rn(q2, __fsub_rn(qh, q1));
+// (sh, sl) += (h, l)
+__device__ __forceinline__ void df_add(float h, float l, float& sh, float& sl) {
+  const float s = __fadd_rn(sh, h);
+  const float bb = __fsub_rn(s, sh);
+  float t = __fadd_rn(__fsub_rn(sh, __fsub_rn(s, bb)), __fsub_rn(h, bb));
+  t = __fadd_rn(t, __fadd_rn(sl, l));
+  sh = __fadd_rn(s, t);
+  sl = __fsub_rn(t, __fsub_rn(sh, s));
 }
 
 __device__ __forceinline__ void split(double v, float& h, float& l) {
@@ -59,76 +65,44 @@ struct BatchHeader {
   int32_t n, precision, valid, generation;
 };
 
-// ---------------------------------------------------------------------------
-// Residual: partial[p] = Ks[rows of this block, k-range p] * X  (double-float), p = blockIdx.y
-struct KxSmem {
-  float Kh[kB][kB + 1], Kl[kB][kB + 1];
-  float Xh[kB][kMaxR + 1], Xl[kB][kMaxR + 1];
+// A solved entry on its way to the blocks after it: two words, each with a tag in its high half (set: 1) and one FP32
+// half of the double-float value in its low half, each stored and loaded as one single-copy-atomic access.
+struct alignas(16) Word {
+  unsigned long long hi, lo;
 };
-
-__global__ void __launch_bounds__(256) batch_kx_kernel(const float* __restrict__ Khi, const float* __restrict__ Klo,
-                                                       int64_t ld, int n, const double* __restrict__ X, int R,
-                                                       double* __restrict__ partial) {
-  extern __shared__ float4 kx_smem[];
-  KxSmem& sm = *reinterpret_cast<KxSmem*>(kx_smem);
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  const int r0 = blockIdx.x * kB;
-  const int ntile = int(ceil_div(n, kB));
-  const int t0 = int(ceil_div(int64_t(ntile) * blockIdx.y, kParts));
-  const int t1 = int(ceil_div(int64_t(ntile) * (blockIdx.y + 1), kParts));
-  float ah[4][4], al[4][4];
-#pragma unroll
-  for (int u = 0; u < 4; ++u)
-#pragma unroll
-    for (int v = 0; v < 4; ++v) ah[u][v] = al[u][v] = 0.f;
-  for (int tt = t0; tt < t1; ++tt) {
-    const int c0 = tt * kB;
-    for (int e = tid; e < kB * kB; e += blockDim.x) {
-      const int i = e >> 6, j = e & 63;
-      const bool ok = r0 + i < n && c0 + j < n;
-      sm.Kh[i][j] = ok ? Khi[int64_t(r0 + i) * ld + c0 + j] : 0.f;
-      sm.Kl[i][j] = ok ? Klo[int64_t(r0 + i) * ld + c0 + j] : 0.f;
-    }
-    for (int e = tid; e < kB * kMaxR; e += blockDim.x) {
-      const int i = e / kMaxR, c = e % kMaxR;
-      const double v = (c0 + i < n && c < R) ? X[int64_t(c0 + i) * R + c] : 0.0;
-      split(v, sm.Xh[i][c], sm.Xl[i][c]);
-    }
-    __syncthreads();
-#pragma unroll 2
-    for (int kk = 0; kk < kB; ++kk) {
-      float a[4], a2[4], b[4], b2[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) { a[u] = sm.Kh[ty * 4 + u][kk]; a2[u] = sm.Kl[ty * 4 + u][kk]; }
-#pragma unroll
-      for (int v = 0; v < 4; ++v) { b[v] = sm.Xh[kk][tx * 4 + v]; b2[v] = sm.Xl[kk][tx * 4 + v]; }
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) df_mac(a[u], a2[u], b[v], b2[v], ah[u][v], al[u][v]);
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int r = r0 + ty * 4 + u;
-    if (r >= n) continue;
-#pragma unroll
-    for (int v = 0; v < 4; ++v) {
-      const int c = tx * 4 + v;
-      if (c < R) partial[(int64_t(blockIdx.y) * n + r) * R + c] = double(ah[u][v]) + double(al[u][v]);
-    }
-  }
+__device__ __forceinline__ void put_word(Word* w, float h, float l) {
+  const unsigned long long tag = 1ull << 32;
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(&w->hi), "l"(tag | __float_as_uint(h)) : "memory");
+  asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(&w->lo), "l"(tag | __float_as_uint(l)) : "memory");
 }
+__device__ __forceinline__ Word get_word(const Word* w) {  // past L1, so that a second look sees new stores
+  Word v;
+  asm volatile("ld.global.cg.v2.u64 {%0, %1}, [%2];" : "=l"(v.hi), "=l"(v.lo) : "l"(w) : "memory");
+  return v;
+}
+__device__ __forceinline__ bool is_set(const Word& w) { return (w.hi >> 32) == 1 && (w.lo >> 32) == 1; }
 
-// Res = Bs - sum_p partial[p]
-__global__ void batch_residual_kernel(const double* __restrict__ Bs, const double* __restrict__ partial, int n, int R,
-                                      double* __restrict__ Res) {
+// Res = Bs - sum_p partial[p] (partials: splits x n x 64)
+__global__ void batch_residual_kernel(const double* __restrict__ Bs, const double* __restrict__ partial, int splits,
+                                      int n, int R, double* __restrict__ Res) {
   const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (e >= int64_t(n) * R) return;
+  const int64_t i = e / R, c = e % R;
   double s = 0.0;
-  for (int p = 0; p < kParts; ++p) s += partial[int64_t(p) * n * R + e];
+  for (int p = 0; p < splits; ++p) s += partial[(int64_t(p) * n + i) * kMaxR + c];
   Res[e] = Bs[e] - s;
+}
+
+// vals[i][c] = sum_p partial[p][i][c]; NaN if the header does not describe a preparation of an n x n system
+__global__ void batch_values_kernel(const double* __restrict__ partial, int splits, int N, int n, int R,
+                                    double* __restrict__ vals, int64_t ldv, const BatchHeader* __restrict__ hdr) {
+  const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (e >= int64_t(N) * R) return;
+  const int64_t i = e / R, c = e % R;
+  double s = 0.0;
+  for (int p = 0; p < splits; ++p) s += partial[(int64_t(p) * N + i) * kMaxR + c];
+  const bool ok = hdr->n == n && hdr->valid == 1;
+  vals[i * ldv + c] = ok ? s : __longlong_as_double(0x7ff8000000000000ll);
 }
 
 // Bs[i][c] = dr_i * Q[i][c] (i < N), 0 for the polynomial rows.  The solve workspace must hold factors of
@@ -147,20 +121,6 @@ __global__ void batch_rhs_kernel(const double* __restrict__ Q, int64_t ldq, int 
   Bs[e] = !ok ? __longlong_as_double(0x7ff8000000000000ll) : (i < N ? dr[i] * Q[int64_t(i) * ldq + c] : 0.0);
 }
 
-// Y[i][c] = X[perm[i]][c]
-__global__ void batch_gather_kernel(const double* __restrict__ X, double* __restrict__ Y,
-                                    const int32_t* __restrict__ perm, int n, int R) {
-  const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (e >= int64_t(n) * R) return;
-  const int i = int(e / R), c = int(e % R);
-  Y[e] = X[int64_t(perm[i]) * R + c];
-}
-
-__global__ void batch_axpy_kernel(double* __restrict__ X, const double* __restrict__ D, int64_t total) {
-  const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (e < total) X[e] += D[e];
-}
-
 // out[i][c] (ld = ldo) = dc_i * X[i][c]
 __global__ void batch_unscale_kernel(const double* __restrict__ X, const double* __restrict__ dc, int n, int R,
                                      double* __restrict__ out, int64_t ldo) {
@@ -170,178 +130,255 @@ __global__ void batch_unscale_kernel(const double* __restrict__ X, const double*
   out[int64_t(i) * ldo + c] = dc[i] * X[e];
 }
 
-// FP64 factors -> hi/lo FP32 planes
-__global__ void split_factors_kernel(const double* __restrict__ F, float* __restrict__ Fh, float* __restrict__ Fl,
-                                     int64_t total) {
-  const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (e < total) split(F[e], Fh[e], Fl[e]);
+// Inverses of the diagonal blocks of a triangular factor F (LOWER: unit lower), 64 x 64 each, and their hi/lo planes
+// (tiles[blk] = {hi, lo}).  Rows and columns beyond n count as the identity.
+struct InverseSmem {
+  double T[kB][kB + 1], I[kB][kB + 1];
+};
+
+template <typename TF, bool LOWER>
+__global__ void __launch_bounds__(256) tri_inverse_kernel(const TF* __restrict__ F, int64_t ldf, int n,
+                                                          double* __restrict__ inv, float* __restrict__ tiles) {
+  extern __shared__ double inv_smem[];
+  InverseSmem& sm = *reinterpret_cast<InverseSmem*>(inv_smem);
+  const int blk = blockIdx.x, r0 = blk * kB, tid = threadIdx.x;
+  for (int e = tid; e < kB * kB; e += blockDim.x) {
+    const int i = e >> 6, j = e & 63;
+    sm.T[i][j] = (r0 + i < n && r0 + j < n) ? double(F[int64_t(r0 + i) * ldf + r0 + j]) : (i == j ? 1.0 : 0.0);
+  }
+  __syncthreads();
+  if (tid < kB) {  // a column of the inverse by substitution
+    const int j = tid;
+    for (int s = 0; s < kB; ++s) {
+      const int i = LOWER ? s : kB - 1 - s;
+      double x = i == j ? 1.0 : 0.0;
+      if (LOWER) {
+        for (int k = j; k < i; ++k) x = fma(-sm.T[i][k], sm.I[k][j], x);
+      } else {
+        for (int k = i + 1; k <= j; ++k) x = fma(-sm.T[i][k], sm.I[k][j], x);
+        x /= sm.T[i][i];
+      }
+      sm.I[i][j] = x;
+    }
+  }
+  __syncthreads();
+  float* out = tiles + int64_t(blk) * 2 * kB * kB;
+  for (int e = tid; e < kB * kB; e += blockDim.x) {
+    const double x = sm.I[e >> 6][e & 63];
+    inv[int64_t(blk) * kB * kB + e] = x;
+    split(x, out[e], out[kB * kB + e]);
+  }
+}
+
+// G = -I_b T for every block T of block row b beside the diagonal (below it in L, above it in U), as hi/lo planes in
+// the place of T; a CTA a block, the lower triangle's inverses in invL, the upper's in invU.
+template <typename TF>
+__global__ void __launch_bounds__(256) tri_premultiply_kernel(const TF* __restrict__ F, int64_t ldf, int n,
+                                                              const double* __restrict__ invL,
+                                                              const double* __restrict__ invU, float* __restrict__ Gh,
+                                                              float* __restrict__ Gl) {
+  extern __shared__ double inv_smem[];
+  InverseSmem& sm = *reinterpret_cast<InverseSmem*>(inv_smem);
+  const int b = blockIdx.y, q = blockIdx.x, tid = threadIdx.x;
+  if (b == q) return;
+  const double* inv = (q < b ? invL : invU) + int64_t(b) * kB * kB;
+  const int r0 = b * kB, c0 = q * kB;
+  for (int e = tid; e < kB * kB; e += blockDim.x) {
+    const int i = e >> 6, j = e & 63;
+    sm.I[i][j] = inv[e];
+    sm.T[i][j] = (r0 + i < n && c0 + j < n) ? double(F[int64_t(r0 + i) * ldf + c0 + j]) : 0.0;
+  }
+  __syncthreads();
+  const int tx = tid & 15, ty = tid >> 4;
+  double acc[4][4] = {};
+#pragma unroll 4
+  for (int k = 0; k < kB; ++k) {
+    double a[4], t[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) { a[u] = -sm.I[ty + 16 * u][k]; t[u] = sm.T[k][tx + 16 * u]; }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int v = 0; v < 4; ++v) acc[u][v] = fma(a[u], t[v], acc[u][v]);
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const int r = r0 + ty + 16 * u, c = c0 + tx + 16 * v;
+      if (r < n && c < ldf) split(c < n ? acc[u][v] : 0.0, Gh[int64_t(r) * ldf + c], Gl[int64_t(r) * ldf + c]);
+    }
 }
 
 // ---------------------------------------------------------------------------
-// Triangular solves of an n x R block in place (LOWER: unit lower, forward; else upper, backward).
-// One CTA per (64-row block, group of 16 right-hand sides), taken in ticket order: the t-th ticket of a
-// group waits (bounded) until the group's t earlier blocks are done, subtracting each finished block's
-// contribution as soon as it is available, then solves its diagonal block warp by warp (two right-hand
-// sides per warp, lanes own rows lane and lane + 32, x_i broadcast by shuffles).
-struct TrsmSmem {
-  float Fh[kB][kB + 1], Fl[kB][kB + 1];
-  float Xh[kB][kRG + 1], Xl[kB][kRG + 1];
+// Triangular solve of n x R right-hand sides (LOWER: unit lower, forward; else upper, backward).
+// One CTA per (64-row block, group of 8 right-hand sides), taken in ticket order.  Block b is
+//   x_b = I_b y_b + sum_q G_bq x_q,   G_bq = -I_b T_bq,
+// with I_b the inverted diagonal block: what is left to do when x_{b-1} arrives is one 64 x 64 product and one
+// hand-off (a substitution inside each block and hand-offs through counters and fences made the chain 32 us a block).
+// Tiles are staged by cp.async one ahead, and the words of a block are read one tile ahead of their use, so blocks
+// solved long ago cost no waiting.
+// Bound by the FP32 pipes for many columns (15 packed instructions per two double-float multiply-adds, which issue every
+// other cycle: 64 columns of n = 6,403 take 1.03 ms a triangle, 0.85 of it at that rate), by the chain for few (8
+// columns: 0.45 ms, 4.4 us a block).
+// A thread owns rows rg + 16 u (u < 4), the columns 2 cg and 2 cg + 1, and every eighth term of the inner sum.
+constexpr int kTriThreads = 512, kKs = 8;
+struct TriSmem {
+  float F[2][2][kB][kLdt];   // [buffer][hi, lo]
+  float Xh[2][kB][kCG], Xl[2][kB][kCG];
 };
 
-template <bool LOWER, bool DF>
-__device__ __forceinline__ void trsm_block(const float* __restrict__ Fh, const float* __restrict__ Fl, int64_t ldf,
-                                           int n, double* X, int R, int t, int g, int* done, DeviceStatus* st,
-                                           TrsmSmem& sm, int& s_done) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nblk = int(ceil_div(n, kB));
-  const int blk = LOWER ? t : nblk - 1 - t;
-  const int r0 = blk * kB;
-  const int rows = min(kB, n - r0);
-  const int cbase = g * kRG;
-  // off-diagonal part: thread owns row tid / 4 and columns (tid % 4) * 4 + {0..3} of the group
-  const int orow = tid >> 2, ocol = (tid & 3) * 4;
-  float ah[4] = {0.f, 0.f, 0.f, 0.f}, al[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int q = 0; q < t; ++q) {
-    const int jb = LOWER ? q : nblk - 1 - q;
-    const int c0 = jb * kB;
-    for (int e = tid; e < kB * kB; e += blockDim.x) {
-      const int i = e >> 6, j = e & 63;
-      const bool ok = r0 + i < n && c0 + j < n;
-      sm.Fh[i][j] = ok ? Fh[int64_t(r0 + i) * ldf + c0 + j] : 0.f;
-      if (DF) sm.Fl[i][j] = ok ? Fl[int64_t(r0 + i) * ldf + c0 + j] : 0.f;
+template <bool LOWER>
+__global__ void __launch_bounds__(kTriThreads) batch_tri_kernel(const float* __restrict__ Gh,
+                                                                const float* __restrict__ Gl, int64_t ldg,
+                                                                const float* __restrict__ tiles, int n, int R,
+                                                                const double* __restrict__ Bin,
+                                                                const int32_t* __restrict__ perm, const Word* win,
+                                                                Word* wout, double* Y, int accumulate, int* ticket,
+                                                                DeviceStatus* st) {
+  extern __shared__ float4 tri_smem[];
+  TriSmem& sm = *reinterpret_cast<TriSmem*>(tri_smem);
+  __shared__ int s_tk;
+  const int tid = threadIdx.x;
+  const int ks = tid & (kKs - 1), rg = (tid >> 3) & 15, cg = tid >> 7;
+  const int G = int(ceil_div(R, kCG)), nblk = int(ceil_div(n, kB));
+  if (tid == 0) s_tk = atomicAdd(ticket, 1);
+  __syncthreads();
+  const int t = s_tk / G, cbase = (s_tk % G) * kCG;
+  if (t >= nblk) return;
+  const int blk = LOWER ? t : nblk - 1 - t, r0 = blk * kB;
+  auto block_at = [&](int q) { return LOWER ? q : nblk - 1 - q; };  // the q-th block to be solved
+
+  // item 0 is the inverse times the right-hand side, item i > 0 the product with the (i-1)-th solved block
+  auto stage = [&](int i) {
+    const float *hi, *lo;
+    int64_t ld;
+    int rows = kB, cols = kB;
+    if (i == 0) {
+      hi = tiles + int64_t(blk) * 2 * kB * kB;
+      lo = hi + kB * kB;
+      ld = kB;
+    } else {
+      const int c0 = block_at(i - 1) * kB;
+      hi = Gh + int64_t(r0) * ldg + c0;
+      lo = Gl + int64_t(r0) * ldg + c0;
+      ld = ldg;
+      rows = n - r0;
+      cols = n - c0;
     }
-    if (tid == 0 && s_done <= q) {
-      volatile int* vc = done + g;
+#pragma unroll
+    for (int k = 0; k < 2 * kB * kB / 4 / kTriThreads; ++k) {
+      const int e = tid + kTriThreads * k, p = e >> 10, row = (e >> 4) & 63, ch = (e & 15) * 4;
+      const bool ok = row < rows && ch < cols;  // the planes' columns from n on are zero
+      const float* src = (p ? lo : hi) + (ok ? int64_t(row) * ld + ch : 0);
+      const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(&sm.F[i & 1][p][row][ch]));
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(ok ? 16 : 0) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  const int xr = tid >> 3, xc = tid & 7;  // the entry of a 64 x 8 block that this thread brings to shared memory
+  auto word_at = [&](int i) -> const Word* {
+    const int row = block_at(i - 1) * kB + xr, c = cbase + xc;
+    return (row < n && c < R) ? wout + int64_t(row) * R + c : nullptr;
+  };
+  auto fetch = [&](int i) {
+    const Word* w = word_at(i);
+    return w ? get_word(w) : Word{1ull << 32, 1ull << 32};
+  };
+
+  stage(0);
+  Word pre{1ull << 32, 1ull << 32};  // the right-hand side's entry, then words one item ahead
+  if (r0 + xr < n && cbase + xc < R) {
+    if (LOWER) {
+      // (a workspace may hold no factors, and then no permutation either)
+      float h, l;
+      split(Bin[int64_t(min(max(perm[r0 + xr], 0), n - 1)) * R + cbase + xc], h, l);
+      pre = Word{(1ull << 32) | __float_as_uint(h), (1ull << 32) | __float_as_uint(l)};
+    } else {
+      pre = get_word(win + int64_t(r0 + xr) * R + cbase + xc);
+    }
+  }
+  float2 ah[4], al[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) ah[u] = al[u] = make_float2(0.f, 0.f);
+  for (int i = 0; i <= t; ++i) {
+    const int b = i & 1;
+    if (i > 0) {
       long long it = 0;
-      int d;
-      while ((d = *vc) <= q) {
+      while (!is_set(pre)) {
         if (++it > spin_limit()) {
           status_error(st, UPDES_ERR_TIMEOUT);
           atomicCAS(&st->timeout_tag, 0, 30);
-          d = q + 1;
           break;
         }
-        __nanosleep(20);
+        if (it > 64) __nanosleep(20);
+        pre = get_word(word_at(i));
       }
-      __threadfence();
-      s_done = d;
     }
+    sm.Xh[b][xr][xc] = __uint_as_float(uint32_t(pre.hi));
+    sm.Xl[b][xr][xc] = __uint_as_float(uint32_t(pre.lo));
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    for (int e = tid; e < kB * kRG; e += blockDim.x) {
-      const int i = e / kRG, c = e % kRG;
-      double v = 0.0;
-      if (c0 + i < n && cbase + c < R) v = __ldcg(X + int64_t(c0 + i) * R + cbase + c);
-      split(v, sm.Xh[i][c], sm.Xl[i][c]);
+    if (i < t) {
+      stage(i + 1);
+      pre = fetch(i + 1);
     }
-    __syncthreads();
-#pragma unroll 4
-    for (int kk = 0; kk < kB; ++kk) {
-      const float a = sm.Fh[orow][kk];
-      const float a2 = DF ? sm.Fl[orow][kk] : 0.f;
 #pragma unroll
-      for (int v = 0; v < 4; ++v) df_mac(a, a2, sm.Xh[kk][ocol + v], sm.Xl[kk][ocol + v], ah[v], al[v]);
-    }
-    __syncthreads();
-  }
-  // right-hand side of this block minus the off-diagonal part
+    for (int k = 0; k < kB / kKs; ++k) {
+      const int kk = kKs * k + ks;
+      const float2 xh = *reinterpret_cast<const float2*>(&sm.Xh[b][kk][2 * cg]);
+      const float2 xl = *reinterpret_cast<const float2*>(&sm.Xl[b][kk][2 * cg]);
 #pragma unroll
-  for (int v = 0; v < 4; ++v) {
-    const int c = ocol + v;
-    double b = 0.0;
-    if (orow < rows && cbase + c < R) b = X[int64_t(r0 + orow) * R + cbase + c] - (double(ah[v]) + double(al[v]));
-    split(b, sm.Xh[orow][c], sm.Xl[orow][c]);
+      for (int u = 0; u < 4; ++u)
+        df_mac2(sm.F[b][0][rg + 16 * u][kk], sm.F[b][1][rg + 16 * u][kk], xh, xl, ah[u], al[u]);
+    }
   }
-  for (int e = tid; e < kB * kB; e += blockDim.x) {
-    const int i = e >> 6, j = e & 63;
-    const bool ok = i < rows && j < rows;
-    sm.Fh[i][j] = ok ? Fh[int64_t(r0 + i) * ldf + r0 + j] : 0.f;
-    if (DF) sm.Fl[i][j] = ok ? Fl[int64_t(r0 + i) * ldf + r0 + j] : 0.f;
+  // The sum over the eight threads of a row: each exchange also halves what a thread keeps, down to one row of a pair
+  // of columns in two threads, so that thread ks ends with row rg + 16 (ks & 3), column 2 cg + (ks >> 2).
+#pragma unroll
+  for (int u = 0; u < 4; u += 2) {  // lanes that differ in bit 0 split rows u, u + 1
+    const bool up = ks & 1;
+    const float2 sh = up ? ah[u] : ah[u + 1], sl = up ? al[u] : al[u + 1];
+    float2 kh = up ? ah[u + 1] : ah[u], kl = up ? al[u + 1] : al[u];
+    df_add(__shfl_xor_sync(0xffffffffu, sh.x, 1), __shfl_xor_sync(0xffffffffu, sl.x, 1), kh.x, kl.x);
+    df_add(__shfl_xor_sync(0xffffffffu, sh.y, 1), __shfl_xor_sync(0xffffffffu, sl.y, 1), kh.y, kl.y);
+    ah[u] = kh;
+    al[u] = kl;
   }
-  __syncthreads();
-  // diagonal block: warp w solves columns 2w, 2w + 1 of the group
+  float2 rh, rl;
   {
-    float bh[2][2], bl[2][2];  // [row slot][column]
-#pragma unroll
-    for (int u = 0; u < 2; ++u)
-#pragma unroll
-      for (int v = 0; v < 2; ++v) {
-        bh[u][v] = sm.Xh[lane + 32 * u][2 * warp + v];
-        bl[u][v] = sm.Xl[lane + 32 * u][2 * warp + v];
-      }
-    for (int s2 = 0; s2 < rows; ++s2) {
-      const int i = LOWER ? s2 : rows - 1 - s2;
-      const int owner = i & 31, slot = i >> 5;
-      float xh[2], xl[2];
-#pragma unroll
-      for (int v = 0; v < 2; ++v) {
-        const float h = slot ? bh[1][v] : bh[0][v];
-        const float l = slot ? bl[1][v] : bl[0][v];
-        xh[v] = __shfl_sync(0xffffffffu, h, owner);
-        xl[v] = __shfl_sync(0xffffffffu, l, owner);
-        if (!LOWER) df_div(xh[v], xl[v], sm.Fh[i][i], DF ? sm.Fl[i][i] : 0.f, xh[v], xl[v]);
-      }
-      if (lane == owner) {
-#pragma unroll
-        for (int v = 0; v < 2; ++v) {
-          if (slot) { bh[1][v] = xh[v]; bl[1][v] = xl[v]; }
-          else { bh[0][v] = xh[v]; bl[0][v] = xl[v]; }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const int r = lane + 32 * u;
-        if (r < rows && (LOWER ? r > i : r < i)) {
-          const float f = -sm.Fh[r][i];
-          const float f2 = DF ? -sm.Fl[r][i] : 0.f;
-#pragma unroll
-          for (int v = 0; v < 2; ++v) df_mac(f, f2, xh[v], xl[v], bh[u][v], bl[u][v]);
-        }
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int r = lane + 32 * u;
-#pragma unroll
-      for (int v = 0; v < 2; ++v) {
-        const int c = cbase + 2 * warp + v;
-        if (r < rows && c < R) X[int64_t(r0 + r) * R + c] = double(bh[u][v]) + double(bl[u][v]);
-      }
+    const bool up = ks & 2;
+    const float2 sh = up ? ah[0] : ah[2], sl = up ? al[0] : al[2];
+    rh = up ? ah[2] : ah[0];
+    rl = up ? al[2] : al[0];
+    df_add(__shfl_xor_sync(0xffffffffu, sh.x, 2), __shfl_xor_sync(0xffffffffu, sl.x, 2), rh.x, rl.x);
+    df_add(__shfl_xor_sync(0xffffffffu, sh.y, 2), __shfl_xor_sync(0xffffffffu, sl.y, 2), rh.y, rl.y);
+  }
+  float h, l;
+  {
+    const bool up = ks & 4;
+    h = up ? rh.y : rh.x;
+    l = up ? rl.y : rl.x;
+    df_add(__shfl_xor_sync(0xffffffffu, up ? rh.x : rh.y, 4), __shfl_xor_sync(0xffffffffu, up ? rl.x : rl.y, 4), h, l);
+  }
+  const int own = r0 + rg + 16 * (ks & 3), c = cbase + 2 * cg + (ks >> 2);
+  if (own < n && c < R) {
+    const int64_t at = int64_t(own) * R + c;
+    put_word(wout + at, h, l);
+    if (!LOWER) {
+      const double x = double(h) + double(l);
+      Y[at] = accumulate ? Y[at] + x : x;
     }
   }
-  __syncthreads();
-  if (tid == 0) {
-    __threadfence();
-    atomicAdd(done + g, 1);
-  }
-}
-
-template <bool LOWER>
-__global__ void __launch_bounds__(256) batch_trsm_kernel(const float* __restrict__ F32, const float* __restrict__ Fh,
-                                                         const float* __restrict__ Fl, int64_t ldf, int n, double* X,
-                                                         int R, int* ticket, int* done, const BatchHeader* hdr,
-                                                         DeviceStatus* st) {
-  __shared__ TrsmSmem sm;
-  __shared__ int s_tk, s_done;
-  const int G = int(ceil_div(R, kRG));
-  const int nblk = int(ceil_div(n, kB));
-  if (threadIdx.x == 0) {
-    s_tk = atomicAdd(ticket, 1);
-    s_done = 0;
-  }
-  __syncthreads();
-  const int tk = s_tk;
-  const int t = tk / G, g = tk % G;
-  if (t >= nblk) return;
-  if (hdr->precision == UPDES_PREC_FP64) trsm_block<LOWER, true>(Fh, Fl, ldf, n, X, R, t, g, done, st, sm, s_done);
-  else trsm_block<LOWER, false>(F32, nullptr, ldf, n, X, R, t, g, done, st, sm, s_done);
 }
 
 // ---------------------------------------------------------------------------
 struct BatchWs {
   BatchHeader* hdr;
-  float *Fh, *Fl;
-  double *Bs, *X, *D, *T, *partial;
-  int* sync;
+  float *Gh, *Gl, *tilesL, *tilesU;  // premultiplied factors, inverted diagonal blocks
+  double *invL, *invU, *Bs, *X, *D, *partial, *chunk;
+  Word* words;  // tickets (the first word), then the words of both solves
+  void *Kd, *Vd, *columns;  // digits of Ks, of the value matrix, of a multiplied block
 };
 
 size_t batch_layout(int n, char* base, BatchWs* w) {
@@ -353,29 +390,46 @@ size_t batch_layout(int n, char* base, BatchWs* w) {
     return p;
   };
   const int64_t ld = updes_matrix_ld(n, 8);
-  const size_t v = size_t(n) * kMaxR * sizeof(double);
+  const size_t v = size_t(n) * kMaxR * sizeof(double), nblk = size_t(ceil_div(n, kB));
   BatchWs b;
   b.hdr = reinterpret_cast<BatchHeader*>(take(sizeof(BatchHeader)));
-  b.Fh = reinterpret_cast<float*>(take(size_t(n) * ld * sizeof(float)));
-  b.Fl = reinterpret_cast<float*>(take(size_t(n) * ld * sizeof(float)));
+  b.Gh = reinterpret_cast<float*>(take(size_t(n) * ld * sizeof(float)));
+  b.Gl = reinterpret_cast<float*>(take(size_t(n) * ld * sizeof(float)));
+  b.tilesL = reinterpret_cast<float*>(take(nblk * 2 * kB * kB * sizeof(float)));
+  b.tilesU = reinterpret_cast<float*>(take(nblk * 2 * kB * kB * sizeof(float)));
+  b.invL = reinterpret_cast<double*>(take(nblk * kB * kB * sizeof(double)));
+  b.invU = reinterpret_cast<double*>(take(nblk * kB * kB * sizeof(double)));
   b.Bs = reinterpret_cast<double*>(take(v));
   b.X = reinterpret_cast<double*>(take(v));
   b.D = reinterpret_cast<double*>(take(v));
-  b.T = reinterpret_cast<double*>(take(v));
-  b.partial = reinterpret_cast<double*>(take(kParts * v));
-  b.sync = reinterpret_cast<int*>(take(2 * (1 + kGroups) * sizeof(int)));
+  b.words = reinterpret_cast<Word*>(take((1 + 2 * size_t(n) * kMaxR) * sizeof(Word)));
+  b.partial = reinterpret_cast<double*>(take(kRhs64MaxSplits * v));
+  b.chunk = reinterpret_cast<double*>(take(size_t(kChunk) * ld * sizeof(double)));
+  b.Kd = take(rhs64_matrix_bytes(n, n));
+  b.Vd = take(rhs64_matrix_bytes(n, n));
+  b.columns = take(rhs64_columns_bytes(n));
   if (w) *w = b;
   return off + 256;
 }
 
-// Opt the residual kernel into its dynamic shared memory on the current device (once per device; a
-// host call that is not a stream operation, made before the first launch).
+// Opt the kernels into their dynamic shared memory on the current device (once per device; host calls that are not
+// stream operations, made before the first launch).
 int batch_kernel_setup() {
-  static std::atomic<unsigned long long> ready{0};
-  return smem_opt_in((const void*)batch_kx_kernel, int(sizeof(KxSmem)), ready);
+  static std::atomic<unsigned long long> done[8];
+  const void* tri[] = {(const void*)batch_tri_kernel<true>, (const void*)batch_tri_kernel<false>};
+  const void* inv[] = {(const void*)tri_inverse_kernel<double, true>, (const void*)tri_inverse_kernel<double, false>,
+                       (const void*)tri_inverse_kernel<float, true>,  (const void*)tri_inverse_kernel<float, false>,
+                       (const void*)tri_premultiply_kernel<double>,   (const void*)tri_premultiply_kernel<float>};
+  for (int i = 0; i < 2; ++i)
+    if (int e = smem_opt_in(tri[i], int(sizeof(TriSmem)), done[i])) return e;
+  for (int i = 0; i < 6; ++i)
+    if (int e = smem_opt_in(inv[i], int(sizeof(InverseSmem)), done[2 + i])) return e;
+  return rhs64_setup();
 }
 
 }  // namespace
+
+int value_rows(const updes_problem* p, int r0, int rows, double* out, int64_t ld, cudaStream_t s);
 
 // Views of the solve workspace the batch needs (defined in solve.cu).
 int solve_ws_views(const updes_problem* p, void* workspace, size_t workspace_bytes, const float** Khi,
@@ -384,25 +438,33 @@ int solve_ws_views(const updes_problem* p, void* workspace, size_t workspace_byt
 
 namespace {
 
-// Y <- M^-1 Y for an n x R block (permute, L, U).
-int batch_precond(int n, int R, const float* F32, const BatchWs& b, int64_t ld, const int32_t* piv, double* Y,
-                  DeviceStatus* st, cudaStream_t s) {
-  const unsigned g = unsigned(ceil_div(int64_t(n) * R, 256));
-  const int nblk = int(ceil_div(n, kB));
-  const int G = int(ceil_div(R, kRG));
-  batch_gather_kernel<<<g, 256, 0, s>>>(Y, b.T, piv + n, n, R);
+// The inverted diagonal blocks and the premultiplied block rows of the factors F.
+template <typename TF>
+int prepare_factors(int n, const TF* F, int64_t ld, const BatchWs& b, cudaStream_t s) {
+  const unsigned nblk = unsigned(ceil_div(n, kB));
+  tri_inverse_kernel<TF, true><<<nblk, 256, sizeof(InverseSmem), s>>>(F, ld, n, b.invL, b.tilesL);
   UPDES_LAUNCH_CHECK();
+  tri_inverse_kernel<TF, false><<<nblk, 256, sizeof(InverseSmem), s>>>(F, ld, n, b.invU, b.tilesU);
+  UPDES_LAUNCH_CHECK();
+  tri_premultiply_kernel<TF><<<dim3(nblk, nblk), 256, sizeof(InverseSmem), s>>>(F, ld, n, b.invL, b.invU, b.Gh, b.Gl);
+  UPDES_LAUNCH_CHECK();
+  return UPDES_OK;
+}
+
+// Y (+)= M^-1 B for n x R blocks (permute, L, U).
+int batch_precond(int n, int R, const BatchWs& b, int64_t ld, const int32_t* piv, const double* B, double* Y,
+                  bool accumulate, DeviceStatus* st, cudaStream_t s) {
+  const unsigned grid = unsigned(ceil_div(n, kB) * ceil_div(R, kCG));
   StatScope sc(kStatTrsv, s, 2.0 * n * n * R, double(n) * n * 8.0);
-  UPDES_CUDA_TRY(cudaMemsetAsync(b.sync, 0, 2 * (1 + kGroups) * sizeof(int), s));
-  int* lo_sync = b.sync;
-  int* up_sync = b.sync + 1 + kGroups;
-  batch_trsm_kernel<true><<<unsigned(nblk * G), 256, 0, s>>>(F32, b.Fh, b.Fl, ld, n, b.T, R, lo_sync, lo_sync + 1,
-                                                             b.hdr, st);
+  int* tickets = reinterpret_cast<int*>(b.words);
+  Word *wL = b.words + 1, *wU = wL + size_t(n) * R;
+  UPDES_CUDA_TRY(cudaMemsetAsync(b.words, 0, (1 + 2 * size_t(n) * R) * sizeof(Word), s));
+  batch_tri_kernel<true><<<grid, kTriThreads, sizeof(TriSmem), s>>>(b.Gh, b.Gl, ld, b.tilesL, n, R, B, piv + n, nullptr, wL,
+                                                            nullptr, 0, tickets, st);
   UPDES_LAUNCH_CHECK();
-  batch_trsm_kernel<false><<<unsigned(nblk * G), 256, 0, s>>>(F32, b.Fh, b.Fl, ld, n, b.T, R, up_sync, up_sync + 1,
-                                                              b.hdr, st);
+  batch_tri_kernel<false><<<grid, kTriThreads, sizeof(TriSmem), s>>>(b.Gh, b.Gl, ld, b.tilesU, n, R, nullptr, nullptr, wL, wU, Y,
+                                                             accumulate, tickets + 1, st);
   UPDES_LAUNCH_CHECK();
-  UPDES_CUDA_TRY(cudaMemcpyAsync(Y, b.T, size_t(n) * R * sizeof(double), cudaMemcpyDeviceToDevice, s));
   return UPDES_OK;
 }
 
@@ -434,11 +496,14 @@ extern "C" int updes_batch_prepare(const updes_problem* p, void* workspace, size
   UPDES_CUDA_TRY(cudaMemcpyAsync(h, state, sizeof h, cudaMemcpyDeviceToHost, s));
   UPDES_CUDA_TRY(cudaStreamSynchronize(s));
   if (h[0] != n || h[2] != 1) return UPDES_ERR_INVALID;  // no factorisation of this system in the workspace
-  if (h[1] == UPDES_PREC_FP64) {
-    const int64_t total = int64_t(n) * ld;
-    split_factors_kernel<<<unsigned(ceil_div(total, 256)), 256, 0, s>>>(F64, b.Fh, b.Fl, total);
-    UPDES_LAUNCH_CHECK();
-  }
+  if ((e = h[1] == UPDES_PREC_FP64 ? prepare_factors(n, F64, ld, b, s) : prepare_factors(n, F32, ld, b, s))) return e;
+  if ((e = rhs64_matrix(nullptr, Khi, Klo, ld, n, n, 0, n, b.Kd, s))) return e;
+  if (!p->supports)  // values on local supports have no batched form
+    for (int r0 = 0; r0 < p->N; r0 += kChunk) {
+      const int rows = std::min(kChunk, p->N - r0);
+      if ((e = value_rows(p, r0, rows, b.chunk, ld, s))) return e;
+      if ((e = rhs64_matrix(b.chunk, nullptr, nullptr, ld, p->N, n, r0, rows, b.Vd, s))) return e;
+    }
   const BatchHeader hd{n, h[1], 1, h[3]};
   UPDES_CUDA_TRY(cudaMemcpyAsync(b.hdr, &hd, sizeof hd, cudaMemcpyHostToDevice, s));
   UPDES_CUDA_TRY(cudaStreamSynchronize(s));
@@ -467,22 +532,43 @@ extern "C" int updes_solve_batch(const updes_problem* p, int32_t R, const double
   const unsigned g = unsigned(ceil_div(total, 256));
   batch_rhs_kernel<<<g, 256, 0, s>>>(Q, ldq, p->N, n, R, dr, b.Bs, state, b.hdr, st);
   UPDES_LAUNCH_CHECK();
-  UPDES_CUDA_TRY(cudaMemcpyAsync(b.X, b.Bs, size_t(total) * 8, cudaMemcpyDeviceToDevice, s));
-  if ((e = batch_precond(n, R, F32, b, ld, piv, b.X, st, s))) return e;
+  if ((e = batch_precond(n, R, b, ld, piv, b.Bs, b.X, false, st, s))) return e;
+  const int splits = rhs64_splits(n, n);
   for (int it = 0; it < sweeps; ++it) {
     {
-      StatScope sc(kStatGemv, s, 2.0 * n * n * R, 8.0 * n * double(ld));
-      batch_kx_kernel<<<dim3(unsigned(ceil_div(n, kB)), kParts), 256, sizeof(KxSmem), s>>>(Khi, Klo, ld, n, b.X, R,
-                                                                                          b.partial);
-      UPDES_LAUNCH_CHECK();
-      batch_residual_kernel<<<g, 256, 0, s>>>(b.Bs, b.partial, n, R, b.D);
+      StatScope sc(kStatGemv, s, 2.0 * n * n * R, 14.0 * n * double(n));
+      if ((e = rhs64_multiply(b.Kd, n, n, b.X, R, R, b.columns, b.partial, splits, st, s))) return e;
+      batch_residual_kernel<<<g, 256, 0, s>>>(b.Bs, b.partial, splits, n, R, b.D);
       UPDES_LAUNCH_CHECK();
     }
-    if ((e = batch_precond(n, R, F32, b, ld, piv, b.D, st, s))) return e;
-    batch_axpy_kernel<<<g, 256, 0, s>>>(b.X, b.D, total);
-    UPDES_LAUNCH_CHECK();
+    if ((e = batch_precond(n, R, b, ld, piv, b.D, b.X, true, st, s))) return e;
   }
   batch_unscale_kernel<<<g, 256, 0, s>>>(b.X, dc, n, R, coeffs, ldc);
+  UPDES_LAUNCH_CHECK();
+  return UPDES_OK;
+}
+
+extern "C" int updes_eval_values_prepared(const updes_problem* p, int32_t R, const double* C, int64_t ldc, double* vals,
+                                          int64_t ldv, void* workspace, size_t workspace_bytes, void* batch_ws,
+                                          size_t batch_ws_bytes, void* stream) {
+  if (!p || !C || !vals || R <= 0 || R > kMaxR || ldc < R || ldv < R || !batch_ws) return UPDES_ERR_INVALID;
+  if (p->supports) return UPDES_ERR_UNSUPPORTED;
+  const int n = p->N + p->M;
+  if (batch_ws_bytes < batch_layout(n, nullptr, nullptr)) return UPDES_ERR_WORKSPACE;
+  const float *Khi, *Klo, *F32;
+  const double *F64, *dr, *dc;
+  const int32_t *piv, *state;
+  int64_t ld;
+  DeviceStatus* st;
+  int e = solve_ws_views(p, workspace, workspace_bytes, &Khi, &Klo, &F32, &F64, &ld, &piv, &dr, &dc, &st, &state);
+  if (e) return e;
+  BatchWs b;
+  batch_layout(n, static_cast<char*>(batch_ws), &b);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int splits = rhs64_splits(p->N, n);
+  if ((e = rhs64_multiply(b.Vd, p->N, n, C, ldc, R, b.columns, b.partial, splits, st, s))) return e;
+  batch_values_kernel<<<unsigned(ceil_div(int64_t(p->N) * R, 256)), 256, 0, s>>>(b.partial, splits, p->N, n, R, vals,
+                                                                               ldv, b.hdr);
   UPDES_LAUNCH_CHECK();
   return UPDES_OK;
 }

@@ -24,3 +24,17 @@ size_t ozaki64_scratch_bytes(int mmax, int ncmax, int Kmax);
 int ozaki64_update(double* C, int64_t ldc, const double* A, int64_t lda, const double* B, int64_t ldb, int m, int nc,
                    int K, void* scratch, size_t scratch_bytes, DeviceStatus* st, cudaStream_t s, int max_ctas = 0,
                    bool a_digits_ready = false);
+
+// A fixed FP64 matrix (m x n) times up to 64 columns on the same digits (gemm_tc64.cu).  rhs64_matrix writes the digits
+// of rows [r0, r0 + rows) into `matrix` (rhs64_matrix_bytes(m, n) bytes), from FP64 rows (A, lda) or, with A null,
+// from the sum of two FP32 planes.  rhs64_multiply leaves the product as `splits` partial sums, each m x 64 (row
+// stride 64), to be added in order; `columns`: scratch of rhs64_columns_bytes(n).  rhs64_setup before a capture.
+constexpr int kRhs64MaxSplits = 16;
+size_t rhs64_matrix_bytes(int m, int n);
+size_t rhs64_columns_bytes(int n);
+int rhs64_splits(int m, int n);
+int rhs64_setup();
+int rhs64_matrix(const double* A, const float* hi, const float* lo, int64_t lda, int m, int n, int r0, int rows,
+                 void* matrix, cudaStream_t s);
+int rhs64_multiply(const void* matrix, int m, int n, const double* X, int64_t ldx, int R, void* columns,
+                   double* partial, int splits, DeviceStatus* st, cudaStream_t s);

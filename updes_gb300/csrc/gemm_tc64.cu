@@ -123,6 +123,25 @@ __device__ __forceinline__ uint32_t bf16_bits(int d) {
 // The exponent written for a row or column whose largest field is emax: its entries are below 2^e.
 __device__ __forceinline__ int scale_exp(int emax) { return emax >= 0x7ff ? kNanExp : emax - 1022; }
 
+// The digits of 8 consecutive entries under the exponent field emax, one 16-byte word into each of the 7 planes.
+__device__ __forceinline__ void write_digits(const double* v, int emax, uint16_t* dst, int64_t plane) {
+  uint32_t w[kDigits][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    int d[kDigits];
+    digits_of(emax >= 0x7ff ? 0.0 : v[i], max(emax, 1), d);
+#pragma unroll
+    for (int p = 0; p < kDigits; ++p) {
+      const uint32_t h = bf16_bits(d[p]);
+      if (i & 1) w[p][i >> 1] |= h << 16;
+      else w[p][i >> 1] = h;
+    }
+  }
+#pragma unroll
+  for (int p = 0; p < kDigits; ++p)
+    *reinterpret_cast<uint4*>(dst + p * plane) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+}
+
 // A (m x K, lda) -> Ad[p][r][k] and Ae[r]; 8 consecutive k a lane, `span` lanes (a power of two >= Kp / 8) a row.
 __device__ __forceinline__ void digits_rows(int bx, const double* __restrict__ A, int64_t lda, int m, int K, int Kp,
                                             int span, uint16_t* __restrict__ Ad, int* __restrict__ Ae) {
@@ -139,21 +158,7 @@ __device__ __forceinline__ void digits_rows(int bx, const double* __restrict__ A
   for (int o = span >> 1; o > 0; o >>= 1) emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, o));
   if (!ok || k0 >= Kp) return;
   if (q == 0) Ae[r] = scale_exp(emax);
-  uint32_t w[kDigits][4];
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    int d[kDigits];
-    digits_of(emax >= 0x7ff ? 0.0 : v[i], max(emax, 1), d);
-#pragma unroll
-    for (int p = 0; p < kDigits; ++p) {
-      const uint32_t h = bf16_bits(d[p]);
-      if (i & 1) w[p][i >> 1] |= h << 16;
-      else w[p][i >> 1] = h;
-    }
-  }
-#pragma unroll
-  for (int p = 0; p < kDigits; ++p)
-    *reinterpret_cast<uint4*>(Ad + (int64_t(p) * m + r) * Kp + k0) = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+  write_digits(v, emax, Ad + int64_t(r) * Kp + k0, int64_t(m) * Kp);
 }
 
 // B (K x nc, ldb) -> Bd[p][c][k] and Be[c]; a lane a column, a warp 32 consecutive k, Kp / 32 warps a group of 32
@@ -180,22 +185,7 @@ __device__ __forceinline__ void digits_cols(int bx, const double* __restrict__ B
   if (part == 0) Be[c] = scale_exp(emax);
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    uint32_t w[kDigits][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      int d[kDigits];
-      digits_of(emax >= 0x7ff ? 0.0 : v[j * 8 + i], max(emax, 1), d);
-#pragma unroll
-      for (int p = 0; p < kDigits; ++p) {
-        const uint32_t h = bf16_bits(d[p]);
-        if (i & 1) w[p][i >> 1] |= h << 16;
-        else w[p][i >> 1] = h;
-      }
-    }
-#pragma unroll
-    for (int p = 0; p < kDigits; ++p)
-      *reinterpret_cast<uint4*>(Bd + (int64_t(p) * nc + c) * Kp + k0 + j * 8) =
-          make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+    write_digits(v + j * 8, emax, Bd + int64_t(c) * Kp + k0 + j * 8, int64_t(nc) * Kp);
   }
 }
 
@@ -235,12 +225,57 @@ __device__ __forceinline__ double to_double(long long v, uint32_t fine) {
   return __longlong_as_double(fine && v != 0 ? b - (8ll << 52) : b);
 }
 
-// c - d 2^(ea + eb - 54); the power as one factor where it is a normal number
-__device__ __forceinline__ double subtract(double c, double d, int ea, int eb) {
+// c + sign d 2^(ea + eb - 54); the power as one factor where it is a normal number
+template <int SIGN>
+__device__ __forceinline__ double add_scaled(double c, double d, int ea, int eb) {
   const int e = ea + eb - 54;
-  if (e > -1022 && e < 1023) return fma(-__longlong_as_double(static_cast<long long>(e + 1023) << 52), d, c);
+  if (e > -1022 && e < 1023) {
+    const double f = __longlong_as_double(static_cast<long long>(e + 1023) << 52);
+    return fma(SIGN > 0 ? f : -f, d, c);
+  }
   if (ea >= kNanExp || eb >= kNanExp) return __longlong_as_double(0x7ff8000000000000ll);
-  return c - scalbn(d, e);
+  return SIGN > 0 ? c + scalbn(d, e) : c - scalbn(d, e);
+}
+
+// The MMAs of one 32-wide k block; `later` is false for the first block of a sum, whose first product in each group
+// overwrites the accumulator.
+__device__ __forceinline__ void mma_stage(uint32_t tmem, const uint8_t* sA, bool later) {
+  const uint64_t a0 = make_desc(smem_u32(sA)), b0 = make_desc(smem_u32(sA + kDigits * kAPlane));
+#pragma unroll
+  for (int a = 0; a < kDigits; ++a)
+#pragma unroll
+    for (int b = 0; b < kDigits && a + b < kGroups; ++b)
+#pragma unroll
+      for (int kk = 0; kk < TK / 16; ++kk) {  // a k-step is 32 bytes: 2 descriptor units
+        const bool first = kk == 0 && (a == 0 || (a == 1 && b == kDigits - 1));
+        mma_acc(tmem + uint32_t((a + b) * TN), a0 + uint64_t(a * (kAPlane >> 4) + kk * 2),
+                b0 + uint64_t(b * (kBPlane >> 4) + kk * 2), first ? uint32_t(later) : 1u);
+      }
+}
+
+// The thread's row of 32 sums as integers.  x is the sum in units of group 5 (at most 2^62), r what groups 6 and 7 add
+// to it, in units of group 7.  Where x has fewer than 54 bits the integer is in units of group 6 instead, so that its
+// conversion to a double is what rounds either way; the result's bit of that column is set then.
+__device__ __forceinline__ uint32_t read_sums(uint32_t taddr, long long* v) {
+  uint32_t fine = 0;
+#pragma unroll
+  for (int ch = 0; ch < kCols / 8; ++ch) {
+    float g[kGroups][8];
+#pragma unroll
+    for (int gi = 0; gi < kGroups; ++gi) tmem_ld8(taddr + uint32_t(gi * TN + ch * 8), g[gi]);
+    tmem_wait_ld();
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      long long x = __float2int_rn(g[0][u]);
+#pragma unroll
+      for (int gi = 1; gi < kGroups - 2; ++gi) x = (x << 8) + __float2int_rn(g[gi][u]);
+      const long long r = (static_cast<long long>(__float2int_rn(g[6][u])) << 8) + __float2int_rn(g[7][u]);
+      const bool f = x < (1ll << 54) && x > -(1ll << 54);
+      v[ch * 8 + u] = f ? (x << 8) + ((r + 128) >> 8) : x + ((r + (1 << 15)) >> 16);
+      fine |= uint32_t(f) << (ch * 8 + u);
+    }
+  }
+  return fine;
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
@@ -323,17 +358,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             break;
           }
           tc_fence_after();
-          const uint8_t* sA = smem + s * kStageBytes;
-          const uint64_t a0 = make_desc(smem_u32(sA)), b0 = make_desc(smem_u32(sA + kDigits * kAPlane));
-          const uint32_t later = kb > 0;
-#pragma unroll
-          for (int a = 0; a < kDigits; ++a)
-#pragma unroll
-            for (int b = 0; b < kDigits && a + b < kGroups; ++b)
-#pragma unroll
-              for (int kk = 0; kk < TK / 16; ++kk)  // a k-step is 32 bytes: 2 descriptor units
-                mma_acc(tmem + uint32_t((a + b) * TN), a0 + uint64_t(a * (kAPlane >> 4) + kk * 2),
-                        b0 + uint64_t(b * (kBPlane >> 4) + kk * 2), ((a == 0 || b == kGroups - 1 - a) && a <= 1 && kk == 0) ? later : 1u);
+          mma_stage(tmem, smem + s * kStageBytes, kb > 0);
           mma_commit(&ctl.empty[s]);
           if (kb == nkb - 1) mma_commit(&ctl.tfull);
           committed = j + 1;
@@ -353,29 +378,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         *abort_flag = 1;
       }
       tc_fence_after();
-      // The sum in units of group 5 (x, at most 2^62) and what groups 6 and 7 add to it (r, in units of group 7).  Where
-      // x has fewer than 54 bits the integer that is converted is in units of group 6 instead, so that the
-      // conversion is what rounds either way; its exponent goes down by 8 then (fine, a bit per column).
       long long v[kCols];
-      uint32_t fine = 0;
-#pragma unroll
-      for (int ch = 0; ch < kCols / 8; ++ch) {
-        float g[kGroups][8];
-#pragma unroll
-        for (int gi = 0; gi < kGroups; ++gi)
-          tmem_ld8(tmem + lane_base + uint32_t(gi * TN + h * kCols + ch * 8), g[gi]);
-        tmem_wait_ld();
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          long long x = __float2int_rn(g[0][u]);
-#pragma unroll
-          for (int gi = 1; gi < kGroups - 2; ++gi) x = (x << 8) + __float2int_rn(g[gi][u]);
-          const long long r = (static_cast<long long>(__float2int_rn(g[6][u])) << 8) + __float2int_rn(g[7][u]);
-          const bool f = x < (1ll << 54) && x > -(1ll << 54);
-          v[ch * 8 + u] = f ? (x << 8) + ((r + 128) >> 8) : x + ((r + (1 << 15)) >> 16);
-          fine |= uint32_t(f) << (ch * 8 + u);
-        }
-      }
+      const uint32_t fine = read_sums(tmem + lane_base + uint32_t(h * kCols), v);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&ctl.tempty);
@@ -398,7 +402,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int i = 0; i < 16; ++i) {
           const int r = r0 + ew * 16 + i;
           if (c < nc && r < m && !*abort_flag)
-            __stcs(cp + int64_t(i) * ldc, subtract(old[i], sV[ew * 16 + i][lane], __ldg(Ae + r), eb));
+            __stcs(cp + int64_t(i) * ldc, add_scaled<-1>(old[i], sV[ew * 16 + i][lane], __ldg(Ae + r), eb));
         }
         if (half == 0) epilogue_barrier();
       }
@@ -421,6 +425,203 @@ __global__ void __launch_bounds__(kThreads, 1)
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
   }
+}
+
+// ---- a fixed matrix times up to 64 columns ------------------------------------------------------------------
+// Y = A X for an m x n matrix whose digits are written once (updes_batch_prepare) and X of at most 64 columns: the
+// same products and sums as above over k blocks of 256, each block's sum rounded once and added in FP64.  A 64-column
+// product reads 14 bytes of digits an entry of A and is bound by its MMAs (34 x 48 cycles for 128 x 64 x 16), about
+// a tenth of what double-float multiply-adds on the FP32 pipes cost.  The k blocks are split over `splits` CTAs a row
+// tile, their sums added in order by the caller.
+constexpr int kBlockK = 256;
+
+__global__ void __launch_bounds__(kThreads, 1)
+    rhs64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                 const int* __restrict__ Ae, const int* __restrict__ Be, double* __restrict__ partial, int m, int nkb,
+                 int splits, DeviceStatus* st) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ Ctrl ctl;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int items = int(ceil_div(m, TM)) * splits;
+  volatile int* abort_flag = &ctl.abort_flag;
+
+  if (tid == 0) {
+    for (int s = 0; s < kStages; ++s) {
+      mbar_init(&ctl.full[s], 1);
+      mbar_init(&ctl.empty[s], 1);
+    }
+    mbar_init(&ctl.tfull, 1);
+    mbar_init(&ctl.tempty, kEpiWarps);
+    ctl.abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl.tmem)),
+                 "r"(kTmemCols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = ctl.tmem;
+  int committed = 0;
+  auto first_block = [&](int item) { return int(int64_t(nkb) * (item % splits) / splits); };
+  auto end_block = [&](int item) { return int(int64_t(nkb) * (item % splits + 1) / splits); };
+
+  if (warp == 0) {
+    if (lane == 0) {
+      const uint64_t stream = l2_policy_evict_first(), keep = l2_policy_evict_last();
+      int j = 0;
+      for (int it = blockIdx.x; it < items && !*abort_flag; it += gridDim.x) {
+        const int r0 = (it / splits) * TM;
+        for (int ks = first_block(it) * (kBlockK / TK); ks < end_block(it) * (kBlockK / TK); ++ks, ++j) {
+          const int s = j % kStages;
+          if (!mbar_wait(&ctl.empty[s], (uint32_t(j / kStages) & 1u) ^ 1u, abort_flag)) {
+            if (!*abort_flag) { status_error(st, UPDES_ERR_TIMEOUT); atomicCAS(&st->timeout_tag, 0, 54); }
+            *abort_flag = 1;
+            break;
+          }
+          uint8_t* sA = smem + s * kStageBytes;
+          mbar_expect_tx(&ctl.full[s], uint32_t(kStageBytes));
+          tma_load_3d(smem_u32(sA), &tmA, ks * TK, r0, 0, &ctl.full[s], stream);
+          tma_load_3d(smem_u32(sA + kDigits * kAPlane), &tmB, ks * TK, 0, 0, &ctl.full[s], keep);
+        }
+      }
+      if (*abort_flag) {
+        // copies still in flight must land before the CTA's shared memory goes away (bounded)
+        for (int jj = (j > kStages ? j - kStages : 0); jj < j; ++jj) {
+          for (long long k = 0; k < (1 << 22); ++k) {
+            if (mbar_try_wait(&ctl.full[jj % kStages], uint32_t(jj / kStages) & 1u)) break;
+            __nanosleep(64);
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      int j = 0, sums = 0;
+      for (int it = blockIdx.x; it < items && !*abort_flag; it += gridDim.x) {
+        for (int kb = first_block(it); kb < end_block(it) && !*abort_flag; ++kb, ++sums) {
+          for (int i = 0; i < kBlockK / TK; ++i, ++j) {
+            const int s = j % kStages;
+            if ((i == 0 && !mbar_wait(&ctl.tempty, (uint32_t(sums) & 1u) ^ 1u, abort_flag)) ||
+                !mbar_wait(&ctl.full[s], uint32_t(j / kStages) & 1u, abort_flag)) {
+              if (!*abort_flag) { status_error(st, UPDES_ERR_TIMEOUT); atomicCAS(&st->timeout_tag, 0, 55); }
+              *abort_flag = 1;
+              break;
+            }
+            tc_fence_after();
+            mma_stage(tmem, smem + s * kStageBytes, i > 0);
+            mma_commit(&ctl.empty[s]);
+            if (i == kBlockK / TK - 1) mma_commit(&ctl.tfull);
+            committed = j + 1;
+          }
+        }
+      }
+    }
+  } else {
+    const int q = warp & 3, h = (warp - 2) >> 2;
+    const uint32_t lane_base = uint32_t(q * 32) << 16;
+    int sums = 0;
+    for (int it = blockIdx.x; it < items && !*abort_flag; it += gridDim.x) {
+      const int r = (it / splits) * TM + q * 32 + lane;
+      double acc[kCols];
+#pragma unroll
+      for (int u = 0; u < kCols; ++u) acc[u] = 0.0;
+      for (int kb = first_block(it); kb < end_block(it); ++kb, ++sums) {
+        const int ea = r < m ? __ldg(Ae + int64_t(kb) * m + r) : 0;
+        // every wait ends in a warp vote, so a warp always leaves together (tcgen05.ld needs all 32 lanes)
+        if (!__all_sync(0xffffffffu, mbar_wait(&ctl.tfull, uint32_t(sums) & 1u, abort_flag))) {
+          if (lane == 0 && !*abort_flag) { status_error(st, UPDES_ERR_TIMEOUT); atomicCAS(&st->timeout_tag, 0, 56); }
+          *abort_flag = 1;
+          break;
+        }
+        tc_fence_after();
+        long long v[kCols];
+        const uint32_t fine = read_sums(tmem + lane_base + uint32_t(h * kCols), v);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&ctl.tempty);
+        const int* be = Be + kb * TN + h * kCols;
+#pragma unroll
+        for (int u = 0; u < kCols; ++u)
+          acc[u] = add_scaled<1>(acc[u], to_double(v[u], (fine >> u) & 1u), ea, __ldg(be + u));
+      }
+      if (r < m && !*abort_flag) {
+        double2* dst = reinterpret_cast<double2*>(partial + (int64_t(it % splits) * m + r) * TN + h * kCols);
+#pragma unroll
+        for (int u = 0; u < kCols; u += 2) dst[u / 2] = make_double2(acc[u], acc[u + 1]);
+      }
+    }
+  }
+
+  __syncthreads();
+  if (warp == 1) {
+    if (ctl.abort_flag && lane == 0 && committed > 0) {
+      // MMAs complete in order: once the last commit has arrived nothing reads tensor memory (bounded)
+      const int jj = committed - 1;
+      for (long long k = 0; k < (1 << 22); ++k) {
+        if (mbar_try_wait(&ctl.empty[jj % kStages], uint32_t(jj / kStages) & 1u)) break;
+        __nanosleep(64);
+      }
+    }
+    __syncwarp();
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+  }
+}
+
+// Digits of rows [r0, r0 + rows) of the m x n matrix, a warp per (row, 256-wide k block), 8 entries a lane: from FP64
+// rows (A, lda, row 0 = row r0) or, with A null, from the sum of two FP32 planes.
+__global__ void __launch_bounds__(256) matrix_digits_kernel(const double* __restrict__ A, const float* __restrict__ hi,
+                                                            const float* __restrict__ lo, int64_t lda, int m, int n,
+                                                            int nkb, int r0, int rows, uint16_t* __restrict__ Ad,
+                                                            int* __restrict__ Ae) {
+  const int64_t w = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (w >= int64_t(rows) * nkb) return;
+  const int i = int(w / nkb), kb = int(w % nkb), k0 = kb * kBlockK + lane * 8;
+  double v[8];
+  int emax = 0;
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    const int64_t at = int64_t(i) * lda + k0 + u;
+    v[u] = k0 + u < n ? (A ? A[at] : double(hi[at]) + double(lo[at])) : 0.0;
+    emax = max(emax, exp_field(v[u]));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, o));
+  if (lane == 0) Ae[int64_t(kb) * m + r0 + i] = scale_exp(emax);
+  const int64_t Kp = int64_t(nkb) * kBlockK;
+  write_digits(v, emax, Ad + int64_t(r0 + i) * Kp + k0, int64_t(m) * Kp);
+}
+
+// Digits of X (n x R, ldx) as 64 columns (those from R on zero): a block per (k block, 8 columns), a warp a column.
+__global__ void __launch_bounds__(256) columns_digits_kernel(const double* __restrict__ X, int64_t ldx, int n, int R,
+                                                             int nkb, uint16_t* __restrict__ Bd,
+                                                             int* __restrict__ Be) {
+  __shared__ double t[kBlockK][9];
+  const int kb = blockIdx.x, c0 = blockIdx.y * 8;
+  for (int e = threadIdx.x; e < kBlockK * 8; e += blockDim.x) {
+    const int k = e >> 3, c = c0 + (e & 7);
+    t[k][e & 7] = (kb * kBlockK + k < n && c < R) ? X[int64_t(kb * kBlockK + k) * ldx + c] : 0.0;
+  }
+  __syncthreads();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double v[8];
+  int emax = 0;
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    v[u] = t[lane * 8 + u][warp];
+    emax = max(emax, exp_field(v[u]));
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) emax = max(emax, __shfl_xor_sync(0xffffffffu, emax, o));
+  if (lane == 0) Be[kb * TN + c0 + warp] = scale_exp(emax);
+  const int64_t Kp = int64_t(nkb) * kBlockK;
+  write_digits(v, emax, Bd + int64_t(c0 + warp) * Kp + kb * kBlockK + lane * 8, TN * Kp);
 }
 
 // 3-D map over digit planes [7][rows][Kp] bf16, box 32 (k) x box_rows x 7, 64B swizzle
@@ -483,6 +684,70 @@ int ozaki64_update(double* C, int64_t ldc, const double* A, int64_t lda, const d
   const int ntiles = int(ceil_div(m, TM) * ceil_div(nc, TN));
   const int grid = std::min(ntiles, max_ctas > 0 ? std::min(max_ctas, num_sms_cached()) : num_sms_cached());
   ozaki64_kernel<<<grid, kThreads, kSmemBytes, s>>>(mapA, mapB, Ae, Be, C, ldc, m, nc, Kp, st);
+  UPDES_LAUNCH_CHECK();
+  return UPDES_OK;
+}
+
+namespace {
+
+struct MatrixDigits {
+  uint16_t* d;
+  int* e;
+};
+int k_blocks(int n) { return int(ceil_div(n, kBlockK)); }
+MatrixDigits matrix_view(void* base, int rows, int n) {
+  char* p = static_cast<char*>(base);
+  return {reinterpret_cast<uint16_t*>(p),
+          reinterpret_cast<int*>(p + al256(kDigits * size_t(rows) * k_blocks(n) * kBlockK * 2))};
+}
+
+}  // namespace
+
+size_t rhs64_matrix_bytes(int m, int n) {
+  return al256(kDigits * size_t(m) * k_blocks(n) * kBlockK * 2) + al256(size_t(m) * k_blocks(n) * 4);
+}
+size_t rhs64_columns_bytes(int n) { return rhs64_matrix_bytes(TN, n); }
+
+// Row tiles times splits are dealt round robin to the SMs: the number of splits with the shortest longest share, a
+// fraction of a block charged for writing and adding each split's sums.
+int rhs64_splits(int m, int n) {
+  const int tiles = int(ceil_div(m, TM)), nkb = k_blocks(n), sms = num_sms_cached();
+  int best = 1;
+  double best_cost = 1e30;
+  for (int s = 1; s <= std::min(nkb, kRhs64MaxSplits); ++s) {
+    const double cost = double(ceil_div(int64_t(tiles) * s, sms) * ceil_div(nkb, s)) + 0.1 * s;
+    if (cost < best_cost) { best_cost = cost; best = s; }
+  }
+  return best;
+}
+
+int rhs64_matrix(const double* A, const float* hi, const float* lo, int64_t lda, int m, int n, int r0, int rows,
+                 void* matrix, cudaStream_t s) {
+  const MatrixDigits v = matrix_view(matrix, m, n);
+  matrix_digits_kernel<<<unsigned(ceil_div(int64_t(rows) * k_blocks(n) * 32, 256)), 256, 0, s>>>(
+      A, hi, lo, lda, m, n, k_blocks(n), r0, rows, v.d, v.e);
+  UPDES_LAUNCH_CHECK();
+  return UPDES_OK;
+}
+
+int rhs64_setup() {
+  static std::atomic<unsigned long long> attr{0};
+  return smem_opt_in((const void*)rhs64_kernel, kStages * kStageBytes + 1024, attr);
+}
+
+int rhs64_multiply(const void* matrix, int m, int n, const double* X, int64_t ldx, int R, void* columns,
+                   double* partial, int splits, DeviceStatus* st, cudaStream_t s) {
+  const int nkb = k_blocks(n);
+  const MatrixDigits a = matrix_view(const_cast<void*>(matrix), m, n), b = matrix_view(columns, TN, n);
+  CUtensorMap mapA, mapB;
+  if (int e = make_map(&mapA, a.d, m, nkb * kBlockK, TM)) return e;
+  if (int e = make_map(&mapB, b.d, TN, nkb * kBlockK, TN)) return e;
+  if (int e = rhs64_setup()) return e;
+  columns_digits_kernel<<<dim3(unsigned(nkb), TN / 8), 256, 0, s>>>(X, ldx, n, R, nkb, b.d, b.e);
+  UPDES_LAUNCH_CHECK();
+  const int items = int(ceil_div(m, TM)) * splits;
+  rhs64_kernel<<<std::min(items, num_sms_cached()), kThreads, kStages * kStageBytes + 1024, s>>>(
+      mapA, mapB, a.e, b.e, partial, m, nkb, splits, st);
   UPDES_LAUNCH_CHECK();
   return UPDES_OK;
 }

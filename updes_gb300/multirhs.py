@@ -8,8 +8,8 @@ factored once (``updes_factor``, FP64 by default: the factorisation is paid once
 while every step applies the factors, so their accuracy is what matters); each
 call then solves R <= 64 right-hand sides together (``updes_solve_batch``: the
 factors applied in double-float arithmetic on the FP32 pipes, a fixed number of
-refinement sweeps with a double-float residual) and evaluates
-``vals = [Phi P] C`` for all of them (``updes_eval_values_batch``).
+refinement sweeps with an exact-product residual) and evaluates
+``vals = [Phi P] C`` for all of them (``updes_eval_values_prepared``).
 Nothing in a step reads back to the host, so ``implicit_steps`` records one step
 into a CUDA graph and replays it.
 """
@@ -79,9 +79,10 @@ class MultiRHSSolver:
 
     def _eval_into(self, C, V, stream):
         lib = _lib.load()
-        st = lib.updes_eval_values_batch(ctypes.byref(self.dp.c), C.shape[1], C.data_ptr(), C.stride(0),
-                                         V.data_ptr(), V.stride(0), stream)
-        _lib.check(st, "updes_eval_values_batch")
+        st = lib.updes_eval_values_prepared(ctypes.byref(self.dp.c), C.shape[1], C.data_ptr(), C.stride(0),
+                                            V.data_ptr(), V.stride(0), self.ws.data_ptr(), self.ws.numel(),
+                                            self.bws.data_ptr(), self.bws.numel(), stream)
+        _lib.check(st, "updes_eval_values_prepared")
 
     def check_status(self):
         """Raise if a device-side wait or the factor check of an earlier batched call failed (syncs)."""
