@@ -23,6 +23,38 @@ __device__ __forceinline__ double ipow(double x, int e) {
   return r;
 }
 
+// ---- a square root with few FP64 operations ---------------------------------------------------------------------
+// GB300's FP64 pipe takes a warp instruction every 64 cycles and scheduler, so an FP64 operation costs as much issue
+// time as some fifty FP32 or integer ones.  Heron's (Newton's) iteration for sqrt(a) therefore starts from a
+// double-float root on the FP32 pipes: a is split by its bits into a float ah and the rest al, y0 is the hardware's
+// approximate 1 / sqrt(ah) (2^-22), and one step in FP32 on the exact residual ah - sh^2 + al gives sh + sl to about
+// 2^-44.  One FP64 step, whose residual is exact by FMA, then leaves the final rounding: 3 FP64 operations.
+constexpr int kRootExp = 70;  // arguments in [2^-70, 2^70); others take the library's functions
+
+// A float's value as a double, by its bits (a zero becomes 2^-127, far below what it is added to).
+__device__ __forceinline__ double bits_to_double(float f) {
+  const unsigned b = __float_as_uint(f);
+  return __hiloint2double(int((b & 0x80000000u) | (((b >> 3) & 0x0fffffffu) + (896u << 20))), int(b << 29));
+}
+__device__ __forceinline__ bool root_range(double a) {
+  return unsigned(__double2hiint(a) - ((1023 - kRootExp) << 20)) < (unsigned(2 * kRootExp) << 20);
+}
+// sqrt(a), a > 0
+__device__ __forceinline__ double root(double a) {
+  if (!root_range(a)) return sqrt(a);
+  const unsigned hi = unsigned(__double2hiint(a)), lo = unsigned(__double2loint(a));
+  const float ah = __uint_as_float(((hi - (896u << 20)) << 3) | (lo >> 29));
+  // the 29 bits below ah: their top 23 as an integer, times 2^(exponent - 46)
+  const float m = __fsub_rn(__uint_as_float(0x4b000000u | ((lo & 0x1fffffffu) >> 6)), 8388608.0f);
+  const float al = __fmul_rn(m, __uint_as_float((__float_as_uint(ah) & 0x7f800000u) - (46u << 23)));
+  float y0;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(ah));
+  const float sh = __fmul_rn(ah, y0), h = 0.5f * y0;
+  const float sl = __fmul_rn(__fadd_rn(__fmaf_rn(-sh, sh, ah), al), h);
+  const double s = bits_to_double(sh) + bits_to_double(sl);
+  return fma(fma(-s, s, a), bits_to_double(h), s);
+}
+
 // r2 = dx^2 + dy^2 > 0 is assumed; the caller handles r2 == 0.
 template <int KIND>
 __device__ __forceinline__ RbfG rbf_g(double r2, double param, int ip) {
