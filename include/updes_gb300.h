@@ -337,8 +337,12 @@ UPDES_API int updes_solve_many(const updes_problem* problems, int32_t count, con
                                updes_solve_info* infos, void* workspace, size_t workspace_bytes, int32_t streams);
 
 /*
- * Many independent systems in ONE persistent launch.  `ctas` CTAs (0 = one
- * per SM) take systems from a device work queue, largest first, and each CTA
+ * Many independent systems in one call of at most two launches.  With
+ * `ctas` = 0, systems that would hold one SM for longer than the average SM's
+ * share of the batch are solved by thread-block clusters of eight CTAs on a
+ * second stream, which `stream` waits for; the others, and with `ctas` > 0
+ * all of them, by `ctas` single CTAs (0 = one per SM).  Both take systems
+ * from device work queues, largest first; a CTA or a cluster
  * runs a system's whole solve by itself: assembly of K (FP64, equilibrated by
  * powers of two) and of the value rows [Phi P]; LU with partial pivoting in
  * panels of panel_width[i] columns (1..64, NULL = 16; chosen per system size
@@ -351,10 +355,13 @@ UPDES_API int updes_solve_many(const updes_problem* problems, int32_t count, con
  * (n_i) and vals[i] (N_i; vals or vals[i] may be NULL).  infos (may be NULL):
  * iters = refinement sweeps, lu_info, converged, backward_error.  Systems
  * must have N + M <= 4096 and no local supports (UPDES_ERR_UNSUPPORTED
- * otherwise).  No CTA waits for another.  The call synchronises `stream`; a
+ * otherwise).  Only the CTAs of one cluster wait for one another.  The order
+ * of the operations on an entry does not depend on who solves a system.  The
+ * call synchronises `stream`; a
  * singular system gives UPDES_ERR_SINGULAR (the others are still solved).
- * workspace: updes_solve_batched_workspace bytes (per CTA, K, the working
- * matrix and the value rows of the largest system: about 24 n_max^2 bytes).
+ * workspace: updes_solve_batched_workspace bytes (per CTA and per cluster, K,
+ * the working matrix and the value rows of its largest system: about
+ * 24 n_max^2 bytes).
  * The reference runs one pde_solver call per system
  * (updes/operators.py:559-618).
  */

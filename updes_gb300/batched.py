@@ -1,9 +1,11 @@
-"""Many independent systems in one persistent launch, with a panel-width autotuner.
+"""Many independent systems in one call, with a panel-width autotuner.
 
 The reference solves each system with its own ``pde_solver`` call (updes/operators.py:559-618).
 ``pde_solver_batched`` prepares every system on the host exactly as ``pde_solver`` does (operator capture,
-boundary rows, right-hand side) and hands them all to ``updes_solve_batched``: one CTA per SM takes systems
-from a device work queue, largest first, and runs each one's assembly, LU, refinement and values by itself.
+boundary rows, right-hand side) and hands them all to ``updes_solve_batched``: systems that would hold one SM for
+longer than the average SM's share of the batch are solved by thread-block clusters of eight CTAs, the others by
+single CTAs beside them.  Either takes systems from a device work queue, largest first, and runs each one's assembly,
+LU, refinement and values by itself.
 
 Precision per system:
 
@@ -19,7 +21,7 @@ Precision per system:
 
 The autotuner (``PanelTuner``) picks the LU panel width per (GPU, kernel, precision, size bucket): it times
 one launch on a single CTA for each candidate width on the largest system of the bucket in the batch, keeps
-the fastest, and caches the choice in memory and, unless disabled, in a JSON file
+the fastest (a cluster uses at least 32 columns), and caches the choice in memory and, unless disabled, in a JSON file
 (``$UPDES_TUNE_CACHE`` or ``~/.cache/updes_gb300/panel_widths.json``).
 """
 from __future__ import annotations
@@ -288,7 +290,7 @@ def _tune_widths(batch, precisions, tuner, max_sweeps):
 
 
 def pde_solver_batched(systems, options=None, precision="auto", max_sweeps=4, ctas=0, tuner="default"):
-    """Solve many independent systems in one persistent launch (``updes_solve_batched``).
+    """Solve many independent systems in one call (``updes_solve_batched``).
 
     ``systems``: dicts with the keyword arguments of ``pde_solver`` (as for ``pde_solver_many``); callable
     boundary conditions are evaluated as in ``pde_solver_jit``.  ``precision``: ``"auto"``, ``"fp32"``,

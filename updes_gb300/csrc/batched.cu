@@ -2,8 +2,9 @@
 //
 // The reference solves each system with its own pde_solver call (updes/operators.py:559-618).  Systems of a
 // few hundred to a few thousand nodes leave most of a GB300 idle one at a time, and a solve made of hundreds
-// of small launches per system is bound by launch and synchronisation latency.  Here one CTA per SM takes
-// systems from a device work queue (largest first) and runs the whole solve of each inside the CTA:
+// of small launches per system is bound by launch and synchronisation latency.  Here CTAs (one per SM), and for the
+// largest systems thread-block clusters of eight, take systems from device work queues (largest first) and run the
+// whole solve of each by themselves:
 //
 //   assembly   K (FP64, closed forms of entries.cuh), equilibrated by powers of two (rows, then columns);
 //              the value matrix A[:N] = [Phi P] for vals, in FP64
@@ -17,8 +18,8 @@
 //              so one or two sweeps reach the floor wherever cond(K) 2^-48 is small
 //   values     coeffs = Dc y, vals = A[:N] coeffs
 //
-// The CTA's scratch (its slice of the workspace) holds K, the working matrix and A for the largest system.
-// Every wait is a CTA barrier; there is no wait between CTAs, so nothing can hang on another CTA.
+// The scratch of a CTA or cluster (its slice of the workspace) holds K, the working matrix and A for the largest
+// system.  Every wait is a CTA or cluster barrier (the CTAs of a cluster run at the same time), so nothing can hang.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -29,6 +30,7 @@
 #include "df.cuh"
 #include "entries.cuh"
 #include "rbf.cuh"
+#include "side_stream.cuh"
 #include "stats.cuh"
 
 int updes_check_problem(const updes_problem* p);
@@ -37,9 +39,13 @@ namespace {
 
 constexpr int kBT = 512;                 // threads per CTA
 constexpr int kWarps = kBT / 32;
-constexpr int kTM = 128, kTN = 64;       // trailing-update tile: 4 x 4 entries per thread
+constexpr int kTM = 64, kTN = 64;        // trailing-update tile of half a CTA: 4 x 4 entries per thread
+constexpr int kTeams = 2;                // half CTAs, each on tiles of its own: one computes while the other loads
 constexpr int kMaxNB = 64;               // widest panel
+constexpr int kCoopNB = 32;              // panel width of a cluster: its panels are short chains whatever their width,
+                                         // and wider panels read the trailing matrix less often
 constexpr int kMaxBatchN = 4096;         // the solve's vectors live in shared memory
+constexpr int kMaxC = 8;                 // CTAs of a cooperative solve
 // A solve counts as converged at a componentwise backward error of 32 FP64 unit roundoffs (the residual is
 // FP64 here, K being kept in FP64), but refinement goes on while the error still halves, down to 2 unit
 // roundoffs: on the r^5 systems of a few hundred nodes the vals only agree with an FP64 LU's to within
@@ -60,15 +66,28 @@ struct BatchOut {
   double backward_error;
 };
 
-// Shared memory of one CTA: the LU's staged tiles, or the solve's two vectors.
-struct SmemLU {
-  double L[kTM][kMaxNB];      // L21 rows of the current row chunk (8-byte elements of either type)
-  double U[kMaxNB][kTN];      // U12 columns of the current column chunk
-  double L11[kMaxNB][kMaxNB]; // unit lower diagonal block of the panel
-  double prow[kMaxNB];        // pivot row of the panel column being eliminated
+// Shared memory of one CTA: a panel's rows, or the update's staged tiles, or the solve's two vectors and a staged block.
+struct TeamTiles {
+  float4 L[kTM][kMaxNB];  // L21 rows of the current row chunk: the elimination's stage_l writes and reads them
+  double U[kMaxNB][kTN];  // U12 columns of the current column chunk (stage_u)
 };
-constexpr size_t kSmemBytes = sizeof(SmemLU) > 2 * kMaxBatchN * sizeof(double) ? sizeof(SmemLU)
-                                                                                 : 2 * kMaxBatchN * sizeof(double);
+union SmemLU {
+  TeamTiles team[kTeams];
+  double L11[kMaxNB][kMaxNB];  // unit lower diagonal block of the panel
+};
+constexpr size_t kSmemBytes = 204 * 1024;
+static_assert(sizeof(SmemLU) <= kSmemBytes && 2 * kMaxBatchN * sizeof(double) + 32 * 33 * 8 <= kSmemBytes, "shared memory");
+
+// The rows of a panel column's exchange.
+struct PanelRows {
+  double cand[2][kMaxNB];  // by column parity: this CTA's best row, and the row at the diagonal if it has it
+  double diag[2][kMaxNB];
+  double prow[kMaxNB], drow[kMaxNB];
+  double inv;              // 1 / pivot in the elimination's type, 0 for an unusable pivot
+  int ok;
+  int piv[kMaxNB];
+  int start[kMaxC + 1];    // first row of every CTA's run
+};
 
 // Element arithmetic of the elimination: FP64, or double-float (F2, 8 bytes like a double).
 struct OpsF64 {
@@ -77,15 +96,21 @@ struct OpsF64 {
   static __device__ __forceinline__ double to_d(T a) { return a; }
   static __device__ __forceinline__ void fms(T& c, T a, T b) { c = fma(-a, b, c); }  // c -= a b
   static __device__ __forceinline__ T mul(T a, T b) { return a * b; }
-  // acc[a][b] -= sum_k L[a][k] U[k][16 b] over a 4 x 4 register tile (L rows ldl apart, U rows ldu apart)
-  static __device__ __forceinline__ void tile_update(T (&acc)[4][4], const T* L, int ldl, const T* U, int ldu,
-                                                     int kb) {
+  // column b (of 4) of thread tc's entries in a tile: a warp's loads of a U row are 16 consecutive entries
+  static __device__ __forceinline__ int column(int tc, int b) { return tc + 16 * b; }
+  static __device__ __forceinline__ void stage_l(TeamTiles& s, int r, int k, T v) {
+    reinterpret_cast<T*>(s.L)[r * kMaxNB + k] = v;
+  }
+  static __device__ __forceinline__ void stage_u(TeamTiles& s, int k, int c, T v) { s.U[k][c] = v; }
+  // acc[a][b] -= sum_k L[row + a][k] U[k][column(tc, b)]
+  static __device__ __forceinline__ void tile_update(T (&acc)[4][4], const TeamTiles& s, int row, int tc, int kb) {
+    const T* L = reinterpret_cast<const T*>(s.L) + row * kMaxNB;
     for (int k = 0; k < kb; ++k) {
       T la[4], ub[4];
 #pragma unroll
-      for (int a = 0; a < 4; ++a) la[a] = L[a * ldl + k];
+      for (int a = 0; a < 4; ++a) la[a] = L[a * kMaxNB + k];
 #pragma unroll
-      for (int b = 0; b < 4; ++b) ub[b] = U[k * ldu + 16 * b];
+      for (int b = 0; b < 4; ++b) ub[b] = s.U[k][column(tc, b)];
 #pragma unroll
       for (int a = 0; a < 4; ++a)
 #pragma unroll
@@ -113,27 +138,37 @@ struct OpsDF {
     c.h = h;
   }
   static __device__ __forceinline__ T mul(T a, T b) { return df_mul(a, b); }
-  // fms on two columns at once with the packed FP32x2 instructions of sm_100+ (one issue slot per pair): the
-  // same operations in the same order as fms, so bitwise the same results; y - x is fma(x, -1, y), which
-  // rounds once like the subtraction
+  // fms on two columns at once with the packed FP32x2 instructions of sm_100+: the same operations, with -a b as the
+  // product of -a (rounding is symmetric) so that nothing is negated, hence bitwise the same results; y - x is
+  // fma(x, -1, y), which rounds once like the subtraction.  A packed instruction takes the FMA pipe two cycles, and so
+  // does every move that puts a pair together: the tiles are staged as the pairs that are read, an L entry as
+  // (h, h, l, l), a row of U as a plane of high and one of low parts (the moves took 40 % of the pipe).
   static __device__ __forceinline__ float2 sub2(float2 y, float2 x) {
     return __ffma2_rn(x, make_float2(-1.f, -1.f), y);
   }
-  static __device__ __forceinline__ void fms2(float2& ch, float2& cl, T a, float2 bh, float2 bl) {
-    const float2 ah = make_float2(a.h, a.h), al = make_float2(a.l, a.l);
-    const float2 p = __fmul2_rn(ah, bh);
-    float2 e = __ffma2_rn(ah, bh, make_float2(-p.x, -p.y));
+  static __device__ __forceinline__ void fms2(float2& ch, float2& cl, float2 ah, float2 nah, float2 al, float2 bh,
+                                              float2 bl) {
+    const float2 np = __fmul2_rn(nah, bh);
+    float2 e = __ffma2_rn(ah, bh, np);
     e = __ffma2_rn(ah, bl, __ffma2_rn(al, bh, e));
-    const float2 s = sub2(ch, p);
+    const float2 s = __fadd2_rn(ch, np);
     const float2 v = sub2(s, ch);
-    float2 t = sub2(sub2(ch, sub2(s, v)), __fadd2_rn(p, v));
+    float2 t = __fadd2_rn(sub2(ch, sub2(s, v)), sub2(np, v));
     t = __fadd2_rn(t, sub2(cl, e));
     const float2 h = __fadd2_rn(s, t);
     cl = sub2(t, sub2(h, s));
     ch = h;
   }
-  static __device__ __forceinline__ void tile_update(T (&acc)[4][4], const T* L, int ldl, const T* U, int ldu,
-                                                     int kb) {
+  static __device__ __forceinline__ int column(int tc, int b) { return 2 * tc + (b & 1) + 32 * (b >> 1); }
+  static __device__ __forceinline__ void stage_l(TeamTiles& s, int r, int k, T v) {
+    s.L[r][k] = make_float4(v.h, v.h, v.l, v.l);
+  }
+  static __device__ __forceinline__ void stage_u(TeamTiles& s, int k, int c, T v) {
+    float* u = reinterpret_cast<float*>(s.U);
+    u[k * kTN + c] = v.h;
+    u[(kMaxNB + k) * kTN + c] = v.l;
+  }
+  static __device__ __forceinline__ void tile_update(T (&acc)[4][4], const TeamTiles& s, int row, int tc, int kb) {
     float2 ch[4][2], cl[4][2];
 #pragma unroll
     for (int a = 0; a < 4; ++a)
@@ -142,21 +177,23 @@ struct OpsDF {
         ch[a][q] = make_float2(acc[a][2 * q].h, acc[a][2 * q + 1].h);
         cl[a][q] = make_float2(acc[a][2 * q].l, acc[a][2 * q + 1].l);
       }
+    const float* u = reinterpret_cast<const float*>(s.U) + 2 * tc;
     for (int k = 0; k < kb; ++k) {
-      T la[4];
-      float2 ubh[2], ubl[2];
-#pragma unroll
-      for (int a = 0; a < 4; ++a) la[a] = L[a * ldl + k];
+      float2 bh[2], bl[2];
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
-        const T u0 = U[k * ldu + 32 * q], u1 = U[k * ldu + 32 * q + 16];
-        ubh[q] = make_float2(u0.h, u1.h);
-        ubl[q] = make_float2(u0.l, u1.l);
+        bh[q] = *reinterpret_cast<const float2*>(u + k * kTN + 32 * q);
+        bl[q] = *reinterpret_cast<const float2*>(u + (kMaxNB + k) * kTN + 32 * q);
       }
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
+      for (int a = 0; a < 4; ++a) {
+        const float4 l = s.L[row + a][k];
+        const float2 ah = make_float2(l.x, l.y), al = make_float2(l.z, l.w);
+        const float2 nah = make_float2(__uint_as_float(__float_as_uint(l.x) ^ 0x80000000u),
+                                       __uint_as_float(__float_as_uint(l.y) ^ 0x80000000u));
 #pragma unroll
-        for (int q = 0; q < 2; ++q) fms2(ch[a][q], cl[a][q], la[a], ubh[q], ubl[q]);
+        for (int q = 0; q < 2; ++q) fms2(ch[a][q], cl[a][q], ah, nah, al, bh[q], bl[q]);
+      }
     }
 #pragma unroll
     for (int a = 0; a < 4; ++a)
@@ -175,24 +212,92 @@ __device__ __forceinline__ double pow2_scale(double m) {
   return ldexp(1.0, -e);
 }
 
-// max over the CTA of (value, -index): the largest value, the smallest index on ties.
-__device__ __forceinline__ void cta_argmax(double& v, int& i, double* red_v, int* red_i) {
+// The CTAs that solve one system: a thread-block cluster (COOP), whose threads share the rows, columns and tiles of
+// every phase, or one CTA by itself.  Either way each entry sees the same operations in the same order, so the results
+// are bitwise the same.
+struct Exchange {
+  double v[2][kMaxC];
+  int i[2][kMaxC];
+};
+
+template <bool COOP>
+struct Group {
+  int rank = 0, ctas = 1;
+  int parity = 0;  // of the exchange slots: one is rewritten two barriers after it was read
+  Exchange* ex = nullptr;
+  __device__ __forceinline__ int thread() const { return COOP ? rank * kBT + int(threadIdx.x) : int(threadIdx.x); }
+  __device__ __forceinline__ int threads() const { return COOP ? ctas * kBT : kBT; }
+  __device__ __forceinline__ int warp() const { return thread() >> 5; }
+  __device__ __forceinline__ int warps() const { return COOP ? ctas * kWarps : kWarps; }
+  __device__ __forceinline__ void sync() const {
+    if constexpr (COOP)
+      asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    else
+      __syncthreads();
+  }
+  // the address of one of this CTA's shared variables in CTA `cta` of the cluster
+  static __device__ __forceinline__ uint32_t remote(const void* p, int cta) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))), "r"(cta));
+    return r;
+  }
+  static __device__ __forceinline__ void put(uint32_t at, double v) {
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(at), "d"(v) : "memory");
+  }
+  // an 8-byte shared variable of CTA `cta`
+  static __device__ __forceinline__ double get(const double* p, int cta) {
+    if constexpr (!COOP) return *p;
+    double v;
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(remote(p, cta)) : "memory");
+    return v;
+  }
+  // every CTA's (v, i) to every CTA (all threads hold the same pair); the group's largest v (none negative: compared by
+  // their bits), smallest i on ties
+  __device__ __forceinline__ void argmax(double& v, int& i) {
+    if constexpr (COOP) {
+      if (int(threadIdx.x) < ctas) {
+        put(remote(&ex->v[parity][rank], int(threadIdx.x)), v);
+        asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(remote(&ex->i[parity][rank], int(threadIdx.x))), "r"(i)
+                     : "memory");
+      }
+      sync();
+      unsigned long long k = static_cast<unsigned long long>(__double_as_longlong(ex->v[parity][0]));
+      i = ex->i[parity][0];
+      for (int c = 1; c < ctas; ++c) {
+        const unsigned long long ok = static_cast<unsigned long long>(__double_as_longlong(ex->v[parity][c]));
+        const int oi = ex->i[parity][c];
+        if (ok > k || (ok == k && oi < i)) { k = ok; i = oi; }
+      }
+      v = __longlong_as_double(static_cast<long long>(k));
+      parity ^= 1;
+    }
+  }
+};
+
+// Order key of a pivot candidate's |a|: its bits + 1, which order like the values (NaN counts as infinity, so it wins and
+// surfaces as a bad pivot); 0 for no candidate.  Integers, because the FP64 pipe takes a comparison 64 cycles.
+using Key = unsigned long long;
+__device__ __forceinline__ Key key_of(double a) {
+  return min(static_cast<Key>(__double_as_longlong(a)) & 0x7fffffffffffffffull, Key(0x7ff0000000000000ull)) + 1;
+}
+// The warp's largest key and the smallest row that has it.
+__device__ __forceinline__ void warp_best(Key& key, int& row) {
+  const unsigned hi = unsigned(key >> 32), lo = unsigned(key);
+  const unsigned hm = __reduce_max_sync(0xffffffffu, hi);
+  const unsigned lm = __reduce_max_sync(0xffffffffu, hi == hm ? lo : 0u);
+  row = __reduce_min_sync(0xffffffffu, (hi == hm && lo == lm) ? row : 0x7fffffff);
+  key = (Key(hm) << 32) | lm;
+}
+// The group's best candidate from every thread's.
+template <bool COOP>
+__device__ __forceinline__ void group_best(Key& key, int& row, Key* red_k, int* red_i, Group<COOP>& grp) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int o = 16; o > 0; o >>= 1) {
-    const double ov = __shfl_xor_sync(0xffffffffu, v, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, i, o);
-    if (ov > v || (ov == v && oi < i)) { v = ov; i = oi; }
-  }
-  if (lane == 0) { red_v[w] = v; red_i[w] = i; }
+  warp_best(key, row);
+  if (lane == 0) { red_k[w] = key; red_i[w] = row; }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int k = 1; k < kWarps; ++k)
-      if (red_v[k] > red_v[0] || (red_v[k] == red_v[0] && red_i[k] < red_i[0])) { red_v[0] = red_v[k]; red_i[0] = red_i[k]; }
-  }
-  __syncthreads();
-  v = red_v[0];
-  i = red_i[0];
-  __syncthreads();
+  key = red_k[lane & (kWarps - 1)];
+  row = red_i[lane & (kWarps - 1)];
+  warp_best(key, row);
 }
 
 __device__ __forceinline__ double cta_max(double v, double* red_v) {
@@ -212,13 +317,13 @@ __device__ __forceinline__ double cta_max(double v, double* red_v) {
 
 // K (n x ld, FP64) and A[:N] (N x ld, FP64) of one system, K equilibrated in place: dr (rows) and dc
 // (columns) are the powers of two applied, b = Dr [q; 0].  One warp per row.
-template <int KIND>
+template <int KIND, bool COOP>
 __device__ void assemble_system(const BatchSys& sys, double* K, double* A, int64_t ld, double* dr, double* dc,
-                                double* b, double* red_v) {
+                                double* b, double* part, const Group<COOP>& grp) {
   const updes_problem& p = sys.p;
-  const int n = sys.n, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n = sys.n, lane = threadIdx.x & 31;
   const int ip = (KIND == UPDES_RBF_POLYHARMONIC) ? 2 * int(p.rbf_param) + 1 : int(p.rbf_param);
-  for (int r = warp; r < n; r += kWarps) {
+  for (int r = grp.warp(); r < n; r += grp.warps()) {
     const RowInfo ri = load_row(p, r);
     double* Kr = K + int64_t(r) * ld;
     double* Ar = A + int64_t(r) * ld;
@@ -259,22 +364,33 @@ __device__ void assemble_system(const BatchSys& sys, double* K, double* A, int64
       }
     }
   }
-  __syncthreads();
-  // column powers of two over the row-scaled K, applied in place
+  grp.sync();
+  // column powers of two over the row-scaled K: a CTA takes a range of rows (a maximum does not depend on the order)
+  const int r0 = int(int64_t(n) * grp.rank / grp.ctas), r1 = int(int64_t(n) * (grp.rank + 1) / grp.ctas);
   for (int c = threadIdx.x; c < n; c += kBT) {
     double mx = 0.0;
-    for (int r = 0; r < n; ++r) mx = fmax(mx, fabs(K[int64_t(r) * ld + c]));
-    dc[c] = pow2_scale(mx);
+#pragma unroll 8
+    for (int r = r0; r < r1; ++r) mx = fmax(mx, fabs(K[int64_t(r) * ld + c]));
+    if constexpr (COOP) part[int64_t(grp.rank) * n + c] = mx;
+    else dc[c] = pow2_scale(mx);
   }
-  __syncthreads();
-  (void)red_v;
+  grp.sync();
+  if constexpr (COOP) {
+    for (int c = grp.thread(); c < n; c += grp.threads()) {
+      double mx = 0.0;
+      for (int k = 0; k < grp.ctas; ++k) mx = fmax(mx, part[int64_t(k) * n + c]);
+      dc[c] = pow2_scale(mx);
+    }
+    grp.sync();
+  }
 }
 
 // W = K (scaled) converted to the elimination's type.
-template <class Ops>
-__device__ void scale_columns_to_w(const BatchSys& sys, double* K, typename Ops::T* W, int64_t ld, const double* dc) {
+template <class Ops, bool COOP>
+__device__ void scale_columns_to_w(const BatchSys& sys, double* K, typename Ops::T* W, int64_t ld, const double* dc,
+                                   const Group<COOP>& grp) {
   const int n = sys.n;
-  for (int r = threadIdx.x >> 5; r < n; r += kWarps) {
+  for (int r = grp.warp(); r < n; r += grp.warps()) {
     double* Kr = K + int64_t(r) * ld;
     typename Ops::T* Wr = W + int64_t(r) * ld;
     for (int c = threadIdx.x & 31; c < n; c += 32) {
@@ -283,209 +399,329 @@ __device__ void scale_columns_to_w(const BatchSys& sys, double* K, typename Ops:
       Wr[c] = Ops::from_d(v);
     }
   }
-  __syncthreads();
+  grp.sync();
 }
 
 // ---- LU -----------------------------------------------------------------------------------------------------
 
-template <class Ops>
-__device__ int cta_lu(typename Ops::T* W, int64_t ld, int n, int nb, int32_t* piv, SmemLU& sm, double* red_v,
-                      int* red_i) {
+// Panel [k0, k0 + kb) of the rows [k0, n), in shared memory: the group's CTAs hold consecutive runs of rows.  Per
+// column: CTA maximum (taken while the column was updated), the best row and the diagonal row staged, one cluster
+// barrier, the winner's row and the diagonal row fetched, the interchange and the update of the CTA's own rows, a
+// thread per row.  The interchanges of the columns outside the panel follow at its end, a thread per column.
+// (With the rows in global memory, a row per thread, and every interchange at once a column took 15 to 20 us on eight
+// CTAs, this about 3.)
+template <class Ops, bool COOP>
+__device__ int group_panel(typename Ops::T* W, int64_t ld, int n, int k0, int kb, int32_t* piv, SmemLU& sm,
+                           PanelRows& pr, Key* red_k, int* red_i, Group<COOP>& grp) {
   using T = typename Ops::T;
+  static_assert(sizeof(T) == 8, "rows travel as 8-byte words");
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int m = n - k0, ldt = kb | 1;
+  if (tid <= grp.ctas) pr.start[tid] = k0 + int(int64_t(m) * tid / grp.ctas);
+  __syncthreads();
+  const int rlo = pr.start[grp.rank], rows = pr.start[grp.rank + 1] - rlo;
+  T* tile = reinterpret_cast<T*>(&sm);
+  T* prow = reinterpret_cast<T*>(pr.prow);
+  T* drow = reinterpret_cast<T*>(pr.drow);
+  for (int l = warp; l < rows; l += kWarps)
+    for (int c = lane; c < kb; c += 32) tile[l * ldt + c] = W[int64_t(rlo + l) * ld + k0 + c];
+  __syncthreads();
   int info = 0;
-  T* L = reinterpret_cast<T*>(&sm.L[0][0]);
-  T* U = reinterpret_cast<T*>(&sm.U[0][0]);
+  Key bk = 0;
+  int bi = n;
+  auto candidate = [&](T x, int row) {
+    const Key k = key_of(Ops::to_d(x));
+    if (k > bk) { bk = k; bi = row; }
+  };
+  for (int l = tid; l < rows; l += kBT) candidate(tile[l * ldt], rlo + l);
+  for (int j = 0; j < kb; ++j) {
+    const int par = j & 1, dg = k0 + j;
+    group_best(bk, bi, red_k, red_i, grp);
+    if (tid < kb && bi >= rlo && bi < rlo + rows)
+      reinterpret_cast<T*>(pr.cand[par])[tid] = tile[(bi - rlo) * ldt + tid];
+    if (tid >= 64 && tid - 64 < kb && dg >= rlo && dg < rlo + rows)
+      reinterpret_cast<T*>(pr.diag[par])[tid - 64] = tile[(dg - rlo) * ldt + tid - 64];
+    if constexpr (COOP) {
+      double v = __longlong_as_double(static_cast<long long>(bk));  // (a key travels and compares as its bits)
+      grp.argmax(v, bi);
+    } else {
+      __syncthreads();
+    }
+    const int p = bi < n ? bi : dg;
+    if (tid < 128 && (tid & 63) < kb) {
+      // the owner of row r: the last CTA whose run starts at or before it
+      const int c = tid & 63, r = tid < 64 ? p : dg;
+      int owner = 0;
+      for (int q = 1; q < grp.ctas; ++q)
+        if (pr.start[q] <= r) owner = q;
+      const double* from = tid < 64 ? (bi < n ? pr.cand[par] : pr.diag[par]) : pr.diag[par];
+      (tid < 64 ? pr.prow : pr.drow)[c] = Group<COOP>::get(from + c, owner);
+      if (tid == j) {  // one thread's division, while the rows are interchanged
+        const double pv = Ops::to_d(prow[j]);
+        const bool ok = pv != 0.0 && isfinite(pv);
+        reinterpret_cast<T&>(pr.inv) = Ops::from_d(ok ? 1.0 / pv : 0.0);
+        pr.ok = ok;
+        pr.piv[j] = p;
+      }
+    }
+    __syncthreads();
+    if (p != dg) {  // the interchange inside the panel
+      if (tid < kb && dg >= rlo && dg < rlo + rows) tile[(dg - rlo) * ldt + tid] = prow[tid];
+      if (tid >= 64 && tid - 64 < kb && p >= rlo && p < rlo + rows) tile[(p - rlo) * ldt + tid - 64] = drow[tid - 64];
+    }
+    __syncthreads();
+    bk = 0;
+    bi = n;
+    const T inv = reinterpret_cast<const T&>(pr.inv);
+    const bool ok = pr.ok;
+    if (tid == 0 && !ok && info == 0) info = dg + 1;
+    for (int l = max(0, dg + 1 - rlo) + tid; l < rows; l += kBT) {
+      T* row = tile + l * ldt;
+      if (ok) {
+        const T x = Ops::mul(row[j], inv);
+        row[j] = x;
+        for (int c = j + 1; c < kb; ++c) Ops::fms(row[c], x, prow[c]);
+      }
+      if (j + 1 < kb) candidate(row[j + 1], rlo + l);
+    }
+  }
+  __syncthreads();
+  for (int l = warp; l < rows; l += kWarps)
+    for (int c = lane; c < kb; c += 32) W[int64_t(rlo + l) * ld + k0 + c] = tile[l * ldt + c];
+  if (grp.rank == 0 && tid < kb) piv[k0 + tid] = pr.piv[tid];
+  for (int c0 = grp.thread(); c0 < n - kb; c0 += grp.threads()) {
+    T* col = W + (c0 < k0 ? c0 : c0 + kb);
+    for (int j = 0; j < kb; ++j) {
+      const int p = pr.piv[j];
+      if (p != k0 + j) {
+        const T a = col[int64_t(k0 + j) * ld], b = col[int64_t(p) * ld];
+        col[int64_t(k0 + j) * ld] = b;
+        col[int64_t(p) * ld] = a;
+      }
+    }
+  }
+  grp.sync();
+  return info;
+}
+
+template <class Ops, bool COOP>
+__device__ int group_lu(typename Ops::T* W, int64_t ld, int n, int nb_max, int32_t* piv, SmemLU& sm, PanelRows& pr,
+                        Key* red_k, int* red_i, Group<COOP>& grp) {
+  using T = typename Ops::T;
+  const int tid = threadIdx.x, team = tid / (kBT / kTeams), ttid = tid % (kBT / kTeams);
+  int info = 0;
+  TeamTiles& tiles_s = sm.team[team];
   T* L11 = reinterpret_cast<T*>(&sm.L11[0][0]);
-  T* prow = reinterpret_cast<T*>(&sm.prow[0]);
-  for (int k0 = 0; k0 < n; k0 += nb) {
-    const int kb = min(nb, n - k0);
+  auto team_sync = [&] { asm volatile("bar.sync %0, %1;" ::"r"(1 + team), "n"(kBT / kTeams) : "memory"); };
+  int kb;
+  for (int k0 = 0; k0 < n; k0 += kb) {
+    // the widest panel whose rows fit in shared memory (an entry's operations do not depend on the width)
+    const int rows = (n - k0 + grp.ctas - 1) / grp.ctas;
+    kb = min(nb_max, n - k0);
+    while (size_t(rows) * (kb | 1) * sizeof(T) > kSmemBytes) kb = (kb + 1) / 2;
     const int k1 = k0 + kb;
-    // ---- panel: columns [k0, k1), rows [k0, n).  One thread per row for the scaling and the rank-1
-    // update (its row's panel entries are adjacent, so after the first access they come from L1, and the
-    // CTA's 512 rows are in flight at once); the candidate for the next column's pivot is taken on the way.
-    double bv = -1.0;
-    int bi = n;
-    for (int i = k0 + tid; i < n; i += kBT) {
-      double v = fabs(Ops::to_d(W[int64_t(i) * ld + k0]));
-      if (v != v) v = INFINITY;  // NaN wins, so it surfaces as a bad pivot
-      if (v > bv) { bv = v; bi = i; }
-    }
-    for (int j = k0; j < k1; ++j) {
-      cta_argmax(bv, bi, red_v, red_i);
-      const int p = bi < n ? bi : j;
-      if (p != j)
-        for (int c = tid; c < n; c += kBT) {
-          T* a = W + int64_t(j) * ld + c;
-          T* b = W + int64_t(p) * ld + c;
-          const T t = *a;
-          *a = *b;
-          *b = t;
-        }
-      __syncthreads();
-      const double pv = Ops::to_d(W[int64_t(j) * ld + j]);
-      const bool ok = pv != 0.0 && isfinite(pv);
-      if (tid == 0) {
-        piv[j] = p;
-        if (!ok && info == 0) info = j + 1;
-      }
-      for (int c = j + 1 + tid; c < k1; c += kBT) prow[c - k0] = W[int64_t(j) * ld + c];
-      __syncthreads();
-      bv = -1.0;
-      bi = n;
-      const T inv = Ops::from_d(ok ? 1.0 / pv : 0.0);
-      // rows below: scale column j and update the panel's columns (j, k1), one thread per row; the row's
-      // remaining panel entries are loaded together (one round trip), updated in a local copy and stored
-      // back, and the candidate for the next column's pivot is taken on the way.  (A warp-per-row mapping
-      // with coalesced accesses and eight rows in flight per warp measured slower on GB300.)
-      for (int i = j + 1 + tid; i < n; i += kBT) {
-        T* Wi = W + int64_t(i) * ld;
-        if (ok) {
-          T rowv[kMaxNB];
-          const int cnt = k1 - j;  // columns j .. k1 - 1
-          for (int c = 0; c < cnt; ++c) rowv[c] = Wi[j + c];
-          const T l = Ops::mul(rowv[0], inv);
-          rowv[0] = l;
-          for (int c = 1; c < cnt; ++c) Ops::fms(rowv[c], l, prow[j + c - k0]);
-          for (int c = 0; c < cnt; ++c) Wi[j + c] = rowv[c];
-          if (cnt > 1) {
-            double v = fabs(Ops::to_d(rowv[1]));
-            if (v != v) v = INFINITY;
-            if (v > bv) { bv = v; bi = i; }
-          }
-        } else if (j + 1 < k1) {
-          double v = fabs(Ops::to_d(Wi[j + 1]));
-          if (v != v) v = INFINITY;
-          if (v > bv) { bv = v; bi = i; }
-        }
-      }
-      __syncthreads();
-    }
+    const int e = group_panel<Ops>(W, ld, n, k0, kb, piv, sm, pr, red_k, red_i, grp);
+    if (info == 0) info = e;
     if (k1 >= n) break;
-    // ---- U12 = L11^-1 A12 (rows [k0, k1), columns [k1, n))
+    // ---- U12 = L11^-1 A12 (rows [k0, k1), columns [k1, n)), a thread per column, 16 rows at a time in registers
     for (int e = tid; e < kb * kb; e += kBT) {
       const int r = e / kb, c = e % kb;
       L11[r * kMaxNB + c] = W[int64_t(k0 + r) * ld + k0 + c];
     }
     __syncthreads();
-    for (int c = k1 + tid; c < n; c += kBT) {
-      T col[kMaxNB];
-      for (int r = 0; r < kb; ++r) col[r] = W[int64_t(k0 + r) * ld + c];
-      for (int r = 1; r < kb; ++r)
-        for (int t = 0; t < r; ++t) Ops::fms(col[r], L11[r * kMaxNB + t], col[t]);
-      for (int r = 1; r < kb; ++r) W[int64_t(k0 + r) * ld + c] = col[r];
-    }
-    __syncthreads();
-    // ---- A22 -= L21 U12 in 128 x 64 tiles, 4 x 4 entries per thread
-    const int tr = tid >> 4, tc = tid & 15;
-    for (int r0 = k1; r0 < n; r0 += kTM) {
-      const int rows = min(kTM, n - r0);
-      for (int e = tid; e < kTM * kb; e += kBT) {
-        const int r = e / kb, c = e % kb;
-        if (r < rows) L[r * kMaxNB + c] = W[int64_t(r0 + r) * ld + k0 + c];
-      }
-      for (int c0 = k1; c0 < n; c0 += kTN) {
-        const int cols = min(kTN, n - c0);
-        __syncthreads();  // the previous tile is done with U (and L has been staged)
-        for (int e = tid; e < kb * kTN; e += kBT) {
-          const int r = e / kTN, c = e % kTN;
-          if (c < cols) U[r * kTN + c] = W[int64_t(k0 + r) * ld + c0 + c];
+    for (int c = k1 + grp.thread(); c < n; c += grp.threads()) {
+      T* col = W + int64_t(k0) * ld + c;
+      for (int rb = 0; rb < kb; rb += 16) {
+        T x[16];
+#pragma unroll
+        for (int r = 0; r < 16; ++r) x[r] = rb + r < kb ? col[int64_t(rb + r) * ld] : Ops::from_d(0.0);
+        for (int t = 0; t < rb; ++t) {
+          const T xt = col[int64_t(t) * ld];
+#pragma unroll
+          for (int r = 0; r < 16; ++r)
+            if (rb + r < kb) Ops::fms(x[r], L11[(rb + r) * kMaxNB + t], xt);
         }
-        __syncthreads();
-        // thread (tr, tc) owns rows 4 tr .. 4 tr + 3 and columns tc + 16 b: a warp's loads of a U row are then
-        // 16 consecutive entries (no shared-memory bank conflicts), and its C accesses 128-byte row segments
-        T acc[4][4];
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
+        for (int r = 1; r < 16; ++r)
+          if (rb + r < kb)
 #pragma unroll
-          for (int b = 0; b < 4; ++b) {
-            const int r = 4 * tr + a, c = tc + 16 * b;
-            acc[a][b] = (r < rows && c < cols) ? W[int64_t(r0 + r) * ld + c0 + c] : Ops::from_d(0.0);
-          }
-        Ops::tile_update(acc, L + (4 * tr) * kMaxNB, kMaxNB, U + tc, kTN, kb);
+            for (int t = 0; t < r; ++t) Ops::fms(x[r], L11[(rb + r) * kMaxNB + rb + t], x[t]);
 #pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b) {
-            const int r = 4 * tr + a, c = tc + 16 * b;
-            if (r < rows && c < cols) W[int64_t(r0 + r) * ld + c0 + c] = acc[a][b];
-          }
+        for (int r = 0; r < 16; ++r)
+          if (rb + r < kb) col[int64_t(rb + r) * ld] = x[r];
       }
-      __syncthreads();  // L is restaged for the next row chunk
     }
+    grp.sync();
+    // ---- A22 -= L21 U12 in 64 x 64 tiles, 4 x 4 entries per thread; half a CTA takes a run of consecutive tiles, so that
+    // it stages the rows of L21 seldom
+    const int tr = ttid >> 4, tc = ttid & 15;
+    const int tiles_c = (n - k1 + kTN - 1) / kTN, tiles = (n - k1 + kTM - 1) / kTM * tiles_c;
+    const int who = grp.rank * kTeams + team, all = grp.ctas * kTeams;
+    const int t0 = int(int64_t(tiles) * who / all), t1 = int(int64_t(tiles) * (who + 1) / all);
+    int staged = -1;
+    for (int t = t0; t < t1; ++t) {
+      const int r0 = k1 + t / tiles_c * kTM, c0 = k1 + t % tiles_c * kTN;
+      const int rows_t = min(kTM, n - r0), cols = min(kTN, n - c0);
+      // thread (tr, tc) owns rows 4 tr .. 4 tr + 3 and four columns
+      T acc[4][4];
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const int r = 4 * tr + a, c = Ops::column(tc, b);
+          acc[a][b] = (r < rows_t && c < cols) ? W[int64_t(r0 + r) * ld + c0 + c] : Ops::from_d(0.0);
+        }
+      team_sync();  // the previous tile is done with L and U
+      if (staged != r0) {
+        for (int e = ttid; e < kTM * kb; e += kBT / kTeams) {
+          const int r = e / kb, c = e % kb;
+          if (r < rows_t) Ops::stage_l(tiles_s, r, c, W[int64_t(r0 + r) * ld + k0 + c]);
+        }
+        staged = r0;
+      }
+      for (int e = ttid; e < kb * kTN; e += kBT / kTeams) {
+        const int r = e / kTN, c = e % kTN;
+        if (c < cols) Ops::stage_u(tiles_s, r, c, W[int64_t(k0 + r) * ld + c0 + c]);
+      }
+      team_sync();
+      Ops::tile_update(acc, tiles_s, 4 * tr, tc, kb);
+#pragma unroll
+      for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+          const int r = 4 * tr + a, c = Ops::column(tc, b);
+          if (r < rows_t && c < cols) W[int64_t(r0 + r) * ld + c0 + c] = acc[a][b];
+        }
+    }
+    grp.sync();  // the next panel reads what other CTAs updated, and writes over the staged tiles
   }
-  __syncthreads();
   return info;
 }
 
 // ---- triangular solves on a shared-memory vector ------------------------------------------------------------
 
-// v = U^-1 L^-1 P v with the factors in W (LAPACK layout: piv[j] is the row swapped with j at step j).  The
-// forward and backward substitutions go by blocks of 32 rows: warp 0 solves a block's diagonal part, then all
-// warps subtract the block's columns from the rows still to come (one warp per row, lanes over the block's
-// columns, coalesced).
-template <class Ops>
-__device__ void cta_lu_solve(const typename Ops::T* W, int64_t ld, int n, const int32_t* piv, double* v) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0)
+// The row permutation of the interchanges: perm[i] is the row that ends up at i.  One thread, on shared memory (scratch:
+// 2 n ints).
+__device__ void permutation(const int32_t* piv, int n, int32_t* perm, int* scratch) {
+  int *sp = scratch, *row = scratch + n;
+  for (int i = threadIdx.x; i < n; i += kBT) {
+    sp[i] = piv[i];
+    row[i] = i;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0)
     for (int j = 0; j < n; ++j) {
-      const int p = piv[j];
-      if (p != j) { const double t = v[j]; v[j] = v[p]; v[p] = t; }
+      const int p = sp[j];
+      if (p != j) { const int t = row[j]; row[j] = row[p]; row[p] = t; }
     }
   __syncthreads();
-  // forward: unit lower
-  for (int b0 = 0; b0 < n; b0 += 32) {
-    const int bs = min(32, n - b0);
-    if (warp == 0) {
-      double xv = lane < bs ? v[b0 + lane] : 0.0;
-      for (int r = 1; r < bs; ++r) {
-        const double lr = lane < r ? Ops::to_d(W[int64_t(b0 + r) * ld + b0 + lane]) : 0.0;
-        double s = lr * xv;
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == r) xv -= s;
-      }
-      if (lane < bs) v[b0 + lane] = xv;
-    }
-    __syncthreads();
-    const double xb = lane < bs ? v[b0 + lane] : 0.0;
-    for (int i = b0 + bs + warp; i < n; i += kWarps) {
-      double s = lane < bs ? Ops::to_d(W[int64_t(i) * ld + b0 + lane]) * xb : 0.0;
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == 0) v[i] -= s;
-    }
-    __syncthreads();
-  }
-  // backward: upper with its diagonal
+  for (int i = threadIdx.x; i < n; i += kBT) perm[i] = row[i];
+  __syncthreads();
+}
+
+// v = U^-1 L^-1 v (v already permuted) with the factors in W.  The forward and backward substitutions go by blocks of 32
+// rows: warp 0 solves a block's diagonal part (staged in shared memory), then all warps subtract the block's columns
+// from the rows still to come (one warp per row, lanes over the block's columns, coalesced, four rows at a time).  In a
+// cluster every CTA holds v, block b is solved and its rows are kept up to date by CTA b % ctas, and each solved block
+// goes to all of them.
+template <class Ops, bool COOP>
+__device__ void group_lu_solve(const typename Ops::T* W, int64_t ld, int n, double* v, typename Ops::T (*diag)[33],
+                               const Group<COOP>& grp) {
+  using T = typename Ops::T;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nblk = (n + 31) / 32;
-  for (int bb = nblk - 1; bb >= 0; --bb) {
-    const int b0 = bb * 32, bs = min(32, n - b0);
-    if (warp == 0) {
-      double xv = lane < bs ? v[b0 + lane] : 0.0;
-      for (int r = bs - 1; r >= 0; --r) {
-        const double ur = (lane > r && lane < bs) ? Ops::to_d(W[int64_t(b0 + r) * ld + b0 + lane]) : 0.0;
-        double s = ur * xv;
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == r) xv = (xv - s) / Ops::to_d(W[int64_t(b0 + r) * ld + b0 + r]);
-      }
-      if (lane < bs) v[b0 + lane] = xv;
+  auto stage = [&](int b0, int bs) {
+    for (int e = tid; e < 32 * 32; e += kBT) {
+      const int r = e >> 5, c = e & 31;
+      if (r < bs && c < bs) diag[r][c] = W[int64_t(b0 + r) * ld + b0 + c];
     }
     __syncthreads();
+  };
+  auto publish = [&](int b0, int bs, double xv) {
+    if (lane < bs) {
+      v[b0 + lane] = xv;
+      if constexpr (COOP)
+        for (int c = 0; c < grp.ctas; ++c)
+          if (c != grp.rank) Group<COOP>::put(Group<COOP>::remote(&v[b0 + lane], c), xv);
+    }
+  };
+  // Rows of the blocks [q0, q1) that this CTA keeps: v[i] -= sum over the block at b0 of W[i][b0 + .] v[b0 + .], 16 rows a
+  // warp.  The sums run over the lanes in halves (16, 8, 4, 2, 1 apart); each exchange also halves the rows that a lane
+  // goes on with, which leaves the same additions in the same order but a third of the FP64 instructions.
+  auto subtract = [&](int q0, int q1, int b0, int bs) {
     const double xb = lane < bs ? v[b0 + lane] : 0.0;
-    for (int i = warp; i < b0; i += kWarps) {
-      double s = lane < bs ? Ops::to_d(W[int64_t(i) * ld + b0 + lane]) * xb : 0.0;
-      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (lane == 0) v[i] -= s;
+    const int first = COOP ? q0 + ((grp.rank - q0) % grp.ctas + grp.ctas) % grp.ctas : q0;
+    const int step = COOP ? grp.ctas : 1;
+    const int halves = first < q1 ? (q1 - first + step - 1) / step * 2 : 0;
+    for (int k = warp; k < halves; k += kWarps) {
+      const int i0 = (first + (k >> 1) * step) * 32 + (k & 1) * 16;
+      double s[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u)
+        s[u] = (i0 + u < n && lane < bs) ? Ops::to_d(W[int64_t(i0 + u) * ld + b0 + lane]) * xb : 0.0;
+#pragma unroll
+      for (int h = 8; h > 0; h >>= 1) {  // lanes 2 h apart exchange; the upper one keeps the rows from h on
+        const bool up = lane & (2 * h);
+#pragma unroll
+        for (int u = 0; u < h; ++u) {
+          const double mine = up ? s[u + h] : s[u], theirs = up ? s[u] : s[u + h];
+          s[u] = mine + __shfl_xor_sync(0xffffffffu, theirs, 2 * h);
+        }
+      }
+      const double total = s[0] + __shfl_xor_sync(0xffffffffu, s[0], 1);
+      const int row = i0 + (lane >> 1);
+      if ((lane & 1) == 0 && row < n) v[row] -= total;
     }
-    __syncthreads();
+  };
+  // forward: unit lower
+  for (int q = 0; q < nblk; ++q) {
+    const int b0 = q * 32, bs = min(32, n - b0);
+    if (!COOP || grp.rank == q % grp.ctas) {
+      stage(b0, bs);  // (its barrier also completes this CTA's updates of the block's rows)
+      if (warp == 0) {
+        double xv = lane < bs ? v[b0 + lane] : 0.0;
+        for (int r = 1; r < bs; ++r) {
+          const double lr = lane < r ? Ops::to_d(diag[r][lane]) : 0.0;
+          double s = lr * xv;
+          for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+          if (lane == r) xv -= s;
+        }
+        publish(b0, bs, xv);
+      }
+    }
+    grp.sync();
+    subtract(q + 1, nblk, b0, bs);
   }
+  grp.sync();
+  // backward: upper with its diagonal
+  for (int q = nblk - 1; q >= 0; --q) {
+    const int b0 = q * 32, bs = min(32, n - b0);
+    if (!COOP || grp.rank == q % grp.ctas) {
+      stage(b0, bs);
+      if (warp == 0) {
+        double xv = lane < bs ? v[b0 + lane] : 0.0;
+        for (int r = bs - 1; r >= 0; --r) {
+          const double ur = (lane > r && lane < bs) ? Ops::to_d(diag[r][lane]) : 0.0;
+          double s = ur * xv;
+          for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+          if (lane == r) xv = (xv - s) / Ops::to_d(diag[r][r]);
+        }
+        publish(b0, bs, xv);
+      }
+    }
+    grp.sync();
+    subtract(0, q, b0, bs);
+  }
+  grp.sync();
 }
 
 // r = b - K y (FP64, K the equilibrated matrix), returns max_i |r_i| / max_i (|K| |y| + |b|)_i.
-__device__ double cta_residual(const double* K, int64_t ld, int n, const double* y, const double* b, double* r,
-                               double* red_v) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+template <bool COOP>
+__device__ double group_residual(const double* K, int64_t ld, int n, const double* y, const double* b, double* r,
+                                 double* red_v, Group<COOP>& grp) {
+  const int lane = threadIdx.x & 31;
   double rmax = 0.0, smax = 0.0;
-  for (int i = warp; i < n; i += kWarps) {
+  for (int i = grp.warp(); i < n; i += grp.warps()) {
     const double* Ki = K + int64_t(i) * ld;
     double s = 0.0, a = 0.0;
     for (int c = lane; c < n; c += 32) {
@@ -506,18 +742,20 @@ __device__ double cta_residual(const double* K, int64_t ld, int n, const double*
   }
   rmax = cta_max(rmax, red_v);
   smax = cta_max(smax, red_v);
+  int unused = 0;
+  grp.argmax(rmax, unused);  // (its barrier also completes r for the other CTAs)
+  grp.argmax(smax, unused);
   return smax > 0.0 ? rmax / smax : rmax;
 }
 
 // ---- one system -------------------------------------------------------------------------------------------------
 
-template <class Ops>
-__device__ void solve_system(const BatchSys& sys, char* slice, int64_t ld_max, SmemLU& sm, double* red_v, int* red_i,
-                             BatchOut* out) {
+template <class Ops, bool COOP>
+__device__ void solve_system(const BatchSys& sys, char* slice, SmemLU& sm, PanelRows& pr, double* red_v, int* red_i,
+                             BatchOut* out, Group<COOP>& grp) {
   using T = typename Ops::T;
   const int n = sys.n;
   const int64_t ld = (int64_t(n) + 3) & ~int64_t(3);
-  (void)ld_max;
   double* K = reinterpret_cast<double*>(slice);
   T* W = reinterpret_cast<T*>(K + int64_t(n) * ld);
   double* A = reinterpret_cast<double*>(W + int64_t(n) * ld);
@@ -526,45 +764,50 @@ __device__ void solve_system(const BatchSys& sys, char* slice, int64_t ld_max, S
   double* b = dc + n;
   double* rv = b + n;
   int32_t* piv = reinterpret_cast<int32_t*>(rv + n);
+  int32_t* perm = piv + n;
+  double* part = reinterpret_cast<double*>(W);  // column maxima by CTA, before W is written
   switch (sys.p.rbf) {
-    case UPDES_RBF_POLYHARMONIC: assemble_system<UPDES_RBF_POLYHARMONIC>(sys, K, A, ld, dr, dc, b, red_v); break;
-    case UPDES_RBF_GAUSSIAN: assemble_system<UPDES_RBF_GAUSSIAN>(sys, K, A, ld, dr, dc, b, red_v); break;
-    case UPDES_RBF_MULTIQUADRIC: assemble_system<UPDES_RBF_MULTIQUADRIC>(sys, K, A, ld, dr, dc, b, red_v); break;
+    case UPDES_RBF_POLYHARMONIC: assemble_system<UPDES_RBF_POLYHARMONIC>(sys, K, A, ld, dr, dc, b, part, grp); break;
+    case UPDES_RBF_GAUSSIAN: assemble_system<UPDES_RBF_GAUSSIAN>(sys, K, A, ld, dr, dc, b, part, grp); break;
+    case UPDES_RBF_MULTIQUADRIC: assemble_system<UPDES_RBF_MULTIQUADRIC>(sys, K, A, ld, dr, dc, b, part, grp); break;
     case UPDES_RBF_INVERSE_MULTIQUADRIC:
-      assemble_system<UPDES_RBF_INVERSE_MULTIQUADRIC>(sys, K, A, ld, dr, dc, b, red_v); break;
-    default: assemble_system<UPDES_RBF_THIN_PLATE>(sys, K, A, ld, dr, dc, b, red_v); break;
+      assemble_system<UPDES_RBF_INVERSE_MULTIQUADRIC>(sys, K, A, ld, dr, dc, b, part, grp); break;
+    default: assemble_system<UPDES_RBF_THIN_PLATE>(sys, K, A, ld, dr, dc, b, part, grp); break;
   }
-  scale_columns_to_w<Ops>(sys, K, W, ld, dc);
-  const int info = cta_lu<Ops>(W, ld, n, sys.nb, piv, sm, red_v, red_i);
-  // the solve's vectors: y and the correction, in shared memory
+  scale_columns_to_w<Ops>(sys, K, W, ld, dc, grp);
+  const int info = group_lu<Ops>(W, ld, n, COOP ? max(sys.nb, kCoopNB) : sys.nb, piv, sm, pr, reinterpret_cast<Key*>(red_v), red_i, grp);
+  // shared memory from here on: y and the correction, a staged diagonal block
   double* y = reinterpret_cast<double*>(&sm);
   double* d = y + kMaxBatchN;
-  for (int i = threadIdx.x; i < n; i += kBT) y[i] = b[i];
-  __syncthreads();
-  cta_lu_solve<Ops>(W, ld, n, piv, y);
+  T(*diag)[33] = reinterpret_cast<T(*)[33]>(d + kMaxBatchN);
+  if (grp.rank == 0) permutation(piv, n, perm, reinterpret_cast<int*>(&sm));
+  grp.sync();
+  for (int i = threadIdx.x; i < n; i += kBT) y[i] = b[perm[i]];
+  grp.sync();
+  group_lu_solve<Ops>(W, ld, n, y, diag, grp);
   int sweeps = 0;
-  double bwd = cta_residual(K, ld, n, y, b, rv, red_v);
+  double bwd = group_residual(K, ld, n, y, b, rv, red_v, grp);
   double last = INFINITY;
   while (bwd > kBwdStop && sweeps < sys.max_sweeps && bwd < 0.5 * last) {
-    for (int i = threadIdx.x; i < n; i += kBT) d[i] = rv[i];
-    __syncthreads();
-    cta_lu_solve<Ops>(W, ld, n, piv, d);
+    for (int i = threadIdx.x; i < n; i += kBT) d[i] = rv[perm[i]];
+    grp.sync();
+    group_lu_solve<Ops>(W, ld, n, d, diag, grp);
     for (int i = threadIdx.x; i < n; i += kBT) y[i] += d[i];
     __syncthreads();
     last = bwd;
-    bwd = cta_residual(K, ld, n, y, b, rv, red_v);
+    bwd = group_residual(K, ld, n, y, b, rv, red_v, grp);
     ++sweeps;
   }
   // coeffs = Dc y; vals = A[:N] coeffs
   for (int i = threadIdx.x; i < n; i += kBT) {
     const double c = dc[i] * y[i];
-    sys.coeffs[i] = c;
+    if (grp.rank == 0) sys.coeffs[i] = c;
     y[i] = c;
   }
   __syncthreads();
   if (sys.vals) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int i = warp; i < sys.p.N; i += kWarps) {
+    const int lane = threadIdx.x & 31;
+    for (int i = grp.warp(); i < sys.p.N; i += grp.warps()) {
       const double* Ai = A + int64_t(i) * ld;
       double s = 0.0;
       for (int c = lane; c < n; c += 32) s = fma(Ai[c], y[c], s);
@@ -572,47 +815,67 @@ __device__ void solve_system(const BatchSys& sys, char* slice, int64_t ld_max, S
       if (lane == 0) sys.vals[i] = s;
     }
   }
-  if (threadIdx.x == 0) {
+  if (grp.thread() == 0) {
     out->lu_info = info;
     out->sweeps = sweeps;
     out->backward_error = bwd;
     out->converged = (info == 0 && bwd <= kBwdFloorB) ? 1 : 0;
     out->done = 1;
   }
-  __syncthreads();
+  grp.sync();
 }
 
+// COOP: each cluster takes systems from the queue and solves them together, in the slice of its own; else each CTA.
+template <bool COOP>
 __global__ void __launch_bounds__(kBT) batched_solve_kernel(const BatchSys* __restrict__ systems,
                                                             const int32_t* __restrict__ order, int count,
                                                             int* __restrict__ queue, char* __restrict__ scratch,
-                                                            size_t slice_bytes, int64_t ld_max,
-                                                            BatchOut* __restrict__ outs) {
+                                                            size_t slice_bytes, BatchOut* __restrict__ outs) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SmemLU& sm = *reinterpret_cast<SmemLU*>(smem_raw);
   __shared__ double red_v[kWarps];
   __shared__ int red_i[kWarps];
   __shared__ int s_next;
-  char* slice = scratch + size_t(blockIdx.x) * slice_bytes;
+  __shared__ Exchange ex;
+  __shared__ PanelRows pr;
+  Group<COOP> grp;
+  int team = blockIdx.x;
+  if constexpr (COOP) {
+    uint32_t rank, ctas;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ctas));
+    grp.rank = int(rank);
+    grp.ctas = int(ctas);
+    grp.ex = &ex;
+    team = blockIdx.x / int(ctas);
+  }
+  char* slice = scratch + size_t(team) * slice_bytes;
   for (;;) {
-    if (threadIdx.x == 0) s_next = atomicAdd(queue, 1);
-    __syncthreads();
+    if (grp.rank == 0 && threadIdx.x == 0) {
+      const int k = atomicAdd(queue, 1);
+      s_next = k;
+      if constexpr (COOP)
+        for (int c = 1; c < grp.ctas; ++c)
+          asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(Group<COOP>::remote(&s_next, c)), "r"(k) : "memory");
+    }
+    grp.sync();
     const int k = s_next;
-    __syncthreads();
+    grp.sync();
     if (k >= count) break;
     const int i = order[k];
     const BatchSys sys = systems[i];
-    if (sys.precision == UPDES_PREC_FP64) solve_system<OpsF64>(sys, slice, ld_max, sm, red_v, red_i, outs + i);
-    else solve_system<OpsDF>(sys, slice, ld_max, sm, red_v, red_i, outs + i);
+    if (sys.precision == UPDES_PREC_FP64) solve_system<OpsF64>(sys, slice, sm, pr, red_v, red_i, outs + i, grp);
+    else solve_system<OpsDF>(sys, slice, sm, pr, red_v, red_i, outs + i, grp);
   }
 }
 
 size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
-// Bytes of one CTA's slice for systems of at most n_max unknowns: K, W and A (n x ld, 8 bytes each),
-// four n-vectors and the pivots.
+// Bytes of one CTA's (cluster's) slice for systems of at most n_max unknowns: K, W and A (n x ld, 8 bytes each),
+// four n-vectors, the pivots and the permutation.
 size_t slice_bytes_for(int n_max) {
   const size_t ld = (size_t(n_max) + 3) & ~size_t(3);
-  return align256(3 * size_t(n_max) * ld * 8 + 4 * size_t(n_max) * 8 + size_t(n_max) * 4);
+  return align256(3 * size_t(n_max) * ld * 8 + 4 * size_t(n_max) * 8 + 2 * size_t(n_max) * 4);
 }
 
 int batch_n_max(const updes_problem* problems, int32_t count, int* n_max) {
@@ -635,7 +898,78 @@ int sm_count() {
   return sms;
 }
 
-std::atomic<unsigned long long> g_batched_smem_done{0};
+std::atomic<unsigned long long> g_batched_smem_done[2];
+
+// Who solves what, from the sizes alone.  A system that would keep one SM busy for longer than the average SM's share of
+// the batch (costs as n^3) is solved by clusters: with one CTA a system the launch lasts as long as its largest one (256
+// clouds of up to 2,025 nodes: 376 ms; so split 118, at half the limit 135, at twice 154).  A cluster takes n = 2,031
+// from 353 to 49 ms, n = 790 from 30 to 8.6, n = 406 from 7.3 to 3.6, n = 202 only from 2.2 to 1.7, and below that
+// nothing; two rounds of clusters (17 systems) take 18.8 ms against 37.6 at n = 790, 7.2 against 8.4 at 406 and 3.6
+// against 3.5 at 202.  So systems of fewer than 384 unknowns always take one CTA each, as those within the share do, on
+// the SMs that no cluster holds and then on those that are done.  With a CTA count given by the caller every system
+// takes one CTA.
+constexpr int kCoopMinN = 384;
+
+struct Split {
+  int n_coop = 0, n_single = 0;      // largest size of either kind
+  int coop = 0, single = 0;          // systems
+  int teams = 0, ctas = 0;           // clusters; CTAs for the others
+  double limit = 0.0;                // n^3 above which a system is solved by a cluster
+  bool by_cluster(int n) const { return n >= kCoopMinN && double(n) * n * n > limit; }
+  size_t coop_slice() const { return coop ? slice_bytes_for(n_coop) : 0; }
+  size_t single_slice() const { return single ? slice_bytes_for(n_single) : 0; }
+  size_t slices() const { return coop_slice() * size_t(teams) + single_slice() * size_t(ctas); }
+};
+
+// Clusters of kMaxC CTAs that fit the device at once (0: none).
+int max_teams() {
+  static std::atomic<int> known[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  if (const int v = known[dev].load()) return v - 1;
+  const void* kern = (const void*)batched_solve_kernel<true>;
+  int n = 0;
+  if (smem_opt_in(kern, int(kSmemBytes), g_batched_smem_done[1]) == UPDES_OK) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim = {unsigned(kMaxC), 1, 1};
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kMaxC);
+    cfg.blockDim = dim3(kBT);
+    cfg.dynamicSmemBytes = kSmemBytes;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) n = 0;
+    (void)cudaGetLastError();
+  }
+  known[dev].store(n + 1);
+  return n;
+}
+
+Split split_batch(const updes_problem* problems, int32_t count, int32_t ctas) {
+  Split s;
+  const int sms = sm_count(), teams = ctas > 0 ? 0 : max_teams();
+  auto cost = [&](int32_t i) {
+    const double n = double(problems[i].N) + problems[i].M;
+    return n * n * n;
+  };
+  double total = 0.0;
+  for (int32_t i = 0; i < count; ++i) total += cost(i);
+  s.limit = teams > 0 ? total / std::max(sms, 1) : INFINITY;
+  for (int32_t i = 0; i < count; ++i) {
+    const int n = problems[i].N + problems[i].M;
+    if (s.by_cluster(n)) {
+      ++s.coop;
+      s.n_coop = std::max(s.n_coop, n);
+    } else {
+      ++s.single;
+      s.n_single = std::max(s.n_single, n);
+    }
+  }
+  s.teams = std::min(teams, s.coop);
+  s.ctas = std::min(ctas > 0 ? int(ctas) : sms, s.single);
+  return s;
+}
 
 }  // namespace
 
@@ -645,10 +979,9 @@ extern "C" int updes_solve_batched_workspace(const updes_problem* problems, int3
   int n_max = 0;
   const int e = batch_n_max(problems, count, &n_max);
   if (e) return e;
-  const int c = std::min<int>(ctas > 0 ? ctas : sm_count(), count);
-  if (c <= 0) return UPDES_ERR_CUDA;
-  *bytes = slice_bytes_for(n_max) * size_t(c) + align256(size_t(count) * (sizeof(BatchSys) + sizeof(BatchOut) + 4)) +
-           1024;
+  if (sm_count() <= 0) return UPDES_ERR_CUDA;
+  *bytes = split_batch(problems, count, ctas).slices() +
+           align256(size_t(count) * (sizeof(BatchSys) + sizeof(BatchOut) + 4)) + 1024;
   return UPDES_OK;
 }
 
@@ -660,10 +993,10 @@ extern "C" int updes_solve_batched(const updes_problem* problems, int32_t count,
   int n_max = 0;
   int e = batch_n_max(problems, count, &n_max);
   if (e) return e;
-  const int nctas = std::min<int>(ctas > 0 ? ctas : sm_count(), count);
-  if (nctas <= 0) return UPDES_ERR_CUDA;
+  if (sm_count() <= 0) return UPDES_ERR_CUDA;
+  const Split split = split_batch(problems, count, ctas);
   size_t need = 0;
-  if ((e = updes_solve_batched_workspace(problems, count, nctas, &need))) return e;
+  if ((e = updes_solve_batched_workspace(problems, count, ctas, &need))) return e;
   if (workspace_bytes < need) return UPDES_ERR_WORKSPACE;
   std::vector<BatchSys> sys(count);
   for (int32_t i = 0; i < count; ++i) {
@@ -680,18 +1013,18 @@ extern "C" int updes_solve_batched(const updes_problem* problems, int32_t count,
     sys[i].precision = pr;
     sys[i].max_sweeps = max_sweeps;
   }
-  // largest systems first (their solves are the longest)
+  // the clusters' systems, then the others, each largest first (their solves are the longest)
   std::vector<int32_t> order(count);
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) {
+    const bool ta = split.by_cluster(sys[a].n), tb = split.by_cluster(sys[b].n);
+    if (ta != tb) return ta;
     const double ca = double(sys[a].n) * sys[a].n * sys[a].n * (sys[a].precision == UPDES_PREC_FP64 ? 6.0 : 1.0);
     const double cb = double(sys[b].n) * sys[b].n * sys[b].n * (sys[b].precision == UPDES_PREC_FP64 ? 6.0 : 1.0);
     return ca > cb;
   });
   char* base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(workspace) + 255) & ~uintptr_t(255));
-  const size_t slice = slice_bytes_for(n_max);
-  char* scratch = base;
-  char* meta = base + slice * size_t(nctas);
+  char* meta = base + split.slices();
   BatchSys* d_sys = reinterpret_cast<BatchSys*>(meta);
   BatchOut* d_out = reinterpret_cast<BatchOut*>(meta + align256(size_t(count) * sizeof(BatchSys)));
   int32_t* d_order = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(d_out) + align256(size_t(count) * sizeof(BatchOut)));
@@ -700,16 +1033,37 @@ extern "C" int updes_solve_batched(const updes_problem* problems, int32_t count,
   UPDES_CUDA_TRY(cudaMemcpyAsync(d_sys, sys.data(), sizeof(BatchSys) * count, cudaMemcpyHostToDevice, s));
   UPDES_CUDA_TRY(cudaMemcpyAsync(d_order, order.data(), sizeof(int32_t) * count, cudaMemcpyHostToDevice, s));
   UPDES_CUDA_TRY(cudaMemsetAsync(d_out, 0, sizeof(BatchOut) * count, s));
-  UPDES_CUDA_TRY(cudaMemsetAsync(d_queue, 0, sizeof(int), s));
-  if ((e = smem_opt_in(reinterpret_cast<const void*>(&batched_solve_kernel), int(kSmemBytes), g_batched_smem_done)))
-    return e;
+  UPDES_CUDA_TRY(cudaMemsetAsync(d_queue, 0, 2 * sizeof(int), s));
+  if ((e = smem_opt_in((const void*)batched_solve_kernel<false>, int(kSmemBytes), g_batched_smem_done[0]))) return e;
   {
     double flops = 0.0;
     for (const auto& x : sys) flops += 2.0 / 3.0 * double(x.n) * x.n * x.n;
     StatScope sc(kStatOther, s, flops, 0.0);
-    batched_solve_kernel<<<nctas, kBT, kSmemBytes, s>>>(d_sys, d_order, count, d_queue, scratch, slice,
-                                                         int64_t((n_max + 3) & ~3), d_out);
-    UPDES_LAUNCH_CHECK();
+    SideStream side;
+    const bool both = split.teams > 0 && split.ctas > 0;
+    if (both && ((e = side.create(s)) || (e = side.start()))) return e;
+    if (split.teams > 0) {
+      cudaLaunchAttribute at{};
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim = {unsigned(kMaxC), 1, 1};
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(unsigned(split.teams * kMaxC));
+      cfg.blockDim = dim3(kBT);
+      cfg.dynamicSmemBytes = kSmemBytes;
+      cfg.stream = both ? side.side : s;  // of higher priority: the clusters start first
+      cfg.attrs = &at;
+      cfg.numAttrs = 1;
+      UPDES_CUDA_TRY(cudaLaunchKernelEx(&cfg, batched_solve_kernel<true>, (const BatchSys*)d_sys, (const int32_t*)d_order,
+                                        split.coop, d_queue, base, split.coop_slice(), d_out));
+      stats_count_launch(1);
+    }
+    if (split.ctas > 0) {
+      batched_solve_kernel<false><<<split.ctas, kBT, kSmemBytes, s>>>(
+          d_sys, d_order + split.coop, split.single, d_queue + 1, base + split.coop_slice() * size_t(split.teams),
+          split.single_slice(), d_out);
+      UPDES_LAUNCH_CHECK();
+    }
+    if (both && (e = side.finish())) return e;
   }
   std::vector<BatchOut> outs(count);
   UPDES_CUDA_TRY(cudaMemcpyAsync(outs.data(), d_out, sizeof(BatchOut) * count, cudaMemcpyDeviceToHost, s));

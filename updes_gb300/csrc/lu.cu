@@ -17,6 +17,7 @@
 
 #include "common.cuh"
 #include "lu.cuh"
+#include "side_stream.cuh"
 #include "stats.cuh"
 #include "gemm_tc.cuh"
 
@@ -845,44 +846,6 @@ size_t lu_df_workspace_bytes(int n) {
 }
 
 namespace {
-
-// The second stream of the look-ahead and the two events that fork it from and join it back to the caller's
-// stream.  The destructor joins as well, so that every return path leaves the caller's stream ordered after
-// all work of the factorisation.
-struct SideStream {
-  cudaStream_t main = nullptr, side = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr;
-  int create(cudaStream_t s) {
-    main = s;
-    int least = 0, greatest = 0;
-    UPDES_CUDA_TRY(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-    UPDES_CUDA_TRY(cudaStreamCreateWithPriority(&side, cudaStreamNonBlocking, greatest));
-    UPDES_CUDA_TRY(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
-    UPDES_CUDA_TRY(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
-    return UPDES_OK;
-  }
-  int start() {  // the side stream waits for all work issued on the caller's stream so far
-    UPDES_CUDA_TRY(cudaEventRecord(fork, main));
-    UPDES_CUDA_TRY(cudaStreamWaitEvent(side, fork, 0));
-    return UPDES_OK;
-  }
-  int finish() {  // the caller's stream waits for all work issued on the side stream so far
-    UPDES_CUDA_TRY(cudaEventRecord(join, side));
-    UPDES_CUDA_TRY(cudaStreamWaitEvent(main, join, 0));
-    return UPDES_OK;
-  }
-  ~SideStream() {
-    bool bad = false;
-    if (side && join) {
-      bad |= cudaEventRecord(join, side) != cudaSuccess;
-      bad |= cudaStreamWaitEvent(main, join, 0) != cudaSuccess;
-    }
-    if (fork) bad |= cudaEventDestroy(fork) != cudaSuccess;
-    if (join) bad |= cudaEventDestroy(join) != cudaSuccess;
-    if (side) bad |= cudaStreamDestroy(side) != cudaSuccess;
-    if (bad) (void)cudaGetLastError();
-  }
-};
 
 void add_swap_job(SwapJobs& j, int64_t& maxc, float* plane, int64_t c0, int64_t c1) {
   if (c1 <= c0) return;
