@@ -8,8 +8,8 @@
 int ozaki_update(float* Chi, float* Clo, int64_t ldc, const float* A, int64_t lda, const float* B, int64_t ldb,
                  int m, int nc, int K, DeviceStatus* st, cudaStream_t s);
 
-// The persistent, warp-specialised version (gemm_tc3.cu): digits written once per update into `scratch`
-// (ozaki3_scratch_bytes(m, nc, K) bytes, 256-byte aligned), 8 digit products, TMA-fed.  The kernel keeps one
+// The persistent, warp-specialised version (gemm_tc3.cu), K <= 256: digits written once per update into `scratch`
+// (ozaki3_scratch_bytes(m, nc, K) bytes, 256-byte aligned), 8 products of FP16 digits, fed by bulk copies.  The kernel keeps one
 // CTA per SM; `max_ctas` > 0 caps its grid so that work on another stream keeps the remaining SMs.
 size_t ozaki3_scratch_bytes(int mmax, int ncmax, int Kmax);
 // a_digits_ready: the previous update on `scratch` had the same A (same m, K and values), whose digits and

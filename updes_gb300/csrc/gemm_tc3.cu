@@ -1,35 +1,46 @@
 // Tensor-core trailing update of the mixed-precision LU, persistent and warp-specialised (sm_103a).
 //
 //   C  <-  C - A * B        C: FP32 hi/lo pairs ("double-float", ~48 bits)
-//                           A: m x K FP32 (L factor block), B: K x nc FP32 (U factor block)
+//                           A: m x K FP32 (L factor block), B: K x nc FP32 (U factor block), K <= 256
 //
-// Numerics.  Every FP32 operand is written as 3 bf16 integer digits under a power-of-two scale shared by a
-// row of A (a column of B) over each 64-wide k block:
-//   a = 2^(e-8) * (d0 + 2^-9 d1 + 2^-18 d2),   |d_i| <= 256 (exact in bf16),
-// exact for entries within a factor 4 of the block's row maximum and cut at 2^-26 of it otherwise.  Digit
-// products are <= 2^16 and a 64-term sum is <= 2^22; the products of equal weight 2^-9g (g = a + b) are
-// summed in one FP32 tensor-memory accumulator, at most 3 of them, so every accumulator holds an exact
-// integer below 2^24 and the tensor cores add no rounding.  The product d2 * e2 (weight 2^-36) lies ten
-// bits below the digit cut and is left out: 8 products, 4 accumulators.  The epilogue folds the four
-// exact group sums of each k block into per-thread double-float accumulators with error-free
-// transformations (FP32 ALU: GB300's FP64 rate is low), and subtracts the result from C once per tile.
+// Numerics.  Every FP32 operand is written as 3 FP16 numbers under a power-of-two scale shared by a row of A (a
+// column of B) over the whole K:
+//   a = 2^(e-8) * (d0 + d1 + d2),  d0 an integer, |d0| <= 256;  d1 a multiple of 2^-12, |d1| <= 2^-1;  |d2| <= 2^-13,
+// exact but for d2's rounding to 11 bits, at most 2^-33 of the row's maximum.  The products go to three FP32
+// tensor-memory accumulators by their size: g0 = d0 e0, g1 = d0 e1 + d1 e0, g2 = d0 e2 + d1 e1 + d2 e0 + d1 e2 + d2 e1.
+// The 256 products d0 e0 add up to an integer of at most 2^24: the tensor cores add no rounding to g0.  g1 is a multiple
+// of 2^-12, exact up to 2^12; at its largest, 2^16 (every entry of both operands near its maximum, with the same
+// remainder), a step drops at most 2^-8, 2^-32 of that sum's g0.  g2 is rounded below 2^-16 of its 2^8.  d2 e2 (2^-26,
+// 2^-42 of the largest product) is left out: 8 products.  The epilogue forms g0 + g1 + g2 as a double-float with
+// error-free transformations (FP32 ALU: GB300's FP64 rate is low) and subtracts it from C, once per tile.
+// Measured against 64 bits, relative to |A||B|, K = 256, and beside it three 9-bit integer digits under a scale per 64 of
+// K: normal entries 2^-37.8 (2^-29.1), columns graded by 2^-16 2^-32.8 (2^-27.6), cosines falling as 1/k 2^-33.1
+// (2^-27.6), entries spread over 2^20 2^-29.6 (2^-23.9), within a factor of 4 2^-40.4 (2^-40.2), constant rows and columns
+// 2^-29.1 (2^-36.4).  As a preconditioner the factors are the better for it: 7-8 iterations at n = 22,506 for 9-11.  The small
+// entries of a graded block matter to the Schur complement: with d1 cut at 2^-8 (g1 always exact) it took 14-25.
 //
-// Structure.  A pre-pass writes the digits once per update (A as [3][m][Kp] bf16, B transposed as
-// [3][nc][Kp] bf16, Kp = K rounded up to 64, zero padded) and the scales.  The main kernel is persistent
-// (one CTA per SM, tiles of 128 x 64 taken round robin) with three roles:
-//   warp 0      TMA producer: the 3 + 3 digit tiles of a k block into a 2-stage ring (128B swizzle, 72 KB
-//               a stage, the most that fits beside the C tile);
-//   warp 1      MMA issuer: 8 products x 4 k-steps of tcgen05.mma (kind::f16, M=128, N=64) into one of
-//               two accumulator sets (4 groups x 64 columns each, 512 TMEM columns in all);
-//   warps 2-17  epilogue: tcgen05.ld of the 4 groups, fold, and at the end of a tile C -= acc on the C tile
-//               in shared memory; one of its threads stores the tile by TMA and, once the store has read
-//               the buffer, loads the next tile's C into it.
-// The fold of one k block runs while the tensor cores work on the next, the C read-modify-write of a tile
-// overlaps the MMAs of the following tile, and the operand stream never waits for the C buffer.  Every mbarrier wait is bounded; a timeout sets the status
-// word and an abort flag that every role checks, and tensor memory is freed on every path.
+// What bounds it.  Shared memory: each tcgen05.mma reads both its operands from there, TMA writes them, and C passes
+// it four times, all at 128 bytes a clock.  The previous form (tiles of 128 x 64, 8 products, a fold of four
+// accumulators per 64 of K) moved 2.6 MB for a 128 x 128 x 256 piece, 21,000 clocks, and took 25,600.  So the tiles are
+// 128 x 128, the digit planes of B lie side by side so that one instruction of N = 256 forms d0 [e0 e1] in the
+// neighbouring accumulators [g0 g1] and another d1 [e0 e1] in [g1 g2] (A is read once for two products), and one scale
+// per K leaves one fold per tile: 1.8 MB, 14,400 clocks; 20,000 x 20,000 x 256 takes 1,300 us (15,400 clocks a piece)
+// against 2,165.  C without an eviction hint: evict-first costs 10 %.
+//
+// Structure.  A pre-pass writes the digits once per update, laid out as the stages hold them, and the scales.  The main
+// kernel is persistent (one CTA per SM, tiles of 128 x TN taken round robin) with three roles:
+//   warp 0      producer: two bulk copies per 32 of K into a ring of stages (64B swizzle, 48 KB a stage);
+//   warp 1      MMA issuer: 6 instructions of tcgen05.mma (kind::f16, M=128) per 16 of K into the three accumulators
+//               of TN columns each;
+//   warps 2-9   epilogue, a 32-row x TN/2-column piece of the tile each: tcgen05.ld, fold, then C -= acc on 32 columns
+//               at a time in the warp's own buffer, which its first lane loads and stores by TMA.
+// There is one accumulator set (384 of the 512 TMEM columns).  The last stage of a tile issues g0's and g1's products first
+// and commits them, so that the epilogue reads them while g2's run; the next tile's first instructions only wait
+// for those.  The fold and the C traffic run beside the next tile's MMAs.  Every mbarrier wait is bounded; a
+// timeout sets the status word and an abort flag that every role checks, and tensor memory is freed on every path.
 #include <atomic>
 
-#include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include "gemm_tc.cuh"
 #include "stats.cuh"
@@ -37,32 +48,40 @@
 
 namespace {
 
-constexpr int TM = 128, TN = 64, TK = 64;
-constexpr int kDigits = 3, kGroups = 4;  // 8 digit products
-constexpr int kStages = 2;  // equal to the number of accumulator sets (one barrier serves both)
-// epilogue: kEpiWarps warps, four per lane quarter of the tile (the warps a TMEM lane quarter allows), each
-// with kEpiCols columns
-constexpr int kEpiWarps = 16, kEpiCols = TN / (kEpiWarps / 4);
+constexpr int TM = 128, TK = 32;
+constexpr int kMaxK = 256;   // one exact accumulation
+constexpr int kKpUnit = 64;  // K is padded to this
+constexpr int kDigits = 3, kGroups = 3;
+constexpr int kEpiWarps = 8;
 constexpr int kWarps = 2 + kEpiWarps, kThreads = kWarps * 32;
-constexpr uint32_t kTmemCols = 512;  // 2 sets x 4 groups x 64 columns
-constexpr int kATile = TM * TK * 2;  // 16 KB per digit plane
-constexpr int kBTile = TN * TK * 2;  //  8 KB per digit plane
-constexpr int kStageBytes = kDigits * (kATile + kBTile);  // 72 KB
-constexpr int kCHalf = TM * 32 * 4;                         // 16 KB: 128 rows x 32 FP32 (one 128-B swizzled box)
-constexpr int kCBytes = 4 * kCHalf;                         // C tile: {hi, lo} x {columns 0-31, 32-63}
-constexpr int kSmemBytes = kStages * kStageBytes + kCBytes + 1024;
-static_assert(kSmemBytes <= 227 * 1024, "shared memory");
+constexpr uint32_t kTmemCols = 512;
+constexpr int kATile = TM * TK * 2;           // 8 KB per digit plane
+constexpr int kCBox = 32 * 32 * 4;            // 32 rows x 32 FP32 (128-byte rows): 4 KB
+constexpr int kCBytes = kEpiWarps * 2 * kCBox;  // {hi, lo} per epilogue warp
 
-// instruction descriptor: D = F32, A = B = BF16, both K-major, N = 64, M = 128
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(TN >> 3) << 17) | (uint32_t(TM >> 4) << 24);
+template <int TN>
+struct Cfg {
+  static constexpr int kStages = TN == 128 ? 3 : 4;
+  static constexpr int kBTile = TN * TK * 2;
+  static constexpr int kStageBytes = kDigits * (kATile + kBTile);  // 48 KB (TN = 64: 36 KB)
+  static constexpr int kSmemBytes = kStages * kStageBytes + kCBytes + 1024;
+  static constexpr int kCols = TN / 2;  // columns of an epilogue warp
+  static_assert(kSmemBytes <= 227 * 1024, "shared memory");
+  static_assert(kGroups * TN <= int(kTmemCols), "tensor memory");
+};
 
-// tcgen05 shared-memory matrix descriptor: K-major, 128B swizzle, 8-row groups 1024 B apart.
+// instruction descriptor: D = F32, A = B = F16, both K-major, M = 128
+__host__ __device__ constexpr uint32_t idesc(int n) {
+  return (1u << 4) | (uint32_t(n >> 3) << 17) | (uint32_t(TM >> 4) << 24);
+}
+
+// tcgen05 shared-memory matrix descriptor: K-major, 64B swizzle, 8-row groups 512 B apart.
 __device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
   uint64_t d = uint64_t((saddr & 0x3FFFFu) >> 4);
   d |= uint64_t(1) << 16;
-  d |= uint64_t(1024 >> 4) << 32;
+  d |= uint64_t(512 >> 4) << 32;
   d |= uint64_t(1) << 46;
-  d |= uint64_t(2) << 61;
+  d |= uint64_t(4) << 61;
   return d;
 }
 
@@ -89,152 +108,169 @@ __device__ __forceinline__ void fast_two_sum2(float2 a, float2 b, float2& s, flo
   e = sub2(b, sub2(s, a));
 }
 
-// The 32 MMAs of one k block: digit products (a, b) with a + b <= 3 (d2 * e2 is below the digit cut), four
-// k-steps of 16 each, into accumulator group a + b.  Descriptors are built once; every operand offset is a
-// compile-time constant added to them (descriptor address units are 16 bytes: a digit plane of A is 1024
-// units, of B 512, a k-step 2), so the issuing thread keeps pace with the tensor pipe.
-template <int A, int B>
-__device__ __forceinline__ void mma_product(uint32_t tset, uint64_t a0, uint64_t b0) {
-  constexpr int g = A + B;
-  constexpr bool first = (A == (g > 2 ? g - 2 : 0));  // the group's first product overwrites it
-  const uint32_t d = tset + uint32_t(g * TN);
+// The digits of one FP32 value under `scale` (|v * scale| <= 256): every step is exact but the last conversion.
+__device__ __forceinline__ void split3(float v, float scale, float (&d)[kDigits]) {
+  const float x = __fmul_rn(v, scale);
+  d[0] = rintf(x);
+  const float y = __fmul_rn(__fsub_rn(x, d[0]), 4096.f);
+  const float i1 = rintf(y);  // |i1| <= 2048: 11 bits and a sign, exact in FP16
+  d[1] = __fmul_rn(i1, 0x1p-12f);
+  d[2] = __fmul_rn(__fsub_rn(y, i1), 0x1p-12f);
+}
+
+// Digits lie as the stages of the main kernel hold them: for each tile of `rows` rows (columns of B) and each 32 of K
+// one contiguous piece [plane][row][32], with 64-byte rows in the 64B swizzle (16-byte chunk c of row r at c ^ ((r >> 1) & 3)).
+// Element offset of (row r of tile t, k) in plane p.
+__device__ __forceinline__ int64_t digit_at(int64_t t, int r, int p, int k, int nks, int rows) {
+  return ((t * nks + k / TK) * kDigits + p) * int64_t(rows * TK) + r * TK + ((((k % TK) >> 3) ^ ((r >> 1) & 3)) << 3) + (k & 7);
+}
+
+// `NK` k-steps of 16 from one stage for operands A and B (descriptors of their first rows): D (+)= A B.  Descriptors
+// are built once per stage; every operand offset is a compile-time constant added to them (address units of 16 bytes).
+template <int NK, bool FIRST>
+__device__ __forceinline__ void mma_steps(uint32_t d, uint64_t a0, uint64_t b0, uint32_t id) {
 #pragma unroll
-  for (int kk = 0; kk < TK / 16; ++kk) {
-    const uint64_t ad = a0 + uint64_t(A * (kATile >> 4) + kk * 2), bd = b0 + uint64_t(B * (kBTile >> 4) + kk * 2);
-    if (first && kk == 0) mma_bf16<false>(d, ad, bd, kIdesc);
-    else mma_bf16<true>(d, ad, bd, kIdesc);
+  for (int kk = 0; kk < NK; ++kk) {
+    if (FIRST && kk == 0) mma_bf16<false>(d, a0, b0, id);  // kind::f16: the descriptor says FP16
+    else mma_bf16<true>(d, a0 + uint64_t(kk * 2), b0 + uint64_t(kk * 2), id);
   }
 }
 
 // ---- digit pre-pass ------------------------------------------------------------------------------------
-// A (m x K, lda) -> Ad[p][r][k] (bf16, p < 3, k < Kp) and As[r][kb] = 2^(e-8), one warp per (row, k block);
-// bx is the block's index among the row part's blocks.
+// A (m x K, lda) -> Ad (see digit_at) and As[r] = 2^(e-8), one warp per row; bx is the block's index among the row
+// part's blocks.
 __device__ __forceinline__ void digits_rows(int bx, const float* __restrict__ A, int64_t lda, int m, int K, int Kp,
-                                            __nv_bfloat16* __restrict__ Ad, float* __restrict__ As) {
-  const int64_t w = (int64_t(bx) * blockDim.x + threadIdx.x) >> 5;
+                                            __half* __restrict__ Ad, float* __restrict__ As) {
+  const int64_t r = (int64_t(bx) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
-  const int nkb = Kp / TK;
-  if (w >= int64_t(m) * nkb) return;
-  const int r = int(w / nkb), kb = int(w % nkb);
-  float v[2];
+  if (r >= m) return;
+  float v[kMaxK / 64][2];
+  float mx = 0.f;
 #pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    const int k = kb * TK + lane + 32 * u;
-    v[u] = k < K ? A[int64_t(r) * lda + k] : 0.f;
-  }
-  float mx = fmaxf(fabsf(v[0]), fabsf(v[1]));
+  for (int u = 0; u < kMaxK / 64; ++u)
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      const int k = u * 64 + 2 * lane + w;
+      v[u][w] = k < K ? A[r * lda + k] : 0.f;
+      mx = fmaxf(mx, fabsf(v[u][w]));
+    }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   const int e = exp_of(mx);
-  if (lane == 0) As[int64_t(r) * nkb + kb] = pow2f(e - 8);
+  if (lane == 0) As[r] = pow2f(e - 8);
   const float scale = pow2f(8 - e);
 #pragma unroll
-  for (int u = 0; u < 2; ++u) {
-    float x = __fmul_rn(v[u], scale);  // exact, |x| <= 256
-    const int64_t base = int64_t(r) * Kp + kb * TK + lane + 32 * u;
+  for (int u = 0; u < kMaxK / 64; ++u) {
+    if (u * 64 >= Kp) break;
+    float da[kDigits], db[kDigits];
+    split3(v[u][0], scale, da);
+    split3(v[u][1], scale, db);
 #pragma unroll
-    for (int p = 0; p < kDigits; ++p) {
-      const float d = rintf(x);
-      Ad[int64_t(p) * m * Kp + base] = __float2bfloat16_rn(d);
-      x = __fmul_rn(__fsub_rn(x, d), 512.f);  // exact
-    }
+    for (int p = 0; p < kDigits; ++p)
+      *reinterpret_cast<__half2*>(Ad + digit_at(r / TM, int(r % TM), p, u * 64 + 2 * lane, Kp / TK, TM)) =
+          __floats2half2_rn(da[p], db[p]);
   }
 }
 
-// B (K x nc, ldb) -> Bd[p][c][k] (bf16, transposed) and Bs[kb][c] (row stride ncp = nc rounded up to TN, the
-// padding columns 0); a CTA per (64 k, 64 columns) tile: column tile bx, k block kb.
-__device__ __forceinline__ void digits_cols(int bx, int kb, const float* __restrict__ B, int64_t ldb, int nc, int K,
-                                            int Kp, __nv_bfloat16* __restrict__ Bd, float* __restrict__ Bs) {
-  __shared__ float t[TK][TN + 1];
-  const int c0 = bx * TN;
-  for (int e = threadIdx.x; e < TK * TN; e += blockDim.x) {
-    const int k = e / TN, c = e % TN;
-    const int gk = kb * TK + k, gc = c0 + c;
-    t[k][c] = (gk < K && gc < nc) ? B[int64_t(gk) * ldb + gc] : 0.f;
-  }
-  __syncthreads();
+// B (K x nc, ldb) -> Bd (transposed, in tiles of TN columns) and Bs[c]; a CTA per 32 columns.
+__device__ __forceinline__ void digits_cols(int bx, const float* __restrict__ B, int64_t ldb, int nc, int K, int Kp, int TN,
+                                            __half* __restrict__ Bd, float* __restrict__ Bs) {
+  __shared__ float t[kMaxK][33];
+  const int c0 = bx * 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t ncp = ceil_div(nc, TN) * TN;
-  for (int c = warp; c < TN; c += blockDim.x / 32) {
-    const int gc = c0 + c;
-    if (gc >= nc) {
-      if (lane == 0) Bs[kb * ncp + gc] = 0.f;
-      continue;
-    }
-    float v[2] = {t[lane][c], t[lane + 32][c]};
-    float mx = fmaxf(fabsf(v[0]), fabsf(v[1]));
+#pragma unroll 16  // loads in flight together: the pass is short and mostly their latency
+  for (int k = warp; k < Kp; k += 8)
+    t[k][lane] = (k < K && c0 + lane < nc) ? B[int64_t(k) * ldb + c0 + lane] : 0.f;
+  __syncthreads();
+  for (int c = warp; c < 32; c += blockDim.x / 32) {
+    const int64_t gc = c0 + c;
+    if (gc >= nc) continue;
+    float mx = 0.f;
+    for (int k = lane; k < Kp; k += 32) mx = fmaxf(mx, fabsf(t[k][c]));
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     const int e = exp_of(mx);
-    if (lane == 0) Bs[kb * ncp + gc] = pow2f(e - 8);
+    if (lane == 0) Bs[gc] = pow2f(e - 8);
     const float scale = pow2f(8 - e);
+    for (int k = 2 * lane; k < Kp; k += 64) {
+      float da[kDigits], db[kDigits];
+      split3(t[k][c], scale, da);
+      split3(t[k + 1][c], scale, db);
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      float x = __fmul_rn(v[u], scale);
-      const int64_t base = int64_t(gc) * Kp + kb * TK + lane + 32 * u;
-#pragma unroll
-      for (int p = 0; p < kDigits; ++p) {
-        const float d = rintf(x);
-        Bd[int64_t(p) * nc * Kp + base] = __float2bfloat16_rn(d);
-        x = __fmul_rn(__fsub_rn(x, d), 512.f);
-      }
+      for (int p = 0; p < kDigits; ++p)
+        *reinterpret_cast<__half2*>(Bd + digit_at(gc / TN, int(gc % TN), p, k, Kp / TK, TN)) =
+            __floats2half2_rn(da[p], db[p]);
     }
   }
 }
 
-// Both digit passes of one update in a single launch: blocks [0, row_blocks) take the rows of A, the next
-// col_tiles x nkb blocks the (column tile, k block) tiles of B.
+// Both digit passes of one update in a single launch: blocks [0, row_blocks) take the rows of A, the others the
+// column tiles of B.
 __global__ void __launch_bounds__(256) digits_kernel(const float* __restrict__ A, int64_t lda, int m,
                                                      const float* __restrict__ B, int64_t ldb, int nc, int K, int Kp,
-                                                     int row_blocks, int col_tiles, __nv_bfloat16* __restrict__ Ad,
-                                                     float* __restrict__ As, __nv_bfloat16* __restrict__ Bd,
-                                                     float* __restrict__ Bs) {
+                                                     int TN, int row_blocks, __half* __restrict__ Ad, float* __restrict__ As,
+                                                     __half* __restrict__ Bd, float* __restrict__ Bs) {
   const int b = int(blockIdx.x);
-  if (b < row_blocks) {
-    digits_rows(b, A, lda, m, K, Kp, Ad, As);
-  } else {
-    const int q = b - row_blocks;
-    digits_cols(q % col_tiles, q / col_tiles, B, ldb, nc, K, Kp, Bd, Bs);
-  }
+  if (b < row_blocks) digits_rows(b, A, lda, m, K, Kp, Ad, As);
+  else digits_cols(b - row_blocks, B, ldb, nc, K, Kp, TN, Bd, Bs);
 }
 
 // ---- main kernel ---------------------------------------------------------------------------------------
 struct Ctrl {
-  // With two stages and two accumulator sets, k block j uses stage j % 2 and set j % 2: the one commit of its
-  // MMAs (tfull[j % 2]) both hands the set to the epilogue and frees the stage for the producer.
-  uint64_t full[kStages], tfull[2], tempty[2], cfull, cready;
+  uint64_t full[4], empty[4];  // operand stages: filled by TMA / their MMAs are done
+  uint64_t hi_done, lo_done;   // the tile's g0 and g1 / g2 are complete
+  uint64_t hi_free, lo_free;   // every epilogue warp has read them
+  uint64_t cfull[kEpiWarps];   // a warp's piece of C has arrived
   uint32_t tmem;
   int abort_flag;
 };
 
-// 18 warps: a sub-partition holds up to 5 of them in its 16,384 registers, so at most 96 registers a thread
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
+  uint32_t r[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// A contiguous copy into shared memory that completes on an mbarrier (16-byte aligned, a multiple of 16 bytes).
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint64_t* bar, uint64_t policy) {
+  asm volatile(
+      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(dst),
+      "l"(src), "r"(bytes), "r"(smem_u32(bar)), "l"(policy)
+      : "memory");
+}
+
+template <int TN>
 __global__ void __launch_bounds__(kThreads, 1)
-    ozaki3_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                  const __grid_constant__ CUtensorMap tmCh, const __grid_constant__ CUtensorMap tmCl,
-                  const float* __restrict__ As, const float* __restrict__ Bs, int m, int nc, int Kp,
+    ozaki3_kernel(const __grid_constant__ CUtensorMap tmCh, const __grid_constant__ CUtensorMap tmCl,
+                  const __half* __restrict__ Ad, const __half* __restrict__ Bd, const float* __restrict__ As, const float* __restrict__ Bs, int m, int nc, int Kp,
                   DeviceStatus* st) {
+  using C = Cfg<TN>;
+  constexpr int kStages = C::kStages, kBTile = C::kBTile, kStageBytes = C::kStageBytes, kCols = C::kCols;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sC = smem + kStages * kStageBytes;  // C tile, 128B-swizzled boxes: hi[0:32], hi[32:64], lo[0:32], lo[32:64]
   __shared__ Ctrl ctl;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int tiles_n = int(ceil_div(nc, TN)), tiles_m = int(ceil_div(m, TM));
   const int ntiles = tiles_n * tiles_m;
-  const int64_t ncp = int64_t(tiles_n) * TN;  // row stride of the column scales
-  const int nkb = Kp / TK;
+  const int nks = Kp / TK;  // at least 2
   volatile int* abort_flag = &ctl.abort_flag;
-  const uint64_t pol_keep = l2_policy_evict_last(), pol_stream = l2_policy_evict_first();
 
   if (tid == 0) {
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&ctl.full[s], 1);
+      mbar_init(&ctl.empty[s], 1);
     }
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(&ctl.tfull[s], 1);
-      mbar_init(&ctl.tempty[s], kEpiWarps);
-    }
-    mbar_init(&ctl.cfull, 1);
-    mbar_init(&ctl.cready, kEpiWarps);
+    mbar_init(&ctl.hi_done, 1);
+    mbar_init(&ctl.lo_done, 1);
+    mbar_init(&ctl.hi_free, kEpiWarps);
+    mbar_init(&ctl.lo_free, kEpiWarps);
+    for (int w = 0; w < kEpiWarps; ++w) mbar_init(&ctl.cfull[w], 1);
     ctl.abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -248,34 +284,30 @@ __global__ void __launch_bounds__(kThreads, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = ctl.tmem;
-  int last_commit = -1;  // MMA issuer: index of the last committed k block
+  int last_commit = -1;  // MMA issuer: index of the last committed stage
+  auto give_up = [&](int tag) {
+    if (!*abort_flag) { status_error(st, UPDES_ERR_TIMEOUT); atomicCAS(&st->timeout_tag, 0, tag); }
+    *abort_flag = 1;
+  };
 
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (lane == 0) {
-      asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmA)) : "memory");
-      asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmB)) : "memory");
-      asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmCh)) : "memory");
-      asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(&tmCl)) : "memory");
+      const uint64_t pol_keep = l2_policy_evict_last();
       int j = 0;
       for (int t = blockIdx.x; t < ntiles && !*abort_flag; t += gridDim.x) {
-        const int r0 = (t / tiles_n) * TM, c0 = (t % tiles_n) * TN;
-        for (int kb = 0; kb < nkb; ++kb, ++j) {
+        const uint8_t* gA = reinterpret_cast<const uint8_t*>(Ad) + int64_t(t / tiles_n) * nks * (kDigits * kATile);
+        const uint8_t* gB = reinterpret_cast<const uint8_t*>(Bd) + int64_t(t % tiles_n) * nks * (kDigits * kBTile);
+        for (int ks = 0; ks < nks; ++ks, ++j) {
           const int s = j % kStages;
-          const uint32_t ph = uint32_t(j / kStages) & 1u;
-          if (!mbar_wait(&ctl.tfull[s], ph ^ 1u, abort_flag)) {  // k block j - 2's MMAs are done
-            if (!*abort_flag) { status_error(st, UPDES_ERR_TIMEOUT); atomicCAS(&st->timeout_tag, 0, 41); }
-            *abort_flag = 1;
+          if (!mbar_wait(&ctl.empty[s], (uint32_t(j / kStages) & 1u) ^ 1u, abort_flag)) {
+            give_up(41);
             break;
           }
           uint8_t* sA = smem + s * kStageBytes;
-          uint8_t* sB = sA + kDigits * kATile;
           mbar_expect_tx(&ctl.full[s], uint32_t(kStageBytes));
-#pragma unroll
-          for (int p = 0; p < kDigits; ++p) {
-            tma_load_3d(smem_u32(sA + p * kATile), &tmA, kb * TK, r0, p, &ctl.full[s], pol_keep);
-            tma_load_3d(smem_u32(sB + p * kBTile), &tmB, kb * TK, c0, p, &ctl.full[s], pol_keep);
-          }
+          bulk_load(smem_u32(sA), gA + ks * (kDigits * kATile), kDigits * kATile, &ctl.full[s], pol_keep);
+          bulk_load(smem_u32(sA + kDigits * kATile), gB + ks * (kDigits * kBTile), kDigits * kBTile, &ctl.full[s], pol_keep);
         }
       }
       if (*abort_flag) {
@@ -291,180 +323,192 @@ __global__ void __launch_bounds__(kThreads, 1)
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     if (lane == 0) {
-      int j = 0;
-      for (int t = blockIdx.x; t < ntiles && !*abort_flag; t += gridDim.x) {
-        for (int kb = 0; kb < nkb; ++kb, ++j) {
-          const int s = j % kStages, set = j & 1;
-          const uint32_t ph = uint32_t(j / kStages) & 1u, tph = uint32_t(j >> 1) & 1u;
-          if (!mbar_wait(&ctl.full[s], ph, abort_flag) || !mbar_wait(&ctl.tempty[set], tph ^ 1u, abort_flag)) {
-            if (!*abort_flag) { status_error(st, UPDES_ERR_TIMEOUT); atomicCAS(&st->timeout_tag, 0, 42); }
-            *abort_flag = 1;
+      constexpr int NK = TK / 16;
+      constexpr uint32_t id1 = idesc(TN), id2 = idesc(2 * TN);
+      const uint32_t g01 = tmem, g12 = tmem + uint32_t(TN), g2 = tmem + uint32_t(2 * TN);
+      int j = 0, tl = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < ntiles && ok && !*abort_flag; t += gridDim.x, ++tl) {
+        for (int ks = 0; ks < nks; ++ks, ++j) {
+          const int s = j % kStages;
+          ok = mbar_wait(&ctl.full[s], uint32_t(j / kStages) & 1u, abort_flag) &&
+               (ks != 0 || mbar_wait(&ctl.hi_free, (uint32_t(tl) & 1u) ^ 1u, abort_flag));
+          if (!ok) {
+            give_up(42);
             break;
           }
           tc_fence_after();
           const uint8_t* sA = smem + s * kStageBytes;
-          const uint64_t a0 = make_desc(smem_u32(sA)), b0 = make_desc(smem_u32(sA + kDigits * kATile));
-          const uint32_t tset = tmem + uint32_t(set * kGroups * TN);
-          mma_product<0, 0>(tset, a0, b0);
-          mma_product<0, 1>(tset, a0, b0);
-          mma_product<1, 0>(tset, a0, b0);
-          mma_product<0, 2>(tset, a0, b0);
-          mma_product<1, 1>(tset, a0, b0);
-          mma_product<2, 0>(tset, a0, b0);
-          mma_product<1, 2>(tset, a0, b0);
-          mma_product<2, 1>(tset, a0, b0);
-          mma_commit(&ctl.tfull[set]);
+          const uint64_t a0 = make_desc(smem_u32(sA)), a1 = a0 + uint64_t(kATile >> 4), a2 = a0 + uint64_t(2 * (kATile >> 4));
+          const uint64_t b0 = make_desc(smem_u32(sA + kDigits * kATile)), b1 = b0 + uint64_t(kBTile >> 4),
+                         b2 = b0 + uint64_t(2 * (kBTile >> 4));
+          if (ks == 0) {
+            mma_steps<NK, true>(g01, a0, b0, id2);  // d0 [e0 e1] -> [g0 g1]
+            ok = mbar_wait(&ctl.lo_free, (uint32_t(tl) & 1u) ^ 1u, abort_flag);
+            if (ok) {
+              tc_fence_after();
+              mma_steps<NK, true>(g2, a0, b2, id1);    // d0 e2 -> g2
+              mma_steps<NK, false>(g12, a1, b0, id2);  // d1 [e0 e1] -> [g1 g2]
+              mma_steps<NK, false>(g2, a1, b2, id1);   // d1 e2 -> g2
+              mma_steps<NK, false>(g2, a2, b0, id1);   // d2 e0 -> g2
+              mma_steps<NK, false>(g2, a2, b1, id1);   // d2 e1 -> g2
+            }
+          } else {
+            mma_steps<NK, false>(g01, a0, b0, id2);
+            mma_steps<NK, false>(g12, a1, b0, id2);
+            if (ks == nks - 1) mma_commit(&ctl.hi_done);
+            mma_steps<NK, false>(g2, a0, b2, id1);
+            mma_steps<NK, false>(g2, a1, b2, id1);
+            mma_steps<NK, false>(g2, a2, b0, id1);
+            mma_steps<NK, false>(g2, a2, b1, id1);
+            if (ks == nks - 1) mma_commit(&ctl.lo_done);
+          }
+          mma_commit(&ctl.empty[s]);
           last_commit = j;
+          if (!ok) {
+            give_up(44);
+            break;
+          }
         }
       }
     }
   } else {
     // ---------------- epilogue: lane quarter q = warp % 4, column group h ----------------
-    const int q = warp & 3, h = (warp - 2) >> 2;
-    const int row_in_tile = q * 32 + lane;
-    const int colbase = h * kEpiCols;
-    const uint32_t lane_base = uint32_t(q * 32) << 16;
-    int j = 0, tl = 0;
-    // the storer stores each tile's C and, as soon as the store has read the buffer, loads the next tile's C
-    // into it, so that the operand stream of the producer never waits on the C buffer
-    const bool storer = (warp == 2 && lane == 0);
-    int c_pending = -1;  // storer: local index of the tile whose C load is in flight and not yet waited for
-    auto load_c = [&](int t_next, int tl_next) {
-      const int r0n = (t_next / tiles_n) * TM, c0n = (t_next % tiles_n) * TN;
-      mbar_expect_tx(&ctl.cfull, uint32_t(kCBytes));
-      tma_load_2d(smem_u32(sC), &tmCh, c0n, r0n, &ctl.cfull, pol_stream);
-      tma_load_2d(smem_u32(sC + kCHalf), &tmCh, c0n + 32, r0n, &ctl.cfull, pol_stream);
-      tma_load_2d(smem_u32(sC + 2 * kCHalf), &tmCl, c0n, r0n, &ctl.cfull, pol_stream);
-      tma_load_2d(smem_u32(sC + 3 * kCHalf), &tmCl, c0n + 32, r0n, &ctl.cfull, pol_stream);
-      c_pending = tl_next;
+    const int q = warp & 3, h = (warp - 2) >> 2, ew = warp - 2;
+    const uint64_t pol_c = l2_policy_unchanged();
+    uint8_t* bufh = smem + kStages * kStageBytes + ew * 2 * kCBox;
+    uint8_t* bufl = bufh + kCBox;
+    uint64_t* cbar = &ctl.cfull[ew];
+    const uint32_t lane_base = (uint32_t(q * 32) << 16) + uint32_t(h * kCols);
+    int loads = 0, waited = 0;  // pieces of C requested / taken over
+    // the warp's pieces of C, 32 columns each, in the order in which it takes them: (tile, slice), those inside C only
+    auto piece_in = [&](int t, int sl) {
+      return t < ntiles && (t / tiles_n) * TM + q * 32 < m && (t % tiles_n) * TN + h * kCols + sl * 32 < nc;
     };
-    if (storer && blockIdx.x < ntiles) load_c(blockIdx.x, 0);
-    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++tl) {
-      const int r0 = (t / tiles_n) * TM, c0 = (t % tiles_n) * TN;
-      const int gr = r0 + row_in_tile;
-      // accumulators of the thread's row over its kEpiCols columns, as column pairs
-      float2 acc_h[kEpiCols / 2], acc_l[kEpiCols / 2];
-#pragma unroll
-      for (int u = 0; u < kEpiCols / 2; ++u) { acc_h[u] = make_float2(0.f, 0.f); acc_l[u] = make_float2(0.f, 0.f); }
-      bool ok = true;
-      for (int kb = 0; kb < nkb; ++kb, ++j) {
-        const int set = j & 1;
-        const uint32_t tph = uint32_t(j >> 1) & 1u;
-        // scales of this k block: the row's (loaded before the wait) and, per chunk of four columns, the
-        // columns' (the same 16-byte vector for every lane: one broadcast load)
-        const float sa = gr < m ? __ldg(As + int64_t(gr) * nkb + kb) : 0.f;
-        const float4* sbp = reinterpret_cast<const float4*>(Bs + int64_t(kb) * ncp + c0 + colbase);
-        // every wait ends in a warp vote, so a warp always leaves together (tcgen05.ld needs all 32 lanes)
-        if (!__all_sync(0xffffffffu, mbar_wait(&ctl.tfull[set], tph, abort_flag))) {
-          if (lane == 0 && !*abort_flag) { status_error(st, UPDES_ERR_TIMEOUT); atomicCAS(&st->timeout_tag, 0, 43); }
-          *abort_flag = 1;
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-#pragma unroll
-        for (int ch = 0; ch < kEpiCols / 4; ++ch) {
-          const int col = colbase + ch * 4;
-          const float4 s4 = __ldg(sbp + ch);
-          float g[kGroups][4];
-#pragma unroll
-          for (int gi = 0; gi < kGroups; ++gi)
-            tmem_ld4(tmem + lane_base + uint32_t(set * kGroups * TN + gi * TN + col), g[gi]);
-          tmem_wait_ld();
-          if (ch == kEpiCols / 4 - 1) {
-            // every chunk has been read: release the accumulator set to the MMA issuer
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&ctl.tempty[set]);
-          }
-          const float2 c9 = make_float2(1.953125e-3f, 1.953125e-3f);          // 2^-9
-          const float2 c18 = make_float2(3.814697265625e-06f, 3.814697265625e-06f);  // 2^-18
-          const float2 sa2 = make_float2(sa, sa);
-#pragma unroll
-          for (int u = 0; u < 4; u += 2) {
-            const int cu = ch * 4 + u;  // the pair's first column among the thread's kEpiCols
-            const float2 sb2 = u ? make_float2(s4.z, s4.w) : make_float2(s4.x, s4.y);
-            // k-block value = g0 + 2^-9 g1 + 2^-18 (g2 + 2^-9 g3): g0 + 2^-9 g1 exactly as (hh, ll); the two
-            // small groups merged in one rounding (about 2^-40 of the block's scale, far below the digit cut)
-            float2 hh, ll;
-            two_sum2(make_float2(g[0][u], g[0][u + 1]), __fmul2_rn(make_float2(g[1][u], g[1][u + 1]), c9), hh, ll);
-            const float2 g23 = __ffma2_rn(make_float2(g[3][u], g[3][u + 1]), c9, make_float2(g[2][u], g[2][u + 1]));
-            ll = __ffma2_rn(g23, c18, ll);
-            const float2 sc = __fmul2_rn(sa2, sb2);  // powers of two: exact
-            hh = __fmul2_rn(hh, sc);
-            ll = __fmul2_rn(ll, sc);
-            // acc += (hh, ll); the low word is renormalised by the final update of C (K <= 1024: at most 16 blocks)
-            float2 s1, t1;
-            two_sum2(acc_h[cu >> 1], hh, s1, t1);
-            acc_h[cu >> 1] = s1;
-            acc_l[cu >> 1] = __fadd2_rn(acc_l[cu >> 1], __fadd2_rn(t1, ll));
-          }
-        }
+    auto load_c = [&](int t, int sl) {
+      const int y = (t / tiles_n) * TM + q * 32, x = (t % tiles_n) * TN + h * kCols + sl * 32;
+      if (lane == 0) {
+        mbar_expect_tx(cbar, uint32_t(2 * kCBox));
+        tma_load_2d(smem_u32(bufh), &tmCh, x, y, cbar, pol_c);
+        tma_load_2d(smem_u32(bufl), &tmCl, x, y, cbar, pol_c);
       }
-      if (!ok) break;
-      // ---- C -= acc in shared memory (the tile arrived by TMA), then one thread stores it back ----
-      if (!__all_sync(0xffffffffu, mbar_wait(&ctl.cfull, uint32_t(tl) & 1u, abort_flag))) {
-        if (lane == 0 && !*abort_flag) { status_error(st, UPDES_ERR_TIMEOUT); atomicCAS(&st->timeout_tag, 0, 45); }
-        *abort_flag = 1;
+      ++loads;
+    };
+    auto load_first = [&](int t) {  // of tile t or the next of the CTA's tiles in which the warp has one
+      while (t < ntiles && !piece_in(t, 0)) t += int(gridDim.x);
+      if (t < ntiles) load_c(t, 0);
+    };
+    load_first(int(blockIdx.x));
+    int tl = 0;
+    for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++tl) {
+      const int r0 = (t / tiles_n) * TM + q * 32, c0 = (t % tiles_n) * TN + h * kCols;
+      const uint32_t ph = uint32_t(tl) & 1u;
+      const float sa = r0 + lane < m ? -__ldg(As + r0 + lane) : 0.f;
+      float2 gh[kCols / 2], gl[kCols / 2];  // the row's sums over the warp's columns, as column pairs
+      // every wait ends in a warp vote, so a warp always leaves together (tcgen05.ld needs all 32 lanes)
+      if (!__all_sync(0xffffffffu, mbar_wait(&ctl.hi_done, ph, abort_flag))) {
+        if (lane == 0) give_up(43);
         break;
       }
-      if (storer) c_pending = -1;
-      {
-        // this thread's row in the 128B-swizzled boxes: 16-byte chunk q of row r sits at chunk q ^ (r & 7)
-        const int r = row_in_tile;
-        const int half = colbase >> 5, qbase = (colbase & 31) >> 2;  // box and first 16-byte chunk
-        uint8_t* hrow = sC + half * kCHalf + (r >> 3) * 1024 + (r & 7) * 128;
-        uint8_t* lrow = hrow + 2 * kCHalf;
+      tc_fence_after();
 #pragma unroll
-        for (int qq = 0; qq < kEpiCols / 4; ++qq) {
-          const int off = (((qbase + qq) ^ (r & 7)) << 4);
+      for (int u = 0; u < kCols / 2; u += 8) {
+        tmem_ld16(tmem + lane_base + uint32_t(2 * u), reinterpret_cast<float*>(gh + u));
+        tmem_ld16(tmem + lane_base + uint32_t(TN + 2 * u), reinterpret_cast<float*>(gl + u));
+      }
+      tmem_wait_ld();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl.hi_free);
+#pragma unroll
+      for (int u = 0; u < kCols / 2; ++u) {
+        float2 s, e;
+        two_sum2(gh[u], gl[u], s, e);
+        gh[u] = s;
+        gl[u] = e;
+      }
+      if (!__all_sync(0xffffffffu, mbar_wait(&ctl.lo_done, ph, abort_flag))) {
+        if (lane == 0) give_up(47);
+        break;
+      }
+      tc_fence_after();
+#pragma unroll
+      for (int u = 0; u < kCols / 2; u += 8) {
+        float2 g[8];
+        tmem_ld16(tmem + lane_base + uint32_t(2 * TN + 2 * u), reinterpret_cast<float*>(g));
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) gl[u + i] = __fadd2_rn(gl[u + i], g[i]);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&ctl.lo_free);
+      // ---- C -= sums, 32 columns at a time ----
+      bool ok = true;
+#pragma unroll
+      for (int sl = 0; sl < kCols / 32; ++sl) {
+        if (!ok || !piece_in(t, sl)) continue;
+        // the columns' scales, the same for every lane (those of columns beyond nc are scratch bytes of no effect: the
+        // store leaves these columns out)
+        const float4* sb = reinterpret_cast<const float4*>(Bs + c0 + sl * 32);
+        ok = __all_sync(0xffffffffu, mbar_wait(cbar, uint32_t(waited) & 1u, abort_flag));
+        if (!ok) {
+          if (lane == 0) give_up(45);
+          continue;
+        }
+        ++waited;
+        // the lane's row in the 128B-swizzled boxes: 16-byte chunk c of row r sits at chunk c ^ (r & 7)
+        uint8_t* hrow = bufh + lane * 128;
+        uint8_t* lrow = bufl + lane * 128;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const int off = ((c ^ (lane & 7)) << 4);
+          const float4 sb4 = __ldg(sb + c);
           const float4 hv = *reinterpret_cast<float4*>(hrow + off), lv = *reinterpret_cast<float4*>(lrow + off);
           float2 hx[2] = {make_float2(hv.x, hv.y), make_float2(hv.z, hv.w)};
           float2 lx[2] = {make_float2(lv.x, lv.y), make_float2(lv.z, lv.w)};
 #pragma unroll
           for (int u = 0; u < 2; ++u) {
+            const int pi = sl * 16 + c * 2 + u;
+            // minus the product of the scales, a power of two: exact
+            const float2 sc = __fmul2_rn(make_float2(sa, sa), u ? make_float2(sb4.z, sb4.w) : make_float2(sb4.x, sb4.y));
             float2 sx, tx;
-            two_sum2(hx[u], make_float2(-acc_h[qq * 2 + u].x, -acc_h[qq * 2 + u].y), sx, tx);
-            tx = __fadd2_rn(tx, sub2(lx[u], acc_l[qq * 2 + u]));
+            two_sum2(hx[u], __fmul2_rn(gh[pi], sc), sx, tx);
+            tx = __fadd2_rn(tx, __ffma2_rn(gl[pi], sc, lx[u]));
             fast_two_sum2(sx, tx, hx[u], lx[u]);
           }
           *reinterpret_cast<float4*>(hrow + off) = make_float4(hx[0].x, hx[0].y, hx[1].x, hx[1].y);
           *reinterpret_cast<float4*>(lrow + off) = make_float4(lx[0].x, lx[0].y, lx[1].x, lx[1].y);
         }
-      }
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic writes -> visible to TMA
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&ctl.cready);
-      bool stop = false;
-      if (storer) {
-        if (!mbar_wait(&ctl.cready, uint32_t(tl) & 1u, abort_flag)) {
-          if (!*abort_flag) { status_error(st, UPDES_ERR_TIMEOUT); atomicCAS(&st->timeout_tag, 0, 46); }
-          *abort_flag = 1;
-          stop = true;
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // generic accesses before TMA's
+        __syncwarp();
+        if (lane == 0) {
+          // rows >= m and columns >= nc are outside the tensor and are not written
+          tma_store_2d(&tmCh, c0 + sl * 32, r0, smem_u32(bufh), pol_c);
+          tma_store_2d(&tmCl, c0 + sl * 32, r0, smem_u32(bufl), pol_c);
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the buffer has been read
+        }
+        // the warp's next piece: the tile's next slice or the first one of a later tile
+        if (sl + 1 < kCols / 32 && piece_in(t, sl + 1)) {
+          load_c(t, sl + 1);
+        } else {
+          load_first(t + int(gridDim.x));
         }
       }
-      if (storer && !stop) {
-        // rows >= m and columns >= nc are outside the tensor and are not written
-        tma_store_2d(&tmCh, c0, r0, smem_u32(sC), pol_stream);
-        tma_store_2d(&tmCh, c0 + 32, r0, smem_u32(sC + kCHalf), pol_stream);
-        tma_store_2d(&tmCl, c0, r0, smem_u32(sC + 2 * kCHalf), pol_stream);
-        tma_store_2d(&tmCl, c0 + 32, r0, smem_u32(sC + 3 * kCHalf), pol_stream);
-        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");  // the buffer has been read
-        if (t + int(gridDim.x) < ntiles && !*abort_flag) load_c(t + int(gridDim.x), tl + 1);
-      }
-      if (__any_sync(0xffffffffu, stop)) break;  // the whole warp leaves together
+      if (!ok) break;
     }
-    if (storer) {
+    if (lane == 0) {
       asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // stores complete before exit
-      if (c_pending >= 0) {
+      if (loads > waited) {
         // a C load still in flight (only after an abort) must land before shared memory goes away (bounded)
         for (long long it = 0; it < (1 << 22); ++it) {
-          if (mbar_try_wait(&ctl.cfull, uint32_t(c_pending) & 1u)) break;
+          if (mbar_try_wait(cbar, uint32_t(waited) & 1u)) break;
           __nanosleep(64);
         }
       }
     }
+    __syncwarp();
   }
 
   // ---- teardown: all roles done; make sure no MMA is in flight before tensor memory is freed ----
@@ -473,7 +517,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     if (ctl.abort_flag && lane == 0 && last_commit >= 0) {
       // MMAs complete in order: once the last commit has arrived nothing reads tensor memory (bounded)
       for (long long it = 0; it < (1 << 22); ++it) {
-        if (mbar_try_wait(&ctl.tfull[last_commit & 1], uint32_t(last_commit >> 1) & 1u)) break;
+        if (mbar_try_wait(&ctl.empty[last_commit % kStages], uint32_t(last_commit / kStages) & 1u)) break;
         __nanosleep(64);
       }
     }
@@ -483,27 +527,13 @@ __global__ void __launch_bounds__(kThreads, 1)
   }
 }
 
-// 3-D map over digit planes [3][rows][Kp] bf16, box 64 (k) x box_rows x 1, 128B swizzle
-int make_map(CUtensorMap* map, void* base, int rows, int Kp, int box_rows) {
-  cuuint64_t dims[3] = {cuuint64_t(Kp), cuuint64_t(rows), cuuint64_t(kDigits)};
-  cuuint64_t strides[2] = {cuuint64_t(Kp) * 2, cuuint64_t(rows) * Kp * 2};
-  cuuint32_t box[3] = {cuuint32_t(TK), cuuint32_t(box_rows), 1};
-  cuuint32_t estr[3] = {1, 1, 1};
-  const EncodeTiledFn fn = encode_tiled();
-  if (!fn) return UPDES_ERR_CUDA;
-  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base, dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? UPDES_OK : UPDES_ERR_CUDA;
-}
-
-// 2-D map over an FP32 plane (rows x cols, row stride ld elements), box 32 columns x 128 rows, 128B swizzle
+// 2-D map over an FP32 plane (rows x cols, row stride ld elements), box 32 columns x 32 rows, 128B swizzle
 int make_map_c(CUtensorMap* map, float* base, int rows, int cols, int64_t ld) {
   const EncodeTiledFn fn = encode_tiled();
   if (!fn) return UPDES_ERR_CUDA;
   cuuint64_t dims[2] = {cuuint64_t(cols), cuuint64_t(rows)};
   cuuint64_t strides[1] = {cuuint64_t(ld) * 4};
-  cuuint32_t box[2] = {32, cuuint32_t(TM)};
+  cuuint32_t box[2] = {32, 32};
   cuuint32_t estr[2] = {1, 1};
   const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, base, dims, strides, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -511,58 +541,67 @@ int make_map_c(CUtensorMap* map, float* base, int rows, int cols, int64_t ld) {
   return r == CUDA_SUCCESS ? UPDES_OK : UPDES_ERR_CUDA;
 }
 
+template <int TN>
+int launch_update(const CUtensorMap (&maps)[2], const __half* Ad, const __half* Bd, const float* As, const float* Bs, int m, int nc, int Kp, int ctas,
+                  DeviceStatus* st, cudaStream_t s) {
+  static std::atomic<unsigned long long> attr{0};
+  if (int e = smem_opt_in((const void*)ozaki3_kernel<TN>, Cfg<TN>::kSmemBytes, attr)) return e;
+  const int64_t ntiles = ceil_div(m, TM) * ceil_div(nc, TN);
+  ozaki3_kernel<TN><<<unsigned(std::min<int64_t>(ntiles, ctas)), kThreads, Cfg<TN>::kSmemBytes, s>>>(
+      maps[0], maps[1], Ad, Bd, As, Bs, m, nc, Kp, st);
+  UPDES_LAUNCH_CHECK();
+  return UPDES_OK;
+}
+
 }  // namespace
 
 size_t ozaki3_scratch_bytes(int mmax, int ncmax, int Kmax) {
-  const size_t Kp = size_t(ceil_div(Kmax, TK)) * TK;
+  const size_t Kp = size_t(ceil_div(Kmax, kKpUnit)) * kKpUnit;
   auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
-  return al(kDigits * size_t(mmax) * Kp * 2) + al(kDigits * size_t(ncmax) * Kp * 2) + al(size_t(mmax) * (Kp / TK) * 4) +
-         al(size_t(ceil_div(ncmax, TN)) * TN * (Kp / TK) * 4) + 256;
+  const size_t mp = size_t(ceil_div(mmax, TM)) * TM, ncp = size_t(ceil_div(ncmax, 128)) * 128;  // whole tiles
+  return al(kDigits * mp * Kp * 2) + al(kDigits * ncp * Kp * 2) + al(mp * 4) + al(ncp * 4) + 256;
 }
 
 int ozaki3_update(float* Chi, float* Clo, int64_t ldc, const float* A, int64_t lda, const float* B, int64_t ldb,
                   int m, int nc, int K, void* scratch, size_t scratch_bytes, DeviceStatus* st, cudaStream_t s,
                   int max_ctas, bool a_digits_ready) {
   if (m <= 0 || nc <= 0 || K <= 0) return UPDES_OK;
-  // the tile accumulator's low word is left unnormalised across k blocks: a few blocks only
-  if (K > 1024) return UPDES_ERR_UNSUPPORTED;
+  if (K > kMaxK) return UPDES_ERR_UNSUPPORTED;
   if (!scratch || scratch_bytes < ozaki3_scratch_bytes(m, nc, K)) return UPDES_ERR_WORKSPACE;
   if ((reinterpret_cast<uintptr_t>(scratch) & 255) != 0) return UPDES_ERR_INVALID;
   // C goes through TMA: 16-byte aligned planes and row stride (else the caller uses the other kernel)
   if (((reinterpret_cast<uintptr_t>(Chi) | reinterpret_cast<uintptr_t>(Clo)) & 15) != 0 || (ldc & 3) != 0)
     return UPDES_ERR_UNSUPPORTED;
-  const int Kp = int(ceil_div(K, TK)) * TK, nkb = Kp / TK;
+  const int Kp = int(ceil_div(K, kKpUnit)) * kKpUnit;
   auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
   // A's digits and scales first: their place depends only on m and K, so an update with the same A can reuse them
+  const size_t mp = size_t(ceil_div(m, TM)) * TM, ncp = size_t(ceil_div(nc, 128)) * 128;
   char* p = static_cast<char*>(scratch);
-  __nv_bfloat16* Ad = reinterpret_cast<__nv_bfloat16*>(p);
-  p += al(kDigits * size_t(m) * Kp * 2);
+  __half* Ad = reinterpret_cast<__half*>(p);
+  p += al(kDigits * mp * Kp * 2);
   float* As = reinterpret_cast<float*>(p);
-  p += al(size_t(m) * nkb * 4);
-  __nv_bfloat16* Bd = reinterpret_cast<__nv_bfloat16*>(p);
-  p += al(kDigits * size_t(nc) * Kp * 2);
+  p += al(mp * 4);
+  __half* Bd = reinterpret_cast<__half*>(p);
+  p += al(kDigits * ncp * Kp * 2);
   float* Bs = reinterpret_cast<float*>(p);
 
-  static std::atomic<unsigned long long> attr{0};
-  if (int e = smem_opt_in((const void*)ozaki3_kernel, kSmemBytes, attr)) return e;
-  CUtensorMap mapA, mapB, mapCh, mapCl;
-  int e = make_map(&mapA, Ad, m, Kp, TM);
+  const int ctas = max_ctas > 0 ? std::min(max_ctas, num_sms_cached()) : num_sms_cached();
+  // Tiles of 128 columns unless tiles of 64, which take about 0.55 of their time, finish in fewer rounds for it: with at
+  // most one tile a CTA (1,000 x 1,000 x 256: 21 us against 25), or where much of the last 128 columns is empty
+  // (20,000 x 192 x 64: 30 against 35).  With many rounds the wide tiles win (3,000 x 3,000 x 256: 49 against 59).
+  const int64_t rows = ceil_div(m, TM), w128 = ceil_div(rows * ceil_div(nc, 128), ctas),
+                w64 = ceil_div(rows * ceil_div(nc, 64), ctas);
+  const bool wide = 9 * w128 <= 5 * w64;
+  CUtensorMap maps[2];
+  int e = make_map_c(&maps[0], Chi, m, nc, ldc);
   if (e) return e;
-  if ((e = make_map(&mapB, Bd, nc, Kp, TN))) return e;
-  if ((e = make_map_c(&mapCh, Chi, m, nc, ldc))) return e;
-  if ((e = make_map_c(&mapCl, Clo, m, nc, ldc))) return e;
+  if ((e = make_map_c(&maps[1], Clo, m, nc, ldc))) return e;
 
   StatScope sc(kStatGemm, s, 2.0 * m * double(nc) * K, double(m) * nc * 16.0 + (double(m) + nc) * K * 4.0);
-  {
-    const int64_t warps = int64_t(m) * nkb;
-    const int row_blocks = a_digits_ready ? 0 : int(ceil_div(warps * 32, 256)), col_tiles = int(ceil_div(nc, TN));
-    digits_kernel<<<unsigned(row_blocks + col_tiles * nkb), 256, 0, s>>>(A, lda, m, B, ldb, nc, K, Kp, row_blocks,
-                                                                      col_tiles, Ad, As, Bd, Bs);
-    UPDES_LAUNCH_CHECK();
-  }
-  const int ntiles = int(ceil_div(m, TM) * ceil_div(nc, TN));
-  const int grid = std::min(ntiles, max_ctas > 0 ? std::min(max_ctas, num_sms_cached()) : num_sms_cached());
-  ozaki3_kernel<<<grid, kThreads, kSmemBytes, s>>>(mapA, mapB, mapCh, mapCl, As, Bs, m, nc, Kp, st);
+  const int row_blocks = a_digits_ready ? 0 : int(ceil_div(int64_t(m) * 32, 256));
+  digits_kernel<<<unsigned(row_blocks + ceil_div(nc, 32)), 256, 0, s>>>(A, lda, m, B, ldb, nc, K, Kp, wide ? 128 : 64,
+                                                                        row_blocks, Ad, As, Bd, Bs);
   UPDES_LAUNCH_CHECK();
-  return UPDES_OK;
+  return wide ? launch_update<128>(maps, Ad, Bd, As, Bs, m, nc, Kp, ctas, st, s)
+              : launch_update<64>(maps, Ad, Bd, As, Bs, m, nc, Kp, ctas, st, s);
 }

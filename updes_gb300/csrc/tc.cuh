@@ -76,10 +76,8 @@ __device__ __forceinline__ void tmem_ld4(uint32_t taddr, float* v) {
 
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// L2 eviction policies for the copies below: the digit tiles of L and U are reused by every tile of their
-// row band / column across the whole launch, while each C tile is read and written once; marking C
-// evict-first and the digits evict-last keeps the streamed C planes (gigabytes per launch at n = 22,506) from
-// pushing the digit tiles out of L2 between their uses.
+// L2 eviction policies for the copies below: the digit tiles of L and U are reused by every tile of their row band /
+// column across the whole launch (evict-last), while each C tile is read and written once.
 __device__ __forceinline__ uint64_t l2_policy_evict_last() {
   uint64_t p;
   asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
@@ -88,6 +86,11 @@ __device__ __forceinline__ uint64_t l2_policy_evict_last() {
 __device__ __forceinline__ uint64_t l2_policy_evict_first() {
   uint64_t p;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+__device__ __forceinline__ uint64_t l2_policy_unchanged() {
+  uint64_t p;
+  asm volatile("createpolicy.fractional.L2::evict_unchanged.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
 
