@@ -958,8 +958,8 @@ int lu_factor_df(int n, float* Whi, float* Wlo, int64_t ld, int32_t* piv, void* 
     for (int k = K0, p = 0; k < KE; k += nb, ++p) {
       const int w = std::min(nb, KE - k);
       int32_t* map = block_maps(K0) + p * kSwapMapInts;
-      // on a cluster while its registers hold the rows (up to 12,288), else on up to 32 CTAs that meet in L2: at
-      // 12,000 rows 121 us against 176 for 64 columns, at 4,000 80 against 146, at 600 72 against 130
+      // on a cluster while its registers hold the rows (up to 24,576), else on up to 32 CTAs that meet in L2: at
+      // 20,000 rows 170 us against 260 for 64 columns, at 12,000 118 against 176, at 4,000 80 against 146, at 600 70 against 130
       e = panel_cluster(Whi, ld, n, k, w, piv, map, st, us);
       if (e == UPDES_ERR_UNSUPPORTED) e = launch_panel_f32(Whi, ld, n, k, w, piv, recs, map, st, us);
       if (e == UPDES_ERR_UNSUPPORTED)
