@@ -231,80 +231,53 @@ struct SwapJobs {
   int njobs;
 };
 
-// All row interchanges of a panel in one pass: a CTA per (64-column chunk, job) reads the moved rows of its
-// columns into shared memory, then writes each to its destination (the net permutation from the panel's swap
-// map), so a launch touches only the rows that move.
-__global__ void __launch_bounds__(256) swap_rows_kernel(SwapJobs jobs, int64_t ld, const int32_t* __restrict__ map) {
-  __shared__ float buf[128][64];
-  const int j = blockIdx.y;
-  if (j >= jobs.njobs) return;
-  const int cnt = map[0];
-  const int col = threadIdx.x & 63, r0 = threadIdx.x >> 6;
-  const int64_t c = jobs.c0[j] + int64_t(blockIdx.x) * 64 + col;
-  const bool ok = c < jobs.c1[j];
-  float* plane = jobs.plane[j];
-  for (int q = r0; q < cnt; q += 4)
-    if (ok) buf[q][col] = plane[int64_t(map[129 + q]) * ld + c];
-  __syncthreads();
-  for (int q = r0; q < cnt; q += 4)
-    if (ok) plane[int64_t(map[1 + q]) * ld + c] = buf[q][col];
+// The moved rows of a 64-wide panel's swap map ([0] count, [1..128] destinations, [129..256] sources) for the column
+// of this thread (256 threads: 64 columns, four threads a column): 32 values a thread, all read before any is written
+// (the caller's barrier).  Every load is in flight at once; as a loop over the map, each with its map entry's latency
+// before its own, they took 16 of the 22 us of a launch.
+constexpr int kSwapMapStride = 512;
+struct MapRows {
+  int dst[128], src[128];
+};
+__device__ __forceinline__ int read_map(MapRows& m, const int32_t* __restrict__ map) {
+  const int t = threadIdx.x;
+  if (t < 128) m.dst[t] = map[1 + t];
+  else m.src[t - 128] = map[129 + t - 128];
+  return map[0];
+}
+__device__ __forceinline__ void gather_rows(float (&v)[32], const MapRows& m, int cnt, const float* plane, int64_t ld,
+                                            int64_t c, bool ok) {
+  const int r0 = threadIdx.x >> 6;
+#pragma unroll
+  for (int i = 0; i < 32; ++i) v[i] = (ok && r0 + 4 * i < cnt) ? plane[int64_t(m.src[r0 + 4 * i]) * ld + c] : 0.f;
+}
+__device__ __forceinline__ void scatter_rows(const float (&v)[32], const MapRows& m, int cnt, float* plane, int64_t ld,
+                                             int64_t c, bool ok) {
+  const int r0 = threadIdx.x >> 6;
+#pragma unroll
+  for (int i = 0; i < 32; ++i)
+    if (ok && r0 + 4 * i < cnt) plane[int64_t(m.dst[r0 + 4 * i]) * ld + c] = v[i];
 }
 
-// The interchanges of nmaps consecutive panels (swap maps kSwapMapStride ints apart) in one launch: each CTA
-// applies the maps to its columns in panel order, the order in which separate launches would apply them.
-constexpr int kSwapMapStride = 512;
+// The interchanges of nmaps consecutive panels (swap maps kSwapMapStride ints apart) in one launch, a CTA per
+// (64-column chunk, job): each applies the maps to its columns in panel order, the order in which separate launches
+// would apply them.
 __global__ void __launch_bounds__(256) swap_rows_maps_kernel(SwapJobs jobs, int64_t ld, const int32_t* __restrict__ maps,
                                                              int nmaps) {
-  __shared__ float buf[128][64];
+  __shared__ MapRows rows;
   const int j = blockIdx.y;
   if (j >= jobs.njobs) return;
-  const int col = threadIdx.x & 63, r0 = threadIdx.x >> 6;
-  const int64_t c = jobs.c0[j] + int64_t(blockIdx.x) * 64 + col;
+  const int64_t c = jobs.c0[j] + int64_t(blockIdx.x) * 64 + (threadIdx.x & 63);
   const bool ok = c < jobs.c1[j];
   float* plane = jobs.plane[j];
   for (int m = 0; m < nmaps; ++m) {
-    const int32_t* map = maps + m * kSwapMapStride;
-    const int cnt = map[0];
-    for (int q = r0; q < cnt; q += 4)
-      if (ok) buf[q][col] = plane[int64_t(map[129 + q]) * ld + c];
+    const int cnt = read_map(rows, maps + m * kSwapMapStride);
     __syncthreads();
-    for (int q = r0; q < cnt; q += 4)
-      if (ok) plane[int64_t(map[1 + q]) * ld + c] = buf[q][col];
-    __syncthreads();  // this map's rows are in place (and buf free) before the next map reads them
-  }
-}
-
-// U = L^-1 W on rows [k, k+nb), columns [c0, c1): L unit lower from F (FP32), W double-float.  Each row is
-// w_i - sum_j L_ij x_j accumulated in double-float (exact FP32 products, compensated sums) and rounded once
-// to FP32 into F: FP32 ALU only.
-__global__ void __launch_bounds__(64) trsm_df_kernel(float* Whi, const float* Wlo, int64_t ld, int k, int nb,
-                                                     int64_t c0, int64_t c1) {
-  __shared__ float sL[64][65];
-  __shared__ float sX[64][65];
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-    const int i = e / nb, j = e % nb;
-    sL[i][j] = (j < i) ? Whi[int64_t(k + i) * ld + k + j] : 0.f;
-  }
-  __syncthreads();
-  const int t = threadIdx.x;
-  const int64_t c = c0 + int64_t(blockIdx.x) * blockDim.x + t;
-  if (c >= c1) return;
-  for (int i = 0; i < nb; ++i) {
-    const int64_t idx = int64_t(k + i) * ld + c;
-    float sh = Whi[idx], sl = Wlo[idx];
-    for (int j = 0; j < i; ++j) {
-      const float f = -sL[i][j], xj = sX[j][t];
-      const float p = __fmul_rn(f, xj);
-      const float e = __fmaf_rn(f, xj, -p);
-      const float s2 = __fadd_rn(sh, p);
-      const float bb = __fsub_rn(s2, sh);
-      const float tt = __fadd_rn(__fsub_rn(sh, __fsub_rn(s2, bb)), __fsub_rn(p, bb));
-      sh = s2;
-      sl = __fadd_rn(sl, __fadd_rn(tt, e));
-    }
-    const float xi = __fadd_rn(sh, sl);
-    sX[i][t] = xi;
-    Whi[idx] = xi;
+    float v[32];
+    gather_rows(v, rows, cnt, plane, ld, c, ok);
+    __syncthreads();
+    scatter_rows(v, rows, cnt, plane, ld, c, ok);
+    __syncthreads();  // this map's rows are in place (and the map read) before the next one's
   }
 }
 
@@ -315,27 +288,78 @@ __global__ void __launch_bounds__(64) trsm_df_kernel(float* Whi, const float* Wl
 // Step j (unrolled): the owner of row j rounds it to FP32 (the factor entry), broadcasts it by shuffle, and
 // every lane subtracts L[i][j] * x_j from its rows i > j in double-float arithmetic; the chain is one
 // shuffle per row instead of a 2016-term dependent sum.
+// With the panel's swap map, the interchanges are applied to the columns on the way in (rows that end inside the panel
+// go straight to shared memory); behind the CTAs of [c0, c1) follow those that only interchange: columns
+// [b0, b1) of both planes and [l0, l1) of the FP32 factors (the first plane).
 struct TrsmDfSmem {
   float L[64][65];
   float Xh[64][65], Xl[64][65];
+  MapRows rows;
+};
+struct TrsmDfCols {
+  int64_t c0, c1, b0, b1, l0, l1;
 };
 
 __device__ __forceinline__ float2 trsm_sub2(float2 y, float2 x) { return __ffma2_rn(x, make_float2(-1.f, -1.f), y); }
 
-__global__ void __launch_bounds__(256) trsm_df64_kernel(float* Whi, const float* Wlo, int64_t ld, int k, int64_t c0,
-                                                        int64_t c1) {
+__global__ void __launch_bounds__(256) trsm_df64_kernel(float* Whi, float* Wlo, int64_t ld, int k, TrsmDfCols cols,
+                                                        const int32_t* __restrict__ map) {
   extern __shared__ float4 trsm_df_smem[];
   TrsmDfSmem& sm = *reinterpret_cast<TrsmDfSmem*>(trsm_df_smem);
   const int tid = threadIdx.x, lane = tid & 31;
-  const int64_t cb = c0 + int64_t(blockIdx.x) * 64;
-  for (int e = tid; e < 64 * 64; e += blockDim.x) {
-    const int i = e >> 6, j = e & 63;
-    sm.L[i][j] = (j < i) ? Whi[int64_t(k + i) * ld + k + j] : 0.f;
-    const int64_t c = cb + j;
-    const bool ok = c < c1;
-    sm.Xh[i][j] = ok ? Whi[int64_t(k + i) * ld + c] : 0.f;
-    sm.Xl[i][j] = ok ? Wlo[int64_t(k + i) * ld + c] : 0.f;
+  const int nt = int(ceil_div(cols.c1 - cols.c0, 64)), nb = int(ceil_div(cols.b1 - cols.b0, 64));
+  const int bx = int(blockIdx.x);
+  const bool solve = bx < nt, both = bx < nt + nb;
+  const int64_t cb = solve ? cols.c0 + bx * 64ll : both ? cols.b0 + (bx - nt) * 64ll : cols.l0 + (bx - nt - nb) * 64ll;
+  const int64_t c1 = solve ? cols.c1 : both ? cols.b1 : cols.l1;
+  const int tc = tid & 63, tr = tid >> 6;
+  const bool ok = cb + tc < c1;
+  float lv[16];
+  if (solve) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) lv[i] = tc < tr + 4 * i ? Whi[int64_t(k + tr + 4 * i) * ld + k + tc] : 0.f;
   }
+  if (map) {
+    const int cnt = read_map(sm.rows, map);
+    __syncthreads();
+    float vh[32], vl[32];
+    gather_rows(vh, sm.rows, cnt, Whi, ld, cb + tc, ok);
+    if (both) gather_rows(vl, sm.rows, cnt, Wlo, ld, cb + tc, ok);
+    __syncthreads();
+    if (solve) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) {
+        if (tr + 4 * i >= cnt) continue;
+        const int d = sm.rows.dst[tr + 4 * i];
+        if (d < k + 64) {  // the map lists every row of the panel
+          sm.Xh[d - k][tc] = vh[i];
+          sm.Xl[d - k][tc] = vl[i];
+        } else if (ok) {
+          Whi[int64_t(d) * ld + cb + tc] = vh[i];
+          Wlo[int64_t(d) * ld + cb + tc] = vl[i];
+        }
+      }
+    } else {
+      scatter_rows(vh, sm.rows, cnt, Whi, ld, cb + tc, ok);
+      if (both) scatter_rows(vl, sm.rows, cnt, Wlo, ld, cb + tc, ok);
+      return;
+    }
+  } else {
+    float vh[16], vl[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int64_t at = int64_t(k + tr + 4 * i) * ld + cb + tc;
+      vh[i] = ok ? Whi[at] : 0.f;
+      vl[i] = ok ? Wlo[at] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      sm.Xh[tr + 4 * i][tc] = vh[i];
+      sm.Xl[tr + 4 * i][tc] = vl[i];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i) sm.L[tr + 4 * i][tc] = lv[i];
   __syncthreads();
   const int col = tid >> 2, s = tid & 3;
   const int gbase = lane & ~3;
@@ -370,11 +394,9 @@ __global__ void __launch_bounds__(256) trsm_df64_kernel(float* Whi, const float*
     }
   }
   __syncthreads();
-  for (int e = tid; e < 64 * 64; e += blockDim.x) {
-    const int i = e >> 6, j = e & 63;
-    const int64_t c = cb + j;
-    if (c < c1) Whi[int64_t(k + i) * ld + c] = sm.Xh[i][j];
-  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+    if (ok) Whi[int64_t(k + tr + 4 * i) * ld + cb + tc] = sm.Xh[tr + 4 * i][tc];
 }
 
 // ---- FP64 interchanges and triangular solve ---------------------------------------------------------------
@@ -387,7 +409,6 @@ template <int NBK>
 struct Trsm64Smem {
   double L[NBK][NBK + 1];
   double X[NBK][33];
-  double moved[2 * 32][33];
 };
 
 template <int NBK>
@@ -401,22 +422,39 @@ __global__ void __launch_bounds__(128) trsm64_kernel(double* W, int64_t ld, int 
   const int64_t cb = only_swap ? left + int64_t(blockIdx.x) * 32 : c0 + (int64_t(blockIdx.x) - left_ctas) * 32;
   const int64_t ce = only_swap ? left_end : c1;
   const bool in = cb + lane < ce;
+  // loads in batches that are in flight together: as loops with a load each, their latencies were most of a launch
   if (!only_swap)
-    for (int i = wid; i < NBK; i += 4)
+#pragma unroll
+    for (int t = 0; t < NBK / 4; ++t) {
+      const int i = wid + 4 * t;
+#pragma unroll
       for (int j = lane; j < NBK; j += 32) sm.L[i][j] = (j < i && i < w) ? W[int64_t(k + i) * ld + k + j] : 0.0;
+    }
   if (map) {
     const int cnt = map[0];
-    for (int q = wid; q < cnt; q += 4) sm.moved[q][lane] = in ? W[int64_t(map[129 + q]) * ld + cb + lane] : 0.0;
+    double v[16];
+    int src[16], dst[16];
+#pragma unroll
+    for (int t = 0; t < 16; ++t) {
+      src[t] = wid + 4 * t < cnt ? map[129 + wid + 4 * t] : -1;
+      dst[t] = wid + 4 * t < cnt ? map[1 + wid + 4 * t] : -1;
+    }
+#pragma unroll
+    for (int t = 0; t < 16; ++t) v[t] = (in && src[t] >= 0) ? W[int64_t(src[t]) * ld + cb + lane] : 0.0;
     __syncthreads();
-    for (int q = wid; q < cnt; q += 4) {
-      const int r = map[1 + q];
-      const double v = sm.moved[q][lane];
-      if (!only_swap && r < k + w) sm.X[r - k][lane] = v;  // destinations below k + w are the panel's own rows
-      else if (in) W[int64_t(r) * ld + cb + lane] = v;
+#pragma unroll
+    for (int t = 0; t < 16; ++t) {
+      if (dst[t] < 0) continue;
+      if (!only_swap && dst[t] < k + w) sm.X[dst[t] - k][lane] = v[t];  // the panel's own rows
+      else if (in) W[int64_t(dst[t]) * ld + cb + lane] = v[t];
     }
     for (int i = w + wid; i < NBK; i += 4) sm.X[i][lane] = 0.0;
   } else {
-    for (int i = wid; i < NBK; i += 4) sm.X[i][lane] = (in && i < w) ? W[int64_t(k + i) * ld + cb + lane] : 0.0;
+#pragma unroll
+    for (int t = 0; t < NBK / 4; ++t) {
+      const int i = wid + 4 * t;
+      sm.X[i][lane] = (in && i < w) ? W[int64_t(k + i) * ld + cb + lane] : 0.0;
+    }
   }
   if (only_swap) return;
   __syncthreads();
@@ -446,7 +484,6 @@ __global__ void __launch_bounds__(128) trsm64_kernel(double* W, int64_t ld, int 
 __global__ void __launch_bounds__(256) swap_rows64_maps_kernel(double* W, int64_t ld, const int32_t* __restrict__ maps,
                                                                int nmaps, int64_t a0, int64_t a1, int64_t b0,
                                                                int64_t b1) {
-  __shared__ double buf[64][32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int na = int(ceil_div(a1 - a0, 32));
   const bool first = int(blockIdx.x) < na;
@@ -455,12 +492,20 @@ __global__ void __launch_bounds__(256) swap_rows64_maps_kernel(double* W, int64_
   for (int m = 0; m < nmaps; ++m) {
     const int32_t* map = maps + m * kSwapMapStride;
     const int cnt = map[0];
-    for (int q = wid; q < cnt; q += 8)
-      if (in) buf[q][lane] = W[int64_t(map[129 + q]) * ld + c];
+    double v[8];
+    int src[8], dst[8];
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      src[t] = wid + 8 * t < cnt ? map[129 + wid + 8 * t] : -1;
+      dst[t] = wid + 8 * t < cnt ? map[1 + wid + 8 * t] : -1;
+    }
+#pragma unroll
+    for (int t = 0; t < 8; ++t) v[t] = (in && src[t] >= 0) ? W[int64_t(src[t]) * ld + c] : 0.0;
     __syncthreads();
-    for (int q = wid; q < cnt; q += 8)
-      if (in) W[int64_t(map[1 + q]) * ld + c] = buf[q][lane];
-    __syncthreads();  // this map's rows are in place (and buf free) before the next map reads them
+#pragma unroll
+    for (int t = 0; t < 8; ++t)
+      if (in && dst[t] >= 0) W[int64_t(dst[t]) * ld + c] = v[t];
+    __syncthreads();  // this map's rows are in place before the next map reads them
   }
 }
 
@@ -909,23 +954,14 @@ int lu_factor_df(int n, float* Whi, float* Wlo, int64_t ld, int32_t* piv, void* 
   UPDES_CUDA_TRY(cudaMemsetAsync(recs, 0, 2 * (kMaxPanelCtas + 1) * sizeof(PanelRec), s));
   constexpr int kOuter = kOuterNb;
 
-  auto swap_launch = [&](const SwapJobs& j, int64_t maxc, const int32_t* map, cudaStream_t us) -> int {
-    if (!j.njobs) return UPDES_OK;
-    StatScope sc(kStatOther, us, 0.0, 2.0 * 2 * nb * maxc * 4.0 * j.njobs);
-    swap_rows_kernel<<<dim3(unsigned(ceil_div(maxc, 64)), j.njobs), 256, 0, us>>>(j, ld, map);
-    UPDES_LAUNCH_CHECK();
-    return UPDES_OK;
-  };
-  auto trsm = [&](int k, int w, int64_t c0, int64_t c1, cudaStream_t us) -> int {
-    if (c1 <= c0) return UPDES_OK;
-    StatScope sc(kStatTrsm, us, double(w) * w * (c1 - c0), double(w) * (c1 - c0) * 12.0);
-    if (w == 64) {
-      static std::atomic<unsigned long long> attr{0};
-      if (int e = smem_opt_in((const void*)trsm_df64_kernel, int(sizeof(TrsmDfSmem)), attr)) return e;
-      trsm_df64_kernel<<<unsigned(ceil_div(c1 - c0, 64)), 256, sizeof(TrsmDfSmem), us>>>(Whi, Wlo, ld, k, c0, c1);
-    } else {
-      trsm_df_kernel<<<unsigned(ceil_div(c1 - c0, 64)), 64, 0, us>>>(Whi, Wlo, ld, k, w, c0, c1);
-    }
+  auto trsm = [&](int k, const TrsmDfCols& c, const int32_t* map, cudaStream_t us) -> int {
+    const int64_t grid = ceil_div(c.c1 - c.c0, 64) + ceil_div(c.b1 - c.b0, 64) + ceil_div(c.l1 - c.l0, 64);
+    if (grid == 0) return UPDES_OK;
+    StatScope sc(c.c1 > c.c0 ? kStatTrsm : kStatOther, us, 64.0 * 64.0 * (c.c1 - c.c0),
+                 64.0 * (c.c1 - c.c0) * 12.0 + (map ? 128.0 * 8.0 * (2 * (c.c1 - c.c0 + c.b1 - c.b0) + c.l1 - c.l0) : 0.0));
+    static std::atomic<unsigned long long> attr{0};
+    if (int e = smem_opt_in((const void*)trsm_df64_kernel, int(sizeof(TrsmDfSmem)), attr)) return e;
+    trsm_df64_kernel<<<unsigned(grid), 256, sizeof(TrsmDfSmem), us>>>(Whi, Wlo, ld, k, c, map);
     UPDES_LAUNCH_CHECK();
     return UPDES_OK;
   };
@@ -966,18 +1002,12 @@ int lu_factor_df(int n, float* Whi, float* Wlo, int64_t ld, int32_t* piv, void* 
         e = launch_panel<float, true>(Whi, Wlo, ld, Whi, ld, n, k, w, piv, bar, cand, cand_row, diag_row, map, st,
                                       us);
       if (e) return e;
-      SwapJobs j{};
-      int64_t maxc = 0;
-      add_swap_job(j, maxc, Whi, k + w, deferred ? KE : n);
-      add_swap_job(j, maxc, Wlo, k + w, deferred ? KE : n);
-      add_swap_job(j, maxc, Whi, deferred ? K0 : 0, k);  // factored columns: the FP32 factors only
-      if ((e = swap_launch(j, maxc, map, us))) return e;
-      if (k + w < KE) {
-        if ((e = trsm(k, w, k + w, KE, us))) return e;
-        if ((e = upd(k + w, n, k + w, KE, k, k + w, us, deferred ? digits_la : digits,
-                     deferred ? digits_la_bytes : digits_bytes, ctas)))
-          return e;
-      }
+      // interchanges (on the factored columns, those of the FP32 factors only) and the panel's rows of U in one launch;
+      // a panel narrower than 64 is the last one, with no columns to solve for
+      if ((e = trsm(k, {k + w, KE, KE, deferred ? KE : n, deferred ? K0 : 0, k}, map, us))) return e;
+      if (k + w < KE && (e = upd(k + w, n, k + w, KE, k, k + w, us, deferred ? digits_la : digits,
+                                 deferred ? digits_la_bytes : digits_bytes, ctas)))
+        return e;
     }
     return UPDES_OK;
   };
@@ -1001,7 +1031,7 @@ int lu_factor_df(int n, float* Whi, float* Wlo, int64_t ld, int32_t* piv, void* 
   auto block_row = [&](int K0, int KE, int c0, int c1) -> int {
     for (int b = K0; b < KE; b += nb) {
       const int w = std::min(nb, KE - b);
-      if (int e = trsm(b, w, c0, c1, s)) return e;
+      if (int e = trsm(b, {c0, c1, 0, 0, 0, 0}, nullptr, s)) return e;
       if (b + w < KE)
         if (int e = upd(b + w, KE, c0, c1, b, b + w, s, digits, digits_bytes, 0)) return e;
     }

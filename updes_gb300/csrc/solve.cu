@@ -28,24 +28,31 @@ namespace {
 std::mutex g_err_mu;
 std::string g_last_error;
 
-constexpr int kMaxPermN = 51200;  // permutation built in shared memory
+constexpr int kMaxPermN = 51200;  // interchanges read from shared memory
 
-__global__ void perm_from_piv_kernel(const int32_t* __restrict__ piv, int n, int32_t* __restrict__ perm) {
-  extern __shared__ int32_t sp[];
-  for (int i = threadIdx.x; i < n; i += blockDim.x) sp[i] = i;
+// perm[i] = the row that the interchanges k <-> piv[k] >= k, k = 0 .. n-1, bring to position i: a thread follows its
+// position backwards through them.  Those after step i do not touch it, step i takes it to piv[i], and each earlier one
+// that ends where it stands takes it to k.  A chain of one comparison per step, four steps a shared-memory read, for all positions side
+// by side; applied one after the other by one thread the interchanges took 33 ns each (0.33 ms at n = 10,006).
+__global__ void __launch_bounds__(128) perm_from_piv_kernel(const int32_t* __restrict__ piv, int n,
+                                                            int32_t* __restrict__ perm) {
+  extern __shared__ __align__(16) int32_t sp[];
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, top = min(n, int((blockIdx.x + 1) * blockDim.x));
+  for (int k = threadIdx.x; k < top; k += blockDim.x) sp[k] = piv[k];
   __syncthreads();
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < n; ++i) {
-      const int p = piv[i];
-      if (p != i) {
-        const int a = sp[i];
-        sp[i] = sp[p];
-        sp[p] = a;
-      }
-    }
+  if (i >= n) return;
+  int r = sp[i];
+  int k = i - 1;
+  for (; (k & 3) != 3 && k >= 0; --k)
+    if (r == sp[k]) r = k;
+  for (; k >= 0; k -= 4) {
+    const int4 p = *reinterpret_cast<const int4*>(sp + k - 3);
+    if (r == p.w) r = k;
+    if (r == p.z) r = k - 1;
+    if (r == p.y) r = k - 2;
+    if (r == p.x) r = k - 3;
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < n; i += blockDim.x) perm[i] = sp[i];
+  perm[i] = r;
 }
 
 // out[i] = scale[i] * in[perm[i]] (gather, scale may be null) or out[perm[i]] = in[i] (scatter)
@@ -524,7 +531,7 @@ int perm_core(int n, int32_t* piv, cudaStream_t s) {
   if (n > kMaxPermN) return UPDES_ERR_UNSUPPORTED;
   static std::atomic<unsigned long long> attr{0};
   if (int e = smem_opt_in((const void*)perm_from_piv_kernel, int(kMaxPermN * sizeof(int32_t)), attr)) return e;
-  perm_from_piv_kernel<<<1, 1024, n * sizeof(int32_t), s>>>(piv, n, piv + n);
+  perm_from_piv_kernel<<<unsigned(ceil_div(n, 128)), 128, size_t(n + 3) / 4 * 16, s>>>(piv, n, piv + n);
   UPDES_LAUNCH_CHECK();
   return UPDES_OK;
 }
