@@ -25,13 +25,14 @@
 // and the exponents.  The main kernel is persistent, one CTA an SM, tiles of 128 x 64 round robin:
 //   warp 0     TMA producer: all digits of a 32-wide k block (7 x (8 + 4) KB = 84 KB, 64B swizzle) into a 2-stage
 //              ring.  The whole stage is one box for A and one for B.
-//   warp 1     MMA issuer: 34 products x 2 k-steps of tcgen05.mma (kind::f16, M = 128, N = 64) into 8 groups of 64
-//              columns (all 512 TMEM columns: no second set);
+//   warp 1     MMA issuer: 12 instructions for the 34 products, x 2 k-steps, of tcgen05.mma (kind::f16, M = 128, N up to
+//              256: several digit planes of B side by side) into 8 groups of 64 columns (all 512 TMEM columns: no second set);
 //   warps 2-9  epilogue: read the 8 groups, make 64-bit integers of them and release the accumulators (the MMAs of the
 //              next tile start then, their operands already in the ring); C, 32 columns at a time, through a
 //              shared-memory transposition so that its rows are read and written whole.
-// With N = 64 the operand reads from shared memory (6 KB an MMA) allow two thirds of the tensor peak; the epilogue
-// needs two FP64-pipe operations an element (8,192 cycles a tile) beside the tile's 26,000 cycles of MMAs.
+// Bound by shared memory: a k-step reads 112 KB of operands there (as 34 MMAs of N = 64 it was 204 KB, 26,000 cycles a
+// tile; all updates of an n = 10,006 factorisation then took 52 ms, now 45) and needs 1,088 cycles of MMAs; the epilogue needs two
+// FP64-pipe operations an element (8,192 cycles a tile) beside them.
 #include <algorithm>
 #include <atomic>
 
@@ -55,8 +56,10 @@ constexpr int kSmemBytes = kStages * kStageBytes + kVBytes + 1024;
 static_assert(kSmemBytes <= 226 * 1024, "shared memory");
 constexpr int kNanExp = 1 << 20;  // exponent of a row or column with a non-finite entry
 
-// instruction descriptor: D = F32, A = B = BF16, both K-major, N = 64, M = 128
-constexpr uint32_t kIdesc = (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(TN >> 3) << 17) | (uint32_t(TM >> 4) << 24);
+// instruction descriptor: D = F32, A = B = BF16, both K-major, M = 128
+constexpr uint32_t idesc(int n) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | (uint32_t(n >> 3) << 17) | (uint32_t(TM >> 4) << 24);
+}
 
 // tcgen05 shared-memory matrix descriptor: K-major, 64B swizzle, 8-row groups 512 B apart.
 __device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
@@ -68,11 +71,11 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
   return d;
 }
 
-__device__ __forceinline__ void mma_acc(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t acc) {
+__device__ __forceinline__ void mma_acc(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t id, uint32_t acc) {
   asm volatile(
       "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
       " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(acc)
+      "l"(adesc), "l"(bdesc), "r"(id), "r"(acc)
       : "memory");
 }
 
@@ -238,19 +241,27 @@ __device__ __forceinline__ double add_scaled(double c, double d, int ea, int eb)
 }
 
 // The MMAs of one 32-wide k block; `later` is false for the first block of a sum, whose first product in each group
-// overwrites the accumulator.
+// overwrites the accumulator.  The digit planes of B lie behind one another and so do the groups: one instruction
+// multiplies digit plane a by up to four planes b, b + 1, ... into groups a + b, a + b + 1, ..., 12 instructions for 34
+// products that read A 12 times.
 __device__ __forceinline__ void mma_stage(uint32_t tmem, const uint8_t* sA, bool later) {
   const uint64_t a0 = make_desc(smem_u32(sA)), b0 = make_desc(smem_u32(sA + kDigits * kAPlane));
 #pragma unroll
-  for (int a = 0; a < kDigits; ++a)
+  for (int a = 0; a < kDigits; ++a) {
+    const int planes = kGroups - a < kDigits ? kGroups - a : kDigits;
 #pragma unroll
-    for (int b = 0; b < kDigits && a + b < kGroups; ++b)
+    for (int b = 0; b < planes;) {
+      // group 7 begins with a = 1, b = 6, where groups 5 and 6 have their second product: an instruction of its own
+      const int to = b + 4 < planes ? b + 4 : (a == 1 && b == 4) ? kDigits - 1 : planes;
 #pragma unroll
       for (int kk = 0; kk < TK / 16; ++kk) {  // a k-step is 32 bytes: 2 descriptor units
         const bool first = kk == 0 && (a == 0 || (a == 1 && b == kDigits - 1));
         mma_acc(tmem + uint32_t((a + b) * TN), a0 + uint64_t(a * (kAPlane >> 4) + kk * 2),
-                b0 + uint64_t(b * (kBPlane >> 4) + kk * 2), first ? uint32_t(later) : 1u);
+                b0 + uint64_t(b * (kBPlane >> 4) + kk * 2), idesc((to - b) * TN), first ? uint32_t(later) : 1u);
       }
+      b = to;
+    }
+  }
 }
 
 // The thread's row of 32 sums as integers.  x is the sum in units of group 5 (at most 2^62), r what groups 6 and 7 add
@@ -430,7 +441,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 // ---- a fixed matrix times up to 64 columns ------------------------------------------------------------------
 // Y = A X for an m x n matrix whose digits are written once (updes_batch_prepare) and X of at most 64 columns: the
 // same products and sums as above over k blocks of 256, each block's sum rounded once and added in FP64.  A 64-column
-// product reads 14 bytes of digits an entry of A and is bound by its MMAs (34 x 48 cycles for 128 x 64 x 16), about
+// product reads 14 bytes of digits an entry of A and is bound by its operands' way through shared memory, about
 // a tenth of what double-float multiply-adds on the FP32 pipes cost.  The k blocks are split over `splits` CTAs a row
 // tile, their sums added in order by the caller.
 constexpr int kBlockK = 256;
