@@ -13,17 +13,17 @@ int ozaki_update(float* Chi, float* Clo, int64_t ldc, const float* A, int64_t ld
 // CTA per SM; `max_ctas` > 0 caps its grid so that work on another stream keeps the remaining SMs.
 size_t ozaki3_scratch_bytes(int mmax, int ncmax, int Kmax);
 // a_digits_ready: the previous update on `scratch` had the same A (same m, K and values), whose digits and
-// scales are still there; only B's are written.
+// scales are still there; only B's are written.  early: as in launch_next.
 int ozaki3_update(float* Chi, float* Clo, int64_t ldc, const float* A, int64_t lda, const float* B, int64_t ldb,
                   int m, int nc, int K, void* scratch, size_t scratch_bytes, DeviceStatus* st, cudaStream_t s,
-                  int max_ctas = 0, bool a_digits_ready = false);
+                  int max_ctas = 0, bool a_digits_ready = false, bool early = false);
 
 // C (FP64, ldc) -= A (m x K FP64, lda) * B (K x nc FP64, ldb), K <= 256, from exact products of 7 digits of each
 // operand (gemm_tc64.cu); scratch, max_ctas and a_digits_ready as for ozaki3_update.
 size_t ozaki64_scratch_bytes(int mmax, int ncmax, int Kmax);
 int ozaki64_update(double* C, int64_t ldc, const double* A, int64_t lda, const double* B, int64_t ldb, int m, int nc,
                    int K, void* scratch, size_t scratch_bytes, DeviceStatus* st, cudaStream_t s, int max_ctas = 0,
-                   bool a_digits_ready = false);
+                   bool a_digits_ready = false, bool early = false);
 
 // A fixed FP64 matrix (m x n) times up to 64 columns on the same digits (gemm_tc64.cu).  rhs64_matrix writes the digits
 // of rows [r0, r0 + rows) into `matrix` (rhs64_matrix_bytes(m, n) bytes), from FP64 rows (A, lda) or, with A null,

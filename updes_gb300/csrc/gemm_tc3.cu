@@ -211,6 +211,8 @@ __global__ void __launch_bounds__(256) digits_kernel(const float* __restrict__ A
                                                      int TN, int row_blocks, __half* __restrict__ Ad, float* __restrict__ As,
                                                      __half* __restrict__ Bd, float* __restrict__ Bs) {
   const int b = int(blockIdx.x);
+  allow_next();
+  wait_previous();
   if (b < row_blocks) digits_rows(b, A, lda, m, K, Kp, Ad, As);
   else digits_cols(b - row_blocks, B, ldb, nc, K, Kp, TN, Bd, Bs);
 }
@@ -283,6 +285,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  allow_next();
+  wait_previous();
   const uint32_t tmem = ctl.tmem;
   int last_commit = -1;  // MMA issuer: index of the last committed stage
   auto give_up = [&](int tag) {
@@ -543,14 +547,12 @@ int make_map_c(CUtensorMap* map, float* base, int rows, int cols, int64_t ld) {
 
 template <int TN>
 int launch_update(const CUtensorMap (&maps)[2], const __half* Ad, const __half* Bd, const float* As, const float* Bs, int m, int nc, int Kp, int ctas,
-                  DeviceStatus* st, cudaStream_t s) {
+                  DeviceStatus* st, cudaStream_t s, bool early) {
   static std::atomic<unsigned long long> attr{0};
   if (int e = smem_opt_in((const void*)ozaki3_kernel<TN>, Cfg<TN>::kSmemBytes, attr)) return e;
   const int64_t ntiles = ceil_div(m, TM) * ceil_div(nc, TN);
-  ozaki3_kernel<TN><<<unsigned(std::min<int64_t>(ntiles, ctas)), kThreads, Cfg<TN>::kSmemBytes, s>>>(
-      maps[0], maps[1], Ad, Bd, As, Bs, m, nc, Kp, st);
-  UPDES_LAUNCH_CHECK();
-  return UPDES_OK;
+  return launch_next(early, ozaki3_kernel<TN>, unsigned(std::min<int64_t>(ntiles, ctas)), kThreads, Cfg<TN>::kSmemBytes, s,
+                     maps[0], maps[1], Ad, Bd, As, Bs, m, nc, Kp, st);
 }
 
 }  // namespace
@@ -564,7 +566,7 @@ size_t ozaki3_scratch_bytes(int mmax, int ncmax, int Kmax) {
 
 int ozaki3_update(float* Chi, float* Clo, int64_t ldc, const float* A, int64_t lda, const float* B, int64_t ldb,
                   int m, int nc, int K, void* scratch, size_t scratch_bytes, DeviceStatus* st, cudaStream_t s,
-                  int max_ctas, bool a_digits_ready) {
+                  int max_ctas, bool a_digits_ready, bool early) {
   if (m <= 0 || nc <= 0 || K <= 0) return UPDES_OK;
   if (K > kMaxK) return UPDES_ERR_UNSUPPORTED;
   if (!scratch || scratch_bytes < ozaki3_scratch_bytes(m, nc, K)) return UPDES_ERR_WORKSPACE;
@@ -599,9 +601,9 @@ int ozaki3_update(float* Chi, float* Clo, int64_t ldc, const float* A, int64_t l
 
   StatScope sc(kStatGemm, s, 2.0 * m * double(nc) * K, double(m) * nc * 16.0 + (double(m) + nc) * K * 4.0);
   const int row_blocks = a_digits_ready ? 0 : int(ceil_div(int64_t(m) * 32, 256));
-  digits_kernel<<<unsigned(row_blocks + ceil_div(nc, 32)), 256, 0, s>>>(A, lda, m, B, ldb, nc, K, Kp, wide ? 128 : 64,
-                                                                        row_blocks, Ad, As, Bd, Bs);
-  UPDES_LAUNCH_CHECK();
-  return wide ? launch_update<128>(maps, Ad, Bd, As, Bs, m, nc, Kp, ctas, st, s)
-              : launch_update<64>(maps, Ad, Bd, As, Bs, m, nc, Kp, ctas, st, s);
+  if ((e = launch_next(early && max_ctas == 0, digits_kernel, unsigned(row_blocks + ceil_div(nc, 32)), 256, 0, s, A, lda, m, B, ldb, nc, K, Kp,
+                       wide ? 128 : 64, row_blocks, Ad, As, Bd, Bs)))
+    return e;
+  return wide ? launch_update<128>(maps, Ad, Bd, As, Bs, m, nc, Kp, ctas, st, s, early)
+              : launch_update<64>(maps, Ad, Bd, As, Bs, m, nc, Kp, ctas, st, s, early);
 }

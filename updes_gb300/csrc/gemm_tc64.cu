@@ -198,6 +198,8 @@ __global__ void __launch_bounds__(256) digits64_kernel(const double* __restrict_
                                                        int Kp, int span, int row_blocks, uint16_t* __restrict__ Ad,
                                                        int* __restrict__ Ae, uint16_t* __restrict__ Bd,
                                                        int* __restrict__ Be) {
+  allow_next();
+  wait_previous();
   const int b = int(blockIdx.x);
   if (b < row_blocks) digits_rows(b, A, lda, m, K, Kp, span, Ad, Ae);
   else digits_cols(b - row_blocks, B, ldb, nc, K, Kp, Bd, Be);
@@ -322,6 +324,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  allow_next();
+  wait_previous();
   const uint32_t tmem = ctl.tmem;
   int committed = 0;  // MMA issuer: k blocks committed so far
 
@@ -661,7 +665,7 @@ size_t ozaki64_scratch_bytes(int mmax, int ncmax, int Kmax) {
 
 int ozaki64_update(double* C, int64_t ldc, const double* A, int64_t lda, const double* B, int64_t ldb, int m, int nc,
                    int K, void* scratch, size_t scratch_bytes, DeviceStatus* st, cudaStream_t s, int max_ctas,
-                   bool a_digits_ready) {
+                   bool a_digits_ready, bool early) {
   if (m <= 0 || nc <= 0 || K <= 0) return UPDES_OK;
   if (K > 256) return UPDES_ERR_UNSUPPORTED;
   if (!scratch || scratch_bytes < ozaki64_scratch_bytes(m, nc, K)) return UPDES_ERR_WORKSPACE;
@@ -688,15 +692,13 @@ int ozaki64_update(double* C, int64_t ldc, const double* A, int64_t lda, const d
     while (span < Kp / 8) span *= 2;
     const int row_blocks = a_digits_ready ? 0 : int(ceil_div(int64_t(m) * span, 256));
     const int col_blocks = int(ceil_div(nc, 32 * (8 / (Kp / 32))));
-    digits64_kernel<<<unsigned(row_blocks + col_blocks), 256, 0, s>>>(A, lda, m, B, ldb, nc, K, Kp, span, row_blocks,
-                                                                    Ad, Ae, Bd, Be);
-    UPDES_LAUNCH_CHECK();
+    if (int e = launch_next(early && max_ctas == 0, digits64_kernel, unsigned(row_blocks + col_blocks), 256, 0, s, A, lda, m, B, ldb, nc, K, Kp,
+                            span, row_blocks, Ad, Ae, Bd, Be))
+      return e;
   }
   const int ntiles = int(ceil_div(m, TM) * ceil_div(nc, TN));
   const int grid = std::min(ntiles, max_ctas > 0 ? std::min(max_ctas, num_sms_cached()) : num_sms_cached());
-  ozaki64_kernel<<<grid, kThreads, kSmemBytes, s>>>(mapA, mapB, Ae, Be, C, ldc, m, nc, Kp, st);
-  UPDES_LAUNCH_CHECK();
-  return UPDES_OK;
+  return launch_next(early, ozaki64_kernel, unsigned(grid), kThreads, kSmemBytes, s, mapA, mapB, Ae, Be, C, ldc, m, nc, Kp, st);
 }
 
 namespace {

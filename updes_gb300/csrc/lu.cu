@@ -232,28 +232,27 @@ struct SwapJobs {
 };
 
 // The moved rows of a 64-wide panel's swap map ([0] count, [1..128] destinations, [129..256] sources) for the column
-// of this thread (256 threads: 64 columns, four threads a column): 32 values a thread, all read before any is written
-// (the caller's barrier).  Every load is in flight at once; as a loop over the map, each with its map entry's latency
+// of this thread (four threads a column, r0 = 0 .. 3): 32 values a thread, all read before any is written (the caller's
+// barrier).  Every load is in flight at once; as a loop over the map, each with its map entry's latency
 // before its own, they took 16 of the 22 us of a launch.
 constexpr int kSwapMapStride = 512;
 struct MapRows {
   int dst[128], src[128];
 };
 __device__ __forceinline__ int read_map(MapRows& m, const int32_t* __restrict__ map) {
-  const int t = threadIdx.x;
-  if (t < 128) m.dst[t] = map[1 + t];
-  else m.src[t - 128] = map[129 + t - 128];
+  for (int t = threadIdx.x; t < 128; t += blockDim.x) {
+    m.dst[t] = map[1 + t];
+    m.src[t] = map[129 + t];
+  }
   return map[0];
 }
-__device__ __forceinline__ void gather_rows(float (&v)[32], const MapRows& m, int cnt, const float* plane, int64_t ld,
-                                            int64_t c, bool ok) {
-  const int r0 = threadIdx.x >> 6;
+__device__ __forceinline__ void gather_rows(float (&v)[32], const MapRows& m, int cnt, int r0, const float* plane,
+                                            int64_t ld, int64_t c, bool ok) {
 #pragma unroll
   for (int i = 0; i < 32; ++i) v[i] = (ok && r0 + 4 * i < cnt) ? plane[int64_t(m.src[r0 + 4 * i]) * ld + c] : 0.f;
 }
-__device__ __forceinline__ void scatter_rows(const float (&v)[32], const MapRows& m, int cnt, float* plane, int64_t ld,
-                                             int64_t c, bool ok) {
-  const int r0 = threadIdx.x >> 6;
+__device__ __forceinline__ void scatter_rows(const float (&v)[32], const MapRows& m, int cnt, int r0, float* plane,
+                                             int64_t ld, int64_t c, bool ok) {
 #pragma unroll
   for (int i = 0; i < 32; ++i)
     if (ok && r0 + 4 * i < cnt) plane[int64_t(m.dst[r0 + 4 * i]) * ld + c] = v[i];
@@ -266,22 +265,24 @@ __global__ void __launch_bounds__(256) swap_rows_maps_kernel(SwapJobs jobs, int6
                                                              int nmaps) {
   __shared__ MapRows rows;
   const int j = blockIdx.y;
+  allow_next();
   if (j >= jobs.njobs) return;
   const int64_t c = jobs.c0[j] + int64_t(blockIdx.x) * 64 + (threadIdx.x & 63);
+  const int r0 = threadIdx.x >> 6;
   const bool ok = c < jobs.c1[j];
   float* plane = jobs.plane[j];
   for (int m = 0; m < nmaps; ++m) {
     const int cnt = read_map(rows, maps + m * kSwapMapStride);
     __syncthreads();
     float v[32];
-    gather_rows(v, rows, cnt, plane, ld, c, ok);
+    gather_rows(v, rows, cnt, r0, plane, ld, c, ok);
     __syncthreads();
-    scatter_rows(v, rows, cnt, plane, ld, c, ok);
+    scatter_rows(v, rows, cnt, r0, plane, ld, c, ok);
     __syncthreads();  // this map's rows are in place (and the map read) before the next one's
   }
 }
 
-// U12 = L11^-1 W12 for a full 64-row panel: 64 columns per CTA, 4 lanes per column.  The right-hand sides
+// U12 = L11^-1 W12 for a full 64-row panel: COLS columns per CTA, 4 lanes per column.  The right-hand sides
 // (double-float planes) are staged in shared memory in one coalesced pass; lane s of a column's group keeps
 // rows s, s+4, ..., s+60 in registers, as eight pairs (s + 8q, s + 8q + 4) on the packed FP32x2 instructions
 // of sm_100+ (one issue slot per pair; the same operations as scalar code, so bitwise the same results).
@@ -291,9 +292,10 @@ __global__ void __launch_bounds__(256) swap_rows_maps_kernel(SwapJobs jobs, int6
 // With the panel's swap map, the interchanges are applied to the columns on the way in (rows that end inside the panel
 // go straight to shared memory); behind the CTAs of [c0, c1) follow those that only interchange: columns
 // [b0, b1) of both planes and [l0, l1) of the FP32 factors (the first plane).
+template <int COLS>
 struct TrsmDfSmem {
   float L[64][65];
-  float Xh[64][65], Xl[64][65];
+  float Xh[64][COLS + 1], Xl[64][COLS + 1];
   MapRows rows;
 };
 struct TrsmDfCols {
@@ -302,29 +304,35 @@ struct TrsmDfCols {
 
 __device__ __forceinline__ float2 trsm_sub2(float2 y, float2 x) { return __ffma2_rn(x, make_float2(-1.f, -1.f), y); }
 
-__global__ void __launch_bounds__(256) trsm_df64_kernel(float* Whi, float* Wlo, int64_t ld, int k, TrsmDfCols cols,
-                                                        const int32_t* __restrict__ map) {
+template <int COLS>
+__global__ void __launch_bounds__(4 * COLS) trsm_df64_kernel(float* Whi, float* Wlo, int64_t ld, int k, TrsmDfCols cols,
+                                                             const int32_t* __restrict__ map) {
   extern __shared__ float4 trsm_df_smem[];
-  TrsmDfSmem& sm = *reinterpret_cast<TrsmDfSmem*>(trsm_df_smem);
+  TrsmDfSmem<COLS>& sm = *reinterpret_cast<TrsmDfSmem<COLS>*>(trsm_df_smem);
   const int tid = threadIdx.x, lane = tid & 31;
-  const int nt = int(ceil_div(cols.c1 - cols.c0, 64)), nb = int(ceil_div(cols.b1 - cols.b0, 64));
+  allow_next();
+  wait_previous();
+  const int nt = int(ceil_div(cols.c1 - cols.c0, COLS)), nb = int(ceil_div(cols.b1 - cols.b0, COLS));
   const int bx = int(blockIdx.x);
   const bool solve = bx < nt, both = bx < nt + nb;
-  const int64_t cb = solve ? cols.c0 + bx * 64ll : both ? cols.b0 + (bx - nt) * 64ll : cols.l0 + (bx - nt - nb) * 64ll;
+  const int64_t cb = solve  ? cols.c0 + bx * int64_t(COLS)
+                     : both ? cols.b0 + (bx - nt) * int64_t(COLS) : cols.l0 + (bx - nt - nb) * int64_t(COLS);
   const int64_t c1 = solve ? cols.c1 : both ? cols.b1 : cols.l1;
-  const int tc = tid & 63, tr = tid >> 6;
+  const int tc = tid % COLS, tr = tid / COLS;
   const bool ok = cb + tc < c1;
-  float lv[16];
+  constexpr int LV = 64 * 64 / (4 * COLS);
+  const int lc = tid & 63, lr = tid >> 6, ls = COLS / 16;  // L: rows lr, lr + ls, ... of column lc
+  float lv[LV];
   if (solve) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) lv[i] = tc < tr + 4 * i ? Whi[int64_t(k + tr + 4 * i) * ld + k + tc] : 0.f;
+    for (int i = 0; i < LV; ++i) lv[i] = lc < lr + ls * i ? Whi[int64_t(k + lr + ls * i) * ld + k + lc] : 0.f;
   }
   if (map) {
     const int cnt = read_map(sm.rows, map);
     __syncthreads();
     float vh[32], vl[32];
-    gather_rows(vh, sm.rows, cnt, Whi, ld, cb + tc, ok);
-    if (both) gather_rows(vl, sm.rows, cnt, Wlo, ld, cb + tc, ok);
+    gather_rows(vh, sm.rows, cnt, tr, Whi, ld, cb + tc, ok);
+    if (both) gather_rows(vl, sm.rows, cnt, tr, Wlo, ld, cb + tc, ok);
     __syncthreads();
     if (solve) {
 #pragma unroll
@@ -340,8 +348,8 @@ __global__ void __launch_bounds__(256) trsm_df64_kernel(float* Whi, float* Wlo, 
         }
       }
     } else {
-      scatter_rows(vh, sm.rows, cnt, Whi, ld, cb + tc, ok);
-      if (both) scatter_rows(vl, sm.rows, cnt, Wlo, ld, cb + tc, ok);
+      scatter_rows(vh, sm.rows, cnt, tr, Whi, ld, cb + tc, ok);
+      if (both) scatter_rows(vl, sm.rows, cnt, tr, Wlo, ld, cb + tc, ok);
       return;
     }
   } else {
@@ -359,7 +367,7 @@ __global__ void __launch_bounds__(256) trsm_df64_kernel(float* Whi, float* Wlo, 
     }
   }
 #pragma unroll
-  for (int i = 0; i < 16; ++i) sm.L[tr + 4 * i][tc] = lv[i];
+  for (int i = 0; i < LV; ++i) sm.L[lr + ls * i][lc] = lv[i];
   __syncthreads();
   const int col = tid >> 2, s = tid & 3;
   const int gbase = lane & ~3;
@@ -418,6 +426,8 @@ __global__ void __launch_bounds__(128) trsm64_kernel(double* W, int64_t ld, int 
   extern __shared__ double trsm64_smem[];
   Trsm64Smem<NBK>& sm = *reinterpret_cast<Trsm64Smem<NBK>*>(trsm64_smem);
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  allow_next();
+  wait_previous();
   const bool only_swap = int(blockIdx.x) < left_ctas;
   const int64_t cb = only_swap ? left + int64_t(blockIdx.x) * 32 : c0 + (int64_t(blockIdx.x) - left_ctas) * 32;
   const int64_t ce = only_swap ? left_end : c1;
@@ -484,6 +494,7 @@ __global__ void __launch_bounds__(128) trsm64_kernel(double* W, int64_t ld, int 
 __global__ void __launch_bounds__(256) swap_rows64_maps_kernel(double* W, int64_t ld, const int32_t* __restrict__ maps,
                                                                int nmaps, int64_t a0, int64_t a1, int64_t b0,
                                                                int64_t b1) {
+  allow_next();
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int na = int(ceil_div(a1 - a0, 32));
   const bool first = int(blockIdx.x) < na;
@@ -954,16 +965,15 @@ int lu_factor_df(int n, float* Whi, float* Wlo, int64_t ld, int32_t* piv, void* 
   UPDES_CUDA_TRY(cudaMemsetAsync(recs, 0, 2 * (kMaxPanelCtas + 1) * sizeof(PanelRec), s));
   constexpr int kOuter = kOuterNb;
 
-  auto trsm = [&](int k, const TrsmDfCols& c, const int32_t* map, cudaStream_t us) -> int {
-    const int64_t grid = ceil_div(c.c1 - c.c0, 64) + ceil_div(c.b1 - c.b0, 64) + ceil_div(c.l1 - c.l0, 64);
-    if (grid == 0) return UPDES_OK;
+  auto trsm = [&](int k, const TrsmDfCols& c, const int32_t* map, cudaStream_t us, bool early) -> int {
+    if (c.c1 <= c.c0 && c.b1 <= c.b0 && c.l1 <= c.l0) return UPDES_OK;
+    // 32 columns a CTA: a CTA's own SM bounds it (n = 10,006: 28.75 ms a factorisation, with 64 columns 29.1, with 16 29.3)
+    constexpr int kTrsmCols = 32;
+    const int64_t grid = ceil_div(c.c1 - c.c0, kTrsmCols) + ceil_div(c.b1 - c.b0, kTrsmCols) + ceil_div(c.l1 - c.l0, kTrsmCols);
     StatScope sc(c.c1 > c.c0 ? kStatTrsm : kStatOther, us, 64.0 * 64.0 * (c.c1 - c.c0),
                  64.0 * (c.c1 - c.c0) * 12.0 + (map ? 128.0 * 8.0 * (2 * (c.c1 - c.c0 + c.b1 - c.b0) + c.l1 - c.l0) : 0.0));
-    static std::atomic<unsigned long long> attr{0};
-    if (int e = smem_opt_in((const void*)trsm_df64_kernel, int(sizeof(TrsmDfSmem)), attr)) return e;
-    trsm_df64_kernel<<<unsigned(grid), 256, sizeof(TrsmDfSmem), us>>>(Whi, Wlo, ld, k, c, map);
-    UPDES_LAUNCH_CHECK();
-    return UPDES_OK;
+    return launch_next(early, trsm_df64_kernel<kTrsmCols>, unsigned(grid), 4 * kTrsmCols, sizeof(TrsmDfSmem<kTrsmCols>), us, Whi, Wlo,
+                       ld, k, c, map);
   };
   // W[r0:r1, c0:c1] -= F[r0:r1, kk0:kk1] * F[kk0:kk1, c0:c1] on stream us with digit scratch dg, at most ctas CTAs
   // The digits of the last A written into each scratch (the update after a block writes them for the next
@@ -974,13 +984,13 @@ int lu_factor_df(int n, float* Whi, float* Wlo, int64_t ld, int32_t* piv, void* 
     int r0 = -1, r1 = -1, kk0 = -1, kk1 = -1;
   } a_main, a_side;
   auto upd = [&](int r0, int r1, int c0, int c1, int kk0, int kk1, cudaStream_t us, void* dg, size_t dgb,
-                 int ctas) -> int {
+                 int ctas, bool early) -> int {
     if (!use_v2) {
       ADigits& last = (dg == digits) ? a_main : a_side;
       const bool a_ready = last.dg == dg && last.r0 == r0 && last.r1 == r1 && last.kk0 == kk0 && last.kk1 == kk1;
       const int e3 = ozaki3_update(Whi + int64_t(r0) * ld + c0, Wlo + int64_t(r0) * ld + c0, ld,
                                    Whi + int64_t(r0) * ld + kk0, ld, Whi + int64_t(kk0) * ld + c0, ld, r1 - r0,
-                                   c1 - c0, kk1 - kk0, dg, dgb, st, us, ctas, a_ready);
+                                   c1 - c0, kk1 - kk0, dg, dgb, st, us, ctas, a_ready, early);
       last = e3 == UPDES_OK ? ADigits{dg, r0, r1, kk0, kk1} : ADigits{};
       if (e3 != UPDES_ERR_UNSUPPORTED) return e3;
     }
@@ -996,7 +1006,7 @@ int lu_factor_df(int n, float* Whi, float* Wlo, int64_t ld, int32_t* piv, void* 
       int32_t* map = block_maps(K0) + p * kSwapMapInts;
       // on a cluster while its registers hold the rows (up to 24,576), else on up to 32 CTAs that meet in L2: at
       // 20,000 rows 170 us against 260 for 64 columns, at 12,000 118 against 176, at 4,000 80 against 146, at 600 70 against 130
-      e = panel_cluster(Whi, ld, n, k, w, piv, map, st, us);
+      e = panel_cluster(Whi, ld, n, k, w, piv, map, st, us, !lookahead && k > K0);
       if (e == UPDES_ERR_UNSUPPORTED) e = launch_panel_f32(Whi, ld, n, k, w, piv, recs, map, st, us);
       if (e == UPDES_ERR_UNSUPPORTED)
         e = launch_panel<float, true>(Whi, Wlo, ld, Whi, ld, n, k, w, piv, bar, cand, cand_row, diag_row, map, st,
@@ -1004,9 +1014,9 @@ int lu_factor_df(int n, float* Whi, float* Wlo, int64_t ld, int32_t* piv, void* 
       if (e) return e;
       // interchanges (on the factored columns, those of the FP32 factors only) and the panel's rows of U in one launch;
       // a panel narrower than 64 is the last one, with no columns to solve for
-      if ((e = trsm(k, {k + w, KE, KE, deferred ? KE : n, deferred ? K0 : 0, k}, map, us))) return e;
+      if ((e = trsm(k, {k + w, KE, KE, deferred ? KE : n, deferred ? K0 : 0, k}, map, us, true))) return e;
       if (k + w < KE && (e = upd(k + w, n, k + w, KE, k, k + w, us, deferred ? digits_la : digits,
-                                 deferred ? digits_la_bytes : digits_bytes, ctas)))
+                                 deferred ? digits_la_bytes : digits_bytes, ctas, true)))
         return e;
     }
     return UPDES_OK;
@@ -1031,9 +1041,9 @@ int lu_factor_df(int n, float* Whi, float* Wlo, int64_t ld, int32_t* piv, void* 
   auto block_row = [&](int K0, int KE, int c0, int c1) -> int {
     for (int b = K0; b < KE; b += nb) {
       const int w = std::min(nb, KE - b);
-      if (int e = trsm(b, {c0, c1, 0, 0, 0, 0}, nullptr, s)) return e;
+      if (int e = trsm(b, {c0, c1, 0, 0, 0, 0}, nullptr, s, !lookahead)) return e;
       if (b + w < KE)
-        if (int e = upd(b + w, KE, c0, c1, b, b + w, s, digits, digits_bytes, 0)) return e;
+        if (int e = upd(b + w, KE, c0, c1, b, b + w, s, digits, digits_bytes, 0, !lookahead)) return e;
     }
     return UPDES_OK;
   };
@@ -1054,16 +1064,16 @@ int lu_factor_df(int n, float* Whi, float* Wlo, int64_t ld, int32_t* piv, void* 
     // 22,506).
     if (pending && (e = swaps_deferred(K0, KE, KE, n, true))) return e;
     if ((e = block_row(K0, KE, KE, n))) return e;
-    if ((e = upd(KE, n, KE, KE2, K0, KE, s, digits, digits_bytes, 0))) return e;
+    if ((e = upd(KE, n, KE, KE2, K0, KE, s, digits, digits_bytes, 0, !lookahead))) return e;
     if (lookahead && KE2 < n) {
       // the next block on the side stream; the rest of this step on this stream, on the SMs it leaves
       if ((e = side.start())) return e;
       if ((e = factor_block(KE, KE2, true, side.side, kLookaheadCtas))) return e;
-      if ((e = upd(KE, n, KE2, n, K0, KE, s, digits, digits_bytes, rest_ctas))) return e;
+      if ((e = upd(KE, n, KE2, n, K0, KE, s, digits, digits_bytes, rest_ctas, false))) return e;
       if ((e = side.finish())) return e;
       pending = true;
     } else {
-      if (KE2 < n && (e = upd(KE, n, KE2, n, K0, KE, s, digits, digits_bytes, 0))) return e;
+      if (KE2 < n && (e = upd(KE, n, KE2, n, K0, KE, s, digits, digits_bytes, 0, !lookahead))) return e;
       if ((e = factor_block(KE, KE2, false, s, 0))) return e;
       pending = false;
     }
@@ -1119,26 +1129,25 @@ int lu_factor_64(int n, double* W, int64_t ld, int32_t* piv, void* ws, size_t ws
     static std::atomic<unsigned long long> attr32{0}, attr64{0};
     if (w <= 32) {
       if (int e = smem_opt_in((const void*)trsm64_kernel<32>, int(sizeof(Trsm64Smem<32>)), attr32)) return e;
-      trsm64_kernel<32><<<unsigned(lc + tc), 128, sizeof(Trsm64Smem<32>), us>>>(W, ld, k, w, c0, c1, map, left,
-                                                                               left_end, lc);
+      return launch_next(map || !lookahead, trsm64_kernel<32>, unsigned(lc + tc), 128, sizeof(Trsm64Smem<32>), us, W, ld, k, w, c0, c1, map,
+                         left, left_end, lc);
     } else {
       if (int e = smem_opt_in((const void*)trsm64_kernel<64>, int(sizeof(Trsm64Smem<64>)), attr64)) return e;
-      trsm64_kernel<64><<<unsigned(lc + tc), 128, sizeof(Trsm64Smem<64>), us>>>(W, ld, k, w, c0, c1, map, left,
-                                                                               left_end, lc);
+      return launch_next(map || !lookahead, trsm64_kernel<64>, unsigned(lc + tc), 128, sizeof(Trsm64Smem<64>), us, W, ld, k, w, c0, c1, map,
+                         left, left_end, lc);
     }
-    UPDES_LAUNCH_CHECK();
-    return UPDES_OK;
   };
   // W[r0:r1, c0:c1] -= W[r0:r1, k0:k1] * W[k0:k1, c0:c1]; the digits of A of the last update on `digits` are reused
   // when the rows and k range are the same (the rest of the trailing matrix after the next block's columns)
   struct {
     int r0 = -1, r1 = -1, k0 = -1, k1 = -1;
   } last;
-  auto upd = [&](int r0, int r1, int c0, int c1, int k0, int k1, cudaStream_t us, bool la, int ctas) -> int {
+  auto upd = [&](int r0, int r1, int c0, int c1, int k0, int k1, cudaStream_t us, bool la, int ctas,
+                 bool early) -> int {
     const bool ready = !la && last.r0 == r0 && last.r1 == r1 && last.k0 == k0 && last.k1 == k1;
     const int e = ozaki64_update(W + int64_t(r0) * ld + c0, ld, W + int64_t(r0) * ld + k0, ld,
                                  W + int64_t(k0) * ld + c0, ld, r1 - r0, c1 - c0, k1 - k0, la ? digits_la : digits,
-                                 la ? digits_la_bytes : digits_bytes, st, us, ctas, ready);
+                                 la ? digits_la_bytes : digits_bytes, st, us, ctas, ready, early);
     if (!la) last = {r0, r1, k0, k1};
     return e;
   };
@@ -1148,13 +1157,13 @@ int lu_factor_64(int n, double* W, int64_t ld, int32_t* piv, void* ws, size_t ws
     for (int k = K0, p = 0; k < KE; k += kNb64, ++p) {
       const int w = std::min(kNb64, KE - k);
       int32_t* map = block_maps(K0) + p * kSwapMapInts;
-      int e = panel_cluster(W, ld, n, k, w, piv, map, st, us);
+      int e = panel_cluster(W, ld, n, k, w, piv, map, st, us, !lookahead && k > K0);
       if (e == UPDES_ERR_UNSUPPORTED)
         e = launch_panel<double, false>(W, nullptr, ld, W, ld, n, k, w, piv, bar, cand, cand_row, diag_row, map, st,
                                         us);
       if (e) return e;
       if ((e = trsm(k, w, k + w, KE, map, K0, k, us))) return e;
-      if (k + w < KE && (e = upd(k + w, n, k + w, KE, k, k + w, us, la, ctas))) return e;
+      if (k + w < KE && (e = upd(k + w, n, k + w, KE, k, k + w, us, la, ctas, true))) return e;
     }
     return UPDES_OK;
   };
@@ -1182,16 +1191,16 @@ int lu_factor_64(int n, double* W, int64_t ld, int32_t* piv, void* ws, size_t ws
     for (int b = K0; b < KE; b += kLuNb) {  // block row of U
       const int w = std::min(kLuNb, KE - b);
       if ((e = trsm(b, w, KE, n, nullptr, 0, 0, s))) return e;
-      if (b + w < KE && (e = upd(b + w, KE, KE, n, b, b + w, s, false, 0))) return e;
+      if (b + w < KE && (e = upd(b + w, KE, KE, n, b, b + w, s, false, 0, !lookahead))) return e;
     }
-    if ((e = upd(KE, n, KE, KE2, K0, KE, s, false, 0))) return e;
+    if ((e = upd(KE, n, KE, KE2, K0, KE, s, false, 0, !lookahead))) return e;
     if (lookahead && KE2 < n) {
       if ((e = side.start())) return e;
       if ((e = factor_block(KE, KE2, side.side, true, kLookaheadCtas))) return e;
-      if ((e = upd(KE, n, KE2, n, K0, KE, s, false, rest_ctas))) return e;
+      if ((e = upd(KE, n, KE2, n, K0, KE, s, false, rest_ctas, false))) return e;
       if ((e = side.finish())) return e;
     } else {
-      if (KE2 < n && (e = upd(KE, n, KE2, n, K0, KE, s, false, 0))) return e;
+      if (KE2 < n && (e = upd(KE, n, KE2, n, K0, KE, s, false, 0, !lookahead))) return e;
       if ((e = factor_block(KE, KE2, s, false, 0))) return e;
     }
     K0 = KE;

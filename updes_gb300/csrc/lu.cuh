@@ -12,11 +12,11 @@ int lu_factor_64(int n, double* W, int64_t ld, int32_t* piv, void* ws, size_t ws
 
 // The panel W[k:n, k:k+w] (w <= 64) factored in place on one thread-block cluster (panel.cu): interchanges to
 // piv[k..k+w) and their net permutation to swap_map (257 ints, may be null).  UPDES_ERR_UNSUPPORTED when its rows do
-// not fit the cluster's shared memory.
+// not fit the cluster's shared memory.  after_kernel: launched early, as by launch_next.
 int panel_cluster(float* W, int64_t ld, int n, int k, int w, int32_t* piv, int32_t* swap_map, DeviceStatus* st,
-                  cudaStream_t s);
+                  cudaStream_t s, bool after_kernel);
 int panel_cluster(double* W, int64_t ld, int n, int k, int w, int32_t* piv, int32_t* swap_map, DeviceStatus* st,
-                  cudaStream_t s);
+                  cudaStream_t s, bool after_kernel);
 
 // mode: 0 = L, 1 = U, 2 = U^T, 3 = L^T (x overwritten in place); sync_ws: ceil(n/64)+1 ints.
 // dinv (FP32 factors only, may be null): inverted diagonal blocks from diag_inverse, applied as matvecs

@@ -164,6 +164,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (tid < kCols<T>) zero.row[tid] = T(0);
+  allow_next();
+  wait_previous();
   if (tid == 0) s_failed = 0;
 
   // row r of this thread: local row tid + kThreads * r, its place (the global row it will be written to), the
@@ -578,7 +580,8 @@ int panel_cluster_ctas(int m, int cmax) {
 }
 
 template <typename T>
-int launch(T* W, int64_t ld, int n, int k, int w, int32_t* piv, int32_t* swap_map, DeviceStatus* st, cudaStream_t s) {
+int launch(T* W, int64_t ld, int n, int k, int w, int32_t* piv, int32_t* swap_map, DeviceStatus* st, cudaStream_t s,
+           bool after_kernel) {
   const int m = n - k;
   const int cmax = max_cluster<T>();
   if (cmax == 0 || w > kCols<T> || m < w) return UPDES_ERR_UNSUPPORTED;
@@ -590,16 +593,18 @@ int launch(T* W, int64_t ld, int n, int k, int w, int32_t* piv, int32_t* swap_ma
   PanelKernel<T> kern = kernel_of<T>(per_thread);
   if constexpr (sizeof(T) == 4)
     if (halves) kern = halves_kernel_of(per_thread);
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim = {unsigned(C), 1, 1};
+  cudaLaunchAttribute at[2] = {};
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim = {unsigned(C), 1, 1};
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_next
+  at[1].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(C);
   cfg.blockDim = dim3(kThreads);
   cfg.dynamicSmemBytes = smem_bytes<T>(rows, halves ? kCols<T> / 2 : kCols<T>, halves ? 2 : 1);
   cfg.stream = s;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = after_kernel ? 2 : 1;
   StatScope sc(kStatPanel, s, double(m) * w * w, double(m) * w * 2.0 * sizeof(T));
   UPDES_CUDA_TRY(cudaLaunchKernelEx(&cfg, kern, W, ld, n, k, w, rows, piv, swap_map, st));
   stats_count_launch(1);
@@ -609,11 +614,11 @@ int launch(T* W, int64_t ld, int n, int k, int w, int32_t* piv, int32_t* swap_ma
 }  // namespace
 
 int panel_cluster(float* W, int64_t ld, int n, int k, int w, int32_t* piv, int32_t* swap_map, DeviceStatus* st,
-                  cudaStream_t s) {
-  return launch<float>(W, ld, n, k, w, piv, swap_map, st, s);
+                  cudaStream_t s, bool after_kernel) {
+  return launch<float>(W, ld, n, k, w, piv, swap_map, st, s, after_kernel);
 }
 
 int panel_cluster(double* W, int64_t ld, int n, int k, int w, int32_t* piv, int32_t* swap_map, DeviceStatus* st,
-                  cudaStream_t s) {
-  return launch<double>(W, ld, n, k, w, piv, swap_map, st, s);
+                  cudaStream_t s, bool after_kernel) {
+  return launch<double>(W, ld, n, k, w, piv, swap_map, st, s, after_kernel);
 }
