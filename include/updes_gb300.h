@@ -258,6 +258,19 @@ UPDES_API int updes_solve(const updes_problem* p, const double* q, double* coeff
                 size_t workspace_bytes, void* stream);
 
 /*
+ * updes_solve in two parts, for callers that form the right-hand side while the GPU factors: updes_solve_begin assembles
+ * K and issues the factorisation on `stream` without waiting for it; updes_solve_end, with the same problem, options,
+ * workspace and stream, waits for it and does the rest.  `pending` carries one solve from one to the other and is gone
+ * after updes_solve_end, whatever that returns; with q = NULL it only waits for what was issued.  Nothing else may use
+ * the workspace in between.
+ */
+UPDES_API int updes_solve_begin(const updes_problem* p, const updes_solve_opts* opts, void* workspace,
+                                size_t workspace_bytes, void* stream, void** pending);
+UPDES_API int updes_solve_end(void* pending, const updes_problem* p, const double* q, double* coeffs, double* vals,
+                              const updes_solve_opts* opts, updes_solve_info* info, void* workspace,
+                              size_t workspace_bytes, void* stream);
+
+/*
  * Factor once, solve many.  updes_factor assembles, equilibrates and factors K
  * into `workspace` (layout of updes_solve_workspace); updes_solve_factored then
  * solves nrhs right-hand sides (the columns of the row-major N x nrhs block Q,
@@ -371,6 +384,18 @@ UPDES_API int updes_solve_batched(const updes_problem* problems, int32_t count, 
                                   double* const* coeffs, double* const* vals, const int32_t* precision,
                                   const int32_t* panel_width, int32_t max_sweeps, int32_t ctas,
                                   updes_solve_info* infos, void* workspace, size_t workspace_bytes, void* stream);
+
+/* updes_solve_batched in two parts: the first issues the launches on `stream` without waiting for them, the second, with
+ * the same stream, waits and reports (infos may be NULL).  `pending` carries one batch from one to the other and is gone
+ * after updes_solve_batched_end, whatever that returns.  tables: device memory of updes_solve_batched_tables bytes
+ * that the batch has to itself until then; the workspace may be given to further batches on the same stream. */
+UPDES_API int updes_solve_batched_tables(int32_t count, size_t* bytes);
+UPDES_API int updes_solve_batched_begin(const updes_problem* problems, int32_t count, const double* const* q,
+                                        double* const* coeffs, double* const* vals, const int32_t* precision,
+                                        const int32_t* panel_width, int32_t max_sweeps, int32_t ctas, void* workspace,
+                                        size_t workspace_bytes, void* tables, size_t tables_bytes, void* stream,
+                                        void** pending);
+UPDES_API int updes_solve_batched_end(void* pending, updes_solve_info* infos, void* stream);
 
 /* ---- adjoint (reverse mode through the solve) ------------------------------
  * The reference differentiates pde_solver with jax.grad through inv, the GEMM

@@ -101,6 +101,10 @@ SIGNATURES = {
                                              ctypes.POINTER(_sz)]),
     "updes_solve": (ctypes.c_int, [ctypes.POINTER(Problem), _vp, _vp, _vp, ctypes.POINTER(SolveOpts),
                                    ctypes.POINTER(SolveInfo), _vp, _sz, _vp]),
+    "updes_solve_begin": (ctypes.c_int, [ctypes.POINTER(Problem), ctypes.POINTER(SolveOpts), _vp, _sz, _vp,
+                                         ctypes.POINTER(_vp)]),
+    "updes_solve_end": (ctypes.c_int, [_vp, ctypes.POINTER(Problem), _vp, _vp, _vp, ctypes.POINTER(SolveOpts),
+                                       ctypes.POINTER(SolveInfo), _vp, _sz, _vp]),
     "updes_factor": (ctypes.c_int, [ctypes.POINTER(Problem), ctypes.POINTER(SolveOpts), ctypes.POINTER(SolveInfo),
                                     _vp, _sz, _vp]),
     "updes_solve_factored": (ctypes.c_int, [ctypes.POINTER(Problem), _i32, _vp, _i64, _vp, _i64, _vp, _i64,
@@ -120,6 +124,10 @@ SIGNATURES = {
     "updes_solve_batched_workspace": (ctypes.c_int, [ctypes.POINTER(Problem), _i32, _i32, ctypes.POINTER(_sz)]),
     "updes_solve_batched": (ctypes.c_int, [ctypes.POINTER(Problem), _i32, _vp, _vp, _vp, _vp, _vp, _i32, _i32,
                                            ctypes.POINTER(SolveInfo), _vp, _sz, _vp]),
+    "updes_solve_batched_tables": (ctypes.c_int, [_i32, ctypes.POINTER(_sz)]),
+    "updes_solve_batched_begin": (ctypes.c_int, [ctypes.POINTER(Problem), _i32, _vp, _vp, _vp, _vp, _vp, _i32, _i32,
+                                                 _vp, _sz, _vp, _sz, _vp, ctypes.POINTER(_vp)]),
+    "updes_solve_batched_end": (ctypes.c_int, [_vp, ctypes.POINTER(SolveInfo), _vp]),
     "updes_eval_values_t": (ctypes.c_int, [ctypes.POINTER(Problem), _vp, _vp, _vp]),
     "updes_solve_transpose": (ctypes.c_int, [ctypes.POINTER(Problem), _vp, _vp, ctypes.POINTER(SolveOpts),
                                              ctypes.POINTER(SolveInfo), _vp, _sz, _vp]),

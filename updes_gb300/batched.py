@@ -6,6 +6,8 @@ boundary rows, right-hand side) and hands them all to ``updes_solve_batched``: s
 longer than the average SM's share of the batch are solved by thread-block clusters of eight CTAs, the others by
 single CTAs beside them.  Either takes systems from a device work queue, largest first, and runs each one's assembly,
 LU, refinement and values by itself.
+A batch of 128 systems or more is prepared and launched in up to four parts: the host works on a part while the GPU
+solves those before it.
 
 Precision per system:
 
@@ -187,8 +189,14 @@ class _Batch:
             fh[fo[3]:fo[3] + N] = np.asarray(q, dtype=np.float64)
             ih[io[0]:io[0] + Nb] = np.asarray(kind, dtype=np.int32)
             ih[io[1]:io[1] + 2 * Nb] = np.asarray(bnodes, dtype=np.int32).ravel()
-        self.fbuf = torch.from_numpy(fh).to(dev)
-        self.ibuf = torch.from_numpy(ih).to(dev)
+        # on a stream of their own: an earlier part of the batch may be running on the caller's
+        copies = torch.cuda.Stream(dev)
+        with torch.cuda.stream(copies):
+            self.fbuf = torch.from_numpy(fh).to(dev)
+            self.ibuf = torch.from_numpy(ih).to(dev)
+        copies.synchronize()
+        for b in (self.fbuf, self.ibuf):
+            b.record_stream(torch.cuda.current_stream())
         self.obuf = torch.empty(max(opos, 1), dtype=torch.float64, device=dev)
         fb, ib, ob = self.fbuf.data_ptr(), self.ibuf.data_ptr(), self.obuf.data_ptr()
         keep = (self.fbuf, self.ibuf)
@@ -221,7 +229,11 @@ class _Batch:
         return [(host[co:co + dp.n].copy(), host[vo:vo + dp.N].copy()) for dp, (co, vo) in zip(self.dps, self.o_off)]
 
     def run(self, idx, precisions, widths, max_sweeps, ctas):
-        """Solve the systems ``idx`` (host indices into the batch) in one launch; returns the status."""
+        """Solve the systems ``idx`` (host indices into the batch) in one call; returns the status."""
+        return self.end(self.begin(idx, precisions, widths, max_sweeps, ctas))
+
+    def begin(self, idx, precisions, widths, max_sweeps, ctas):
+        """Issue the solves of the systems ``idx`` without waiting for them; the result goes to ``end``."""
         torch, lib = self.torch, _lib.load()
         c = len(idx)
         sub = lambda arr, T: (T * c)(*[arr[i] for i in idx])
@@ -229,15 +241,26 @@ class _Batch:
         qp, cp, vp = sub(self.qp, ctypes.c_void_p), sub(self.cp, ctypes.c_void_p), sub(self.vp, ctypes.c_void_p)
         prec = (ctypes.c_int32 * c)(*[precisions[i] for i in idx])
         wid = (ctypes.c_int32 * c)(*[widths[i] for i in idx])
-        infos = (_lib.SolveInfo * c)()
-        nbytes = ctypes.c_size_t()
+        nbytes, tbytes = ctypes.c_size_t(), ctypes.c_size_t()
         _lib.check(lib.updes_solve_batched_workspace(probs, c, int(ctas), ctypes.byref(nbytes)),
                    "updes_solve_batched_workspace")
         ws = _workspace(nbytes.value, self.dps[0].device)
+        _lib.check(lib.updes_solve_batched_tables(c, ctypes.byref(tbytes)), "updes_solve_batched_tables")
+        tables = torch.empty(tbytes.value, dtype=torch.uint8, device=self.dps[0].device)
         stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-        st = lib.updes_solve_batched(probs, c, ctypes.cast(qp, ctypes.c_void_p), ctypes.cast(cp, ctypes.c_void_p),
-                                     ctypes.cast(vp, ctypes.c_void_p), prec, wid, int(max_sweeps), int(ctas), infos,
-                                     ws.data_ptr(), ws.numel(), stream)
+        pending = ctypes.c_void_p()
+        _lib.check(lib.updes_solve_batched_begin(probs, c, ctypes.cast(qp, ctypes.c_void_p),
+                                                 ctypes.cast(cp, ctypes.c_void_p), ctypes.cast(vp, ctypes.c_void_p),
+                                                 prec, wid, int(max_sweeps), int(ctas), ws.data_ptr(), ws.numel(),
+                                                 tables.data_ptr(), tables.numel(), stream, ctypes.byref(pending)),
+                   "updes_solve_batched")
+        return idx, pending, stream, (tables, ws)
+
+    def end(self, begun):
+        """Wait for what ``begin`` issued; returns the status."""
+        idx, pending, stream, _ = begun
+        infos = (_lib.SolveInfo * len(idx))()
+        st = _lib.load().updes_solve_batched_end(pending, infos, stream)
         for k, i in enumerate(idx):
             self.infos[i] = infos[k]
         return st
@@ -289,6 +312,37 @@ def _tune_widths(batch, precisions, tuner, max_sweeps):
     return widths
 
 
+def _parts(sizes):
+    """The consecutive parts [first, last) in which a batch is prepared and launched, so that the host prepares a part while
+    the GPU solves those before it (256 clouds: 240 ms of preparation, most of it the callers' functions, beside 118 ms
+    of solves): one part below 128 systems, where a part would not fill the GPU; else four with about 30, 30, 25 and 15 %
+    of the nodes, the last one small because nothing runs beside its solves."""
+    if len(sizes) < 128:
+        return [(0, len(sizes))]
+    total, done, first, parts = sum(sizes), 0, 0, []
+    for i, s in enumerate(sizes):
+        done += s
+        if len(parts) < 3 and done >= (0.30, 0.60, 0.85)[len(parts)] * total:
+            parts.append((first, i + 1))
+            first = i + 1
+    if first < len(sizes):
+        parts.append((first, len(sizes)))
+    return parts
+
+
+def _prepare_part(systems, opts):
+    prepared = []
+    for sysd in systems:
+        bcs = boundary_conditions_func_to_arr(sysd["boundary_conditions"], sysd["cloud"])
+        prepared.append(prepare(sysd["diff_operator"], sysd["rhs_operator"], sysd["cloud"], bcs, sysd["rbf"],
+                                sysd["max_degree"], sysd.get("diff_args"), sysd.get("rhs_args"), opts))
+    for sysd in systems:
+        if getattr(sysd["cloud"], "sorted_local_supports", None) is not None:
+            raise _lib.UpdesError(_lib.ERR_UNSUPPORTED, "updes_solve_batched (local supports)")
+    return _Batch([s["cloud"] for s in systems], [s["rbf"] for s in systems], [s["max_degree"] for s in systems],
+                  prepared, opts.self_term)
+
+
 def pde_solver_batched(systems, options=None, precision="auto", max_sweeps=4, ctas=0, tuner="default"):
     """Solve many independent systems in one call (``updes_solve_batched``).
 
@@ -301,58 +355,68 @@ def pde_solver_batched(systems, options=None, precision="auto", max_sweeps=4, ct
     import time
     torch = _torch()
     opts = options or DEFAULT_OPTIONS
-    t0 = time.perf_counter()
-    prepared = []
-    for sysd in systems:
-        cloud = sysd["cloud"]
-        n = cloud.N + compute_nb_monomials(sysd["max_degree"])
-        if n > MAX_N:
-            raise ValueError(f"system of n = {n} unknowns exceeds the batched solver's limit of {MAX_N}")
-        bcs = boundary_conditions_func_to_arr(sysd["boundary_conditions"], cloud)
-        prepared.append(prepare(sysd["diff_operator"], sysd["rhs_operator"], cloud, bcs, sysd["rbf"],
-                                sysd["max_degree"], sysd.get("diff_args"), sysd.get("rhs_args"), opts))
-    if not prepared:
+    systems = list(systems)
+    if not systems:
         return []
     for sysd in systems:
-        if getattr(sysd["cloud"], "sorted_local_supports", None) is not None:
-            raise _lib.UpdesError(_lib.ERR_UNSUPPORTED, "updes_solve_batched (local supports)")
-    batch = _Batch([s["cloud"] for s in systems], [s["rbf"] for s in systems], [s["max_degree"] for s in systems],
-                   prepared, opts.self_term)
-    dps = batch.dps
-    names = precision if isinstance(precision, (list, tuple)) else [precision] * len(dps)
+        n = sysd["cloud"].N + compute_nb_monomials(sysd["max_degree"])
+        if n > MAX_N:
+            raise ValueError(f"system of n = {n} unknowns exceeds the batched solver's limit of {MAX_N}")
+    names = list(precision) if isinstance(precision, (list, tuple)) else [precision] * len(systems)
     code = {"fp32": _lib.PREC_FP32, "auto": _lib.PREC_FP32, "fp64": _lib.PREC_FP64}
-    precs = [code[p] for p in names]
     tuner = default_tuner() if tuner == "default" else tuner
-    widths = _tune_widths(batch, precs, tuner, max_sweeps) if tuner is not None else [16] * len(dps)
+    parts = []  # (first system, batch, precisions, widths, what begin returned, events around it)
+    prepare_s = 0.0
+    st = _lib.OK
+    try:
+        for first, last in _parts([s["cloud"].N for s in systems]):
+            t0 = time.perf_counter()
+            batch = _prepare_part(systems[first:last], opts)
+            precs = [code[p] for p in names[first:last]]
+            prepare_s += time.perf_counter() - t0
+            widths = _tune_widths(batch, precs, tuner, max_sweeps) if tuner is not None else [16] * batch.count
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            parts.append((first, batch, precs, widths, batch.begin(list(range(batch.count)), precs, widths, max_sweeps,
+                                                                   ctas), (e0, e1)))
+            e1.record()
+    finally:
+        for _, batch, _, _, begun, _ in parts:
+            one = batch.end(begun)
+            if st == _lib.OK or (st == _lib.ERR_SINGULAR and one != _lib.OK):
+                st = one
+    used = ["fp64" if code[nm] == _lib.PREC_FP64 else "fp32" for nm in names]
+    relaunched, relaunch_ms, widths_all = 0, 0.0, []
+    for first, batch, precs, widths, _, _ in parts:
+        redo = [i for i in range(batch.count) if names[first + i] == "auto" and (
+            batch.infos[i].lu_info != 0 or not batch.infos[i].backward_error <= RELAUNCH_BACKWARD_ERROR)]
+        if redo:
+            precs2 = list(precs)
+            for i in redo:
+                precs2[i] = _lib.PREC_FP64
+                used[first + i] = "fp64 (after fp32)"
+            w2 = _tune_widths(batch, precs2, tuner, max_sweeps) if tuner is not None else widths
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            st2 = batch.run(redo, precs2, w2, max_sweeps, ctas)
+            e1.record()
+            e1.synchronize()
+            relaunched, relaunch_ms = relaunched + len(redo), relaunch_ms + e0.elapsed_time(e1)
+            if st == _lib.OK or st == _lib.ERR_SINGULAR:
+                st = st2 if st2 != _lib.OK else st
+        widths_all += widths
     torch.cuda.synchronize()
-    t1 = time.perf_counter()
-    e0, e1, e2 = (torch.cuda.Event(enable_timing=True) for _ in range(3))
-    e0.record()
-    st = batch.run(list(range(len(dps))), precs, widths, max_sweeps, ctas)
-    e1.record()
-    used = ["fp64" if p == _lib.PREC_FP64 else "fp32" for p in precs]
-    redo = [i for i, nm in enumerate(names) if nm == "auto" and (batch.infos[i].lu_info != 0 or not
-                                                                  batch.infos[i].backward_error <= RELAUNCH_BACKWARD_ERROR)]
-    if redo:
-        precs2 = list(precs)
-        for i in redo:
-            precs2[i] = _lib.PREC_FP64
-            used[i] = "fp64 (after fp32)"
-        w2 = _tune_widths(batch, precs2, tuner, max_sweeps) if tuner is not None else widths
-        e1.record()
-        st2 = batch.run(redo, precs2, w2, max_sweeps, ctas)
-        if st == _lib.OK or st == _lib.ERR_SINGULAR:
-            st = st2 if st2 != _lib.OK else st
-    e2.record()
-    torch.cuda.synchronize()
+    dps = [dp for _, batch, _, _, _, _ in parts for dp in batch.dps]
+    infos = [batch.infos[i] for _, batch, _, _, _, _ in parts for i in range(batch.count)]
     LAST_BATCHED_TIMING.clear()
-    LAST_BATCHED_TIMING.update(host_prepare_s=t1 - t0, launch_ms=e0.elapsed_time(e1),
-                               fp64_relaunch_ms=e1.elapsed_time(e2), relaunched=len(redo))
-    LAST_BATCHED_INFO[:] = [dict(batch.infos[i].as_dict(), precision=used[i], panel_width=widths[i])
+    LAST_BATCHED_TIMING.update(host_prepare_s=prepare_s, launch_ms=sum(e[0].elapsed_time(e[1]) for *_, e in parts),
+                               fp64_relaunch_ms=relaunch_ms, relaunched=relaunched)
+    LAST_BATCHED_INFO[:] = [dict(infos[i].as_dict(), precision=used[i], panel_width=widths_all[i])
                             for i in range(len(dps))]
     _lib.check(st, "updes_solve_batched")
     out = []
-    for sysd, dp, (c, v) in zip(systems, dps, batch.results()):
+    results = [r for _, batch, _, _, _, _ in parts for r in batch.results()]
+    for sysd, dp, (c, v) in zip(systems, dps, results):
         cloud, rbf, deg = sysd["cloud"], sysd["rbf"], sysd["max_degree"]
         out.append(SteadySol(v, c, CollocationMatrix(lambda dp=dp, cloud=cloud, rbf=rbf, deg=deg:
                                                      materialize_B(dp, cloud, rbf, deg))))

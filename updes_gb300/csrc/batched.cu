@@ -23,6 +23,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <memory>
+#include <new>
 #include <numeric>
 #include <vector>
 
@@ -973,6 +975,18 @@ Split split_batch(const updes_problem* problems, int32_t count, int32_t ctas) {
 
 }  // namespace
 
+namespace {
+size_t tables_bytes_for(int32_t count) {
+  return align256(size_t(count) * (sizeof(BatchSys) + sizeof(BatchOut) + 4)) + 1024;
+}
+}  // namespace
+
+extern "C" int updes_solve_batched_tables(int32_t count, size_t* bytes) {
+  if (count <= 0 || !bytes) return UPDES_ERR_INVALID;
+  *bytes = tables_bytes_for(count);
+  return UPDES_OK;
+}
+
 extern "C" int updes_solve_batched_workspace(const updes_problem* problems, int32_t count, int32_t ctas,
                                              size_t* bytes) {
   if (!problems || count <= 0 || ctas < 0 || !bytes) return UPDES_ERR_INVALID;
@@ -980,25 +994,39 @@ extern "C" int updes_solve_batched_workspace(const updes_problem* problems, int3
   const int e = batch_n_max(problems, count, &n_max);
   if (e) return e;
   if (sm_count() <= 0) return UPDES_ERR_CUDA;
-  *bytes = split_batch(problems, count, ctas).slices() +
-           align256(size_t(count) * (sizeof(BatchSys) + sizeof(BatchOut) + 4)) + 1024;
+  *bytes = split_batch(problems, count, ctas).slices() + 256 + tables_bytes_for(count);
   return UPDES_OK;
 }
 
-extern "C" int updes_solve_batched(const updes_problem* problems, int32_t count, const double* const* q,
-                                   double* const* coeffs, double* const* vals, const int32_t* precision,
-                                   const int32_t* panel_width, int32_t max_sweeps, int32_t ctas,
-                                   updes_solve_info* infos, void* workspace, size_t workspace_bytes, void* stream) {
+namespace {
+struct PendingBatch {
+  std::vector<BatchSys> sys;  // copied from by the stream
+  std::vector<int32_t> order;
+  const BatchOut* d_out;
+};
+}  // namespace
+
+extern "C" int updes_solve_batched_begin(const updes_problem* problems, int32_t count, const double* const* q,
+                                         double* const* coeffs, double* const* vals, const int32_t* precision,
+                                         const int32_t* panel_width, int32_t max_sweeps, int32_t ctas, void* workspace,
+                                         size_t workspace_bytes, void* tables, size_t tables_bytes, void* stream,
+                                         void** pending) {
+  if (!pending) return UPDES_ERR_INVALID;
+  *pending = nullptr;
+  if (!tables || count <= 0) return UPDES_ERR_INVALID;
+  if (tables_bytes < tables_bytes_for(count)) return UPDES_ERR_WORKSPACE;
   if (!problems || count <= 0 || !q || !coeffs || !workspace || ctas < 0 || max_sweeps < 0) return UPDES_ERR_INVALID;
   int n_max = 0;
   int e = batch_n_max(problems, count, &n_max);
   if (e) return e;
   if (sm_count() <= 0) return UPDES_ERR_CUDA;
   const Split split = split_batch(problems, count, ctas);
-  size_t need = 0;
-  if ((e = updes_solve_batched_workspace(problems, count, ctas, &need))) return e;
-  if (workspace_bytes < need) return UPDES_ERR_WORKSPACE;
-  std::vector<BatchSys> sys(count);
+  if (workspace_bytes < split.slices() + 256) return UPDES_ERR_WORKSPACE;
+  std::unique_ptr<PendingBatch> h(new (std::nothrow) PendingBatch);
+  if (!h) return UPDES_ERR_CUDA;
+  h->sys.resize(count);
+  h->order.resize(count);
+  std::vector<BatchSys>& sys = h->sys;
   for (int32_t i = 0; i < count; ++i) {
     if (!q[i] || !coeffs[i]) return UPDES_ERR_INVALID;
     const int pr = precision ? precision[i] : UPDES_PREC_FP32;
@@ -1014,7 +1042,7 @@ extern "C" int updes_solve_batched(const updes_problem* problems, int32_t count,
     sys[i].max_sweeps = max_sweeps;
   }
   // the clusters' systems, then the others, each largest first (their solves are the longest)
-  std::vector<int32_t> order(count);
+  std::vector<int32_t>& order = h->order;
   std::iota(order.begin(), order.end(), 0);
   std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t b) {
     const bool ta = split.by_cluster(sys[a].n), tb = split.by_cluster(sys[b].n);
@@ -1024,7 +1052,7 @@ extern "C" int updes_solve_batched(const updes_problem* problems, int32_t count,
     return ca > cb;
   });
   char* base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(workspace) + 255) & ~uintptr_t(255));
-  char* meta = base + split.slices();
+  char* meta = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(tables) + 255) & ~uintptr_t(255));
   BatchSys* d_sys = reinterpret_cast<BatchSys*>(meta);
   BatchOut* d_out = reinterpret_cast<BatchOut*>(meta + align256(size_t(count) * sizeof(BatchSys)));
   int32_t* d_order = reinterpret_cast<int32_t*>(reinterpret_cast<char*>(d_out) + align256(size_t(count) * sizeof(BatchOut)));
@@ -1065,8 +1093,18 @@ extern "C" int updes_solve_batched(const updes_problem* problems, int32_t count,
     }
     if (both && (e = side.finish())) return e;
   }
+  h->d_out = d_out;
+  *pending = h.release();
+  return UPDES_OK;
+}
+
+extern "C" int updes_solve_batched_end(void* pending, updes_solve_info* infos, void* stream) {
+  if (!pending) return UPDES_ERR_INVALID;
+  std::unique_ptr<PendingBatch> h(static_cast<PendingBatch*>(pending));
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int32_t count = int32_t(h->sys.size());
   std::vector<BatchOut> outs(count);
-  UPDES_CUDA_TRY(cudaMemcpyAsync(outs.data(), d_out, sizeof(BatchOut) * count, cudaMemcpyDeviceToHost, s));
+  UPDES_CUDA_TRY(cudaMemcpyAsync(outs.data(), h->d_out, sizeof(BatchOut) * count, cudaMemcpyDeviceToHost, s));
   UPDES_CUDA_TRY(cudaStreamSynchronize(s));
   int status = UPDES_OK;
   for (int32_t i = 0; i < count; ++i) {
@@ -1081,4 +1119,20 @@ extern "C" int updes_solve_batched(const updes_problem* problems, int32_t count,
     else if (status == UPDES_OK && outs[i].lu_info) status = UPDES_ERR_SINGULAR;
   }
   return status;
+}
+
+extern "C" int updes_solve_batched(const updes_problem* problems, int32_t count, const double* const* q,
+                                   double* const* coeffs, double* const* vals, const int32_t* precision,
+                                   const int32_t* panel_width, int32_t max_sweeps, int32_t ctas,
+                                   updes_solve_info* infos, void* workspace, size_t workspace_bytes, void* stream) {
+  if (!problems || count <= 0 || !workspace || ctas < 0) return UPDES_ERR_INVALID;
+  size_t need = 0;
+  if (int e = updes_solve_batched_workspace(problems, count, ctas, &need)) return e;
+  if (workspace_bytes < need) return UPDES_ERR_WORKSPACE;
+  // the tables behind the systems' slices
+  const size_t tb = tables_bytes_for(count);
+  void* pending = nullptr;
+  const int e = updes_solve_batched_begin(problems, count, q, coeffs, vals, precision, panel_width, max_sweeps, ctas,
+                                          workspace, need - tb, static_cast<char*>(workspace) + (need - tb), tb, stream, &pending);
+  return e ? e : updes_solve_batched_end(pending, infos, stream);
 }

@@ -9,7 +9,9 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <vector>
 
@@ -762,14 +764,17 @@ int multi_dot(const double* V, int64_t ldv, int nv, const double* w, int n, doub
 struct Timer {
   cudaEvent_t a, b;
   cudaStream_t s;
-  bool ok;
+  bool ok, marked = false;
   explicit Timer(cudaStream_t st) : s(st) {
     ok = cudaEventCreate(&a) == cudaSuccess && cudaEventCreate(&b) == cudaSuccess;
     if (ok) cudaEventRecord(a, s);
   }
+  void mark() {  // the end of what is timed, where stop() comes later
+    if (ok) marked = cudaEventRecord(b, s) == cudaSuccess;
+  }
   double stop() {
     if (!ok) return 0.0;
-    cudaEventRecord(b, s);
+    if (!marked) cudaEventRecord(b, s);
     cudaEventSynchronize(b);
     float ms = 0.f;
     cudaEventElapsedTime(&ms, a, b);
@@ -976,9 +981,7 @@ namespace {
 // Factors of the equilibrated K (double-float planes) at `precision`; records the factored state.
 // planes_ready: the working copy already holds the equilibrated K, written by the assembly: for FP32 factors
 // the planes F32 and Wlo (double-float assembly), for FP64 factors the FP64 matrix W.
-int factor_stage(const SolveWs& w, int n, int precision, updes_solve_info* info, cudaStream_t s,
-                 bool planes_ready = false) {
-  Timer t(s);
+int factor_launch(const SolveWs& w, int n, int precision, cudaStream_t s, bool planes_ready) {
   int e;
   UPDES_CUDA_TRY(cudaMemsetAsync(w.state, 0, 4 * sizeof(int32_t), s));  // invalid until the factors are complete
   const int64_t total = int64_t(n) * w.ld;
@@ -997,7 +1000,12 @@ int factor_stage(const SolveWs& w, int n, int precision, updes_solve_info* info,
     if (!e) e = diag_inverse(n, w.F32, w.ld, w.dinv, s);
     if (!e) e = diag_inverse128(n, w.F32, w.ld, w.dinv, w.dinv128, s);
   }
-  if (e) return e;
+  return e;
+}
+
+// Waits for what factor_launch issued, reports on it and marks the factors as complete.
+int factor_finish(const SolveWs& w, int n, int precision, updes_solve_info* info, cudaStream_t s, Timer& t) {
+  int e;
   DeviceStatus h;
   if ((e = read_status(w.lu.st, s, &h))) return e;
   if (h.error) return h.error;
@@ -1010,6 +1018,12 @@ int factor_stage(const SolveWs& w, int n, int precision, updes_solve_info* info,
   UPDES_CUDA_TRY(cudaMemcpyAsync(w.state, st4, sizeof st4, cudaMemcpyHostToDevice, s));
   UPDES_CUDA_TRY(cudaStreamSynchronize(s));
   return UPDES_OK;
+}
+
+int factor_stage(const SolveWs& w, int n, int precision, updes_solve_info* info, cudaStream_t s, bool planes_ready) {
+  Timer t(s);
+  if (int e = factor_launch(w, n, precision, s, planes_ready)) return e;
+  return factor_finish(w, n, precision, info, s, t);
 }
 
 int read_state(const SolveWs& w, int n, int* precision, cudaStream_t s) {
@@ -1230,6 +1244,62 @@ extern "C" int updes_solve_factored(const updes_problem* p, int32_t nrhs, const 
   }
   *info = agg;
   return agg.converged ? UPDES_OK : UPDES_ERR_NOT_CONVERGED;
+}
+
+namespace {
+struct Pending {
+  Timer t;
+  updes_solve_info info;
+  int n, precision;
+};
+}  // namespace
+
+extern "C" int updes_solve_begin(const updes_problem* p, const updes_solve_opts* opts, void* workspace,
+                                 size_t workspace_bytes, void* stream, void** pending) {
+  SolveWs w;
+  updes_solve_opts o;
+  if (!pending) return UPDES_ERR_INVALID;
+  *pending = nullptr;
+  int e = solve_setup(p, opts, workspace, workspace_bytes, &w, &o);
+  if (e) return e;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  const int n = p->N + p->M;
+  updes_solve_info info;
+  std::memset(&info, 0, sizeof info);
+  bool planes_ready = false;
+  if ((e = assemble_stage(p, w, n, o.precision, &info, s, &planes_ready))) return e;
+  std::unique_ptr<Pending> h(new (std::nothrow) Pending{Timer(s), info, n, o.precision});
+  if (!h) return UPDES_ERR_CUDA;
+  if ((e = factor_launch(w, n, o.precision, s, planes_ready))) return e;
+  h->t.mark();
+  *pending = h.release();
+  return UPDES_OK;
+}
+
+extern "C" int updes_solve_end(void* pending, const updes_problem* p, const double* q, double* coeffs, double* vals,
+                               const updes_solve_opts* opts, updes_solve_info* info, void* workspace,
+                               size_t workspace_bytes, void* stream) {
+  if (!pending) return UPDES_ERR_INVALID;
+  std::unique_ptr<Pending> h(static_cast<Pending*>(pending));
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (!q) {  // given up: nothing of it runs any more when the call returns
+    UPDES_CUDA_TRY(cudaStreamSynchronize(s));
+    return UPDES_OK;
+  }
+  SolveWs w;
+  updes_solve_opts o;
+  int e = solve_setup(p, opts, workspace, workspace_bytes, &w, &o);
+  if (e) return e;
+  const int n = p->N + p->M;
+  if (!coeffs || n != h->n || o.precision != h->precision) return UPDES_ERR_INVALID;
+  updes_solve_info dummy;
+  if (!info) info = &dummy;
+  *info = h->info;
+  if ((e = factor_finish(w, n, o.precision, info, s, h->t))) return e;
+  if ((e = solve_stage(p, w, n, q, 1, coeffs, 1, vals, 1, o, info, s))) return e;
+  if (info->lu_info) return UPDES_ERR_SINGULAR;
+  if (!info->converged) return UPDES_ERR_NOT_CONVERGED;
+  return UPDES_OK;
 }
 
 extern "C" int updes_solve(const updes_problem* p, const double* q, double* coeffs, double* vals,
