@@ -1260,13 +1260,147 @@ __device__ __forceinline__ void df_div1(float bh, float bl, float d, float& qh, 
   ql = __fsub_rn(q2, __fsub_rn(qh, q1));
 }
 
-template <typename TF, int MODE>
-__global__ void __launch_bounds__(256) trsv_kernel(const TF* __restrict__ F, int64_t ldf, int n, double* x,
+// Triangular solve with FP64 factors: x_blk = T_bb^-1 (b - off-diagonal part), block after block along a chain of
+// n / 64 hand-overs, so its time is that chain's latency.  What does not need x comes before the wait: the
+// right-hand side, the diagonal block, and the division by its diagonal (rows scaled by the reciprocals, so a step of the
+// substitution is a shuffle and one multiply-add).  Behind the wait: the last off-diagonal tile (four threads a row:
+// 2,048 cycles of the SM's FP64 pipe, and nine additions a thread to sum a row), 32 rows by one warp, their part of the
+// other 32 by all eight, and those: 7.6 us a block.  With a row's sum over 32 lanes (5,100 cycles), the diagonal block and the
+// divisions behind the wait and two multiply-adds and a product a step it was 15.9.
+constexpr int kTrsv64Smem = (kTB * (kTB + 4) + kTB * (kTB + 1)) * 8;
+template <int MODE>
+__global__ void __launch_bounds__(256) trsv_f64_kernel(const double* __restrict__ F, int64_t ldf, int n, double* x,
+                                                       int* ticket, int* flags, DeviceStatus* st) {
+  extern __shared__ __align__(16) unsigned char trsv_smem[];
+  double(*sT)[kTB + 4] = reinterpret_cast<double(*)[kTB + 4]>(trsv_smem);  // four rows x four threads: distinct banks
+  double(*sD)[kTB + 1] = reinterpret_cast<double(*)[kTB + 1]>(sT + kTB);   // in the order of the solve
+  __shared__ double sx[kTB], sv[kTB], srd[kTB];
+  __shared__ int s_blk, s_done;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int row = tid >> 2, g = tid & 3;
+  const int nblk = int(ceil_div(n, kTB));
+  if (tid == 0) {
+    s_blk = atomicAdd(ticket, 1);
+    s_done = 0;
+  }
+  __syncthreads();
+  const int t = s_blk;
+  if (t >= nblk) return;
+  constexpr bool fwd = (MODE == 0 || MODE == 2), trans = (MODE >= 2), unit = (MODE == 0 || MODE == 3);
+  const int blk = fwd ? t : nblk - 1 - t;
+  const int r0 = blk * kTB;
+  const int rows = min(kTB, n - r0);
+  auto at = [&](int r) { return fwd ? r : kTB - 1 - r; };  // a row's place in the order of the solve (and back)
+  auto load_tile = [&](int c0, double (&pre)[16]) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int a = warp + 8 * (i >> 1), b = lane + 32 * (i & 1);  // row and column in F
+      const int64_t fr = (trans ? c0 : r0) + a, fc = (trans ? r0 : c0) + b;
+      pre[i] = fr < n && fc < n ? F[fr * ldf + fc] : 0.0;
+    }
+  };
+  const double b_own = row < rows ? x[r0 + row] : 0.0;
+  double pre[16];
+  load_tile(r0, pre);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int a = warp + 8 * (i >> 1), b = lane + 32 * (i & 1);
+    sD[at(trans ? b : a)][at(trans ? a : b)] = pre[i];
+  }
+  if (t > 0) load_tile((fwd ? 0 : nblk - 1) * kTB, pre);
+  if (!unit) {
+    __syncthreads();
+    if (tid < kTB) srd[tid] = at(tid) < rows ? 1.0 / sD[tid][tid] : 1.0;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int p = warp + 8 * (i >> 1), c = lane + 32 * (i & 1);
+      if (c < p) sD[p][c] *= srd[p];
+    }
+  }
+  // 32 partial sums a row, eight a thread: a long FP64 chain of n / 4 terms would round more than the sums of a warp's lanes
+  double acc[8] = {};
+  // Blocks finish in ticket order (each waits for all earlier ones), so flags[nblk] counts finished blocks: a CTA
+  // re-reads it only when it needs a block beyond the last count it saw.
+  for (int q = 0; q < t; ++q) {
+    const int c0 = (fwd ? q : nblk - 1 - q) * kTB;
+    __syncthreads();  // the previous tile has been used
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int a = warp + 8 * (i >> 1), b = lane + 32 * (i & 1);
+      sT[trans ? b : a][trans ? a : b] = pre[i];
+    }
+    if (q + 1 < t) load_tile((fwd ? q + 1 : nblk - 2 - q) * kTB, pre);
+    if (tid == 0 && s_done <= q) {
+      volatile int* vc = flags + nblk;
+      long long it = 0;
+      int d;
+      while ((d = *vc) <= q) {
+        if (++it > spin_limit()) {
+          status_error(st, UPDES_ERR_TIMEOUT);
+          atomicCAS(&st->timeout_tag, 0, 10 + MODE);
+          d = q + 1;
+          break;
+        }
+        __nanosleep(20);
+      }
+      __threadfence();
+      s_done = d;
+    }
+    __syncthreads();
+    if (tid < kTB) sx[tid] = c0 + tid < n ? __ldcg(x + c0 + tid) : 0.0;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) acc[i & 7] = fma(sT[row][g + 4 * i], sx[g + 4 * i], acc[i & 7]);
+  }
+  double sum = ((acc[0] + acc[1]) + (acc[2] + acc[3])) + ((acc[4] + acc[5]) + (acc[6] + acc[7]));
+  sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+  sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+  __syncthreads();  // sD and srd are complete
+  if (g == 0) {
+    const double v = b_own - sum;
+    sv[at(row)] = unit ? v : v * srd[at(row)];
+  }
+  __syncthreads();
+  auto solve32 = [&](int p0) {  // rows p0 .. p0 + 31 of the order, a lane each
+    double v = sv[p0 + lane];
+#pragma unroll
+    for (int i = 0; i < 31; ++i) {
+      const double xi = __shfl_sync(0xffffffffu, v, i);
+      const double u = fma(-sD[p0 + lane][p0 + i], xi, v);
+      if (lane > i) v = u;
+    }
+    sv[p0 + lane] = v;
+    const int r = at(p0 + lane);
+    if (r < rows) x[r0 + r] = v;
+  };
+  if (warp == 0) solve32(0);
+  __syncthreads();
+  {
+    const int p = 32 + (tid >> 3), h = tid & 7;
+    double a = 0.0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a = fma(sD[p][h + 8 * i], sv[h + 8 * i], a);
+#pragma unroll
+    for (int o = 1; o <= 4; o <<= 1) a += __shfl_xor_sync(0xffffffffu, a, o);
+    if (h == 0) sv[p] -= a;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    solve32(32);
+    __threadfence();
+    __syncwarp();
+    if (lane == 0) atomicAdd(flags + nblk, 1);  // blocks finish in order: this is block number t
+  }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(256) trsv_kernel(const float* __restrict__ F, int64_t ldf, int n, double* x,
                                                    int* ticket, int* flags, DeviceStatus* st,
                                                    const float* __restrict__ dinv) {
   extern __shared__ __align__(16) unsigned char trsv_smem[];
-  TF(*sT)[kTB + 1] = reinterpret_cast<TF(*)[kTB + 1]>(trsv_smem);
-  double* sxd = reinterpret_cast<double*>(trsv_smem + sizeof(TF) * kTB * (kTB + 1));  // 64
+  float(*sT)[kTB + 1] = reinterpret_cast<float(*)[kTB + 1]>(trsv_smem);
+  double* sxd = reinterpret_cast<double*>(trsv_smem + sizeof(float) * kTB * (kTB + 1));  // 64
   float* sxh = reinterpret_cast<float*>(sxd + kTB);                                    // 64
   float* sxl = sxh + kTB;                                                              // 64
   double* sacc = reinterpret_cast<double*>(sxl + kTB);                                 // 64
@@ -1287,7 +1421,7 @@ __global__ void __launch_bounds__(256) trsv_kernel(const TF* __restrict__ F, int
   // inputs that no other block writes, fetched before any wait: this block's right-hand side and, with
   // dinv, its inverted diagonal block (modes 2 and 3 use the transposes of the U and L inverses)
   const double b_own = (tid < rows) ? x[r0 + tid] : 0.0;
-  if constexpr (sizeof(TF) == 4) {
+  {
     if (dinv) {
       constexpr int which = (MODE == 0 || MODE == 3) ? 0 : 1;  // 0: inv(L_bb), 1: inv(U_bb)
       constexpr bool tr = (MODE >= 2);
@@ -1302,12 +1436,12 @@ __global__ void __launch_bounds__(256) trsv_kernel(const TF* __restrict__ F, int
     }
   }
 
-  auto load_tile = [&](int c0, TF (&pre)[16]) {
+  auto load_tile = [&](int c0, float (&pre)[16]) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       const int e = tid + 256 * i;
       const int a = e >> 6, b = e & 63;  // a: source row in the tile, b: source column
-      TF v = TF(0);
+      float v = 0.f;
       if (!trans) {
         if (r0 + a < n && c0 + b < n) v = F[int64_t(r0 + a) * ldf + c0 + b];
       } else {
@@ -1316,7 +1450,7 @@ __global__ void __launch_bounds__(256) trsv_kernel(const TF* __restrict__ F, int
       pre[i] = v;
     }
   };
-  auto store_tile = [&](const TF (&pre)[16]) {
+  auto store_tile = [&](const float (&pre)[16]) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       const int e = tid + 256 * i;
@@ -1328,10 +1462,9 @@ __global__ void __launch_bounds__(256) trsv_kernel(const TF* __restrict__ F, int
 
   // per-warp rows w*8 .. w*8+7, lane columns lane, lane+32
   float ah[8], al[8];
-  double ad[8];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) { ah[i] = 0.f; al[i] = 0.f; ad[i] = 0.0; }
-  TF pre[16];
+  for (int i = 0; i < 8; ++i) { ah[i] = 0.f; al[i] = 0.f; }
+  float pre[16];
   if (t > 0) load_tile((fwd ? 0 : nblk - 1) * kTB, pre);
   // Blocks finish in ticket order (each waits for all earlier ones), so flags[nblk] counts finished
   // blocks: a CTA re-reads it only when it needs a block beyond the last count it saw.
@@ -1374,13 +1507,12 @@ __global__ void __launch_bounds__(256) trsv_kernel(const TF* __restrict__ F, int
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
         const int cc = lane + 32 * h;
-        if constexpr (sizeof(TF) == 4) df_fma(float(sT[rr][cc]), sxh[cc], sxl[cc], ah[i], al[i]);
-        else ad[i] = fma(double(sT[rr][cc]), sxd[cc], ad[i]);
+        df_fma(sT[rr][cc], sxh[cc], sxl[cc], ah[i], al[i]);
       }
     }
     __syncthreads();
   }
-  if constexpr (sizeof(TF) == 4) {
+  {
     if (dinv) {
       // row sums of the off-diagonal part in double-float (FP32 pipes), kept as two FP32 words
       float* sacc_h = reinterpret_cast<float*>(sacc);
@@ -1446,22 +1578,19 @@ __global__ void __launch_bounds__(256) trsv_kernel(const TF* __restrict__ F, int
   // row sums of the off-diagonal part
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    double v = (sizeof(TF) == 4) ? double(ah[i]) + double(al[i]) : ad[i];
+    double v = double(ah[i]) + double(al[i]);
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     if (lane == 0) sacc[warp * 8 + i] = v;
   }
   // diagonal block
   {
-    TF dpre[16];
+    float dpre[16];
     load_tile(r0, dpre);
     store_tile(dpre);
   }
   __syncthreads();
-  __shared__ double s_rdiag[kTB];
   constexpr bool unit = (MODE == 0 || MODE == 3);
-  if (sizeof(TF) == 8 && !unit && tid < rows) s_rdiag[tid] = 1.0 / double(sT[tid][tid]);
-  __syncthreads();
-  if (sizeof(TF) == 4 && tid < 32) {
+  if (tid < 32) {
     // FP32 factors: the same column-oriented substitution in double-float arithmetic on the FP32 pipes
     // (one warp's FP64 instructions would serialise on the SM's few FP64 units)
     float v0h = 0.f, v0l = 0.f, v1h = 0.f, v1l = 0.f;
@@ -1491,26 +1620,6 @@ __global__ void __launch_bounds__(256) trsv_kernel(const TF* __restrict__ F, int
     }
     if (tid < rows) x[r0 + tid] = double(v0h) + double(v0l);
     if (tid + 32 < rows) x[r0 + tid + 32] = double(v1h) + double(v1l);
-  } else if (sizeof(TF) == 8 && tid < 32) {
-    // column-oriented substitution: lane owns rows lane and lane+32; x_i is broadcast by one shuffle and
-    // every unsolved row is updated right away (no global loads on the dependent chain)
-    double v0 = 0.0, v1 = 0.0;
-    if (tid < rows) v0 = x[r0 + tid] - sacc[tid];
-    if (tid + 32 < rows) v1 = x[r0 + tid + 32] - sacc[tid + 32];
-    for (int s2 = 0; s2 < rows; ++s2) {
-      const int i = fwd ? s2 : rows - 1 - s2;
-      double xi = __shfl_sync(0xffffffffu, (i >> 5) ? v1 : v0, i & 31);
-      if (!unit) xi *= s_rdiag[i];
-      if ((i & 31) == tid) {
-        if (i >> 5) v1 = xi;
-        else v0 = xi;
-      }
-      const int ra = tid, rb = tid + 32;
-      if (fwd ? ra > i : ra < i) v0 -= double(sT[ra][i]) * xi;
-      if (rb < rows && (fwd ? rb > i : rb < i)) v1 -= double(sT[rb][i]) * xi;
-    }
-    if (tid < rows) x[r0 + tid] = v0;
-    if (tid + 32 < rows) x[r0 + tid + 32] = v1;
   }
   __syncthreads();
   if (tid == 0) {
@@ -1986,8 +2095,23 @@ int trsv_impl(int n, const TF* F, int64_t ldf, double* x, int mode, int* sync_ws
   UPDES_CUDA_TRY(cudaMemsetAsync(sync_ws, 0, sizeof(int) * (nblk + 2), s));
   int* ticket = sync_ws;
   int* flags = sync_ws + 1;
-  if (sizeof(TF) != 4) dinv = nullptr;
-  if constexpr (sizeof(TF) == 4) {
+  if constexpr (sizeof(TF) == 8) {
+    static std::atomic<unsigned long long> attr64[4] = {};
+    int e;
+    if ((e = smem_opt_in((const void*)trsv_f64_kernel<0>, kTrsv64Smem, attr64[0])) ||
+        (e = smem_opt_in((const void*)trsv_f64_kernel<1>, kTrsv64Smem, attr64[1])) ||
+        (e = smem_opt_in((const void*)trsv_f64_kernel<2>, kTrsv64Smem, attr64[2])) ||
+        (e = smem_opt_in((const void*)trsv_f64_kernel<3>, kTrsv64Smem, attr64[3])))
+      return e;
+    switch (mode) {
+      case 0: trsv_f64_kernel<0><<<nblk, 256, kTrsv64Smem, s>>>(F, ldf, n, x, ticket, flags, st); break;
+      case 1: trsv_f64_kernel<1><<<nblk, 256, kTrsv64Smem, s>>>(F, ldf, n, x, ticket, flags, st); break;
+      case 2: trsv_f64_kernel<2><<<nblk, 256, kTrsv64Smem, s>>>(F, ldf, n, x, ticket, flags, st); break;
+      default: trsv_f64_kernel<3><<<nblk, 256, kTrsv64Smem, s>>>(F, ldf, n, x, ticket, flags, st); break;
+    }
+    UPDES_LAUNCH_CHECK();
+    return UPDES_OK;
+  } else {
     if (dinv && xh && xl) {
       // UPDES_TRSV_BLOCK=64 selects the 64-row kernel
       static const bool rows128 = [] {
@@ -2045,27 +2169,27 @@ int trsv_impl(int n, const TF* F, int64_t ldf, double* x, int mode, int* sync_ws
       UPDES_LAUNCH_CHECK();
       return UPDES_OK;
     }
+    const size_t smem =
+        sizeof(float) * kTB * (kTB + 1) + kTB * (8 + 4 + 4 + 8) + (dinv ? 2 * sizeof(float) * kTB * (kTB + 1) : 0);
+    {
+      const int big = int(sizeof(float) * kTB * (kTB + 1) + kTB * 24 + 2 * sizeof(float) * kTB * (kTB + 1));
+      static std::atomic<unsigned long long> attr[4] = {};
+      int e;
+      if ((e = smem_opt_in((const void*)trsv_kernel<0>, big, attr[0])) ||
+          (e = smem_opt_in((const void*)trsv_kernel<1>, big, attr[1])) ||
+          (e = smem_opt_in((const void*)trsv_kernel<2>, big, attr[2])) ||
+          (e = smem_opt_in((const void*)trsv_kernel<3>, big, attr[3])))
+        return e;
+    }
+    switch (mode) {
+      case 0: trsv_kernel<0><<<nblk, 256, smem, s>>>(F, ldf, n, x, ticket, flags, st, dinv); break;
+      case 1: trsv_kernel<1><<<nblk, 256, smem, s>>>(F, ldf, n, x, ticket, flags, st, dinv); break;
+      case 2: trsv_kernel<2><<<nblk, 256, smem, s>>>(F, ldf, n, x, ticket, flags, st, dinv); break;
+      default: trsv_kernel<3><<<nblk, 256, smem, s>>>(F, ldf, n, x, ticket, flags, st, dinv); break;
+    }
+    UPDES_LAUNCH_CHECK();
+    return UPDES_OK;
   }
-  const size_t smem =
-      sizeof(TF) * kTB * (kTB + 1) + kTB * (8 + 4 + 4 + 8) + (dinv ? 2 * sizeof(float) * kTB * (kTB + 1) : 0);
-  {
-    const int big = int(sizeof(TF) * kTB * (kTB + 1) + kTB * 24 + 2 * sizeof(float) * kTB * (kTB + 1));
-    static std::atomic<unsigned long long> attr[4] = {};
-    int e;
-    if ((e = smem_opt_in((const void*)trsv_kernel<TF, 0>, big, attr[0])) ||
-        (e = smem_opt_in((const void*)trsv_kernel<TF, 1>, big, attr[1])) ||
-        (e = smem_opt_in((const void*)trsv_kernel<TF, 2>, big, attr[2])) ||
-        (e = smem_opt_in((const void*)trsv_kernel<TF, 3>, big, attr[3])))
-      return e;
-  }
-  switch (mode) {
-    case 0: trsv_kernel<TF, 0><<<nblk, 256, smem, s>>>(F, ldf, n, x, ticket, flags, st, dinv); break;
-    case 1: trsv_kernel<TF, 1><<<nblk, 256, smem, s>>>(F, ldf, n, x, ticket, flags, st, dinv); break;
-    case 2: trsv_kernel<TF, 2><<<nblk, 256, smem, s>>>(F, ldf, n, x, ticket, flags, st, dinv); break;
-    default: trsv_kernel<TF, 3><<<nblk, 256, smem, s>>>(F, ldf, n, x, ticket, flags, st, dinv); break;
-  }
-  UPDES_LAUNCH_CHECK();
-  return UPDES_OK;
 }
 
 template int trsv_impl<double>(int, const double*, int64_t, double*, int, int*, DeviceStatus*, cudaStream_t,
