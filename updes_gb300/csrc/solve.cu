@@ -195,26 +195,6 @@ __global__ void __launch_bounds__(256) gemv_kernel(const double* __restrict__ K,
   }
 }
 
-// partial maxima of |r_i| / a_i (a_i = 0 with r_i = 0 counts as 0)
-__global__ void bwd_partial_kernel(const double* __restrict__ r, const double* __restrict__ a, int n,
-                                   double* __restrict__ partial) {
-  __shared__ double red[8];
-  double m = 0.0;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    const double rr = fabs(r[t]);
-    const double v = a[t] > 0.0 ? rr / a[t] : (rr > 0.0 ? INFINITY : 0.0);
-    m = fmax(m, v != v ? INFINITY : v);
-  }
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    for (int q = 0; q < 8; ++q) t = fmax(t, red[q]);
-    partial[blockIdx.x] = t;
-  }
-}
-
 // Transposed: out_j = dc_j * (bsign * b_j + ksign * sum_i K_ij dr_i x_i), 256 columns per CTA.
 __global__ void __launch_bounds__(256) gemv_t_kernel(const double* __restrict__ K, int64_t ld, int n,
                                                      const double* __restrict__ x, const double* __restrict__ b,
@@ -348,34 +328,100 @@ constexpr double kBwdFloor = 256.0 * 1.1102230246251565e-16;
 // the floor comes first and one cycle of 10 iterations converges; 1e-10 and 1e-14 here measured the same).
 constexpr double kInnerReduction = 1e-6;
 
-// partial[b * nv + i] = sum over block b's chunk of V_i . w
-__global__ void __launch_bounds__(256) multi_dot_kernel(const double* __restrict__ V, int64_t ldv, int nv,
-                                                        const double* __restrict__ w, int n,
-                                                        double* __restrict__ partial) {
+// The last of a grid's CTAs to arrive here (every thread of the CTA gets the answer): it sees what the others wrote
+// before.  *cnt is 0 again afterwards.
+__device__ __forceinline__ bool last_cta(unsigned* cnt) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicInc(cnt, gridDim.x - 1) == gridDim.x - 1;
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+
+// One Gram-Schmidt pass and the sums that the next one needs: w -= V h_in (h_in null: w as it is), then out_i = V_i . w for
+// nv vectors or, with `norm`, out_0 = w . w, in one launch: a CTA per chunk of w, the last of them adds the chunks' sums.
+// At n = 600 an iteration is mostly such launches (as a product, a sum of its parts and an update each, with the host
+// reading three sums, 8 launches and 3 waits; now 3 and 1).
+__global__ void __launch_bounds__(256) gram_schmidt_kernel(const double* __restrict__ V, int64_t ldv, int nv,
+                                                           const double* __restrict__ h_in, double* w, int n, bool norm,
+                                                           double* partial, unsigned* cnt, double* out) {
   __shared__ double red[8];
   const int chunk = int(ceil_div(n, gridDim.x));
   const int lo = blockIdx.x * chunk, hi = min(n, lo + chunk);
-  for (int i = 0; i < nv; ++i) {
+  if (h_in)
+    for (int t = lo + threadIdx.x; t < hi; t += blockDim.x) {
+      double s = 0.0;
+      for (int i = 0; i < nv; ++i) s = fma(h_in[i], V[int64_t(i) * ldv + t], s);
+      w[t] -= s;
+    }
+  const int nd = norm ? 1 : nv;
+  for (int i = 0; i < nd; ++i) {
     double s = 0.0;
-    for (int t = lo + threadIdx.x; t < hi; t += blockDim.x) s = fma(V[int64_t(i) * ldv + t], w[t], s);
+    for (int t = lo + threadIdx.x; t < hi; t += blockDim.x) s = fma(norm ? w[t] : V[int64_t(i) * ldv + t], w[t], s);
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
     __syncthreads();
     if (threadIdx.x == 0) {
       double t = 0.0;
       for (int q = 0; q < 8; ++q) t += red[q];
-      partial[blockIdx.x * nv + i] = t;
+      partial[blockIdx.x * nd + i] = t;
     }
     __syncthreads();
   }
+  if (!last_cta(cnt)) return;
+  for (int i = threadIdx.x >> 5; i < nd; i += 8) {
+    double s = 0.0;
+    for (int b = threadIdx.x & 31; b < gridDim.x; b += 32) s += __ldcg(partial + b * nd + i);
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) out[i] = s;
+  }
 }
 
-__global__ void reduce_partials_kernel(const double* __restrict__ partial, int nblocks, int nv, double* __restrict__ h) {
-  const int i = threadIdx.x;
-  if (i >= nv) return;
-  double s = 0.0;
-  for (int b = 0; b < nblocks; ++b) s += partial[b * nv + i];
-  h[i] = s;
+// r <- b + r (r holds -K x), and out = {max_i |r_i| / (|K||x| + |b|)_i, r . r, b . b}, the last CTA as above.
+__global__ void __launch_bounds__(256) residual_kernel(double* r, const double* __restrict__ b,
+                                                       const double* __restrict__ absr, const double* __restrict__ bsabs,
+                                                       int n, double* partial, unsigned* cnt, double* out) {
+  __shared__ double red[3][8];
+  double m = 0.0, rr = 0.0, bb = 0.0;
+  auto reduce = [&] {
+    for (int o = 16; o > 0; o >>= 1) {
+      m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+      rr += __shfl_xor_sync(0xffffffffu, rr, o);
+      bb += __shfl_xor_sync(0xffffffffu, bb, o);
+    }
+  };
+  const int chunk = int(ceil_div(n, gridDim.x));
+  const int lo = blockIdx.x * chunk, hi = min(n, lo + chunk);
+  for (int t = lo + threadIdx.x; t < hi; t += blockDim.x) {
+    const double bv = b[t], v = bv + r[t], a = bsabs[t] + absr[t];
+    r[t] = v;
+    const double q = a > 0.0 ? fabs(v) / a : (fabs(v) > 0.0 ? INFINITY : 0.0);
+    m = fmax(m, q != q ? INFINITY : q);
+    rr = fma(v, v, rr);
+    bb = fma(bv, bv, bb);
+  }
+  reduce();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (lane == 0) { red[0][wid] = m; red[1][wid] = rr; red[2][wid] = bb; }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    m = rr = bb = 0.0;
+    for (int q = 0; q < 8; ++q) { m = fmax(m, red[0][q]); rr += red[1][q]; bb += red[2][q]; }
+    partial[blockIdx.x * 3] = m;
+    partial[blockIdx.x * 3 + 1] = rr;
+    partial[blockIdx.x * 3 + 2] = bb;
+  }
+  if (!last_cta(cnt) || wid != 0) return;
+  m = rr = bb = 0.0;
+  for (int c = lane; c < gridDim.x; c += 32) {
+    m = fmax(m, __ldcg(partial + c * 3));
+    rr += __ldcg(partial + c * 3 + 1);
+    bb += __ldcg(partial + c * 3 + 2);
+  }
+  reduce();
+  if (lane == 0) { out[0] = m; out[1] = rr; out[2] = bb; }
 }
 
 // w += sign * sum_i h_i V_i ; if out != null writes there instead of w (out = sign * sum_i h_i V_i)
@@ -572,13 +618,13 @@ int factor_core(int n, double* A, int64_t lda, int precision, void* F, int64_t l
 
 // x (contiguous, n) <- A^-1 x or A^-T x using the permutation in piv[n, 2n)
 template <typename TF>
-int solve_core(int n, const TF* F, int64_t ldf, const int32_t* piv, double* x, int trans, const LuWs& w,
+int solve_core(int n, const TF* F, int64_t ldf, const int32_t* piv, const double* b, double* x, int trans, const LuWs& w,
                cudaStream_t s, const float* dinv = nullptr, float* xh = nullptr, float* xl = nullptr,
                const float* dinv128 = nullptr, unsigned long long* xtag = nullptr) {
   const int32_t* perm = piv + n;
   const unsigned g = unsigned(ceil_div(n, 256));
   if (!trans) {
-    permute_kernel<<<g, 256, 0, s>>>(w.tmp, x, 1, 1, perm, n, 0);
+    permute_kernel<<<g, 256, 0, s>>>(w.tmp, b, 1, 1, perm, n, 0);
     UPDES_LAUNCH_CHECK();
     int e = trsv_impl<TF>(n, F, ldf, w.tmp, 0, w.sync, w.st, s, dinv, xh, xl, dinv128, xtag);
     if (e) return e;
@@ -586,7 +632,7 @@ int solve_core(int n, const TF* F, int64_t ldf, const int32_t* piv, double* x, i
     if (e) return e;
     UPDES_CUDA_TRY(cudaMemcpyAsync(x, w.tmp, size_t(n) * 8, cudaMemcpyDeviceToDevice, s));
   } else {
-    UPDES_CUDA_TRY(cudaMemcpyAsync(w.tmp, x, size_t(n) * 8, cudaMemcpyDeviceToDevice, s));
+    UPDES_CUDA_TRY(cudaMemcpyAsync(w.tmp, b, size_t(n) * 8, cudaMemcpyDeviceToDevice, s));
     int e = trsv_impl<TF>(n, F, ldf, w.tmp, 2, w.sync, w.st, s, dinv, xh, xl, dinv128, xtag);
     if (e) return e;
     e = trsv_impl<TF>(n, F, ldf, w.tmp, 3, w.sync, w.st, s, dinv, xh, xl, dinv128, xtag);
@@ -599,8 +645,8 @@ int solve_core(int n, const TF* F, int64_t ldf, const int32_t* piv, double* x, i
 
 int solve_any(int n, const void* F, int64_t ldf, int precision, const int32_t* piv, double* x, int trans,
               const LuWs& w, cudaStream_t s) {
-  if (precision == UPDES_PREC_FP64) return solve_core<double>(n, static_cast<const double*>(F), ldf, piv, x, trans, w, s);
-  return solve_core<float>(n, static_cast<const float*>(F), ldf, piv, x, trans, w, s);
+  if (precision == UPDES_PREC_FP64) return solve_core<double>(n, static_cast<const double*>(F), ldf, piv, x, x, trans, w, s);
+  return solve_core<float>(n, static_cast<const float*>(F), ldf, piv, x, x, trans, w, s);
 }
 
 }  // namespace
@@ -679,6 +725,7 @@ struct SolveWs {
   LuWs lu;
   double *W, *dr, *dc, *bs, *bsabs, *absr, *x, *r, *z, *wv, *V, *Z, *partial, *h;
   double* evp;  // per-tile partial sums of the symmetric value evaluation
+  unsigned* cnt;  // CTAs that have arrived at the end of a reduction (0 between them)
   float *Khi, *Klo;  // equilibrated K as double-float planes (kept for the refinement's residuals)
   float *xh, *xl;    // FP32 planes of the vector a GEMV multiplies
   float* F32;  // hi plane = FP32 factors
@@ -723,7 +770,8 @@ size_t solve_ws_layout(int n, const updes_solve_opts& o, char* base, SolveWs* ou
   const int m = o.restart > 0 ? o.restart : 1;
   w.V = c.take<double>(size_t(m + 1) * n);
   w.partial = c.take<double>(size_t(kDotBlocks) * (m + 2));
-  w.h = c.take<double>(m + 2);
+  w.h = c.take<double>(2 * (m + 2));  // two passes' coefficients and a norm, or a residual's three sums
+  w.cnt = c.take<unsigned>(64);
   w.xtag = c.take<unsigned long long>(2 * size_t(n));
   w.Z = c.take<double>(size_t(m) * n);  // preconditioned basis vectors M^-1 V_j of a restart cycle
   if (out) *out = w;
@@ -748,19 +796,6 @@ updes_solve_opts normalise(const updes_solve_opts* o) {
 }
 
 // h[0..nv) = V[0..nv)^T w (device), then copied to host
-int multi_dot(const double* V, int64_t ldv, int nv, const double* w, int n, double* partial, double* h_dev,
-              double* h_host, cudaStream_t s) {
-  multi_dot_kernel<<<kDotBlocks, 256, 0, s>>>(V, ldv, nv, w, n, partial);
-  UPDES_LAUNCH_CHECK();
-  reduce_partials_kernel<<<1, 256, 0, s>>>(partial, kDotBlocks, nv, h_dev);
-  UPDES_LAUNCH_CHECK();
-  if (h_host) {
-    UPDES_CUDA_TRY(cudaMemcpyAsync(h_host, h_dev, nv * sizeof(double), cudaMemcpyDeviceToHost, s));
-    UPDES_CUDA_TRY(cudaStreamSynchronize(s));
-  }
-  return UPDES_OK;
-}
-
 struct Timer {
   cudaEvent_t a, b;
   cudaStream_t s;
@@ -811,30 +846,21 @@ int apply_K(const SolveWs& w, int n, const double* z, double* out, cudaStream_t 
   return gemv_scaled(w, n, z, 1.0, out, nullptr, s, trans);
 }
 
-// out = bs - Ks x; also returns (on the host) the componentwise backward error
-// max_i |out_i| / (|Ks| |x| + |bs|)_i.
-int residual_scaled(const SolveWs& w, int n, const double* x, double* out, double* bwd, cudaStream_t s,
+// out = bs - Ks x; on the host, sums = {the componentwise backward error max_i |out_i| / (|Ks| |x| + |bs|)_i, ||out||^2,
+// ||bs||^2}.
+int residual_scaled(const SolveWs& w, int n, const double* x, double* out, double* sums, cudaStream_t s,
                     bool trans = false) {
-  int e0 = gemv_scaled(w, n, x, -1.0, out, w.absr, s, trans);
-  if (e0) return e0;
-  axpby_kernel<<<unsigned(ceil_div(n, 256)), 256, 0, s>>>(out, 1.0, w.bs, 1.0, n, nullptr);
+  if (int e = gemv_scaled(w, n, x, -1.0, out, w.absr, s, trans)) return e;
+  residual_kernel<<<kDotBlocks, 256, 0, s>>>(out, w.bs, w.absr, w.bsabs, n, w.partial, w.cnt, w.h);
   UPDES_LAUNCH_CHECK();
-  axpby_kernel<<<unsigned(ceil_div(n, 256)), 256, 0, s>>>(w.absr, 1.0, w.bsabs, 1.0, n, nullptr);
-  UPDES_LAUNCH_CHECK();
-  bwd_partial_kernel<<<kDotBlocks, 256, 0, s>>>(out, w.absr, n, w.partial);
-  UPDES_LAUNCH_CHECK();
-  std::vector<double> part(kDotBlocks);
-  UPDES_CUDA_TRY(cudaMemcpyAsync(part.data(), w.partial, kDotBlocks * sizeof(double), cudaMemcpyDeviceToHost, s));
+  UPDES_CUDA_TRY(cudaMemcpyAsync(sums, w.h, 3 * sizeof(double), cudaMemcpyDeviceToHost, s));
   UPDES_CUDA_TRY(cudaStreamSynchronize(s));
-  double m = 0.0;
-  for (double v : part) m = std::fmax(m, v);
-  *bwd = m;
   return UPDES_OK;
 }
 
-int precond(const SolveWs& w, int n, int precision, double* x, cudaStream_t s, bool trans = false) {
-  if (precision == UPDES_PREC_FP64) return solve_core<double>(n, w.W, w.ld, w.piv, x, trans ? 1 : 0, w.lu, s);
-  return solve_core<float>(n, w.F32, w.ld, w.piv, x, trans ? 1 : 0, w.lu, s, w.dinv, w.xh, w.xl, w.dinv128,
+int precond(const SolveWs& w, int n, int precision, const double* b, double* x, cudaStream_t s, bool trans = false) {
+  if (precision == UPDES_PREC_FP64) return solve_core<double>(n, w.W, w.ld, w.piv, b, x, trans ? 1 : 0, w.lu, s);
+  return solve_core<float>(n, w.F32, w.ld, w.piv, b, x, trans ? 1 : 0, w.lu, s, w.dinv, w.xh, w.xl, w.dinv128,
                            w.xtag);
 }
 
@@ -859,19 +885,15 @@ int gmres(const SolveWs& w, int n, int precision, const updes_solve_opts& o, upd
           cudaStream_t s, bool trans = false) {
   const int m = o.restart;
   const unsigned g = unsigned(ceil_div(n, 256));
-  std::vector<double> H(size_t(m + 1) * m), cs(m), sn(m), gv(m + 1), hcol(m + 2);
-  double bnorm2;
-  int e = multi_dot(w.bs, n, 1, w.bs, n, w.partial, w.h, &bnorm2, s);
-  if (e) return e;
-  const double bnorm = std::sqrt(bnorm2);
+  std::vector<double> H(size_t(m + 1) * m), cs(m), sn(m), gv(m + 1), hcol(m + 2), hh(2 * m + 1);
+  int e;
+  UPDES_CUDA_TRY(cudaMemsetAsync(w.cnt, 0, sizeof(unsigned), s));
   int total = 0, stalls = 0;
   double last_beta = INFINITY;
   for (;;) {
-    double bwd;
-    if ((e = residual_scaled(w, n, w.x, w.r, &bwd, s, trans))) return e;
-    double beta2;
-    if ((e = multi_dot(w.r, n, 1, w.r, n, w.partial, w.h, &beta2, s))) return e;
-    const double beta = std::sqrt(beta2);
+    double sums[3];
+    if ((e = residual_scaled(w, n, w.x, w.r, sums, s, trans))) return e;
+    const double bwd = sums[0], beta = std::sqrt(sums[1]), bnorm = std::sqrt(sums[2]);
     info->rel_residual = bnorm > 0 ? beta / bnorm : beta;
     info->backward_error = bwd;
     if (trace_on())
@@ -903,21 +925,19 @@ int gmres(const SolveWs& w, int n, int precision, const updes_solve_opts& o, upd
       // z_j = M^-1 v_j is kept (flexible GMRES form): the cycle's update is then Z y, with no further solve
       double* vj = w.V + size_t(j) * n;
       double* zj = w.Z + size_t(j) * n;
-      UPDES_CUDA_TRY(cudaMemcpyAsync(zj, vj, size_t(n) * 8, cudaMemcpyDeviceToDevice, s));
-      if ((e = precond(w, n, precision, zj, s, trans))) return e;
+      if ((e = precond(w, n, precision, vj, zj, s, trans))) return e;
       if ((e = apply_K(w, n, zj, w.wv, s, trans))) return e;
-      // CGS2
-      std::fill(hcol.begin(), hcol.end(), 0.0);
-      for (int pass = 0; pass < 2; ++pass) {
-        std::vector<double> hh(j + 1);
-        if ((e = multi_dot(w.V, n, j + 1, w.wv, n, w.partial, w.h, hh.data(), s))) return e;
-        multi_axpy_kernel<<<g, 256, 0, s>>>(w.V, n, j + 1, w.h, -1.0, w.wv, nullptr, n);
+      // CGS2: the two passes' coefficients and the norm of what is left, read together
+      const int nv = j + 1;
+      for (int pass = 0; pass < 3; ++pass) {
+        gram_schmidt_kernel<<<kDotBlocks, 256, 0, s>>>(w.V, n, nv, pass ? w.h + (pass - 1) * nv : nullptr, w.wv, n,
+                                                       pass == 2, w.partial, w.cnt, w.h + pass * nv);
         UPDES_LAUNCH_CHECK();
-        for (int i = 0; i <= j; ++i) hcol[i] += hh[i];
       }
-      double hn2;
-      if ((e = multi_dot(w.wv, n, 1, w.wv, n, w.partial, w.h, &hn2, s))) return e;
-      const double hn = std::sqrt(hn2);
+      UPDES_CUDA_TRY(cudaMemcpyAsync(hh.data(), w.h, (2 * nv + 1) * sizeof(double), cudaMemcpyDeviceToHost, s));
+      UPDES_CUDA_TRY(cudaStreamSynchronize(s));
+      for (int i = 0; i < nv; ++i) hcol[i] = hh[i] + hh[nv + i];
+      const double hn = std::sqrt(hh[2 * nv]);
       hcol[j + 1] = hn;
       if (hn > 0) {
         axpby_kernel<<<g, 256, 0, s>>>(w.V + size_t(j + 1) * n, 1.0 / hn, w.wv, 0.0, n, nullptr);
@@ -1132,8 +1152,7 @@ int solve_stage(const updes_problem* p, const SolveWs& w, int n, const double* q
     }
     abs_kernel<<<g, 256, 0, s>>>(w.bs, w.bsabs, n);
     UPDES_LAUNCH_CHECK();
-    UPDES_CUDA_TRY(cudaMemcpyAsync(w.x, w.bs, size_t(n) * 8, cudaMemcpyDeviceToDevice, s));
-    if ((e = precond(w, n, precision, w.x, s))) return e;
+    if ((e = precond(w, n, precision, w.bs, w.x, s))) return e;
     updes_solve_opts oi = o;
     if (precision == UPDES_PREC_FP64) oi.max_iters = 0;  // plain FP64 LU: report the residual only
     if ((e = gmres(w, n, precision, oi, info, s))) return e;
@@ -1470,7 +1489,7 @@ extern "C" int updes_solve_transpose(const updes_problem* p, const double* g, do
   UPDES_LAUNCH_CHECK();
   UPDES_CUDA_TRY(cudaMemcpyAsync(w.x, w.bs, size_t(n) * 8, cudaMemcpyDeviceToDevice, s));
   int e;
-  if ((e = precond(w, n, precision, w.x, s, true))) return e;
+  if ((e = precond(w, n, precision, w.x, w.x, s, true))) return e;
   updes_solve_opts oi = o;
   if (precision == UPDES_PREC_FP64) oi.max_iters = 0;
   if ((e = gmres(w, n, precision, oi, info, s, true))) return e;
