@@ -31,18 +31,18 @@ constexpr int kChunk = 256;  // value rows staged at a time
 
 __device__ __forceinline__ float2 sub2(float2 y, float2 x) { return __ffma2_rn(x, make_float2(-1.f, -1.f), y); }
 
-// Double-float accumulators of a pair of columns: (sh, sl) += (a + al) * (b + bl), dropping al * bl; renormalised.
-// Packed FP32x2 instructions, one issue slot a pair.
-__device__ __forceinline__ void df_mac2(float a, float al, float2 b, float2 bl, float2& sh, float2& sl) {
+// Double-float accumulators of a pair of columns: (sh, sl) += (a + al) * (b + bl), dropping al * bl; nb = -b.  Packed
+// FP32x2 instructions, 12 of them: the negated product comes from the negated operand (a negation of a pair costs two
+// more), and the pair is renormalised by its owner after a few terms.
+__device__ __forceinline__ void df_mac2(float a, float al, float2 b, float2 nb, float2 bl, float2& sh, float2& sl) {
   const float2 a2 = make_float2(a, a), al2 = make_float2(al, al);
-  const float2 p = __fmul2_rn(a2, b);
-  const float2 e = __ffma2_rn(a2, b, make_float2(-p.x, -p.y));
-  const float2 s = __fadd2_rn(sh, p);
+  const float2 np = __fmul2_rn(a2, nb);
+  const float2 e = __ffma2_rn(a2, b, np);
+  const float2 s = sub2(sh, np);
   const float2 bb = sub2(s, sh);
-  float2 t = __fadd2_rn(sub2(sh, sub2(s, bb)), sub2(p, bb));
-  t = __fadd2_rn(t, __fadd2_rn(sl, __ffma2_rn(a2, bl, __ffma2_rn(al2, b, e))));
-  sh = __fadd2_rn(s, t);
-  sl = sub2(t, sub2(sh, s));
+  const float2 t = sub2(sub2(sh, sub2(s, bb)), __fadd2_rn(np, bb));
+  sl = __fadd2_rn(sl, __fadd2_rn(t, __ffma2_rn(a2, bl, __ffma2_rn(al2, b, e))));
+  sh = s;
 }
 
 // (sh, sl) += (h, l)
@@ -225,6 +225,7 @@ __global__ void __launch_bounds__(256) tri_premultiply_kernel(const TF* __restri
 constexpr int kTriThreads = 512, kKs = 8;
 struct TriSmem {
   float F[2][2][kB][kLdt];   // [buffer][hi, lo]
+  float Xn[2][kB][kCG];  // the high words negated
   float Xh[2][kB][kCG], Xl[2][kB][kCG];
 };
 
@@ -316,6 +317,7 @@ __global__ void __launch_bounds__(kTriThreads) batch_tri_kernel(const float* __r
       }
     }
     sm.Xh[b][xr][xc] = __uint_as_float(uint32_t(pre.hi));
+    sm.Xn[b][xr][xc] = -__uint_as_float(uint32_t(pre.hi));
     sm.Xl[b][xr][xc] = __uint_as_float(uint32_t(pre.lo));
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
@@ -327,10 +329,17 @@ __global__ void __launch_bounds__(kTriThreads) batch_tri_kernel(const float* __r
     for (int k = 0; k < kB / kKs; ++k) {
       const int kk = kKs * k + ks;
       const float2 xh = *reinterpret_cast<const float2*>(&sm.Xh[b][kk][2 * cg]);
+      const float2 xn = *reinterpret_cast<const float2*>(&sm.Xn[b][kk][2 * cg]);
       const float2 xl = *reinterpret_cast<const float2*>(&sm.Xl[b][kk][2 * cg]);
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        df_mac2(sm.F[b][0][rg + 16 * u][kk], sm.F[b][1][rg + 16 * u][kk], xh, xl, ah[u], al[u]);
+        df_mac2(sm.F[b][0][rg + 16 * u][kk], sm.F[b][1][rg + 16 * u][kk], xh, xn, xl, ah[u], al[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {  // eight terms on: renormalised
+      const float2 s = __fadd2_rn(ah[u], al[u]);
+      al[u] = sub2(al[u], sub2(s, ah[u]));
+      ah[u] = s;
     }
   }
   // The sum over the eight threads of a row: each exchange also halves what a thread keeps, down to one row of a pair
