@@ -1089,6 +1089,10 @@ int lu_factor_df(int n, float* Whi, float* Wlo, int64_t ld, int32_t* piv, void* 
 // of 64).  The look-ahead is that of lu_factor_df: the next block on a second stream beside the update of the rest.
 namespace {
 constexpr int kNb64 = 32;
+// Up to this many trailing rows the next block's chain is longer than the update beside it, and its own updates (seven digit
+// planes) gain from 64 SMs instead of 32: n = 3,959 17.9 ms a factorisation against 18.4, 10,006 65.2 against 69.3, 20,000
+// 293 against 297 (with 64 throughout 299).  The mixed path's do not (10,006: 28.3 against 28.4, 22,506: 117 against 108).
+constexpr int kWideSideRows64 = 12288;
 constexpr int kMaps64 = kOuterNb / kNb64;
 }  // namespace
 
@@ -1181,7 +1185,6 @@ int lu_factor_64(int n, double* W, int64_t ld, int32_t* piv, void* ws, size_t ws
   SideStream side;
   int e;
   if (lookahead && (e = side.create(s))) return e;
-  const int rest_ctas = std::max(num_sms() - kLookaheadCtas, num_sms() / 2);
   int K0 = 0, KE = std::min(kOuterNb, n);
   if ((e = factor_block(K0, KE, s, false, 0))) return e;
   for (;;) {
@@ -1196,8 +1199,9 @@ int lu_factor_64(int n, double* W, int64_t ld, int32_t* piv, void* ws, size_t ws
     if ((e = upd(KE, n, KE, KE2, K0, KE, s, false, 0, !lookahead))) return e;
     if (lookahead && KE2 < n) {
       if ((e = side.start())) return e;
-      if ((e = factor_block(KE, KE2, side.side, true, kLookaheadCtas))) return e;
-      if ((e = upd(KE, n, KE2, n, K0, KE, s, false, rest_ctas, false))) return e;
+      const int side_ctas = std::min(n - KE <= kWideSideRows64 ? 2 * kLookaheadCtas : kLookaheadCtas, num_sms() / 2);
+      if ((e = factor_block(KE, KE2, side.side, true, side_ctas))) return e;
+      if ((e = upd(KE, n, KE2, n, K0, KE, s, false, num_sms() - side_ctas, false))) return e;
       if ((e = side.finish())) return e;
     } else {
       if (KE2 < n && (e = upd(KE, n, KE2, n, K0, KE, s, false, 0, !lookahead))) return e;
