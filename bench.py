@@ -294,8 +294,8 @@ def run_ours(args, world, rank, local):
     if dom == "trailing_update":
         # achieved counts the algorithmic flops of the updates, 2 m nc K per launch (the LU's (2/3) n^3 in
         # all), against the measured bf16 sustained peak of the tensor cores the update runs on (it runs
-        # inside a seconds-long step).  Each FP32 operand is written as 3 bf16 integer digits and 8 of the
-        # 3 x 3 digit products are exact tcgen05 MMAs (9 with UPDES_OZAKI=2): tensor_work_* count those.
+        # inside a seconds-long step).  Each FP32 operand is written as 3 FP16 numbers and 8 of the 3 x 3
+        # products are tcgen05 MMAs (9 of bf16 digits with UPDES_OZAKI=2): tensor_work_* count those.
         digit_products = 9 if os.environ.get("UPDES_OZAKI", "") == "2" else 8
         achieved = d["flops"] / (d["ms"] / 1000.0) / 1e12
         peak = peaks.get("bf16_tflops_sustained", 1700.0)
@@ -315,13 +315,13 @@ def run_ours(args, world, rank, local):
                  "measured_in": "a second pass of the same steps with per-launch CUDA events on each launch's "
                                 "stream (the timed region itself runs without them)"})
     # DRAM bytes (read + write) of the update per algorithmic byte (the double-float C planes read and
-    # written once plus the digit operands), from one ncu capture of the update kernel at this workload's size;
-    # applied to this run's average launch.  An estimate, named with its source.
-    dram_per_alg_byte = {"trailing_update": (8.3175e9 / 7.8752e9,
-                                             "ncu dram__bytes_read.sum + dram__bytes_write.sum of the largest "
-                                             "update launch at n = 22,506 (m = 22,250, nc = 21,994, K = 256; "
-                                             "UPDES_LOOKAHEAD=0, launch 8): 4.458 + 3.859 GB against 7.875 GB "
-                                             "algorithmic, scaled by this run's algorithmic bytes per launch")}
+    # written once plus the digit operands), from one ncu capture of the update kernel; applied to this run's
+    # average launch.  An estimate, named with its source.
+    dram_per_alg_byte = {"trailing_update": (1.5852e9 / 1.6205e9,
+                                             "ncu dram__bytes_read.sum + dram__bytes_write.sum of one update of "
+                                             "10,000 x 10,000 x 256 alone on the GPU: 0.836 + 0.749 GB against "
+                                             "1.62 GB algorithmic, scaled by this run's algorithmic bytes per "
+                                             "launch")}
     if dom in dram_per_alg_byte:
         ratio, src = dram_per_alg_byte[dom]
         roof["traffic"] = ratio * d["bytes"] / d["count"]
@@ -511,10 +511,10 @@ def _cfg_control(args, U, torch):
 
 def _cfg_uneven(args, U, torch):
     """Batched uneven clouds: 512 independent systems of 100 to 2,025 nodes.  Per-problem FP64 (each system
-    its own solve, 8 host-driven streams) against the persistent launch (one CTA per SM takes systems from a
-    device queue), mixed ("auto": double-float LU on the FP32 pipes + FP64 refinement, FP64 relaunch of the
+    its own solve, 8 host-driven streams) against one call (clusters and single CTAs take systems from
+    device queues), mixed ("auto": double-float LU on the FP32 pipes + FP64 refinement, FP64 relaunch of the
     systems that do not reach the FP64 floor) and FP64.  Wall clock includes host preparation; the
-    persistent launch's own device time is reported beside it."""
+    call's own device time is reported beside it."""
     from updes_gb300 import batched as B
     from updes_gb300 import workloads as WL
     out = {}

@@ -219,7 +219,7 @@ __global__ void __launch_bounds__(256) tri_premultiply_kernel(const TF* __restri
 // Tiles are staged by cp.async one ahead, and the words of a block are read one tile ahead of their use, so blocks
 // solved long ago cost no waiting.
 // Bound by the FP32 pipes for many columns (15 packed instructions per two double-float multiply-adds, which issue every
-// other cycle: 64 columns of n = 6,403 take 1.03 ms a triangle, 0.85 of it at that rate), by the chain for few (8
+// other cycle: 64 columns of n = 6,406 take 0.96 ms a triangle), by the chain for few (8
 // columns: 0.45 ms, 4.4 us a block).
 // A thread owns rows rg + 16 u (u < 4), the columns 2 cg and 2 cg + 1, and every eighth term of the inner sum.
 constexpr int kTriThreads = 512, kKs = 8;

@@ -19,13 +19,14 @@
 // 2^-29.1 (2^-36.4).  As a preconditioner the factors are the better for it: 7-8 iterations at n = 22,506 for 9-11.  The small
 // entries of a graded block matter to the Schur complement: with d1 cut at 2^-8 (g1 always exact) it took 14-25.
 //
-// What bounds it.  Shared memory: each tcgen05.mma reads both its operands from there, TMA writes them, and C passes
-// it four times, all at 128 bytes a clock.  The previous form (tiles of 128 x 64, 8 products, a fold of four
-// accumulators per 64 of K) moved 2.6 MB for a 128 x 128 x 256 piece, 21,000 clocks, and took 25,600.  So the tiles are
-// 128 x 128, the digit planes of B lie side by side so that one instruction of N = 256 forms d0 [e0 e1] in the
-// neighbouring accumulators [g0 g1] and another d1 [e0 e1] in [g1 g2] (A is read once for two products), and one scale
-// per K leaves one fold per tile: 1.8 MB, 14,400 clocks; 20,000 x 20,000 x 256 takes 1,300 us (15,400 clocks a piece)
-// against 2,165.  C without an eviction hint: evict-first costs 10 %.
+// What bounds it.  The previous form (tiles of 128 x 64, 8 products, a fold of four accumulators per 64 of K) moved 2.6 MB
+// through shared memory for a 128 x 128 x 256 piece and took 25,600 clocks.  So the tiles are 128 x 128, the digit planes
+// of B lie side by side so that one instruction of N = 256 forms d0 [e0 e1] in the neighbouring accumulators [g0 g1] and
+// another d1 [e0 e1] in [g1 g2] (A is read once for two products), and one scale per K leaves one fold per tile: 1.8 MB,
+// 15,400 clocks; 20,000 x 20,000 x 256 takes 1,310 us against 2,165.  Of these the products and the fold take 920 us without
+// C, C's way (load, update, store, a warp after another) 1,390 without most products: the warps' chain over their pieces
+// of C is what is left, with the tensor pipe 54 % and DRAM 60 % busy (n = 10,000).  C without an eviction hint: evict-first
+// costs 10 %; neither prefetching C to L2 nor storing it from registers gains.
 //
 // Structure.  A pre-pass writes the digits once per update, laid out as the stages hold them, and the scales.  The main
 // kernel is persistent (one CTA per SM, tiles of 128 x TN taken round robin) with three roles:
