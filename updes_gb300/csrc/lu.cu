@@ -304,6 +304,45 @@ struct TrsmDfCols {
 
 __device__ __forceinline__ float2 trsm_sub2(float2 y, float2 x) { return __ffma2_rn(x, make_float2(-1.f, -1.f), y); }
 
+// The substitution with four lanes a column (see trsm_df64_kernel): t / 4 is the column, X's rows are overwritten by the
+// solution, rounded to FP32.
+template <int LD>
+__device__ __forceinline__ void solve_df64(const float (*L)[65], float (*Xh)[LD], const float (*Xl)[LD], int tid) {
+  const int lane = tid & 31;
+  const int col = tid >> 2, s = tid & 3;
+  const int gbase = lane & ~3;
+  float2 ah[8], al[8];  // pair q: rows s + 8q (.x) and s + 8q + 4 (.y)
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    ah[q] = make_float2(Xh[s + 8 * q][col], Xh[s + 8 * q + 4][col]);
+    al[q] = make_float2(Xl[s + 8 * q][col], Xl[s + 8 * q + 4][col]);
+  }
+#pragma unroll
+  for (int j = 0; j < 64; ++j) {
+    // row j lives in slot j / 4 of lane j % 4: pair j / 8, half (j / 4) & 1
+    const int q0 = j >> 3;
+    const float mine = ((j >> 2) & 1) ? __fadd_rn(ah[q0].y, al[q0].y) : __fadd_rn(ah[q0].x, al[q0].x);
+    const float xj = __shfl_sync(0xffffffffu, mine, gbase | (j & 3));
+    if (s == (j & 3)) Xh[j][col] = xj;
+    const float2 x2 = make_float2(xj, xj);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      if (8 * q + 7 <= j) continue;  // both rows of this pair are <= j
+      const int i0 = s + 8 * q, i1 = i0 + 4;
+      const float2 f = make_float2(-L[i0][j], -L[i1][j]);
+      const float2 p = __fmul2_rn(f, x2);
+      const float2 e = __ffma2_rn(f, x2, make_float2(-p.x, -p.y));
+      const float2 t0 = __fadd2_rn(ah[q], p);
+      const float2 bb = trsm_sub2(t0, ah[q]);
+      const float2 tt = __fadd2_rn(trsm_sub2(ah[q], trsm_sub2(t0, bb)), trsm_sub2(p, bb));
+      const float2 nl = __fadd2_rn(al[q], __fadd2_rn(tt, e));
+      // rows i <= j keep their values (only a pair straddling j has one)
+      if (i0 > j) { ah[q].x = t0.x; al[q].x = nl.x; }
+      if (i1 > j) { ah[q].y = t0.y; al[q].y = nl.y; }
+    }
+  }
+}
+
 template <int COLS>
 __global__ void __launch_bounds__(4 * COLS) trsm_df64_kernel(float* Whi, float* Wlo, int64_t ld, int k, TrsmDfCols cols,
                                                              const int32_t* __restrict__ map) {
@@ -369,42 +408,130 @@ __global__ void __launch_bounds__(4 * COLS) trsm_df64_kernel(float* Whi, float* 
 #pragma unroll
   for (int i = 0; i < LV; ++i) sm.L[lr + ls * i][lc] = lv[i];
   __syncthreads();
-  const int col = tid >> 2, s = tid & 3;
-  const int gbase = lane & ~3;
-  float2 ah[8], al[8];  // pair q: rows s + 8q (.x) and s + 8q + 4 (.y)
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    ah[q] = make_float2(sm.Xh[s + 8 * q][col], sm.Xh[s + 8 * q + 4][col]);
-    al[q] = make_float2(sm.Xl[s + 8 * q][col], sm.Xl[s + 8 * q + 4][col]);
-  }
-#pragma unroll
-  for (int j = 0; j < 64; ++j) {
-    // row j lives in slot j / 4 of lane j % 4: pair j / 8, half (j / 4) & 1
-    const int q0 = j >> 3;
-    const float mine = ((j >> 2) & 1) ? __fadd_rn(ah[q0].y, al[q0].y) : __fadd_rn(ah[q0].x, al[q0].x);
-    const float xj = __shfl_sync(0xffffffffu, mine, gbase | (j & 3));
-    if (s == (j & 3)) sm.Xh[j][col] = xj;
-    const float2 x2 = make_float2(xj, xj);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      if (8 * q + 7 <= j) continue;  // both rows of this pair are <= j
-      const int i0 = s + 8 * q, i1 = i0 + 4;
-      const float2 f = make_float2(-sm.L[i0][j], -sm.L[i1][j]);
-      const float2 p = __fmul2_rn(f, x2);
-      const float2 e = __ffma2_rn(f, x2, make_float2(-p.x, -p.y));
-      const float2 t0 = __fadd2_rn(ah[q], p);
-      const float2 bb = trsm_sub2(t0, ah[q]);
-      const float2 tt = __fadd2_rn(trsm_sub2(ah[q], trsm_sub2(t0, bb)), trsm_sub2(p, bb));
-      const float2 nl = __fadd2_rn(al[q], __fadd2_rn(tt, e));
-      // rows i <= j keep their values (only a pair straddling j has one)
-      if (i0 > j) { ah[q].x = t0.x; al[q].x = nl.x; }
-      if (i1 > j) { ah[q].y = t0.y; al[q].y = nl.y; }
-    }
-  }
+  solve_df64(sm.L, sm.Xh, sm.Xl, tid);
   __syncthreads();
 #pragma unroll
   for (int i = 0; i < 16; ++i)
     if (ok) Whi[int64_t(k + tr + 4 * i) * ld + cb + tc] = sm.Xh[tr + 4 * i][tc];
+}
+
+// The block row of U for a whole block of 256 rows, 16 columns a CTA: four times a substitution in 64 rows (two warps; the
+// others bring the part of L below) and the update of the rows below it by all warps, in double-float on the FP32
+// pipes (exact products, error-free sums, 10 packed instructions per two terms).
+// As four solves and three updates of two launches each this is 150 to 180 us of launches and short kernels whatever the
+// number of columns, in which the next block cannot begin; here it is the CTA's own chain, about 45 us, up to the columns that fill
+// the SMs once.
+constexpr int kRowCols = 16;
+// Up to this many columns: n = 2,873 5.59 ms a factorisation against 6.19, 5,000 10.8 against 11.6, 10,006 27.6 against
+// 28.3 (with the launches from 4,096 columns on 27.7, never 27.7), 22,506 107.1 against 107.8 (never: 110.8), because many
+// columns are bound by the FP32 pipes here and by the tensor cores there.
+constexpr int kFusedRowCols = 8192;
+struct BlockRowSmem {
+  float Xh[256][kRowCols + 1], Xl[256][kRowCols + 1];
+  float L[64][65];
+  float B[192][65];  // the block of L below the diagonal block
+};
+
+__global__ void __launch_bounds__(256) block_row_df_kernel(float* Whi, const float* __restrict__ Wlo, int64_t ld, int k0,
+                                                           int64_t c0, int64_t c1) {
+  extern __shared__ float4 block_row_smem[];
+  BlockRowSmem& sm = *reinterpret_cast<BlockRowSmem*>(block_row_smem);
+  allow_next();
+  wait_previous();
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tc = tid & 15, tr = tid >> 4;
+  const int64_t c = c0 + int64_t(blockIdx.x) * kRowCols + tc;
+  const bool ok = c < c1;
+  {
+    float vh[16], vl[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int64_t at = int64_t(k0 + tr + 16 * i) * ld + c;
+      vh[i] = ok ? Whi[at] : 0.f;
+      vl[i] = ok ? Wlo[at] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      sm.Xh[tr + 16 * i][tc] = vh[i];
+      sm.Xl[tr + 16 * i][tc] = vl[i];
+    }
+  }
+#pragma unroll 1
+  for (int b = 0; b < 256; b += 64) {
+    const float* src = Whi + int64_t(k0 + b) * ld + k0 + b;
+    {
+      float v[16];
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const int r = warp + 8 * (i >> 1), q = lane + 32 * (i & 1);
+        v[i] = q < r ? src[int64_t(r) * ld + q] : 0.f;
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) sm.L[warp + 8 * (i >> 1)][lane + 32 * (i & 1)] = v[i];
+    }
+    __syncthreads();
+    const int below = 192 - b;
+    if (warp < 2) {
+      solve_df64(sm.L, sm.Xh + b, sm.Xl + b, tid);
+    } else {
+      for (int r0 = warp - 2; r0 < below; r0 += 48) {  // six warps, eight rows of each at a time
+        float v[16];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const int r = r0 + 6 * (i >> 1);
+          v[i] = r < below ? src[int64_t(64 + r) * ld + lane + 32 * (i & 1)] : 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const int r = r0 + 6 * (i >> 1);
+          if (r < below) sm.B[r][lane + 32 * (i & 1)] = v[i];
+        }
+      }
+    }
+    __syncthreads();
+    auto update = [&](auto pairs) {  // rows tr + 32 p and tr + 32 p + 16 below the diagonal block, column tc
+      constexpr int P = decltype(pairs)::value;
+      float2 ah[P], al[P];
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        const int r = b + 64 + tr + 32 * p;
+        ah[p] = make_float2(sm.Xh[r][tc], sm.Xh[r + 16][tc]);
+        al[p] = make_float2(sm.Xl[r][tc], sm.Xl[r + 16][tc]);
+      }
+#pragma unroll 4
+      for (int k = 0; k < 64; ++k) {
+        const float x = sm.Xh[b + k][tc];
+        const float2 x2 = make_float2(x, x), nx = make_float2(-x, -x);
+#pragma unroll
+        for (int p = 0; p < P; ++p) {
+          const float2 l = make_float2(sm.B[tr + 32 * p][k], sm.B[tr + 32 * p + 16][k]);
+          const float2 np = __fmul2_rn(l, nx);
+          const float2 e = __ffma2_rn(l, x2, np);  // what the product lost, with the product's sign
+          const float2 s = __fadd2_rn(ah[p], np);
+          const float2 bb = trsm_sub2(s, ah[p]);
+          const float2 t = __fadd2_rn(trsm_sub2(ah[p], trsm_sub2(s, bb)), trsm_sub2(np, bb));
+          al[p] = __fadd2_rn(al[p], trsm_sub2(t, e));
+          ah[p] = s;
+        }
+      }
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        const int r = b + 64 + tr + 32 * p;
+        const float2 s = __fadd2_rn(ah[p], al[p]), l = trsm_sub2(al[p], trsm_sub2(s, ah[p]));
+        sm.Xh[r][tc] = s.x;
+        sm.Xh[r + 16][tc] = s.y;
+        sm.Xl[r][tc] = l.x;
+        sm.Xl[r + 16][tc] = l.y;
+      }
+    };
+    if (b == 0) update(std::integral_constant<int, 6>{});
+    else if (b == 64) update(std::integral_constant<int, 4>{});
+    else if (b == 128) update(std::integral_constant<int, 2>{});
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+    if (ok) Whi[int64_t(k0 + tr + 16 * i) * ld + c] = sm.Xh[tr + 16 * i][tc];
 }
 
 // ---- FP64 interchanges and triangular solve ---------------------------------------------------------------
@@ -1039,6 +1166,13 @@ int lu_factor_df(int n, float* Whi, float* Wlo, int64_t ld, int32_t* piv, void* 
   };
   // Block row of U for block [K0, KE) on trailing columns [c0, c1).
   auto block_row = [&](int K0, int KE, int c0, int c1) -> int {
+    if (KE - K0 == 256 && c1 - c0 <= kFusedRowCols) {
+      static std::atomic<unsigned long long> attr{0};
+      if (int e = smem_opt_in((const void*)block_row_df_kernel, int(sizeof(BlockRowSmem)), attr)) return e;
+      StatScope sc(kStatTrsm, s, 256.0 * 256.0 * (c1 - c0), 256.0 * (c1 - c0) * 12.0);
+      return launch_next(!lookahead, block_row_df_kernel, unsigned(ceil_div(c1 - c0, kRowCols)), 256, sizeof(BlockRowSmem), s,
+                         Whi, (const float*)Wlo, ld, K0, int64_t(c0), int64_t(c1));
+    }
     for (int b = K0; b < KE; b += nb) {
       const int w = std::min(nb, KE - b);
       if (int e = trsm(b, {c0, c1, 0, 0, 0, 0}, nullptr, s, !lookahead)) return e;
