@@ -1217,9 +1217,54 @@ int lu_factor_df(int n, float* Whi, float* Wlo, int64_t ld, int32_t* piv, void* 
   return UPDES_OK;
 }
 
-// FP64 LU with LAPACK's pivots, in place.  Blocks of 256 columns of 32-wide panels; every update of the block's own
-// columns (K = 32), of the block row of U (K = 64) and of the trailing matrix (K = 256) runs on the tensor cores
-// (gemm_tc64.cu).  Panels are 32 wide because the FP64 pipe of the cluster's SMs bounds them (half the multiply-adds
+// C (m x nc) -= A (m x K) B (K x nc) by FP64 multiply-adds, 64 x 64 tiles, 4 x 4 entries a thread.  Bound by the FP64
+// pipe (two multiply-adds a cycle and SM, 97 % of them reached): 552 ms of an n = 10,006 factorisation, where the digit
+// products of gemm_tc64.cu take 45.  For matrices that nobody has scaled: an FP64 product keeps every entry's own 53 bits,
+// the digits share one power of two along a row of A and a column of B.
+__global__ void __launch_bounds__(256) gemm64_chain_kernel(double* C, const double* __restrict__ A,
+                                                           const double* __restrict__ B, int64_t ld, int m, int nc, int K) {
+  __shared__ double As[32][65];
+  __shared__ double Bs[32][65];
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int r0 = blockIdx.y * 64, c0 = blockIdx.x * 64;
+  double acc[4][4] = {};
+  for (int kb = 0; kb < K; kb += 32) {
+    for (int e = threadIdx.x; e < 64 * 32; e += 256) {
+      const int i = e >> 5, j = e & 31;
+      As[j][i] = (r0 + i < m && kb + j < K) ? A[int64_t(r0 + i) * ld + kb + j] : 0.0;
+      const int kr = e >> 6, cj = e & 63;
+      Bs[kr][cj] = (kb + kr < K && c0 + cj < nc) ? B[int64_t(kb + kr) * ld + c0 + cj] : 0.0;
+    }
+    __syncthreads();
+#pragma unroll 8
+    for (int kk = 0; kk < 32; ++kk) {
+      double a[4], b[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) { a[u] = As[kk][ty + 16 * u]; b[u] = Bs[kk][tx + 16 * u]; }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int v = 0; v < 4; ++v) acc[u][v] = fma(a[u], b[v], acc[u][v]);
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int r = r0 + ty + 16 * u;
+    if (r >= m) continue;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const int c = c0 + tx + 16 * v;
+      if (c < nc) C[int64_t(r) * ld + c] -= acc[u][v];
+    }
+  }
+}
+
+// FP64 LU with LAPACK's pivots, in place.  Blocks of 256 columns of 32-wide panels.  With `digits` every update of the
+// block's own columns (K = 32), of the block row of U (K = 64) and of the trailing matrix (K = 256) runs on the tensor
+// cores (gemm_tc64.cu): for matrices whose rows and columns are scaled so that the entries that share a digit scale are of
+// one size (the solves' equilibrated K).  Without, by FP64 multiply-adds, on one stream.
+// Panels are 32 wide because the FP64 pipe of the cluster's SMs bounds them (half the multiply-adds
 // of 64).  The look-ahead is that of lu_factor_df: the next block on a second stream beside the update of the rest.
 namespace {
 constexpr int kNb64 = 32;
@@ -1236,7 +1281,7 @@ size_t lu_64_workspace_bytes(int n) {
 }
 
 int lu_factor_64(int n, double* W, int64_t ld, int32_t* piv, void* ws, size_t ws_bytes, DeviceStatus* st,
-                 cudaStream_t s) {
+                 cudaStream_t s, bool use_digits) {
   if (ws_bytes < lu_64_workspace_bytes(n)) return UPDES_ERR_WORKSPACE;
   char* base = static_cast<char*>(ws);
   unsigned int* bar = reinterpret_cast<unsigned int*>(base);
@@ -1256,7 +1301,7 @@ int lu_factor_64(int n, double* W, int64_t ld, int32_t* piv, void* ws, size_t ws
   }();
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   UPDES_CUDA_TRY(cudaStreamIsCapturing(s, &cs));
-  const bool lookahead = lookahead_on && n >= kLookaheadMinN && cs == cudaStreamCaptureStatusNone;
+  const bool lookahead = use_digits && lookahead_on && n >= kLookaheadMinN && cs == cudaStreamCaptureStatusNone;
   UPDES_CUDA_TRY(cudaMemsetAsync(bar, 0, 256 + 2 * 1024 * sizeof(Cand), s));  // barrier words and candidate tags
 
   auto trsm = [&](int k, int w, int64_t c0, int64_t c1, const int32_t* map, int64_t left, int64_t left_end,
@@ -1282,6 +1327,15 @@ int lu_factor_64(int n, double* W, int64_t ld, int32_t* piv, void* ws, size_t ws
   } last;
   auto upd = [&](int r0, int r1, int c0, int c1, int k0, int k1, cudaStream_t us, bool la, int ctas,
                  bool early) -> int {
+    if (!use_digits) {
+      const int m = r1 - r0, nc = c1 - c0, K = k1 - k0;
+      if (m <= 0 || nc <= 0 || K <= 0) return UPDES_OK;
+      StatScope sc(kStatGemm, us, 2.0 * m * double(nc) * K, double(m) * nc * 16.0 + (double(m) + nc) * K * 8.0);
+      gemm64_chain_kernel<<<dim3(unsigned(ceil_div(nc, 64)), unsigned(ceil_div(m, 64))), 256, 0, us>>>(
+          W + int64_t(r0) * ld + c0, W + int64_t(r0) * ld + k0, W + int64_t(k0) * ld + c0, ld, m, nc, K);
+      UPDES_LAUNCH_CHECK();
+      return UPDES_OK;
+    }
     const bool ready = !la && last.r0 == r0 && last.r1 == r1 && last.k0 == k0 && last.k1 == k1;
     const int e = ozaki64_update(W + int64_t(r0) * ld + c0, ld, W + int64_t(r0) * ld + k0, ld,
                                  W + int64_t(k0) * ld + c0, ld, r1 - r0, c1 - c0, k1 - k0, la ? digits_la : digits,

@@ -5,10 +5,11 @@
 
 constexpr int kLuNb = 64;  // panel width
 
-// FP64 LU in place, LAPACK's pivot choices (interchanges to piv[0, n)).
+// FP64 LU in place, LAPACK's pivot choices (interchanges to piv[0, n)).  use_digits: the updates on the tensor cores, for
+// a matrix whose rows and columns are scaled (gemm_tc64.cu says to what); else by FP64 multiply-adds, for any.
 size_t lu_64_workspace_bytes(int n);
 int lu_factor_64(int n, double* W, int64_t ld, int32_t* piv, void* ws, size_t ws_bytes, DeviceStatus* st,
-                 cudaStream_t s);
+                 cudaStream_t s, bool use_digits);
 
 // The panel W[k:n, k:k+w] (w <= 64) factored in place on one thread-block cluster (panel.cu): interchanges to
 // piv[k..k+w) and their net permutation to swap_map (257 ints, may be null).  UPDES_ERR_UNSUPPORTED when its rows do

@@ -592,8 +592,9 @@ int factor_df_core(int n, float* hi, float* lo, int64_t ld, int32_t* piv, const 
   return perm_core(n, piv, s);
 }
 
+// scaled: the rows and columns of A are equilibrated (what the FP64 updates on the tensor cores ask for).
 int factor_core(int n, double* A, int64_t lda, int precision, void* F, int64_t ldf, int32_t* piv, const LuWs& w,
-                cudaStream_t s) {
+                cudaStream_t s, bool scaled) {
   if (precision == UPDES_PREC_FP32) {
     if (!w.lo || !F) return UPDES_ERR_INVALID;
     split_df_kernel<<<unsigned(ceil_div(int64_t(n) * ldf, 256)), 256, 0, s>>>(A, lda, static_cast<float*>(F), w.lo,
@@ -610,7 +611,7 @@ int factor_core(int n, double* A, int64_t lda, int precision, void* F, int64_t l
       A = Fd;
       lda = ldf;
     }
-    e = lu_factor_64(n, A, lda, piv, w.panel, w.panel_bytes, w.st, s);
+    e = lu_factor_64(n, A, lda, piv, w.panel, w.panel_bytes, w.st, s, scaled);
   }
   if (e) return e;
   return perm_core(n, piv, s);
@@ -667,7 +668,7 @@ extern "C" int updes_lu_factor(int32_t n, double* A, int64_t lda, int32_t precis
   LuWs w;
   lu_ws_layout(n, precision, static_cast<char*>(workspace), &w);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  int e = factor_core(n, A, lda, precision, F, ldf, piv, w, s);
+  int e = factor_core(n, A, lda, precision, F, ldf, piv, w, s, false);
   if (e) return e;
   DeviceStatus h;
   e = read_status(w.st, s, &h);
@@ -1010,7 +1011,7 @@ int factor_launch(const SolveWs& w, int n, int precision, cudaStream_t s, bool p
       join_df_kernel<<<unsigned(ceil_div(total, 256)), 256, 0, s>>>(w.Khi, w.Klo, w.W, total);
       UPDES_LAUNCH_CHECK();
     }
-    e = factor_core(n, w.W, w.ld, precision, nullptr, w.ld, w.piv, w.lu, s);
+    e = factor_core(n, w.W, w.ld, precision, nullptr, w.ld, w.piv, w.lu, s, true);
   } else {
     if (!planes_ready) {
       UPDES_CUDA_TRY(cudaMemcpyAsync(w.F32, w.Khi, size_t(total) * 4, cudaMemcpyDeviceToDevice, s));
