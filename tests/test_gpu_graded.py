@@ -56,3 +56,82 @@ def test_lu_factor_takes_any_scaling(kind, n):
     PA, L, U = _lu(A)
     wrong = np.abs(PA - L @ U) > 2 * A.shape[0] * 2.0 ** -53 * (np.abs(L) @ np.abs(U))
     assert not wrong.any(), f"{int(wrong.sum())} entries"
+
+
+def _poisson(side, a, precision, nx=30, ny=20, degree=2):
+    import updes_gb300 as U
+    from functools import partial
+    X = _nodes(nx, ny, side)
+    cloud = U.SquareCloud(Nx=nx, Ny=ny, coords=X, facet_types={f: "d" for f in ("South", "West", "North", "East")})
+    x = np.asarray(cloud.sorted_nodes).T / side
+    values = np.sin(x[0]) * np.exp(x[1])
+    bcs = {f: values[np.asarray(cloud.facet_nodes[f])] for f in cloud.facet_types}
+    rhs = lambda x, centers, rbf, fields: np.sin(3.0 * x[0] / side) * np.cosh(2.0 * x[1] / side) / side ** 2
+    lap = lambda x, center, rbf, monomial, fields: U.nodal_laplacian(x, center, rbf, monomial)
+    return U.pde_solver(lap, rhs, cloud, bcs, partial(U.polyharmonic, a=a), degree,
+                        options=U.SolverOptions(precision=precision, reuse_factorization=False))
+
+
+# A domain whose side is a power of two is the unit square's system with exactly scaled coordinates and entries, so the
+# nodal values are those of side 1 up to the errors of an FP64 solution on it.  LAPACK's (CPU, against extended precision,
+# four clouds): 8e-14 for r^3 and 2.3e-12 for r^5; 32 times that for the two solutions compared.
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("a,degree,lapack", [(1, 1, 8e-14), (1, 2, 8e-14), (2, 2, 2.3e-12)])
+@pytest.mark.parametrize("k", [-13, -10, -7, 4])
+def test_the_solution_does_not_depend_on_the_unit_of_length(k, a, degree, lapack, precision):
+    from updes_gb300 import operators
+    want = _poisson(1.0, a, "fp64", degree=degree).vals
+    got = _poisson(2.0 ** k, a, precision, degree=degree).vals
+    # a mixed solve that its refinement certifies (256 u of backward error) is held to that
+    certified = precision == "fp32" and not operators.LAST_INFO["fell_back"]
+    assert np.max(np.abs(got - want)) <= (256 if certified else 1) * 32 * lapack * np.max(np.abs(want))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_the_adjoint_on_a_small_domain(precision):
+    # A cost w . vals is linear in the boundary values, so its gradient times other boundary values is the cost of their
+    # solution.  The gradient itself is a vector of coefficients, which r^3 leaves undetermined beyond eight digits; a
+    # transposed solution of small backward error gives the product as well as a solution gives its values.
+    import torch
+    import updes_gb300 as U
+    from functools import partial
+    from updes_gb300.adjoint import pde_solver_torch
+    lap = lambda x, center, rbf, monomial, fields: U.nodal_laplacian(x, center, rbf, monomial)
+    w = np.random.default_rng(1).standard_normal(600)
+
+    def solve(side, precision, value):
+        cloud = U.SquareCloud(Nx=30, Ny=20, coords=_nodes(30, 20, side),
+                              facet_types={f: "d" for f in ("South", "West", "North", "East")})
+        x = np.asarray(cloud.sorted_nodes).T / side
+        bcs = {f: np.zeros(len(cloud.facet_nodes[f])) for f in cloud.facet_types}
+        control = torch.as_tensor(value(x[0][np.asarray(cloud.facet_nodes["North"])]), device="cuda").requires_grad_()
+        vals, _ = pde_solver_torch(lap, lambda x, centers, rbf, fields: 0.0 * x[0], cloud, dict(bcs, North=control),
+                                   partial(U.polyharmonic, a=1), 1, options=U.SolverOptions(precision=precision))
+        return control, vals
+
+    other = lambda t: np.cos(2.0 * t)
+    control, vals = solve(2.0 ** -10, precision, lambda t: np.sin(np.pi * t))  # fp32 falls back to FP64 on this side
+    gradient, = torch.autograd.grad(torch.dot(torch.as_tensor(w, device="cuda"), vals), [control])
+    control, vals = solve(1.0, "fp64", other)
+    vals = vals.detach().cpu().numpy()
+    got = float(torch.dot(gradient, control.detach()))
+    assert abs(got - w @ vals) <= 64 * 8e-14 * np.abs(w).sum() * np.max(np.abs(vals))
+
+
+def test_far_nodes_do_not_spoil_the_scaling():
+    # a facet whose nodes see the others' Gaussians at 1e-10 only: their rows are all polynomial, and its values come out
+    # as those of the polynomial that the data are (FP64 arithmetic on a CPU: 2.6e-12)
+    import updes_gb300 as U
+    from functools import partial
+    nx, ny = 20, 16
+    ii, jj = np.arange(nx * ny) // ny, np.arange(nx * ny) % ny
+    X = np.stack([np.linspace(0.0, 1.0, nx)[ii], np.linspace(0.0, 1.0, ny)[jj]], axis=-1)
+    X[ii == nx - 1] = np.stack([np.full(ny, 1.4), 6.0 * np.linspace(0.0, 1.0, ny)], axis=-1)
+    cloud = U.SquareCloud(Nx=nx, Ny=ny, coords=X, facet_types={f: "d" for f in ("South", "West", "North", "East")})
+    x = np.asarray(cloud.sorted_nodes).T
+    exact = 1.0 + 0.3 * x[0] - 0.2 * x[1]
+    bcs = {f: exact[np.asarray(cloud.facet_nodes[f])] for f in cloud.facet_types}
+    lap = lambda x, center, rbf, monomial, fields: U.nodal_laplacian(x, center, rbf, monomial)
+    sol = U.pde_solver(lap, lambda x, centers, rbf, fields: 0.0 * x[0], cloud, bcs, partial(U.gaussian, eps=12.0), 1,
+                       options=U.SolverOptions(precision="fp64", reuse_factorization=False))
+    assert np.max(np.abs(sol.vals - exact)) <= 3e-10

@@ -10,8 +10,11 @@
 // column of B) over all of K:
 //   a = 2^(e - 55) * sum_i d_i 2^(8 (6 - i)),   |d_i| <= 128,   |a| < 2^e for the whole row,
 // by rounding the 53-bit significand to a multiple of 2^(e - 55): exact for entries within a factor 8 of the row's
-// largest, cut at 2^-56 of 2^e otherwise (an FP64 rounding of that largest entry is 2^-54).  The digit products of
-// equal weight 2^-8g, g = a + b <= 7 (34 of them), are summed in one FP32 tensor-memory accumulator over all of K:
+// largest, cut at 2^-56 of 2^e otherwise (an FP64 rounding of that largest entry is 2^-54).  The cut is harmless where the
+// entries that meet in a sum are of one size, as in K scaled by solve.cu (row_scale_kernel); where a row's largest entry
+// meets small ones only (graded rows of a matrix that nobody scaled) it loses digits that a chain of FP64 multiply-adds
+// keeps, so such matrices are factored with that (gemm64_chain_kernel in lu.cu).
+// The digit products of equal weight 2^-8g, g = a + b <= 7 (34 of them), are summed in one FP32 accumulator over all of K:
 // 256 products of at most 2^14 each, at most 7 times, so sums stay integers below 2^24.8 and are exact unless
 // nearly every digit of a row and a column is at its limit with one sign, when the error is a unit of that group.
 // Products with g >= 8 lie 2^-64 below 2^(ea + eb) each and are left out.  (The products with g = 7 are needed: the

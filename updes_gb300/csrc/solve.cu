@@ -66,32 +66,121 @@ __global__ void permute_kernel(double* __restrict__ out, const double* __restric
   else out[int64_t(i) * out_stride] = in[int64_t(perm[i]) * in_stride];
 }
 
-// dr[i] = 2^-round(log2(max_j |K_ij|)) (power of two, so scaling is exact)
-__global__ void row_scale_kernel(const double* __restrict__ K, int64_t ld, int n, double* __restrict__ dr) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (warp >= n) return;
-  double m = 0.0;
-  for (int j = lane; j < n; j += 32) m = fmax(m, fabs(K[int64_t(warp) * ld + j]));
-  for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if (lane == 0) {
-    int e = 0;
-    if (m > 0.0 && isfinite(m)) frexp(m, &e);
-    dr[warp] = ldexp(1.0, -e);
-  }
+// A power of two that brings the maximum m into [1/2, 1) (scaling by it is exact); 1 for m = 0 or a non-finite m.
+__device__ __forceinline__ double pow2_scale(double m) {
+  int e = 0;
+  if (m > 0.0 && isfinite(m)) frexp(m, &e);
+  return ldexp(1.0, -e);
 }
 
-// Column maxima of |K| diag(dr) over a chunk of rows per blockIdx.y, combined with an integer atomicMax on the
-// bit patterns (non-negative doubles order like their bits); colmax must start at zero.
+// Scaling of the FP64 factorisation.  Its digit products (gemm_tc64.cu) share one power of two along a row of L and a column
+// of U, so the entries that meet there have to be of one size.  In K = [[op Phi, op P], [P^T, 0]] of a domain of side S they
+// are not: Phi is S^(2a+1) beside the ones of P, and scaled by the whole row's and column's largest entry, the ones, it
+// stays so.  So the kernel block's rows and columns are scaled to their own maxima, each monomial's column and row to the
+// size that its entries then have beside these (monomial_scale_kernel), and only then whole rows and columns: whatever the
+// side, a matrix like the unit square's.  r^3, 600 nodes, side 2^-10: nodal values wrong by 1.6e-7 with whole rows
+// and columns alone, by 4e-14 (as on the unit square) with this.
+
+// Only exponents count, so the passes over K compare those, on integers: the FP64 pipe takes 64 cycles an operation and warp
+// and made a pass 0.6 ms at n = 10,006, memory 0.15.
+
+// e with |v| in [2^(e-1), 2^e); kNoExp for 0 and subnormal numbers.
+constexpr int kNoExp = -(1 << 20);
+__device__ __forceinline__ int exponent_of(double v) {
+  const int f = (__double2hiint(v) >> 20) & 0x7ff;
+  return f ? f - 1022 : kNoExp;
+}
+// the power of two that brings a maximum with that exponent into [1/2, 1); 1 for 0 and for infinities
+__device__ __forceinline__ double scale_by(int e) { return e <= kNoExp / 2 || e >= 1025 ? 1.0 : ldexp(1.0, -e); }
+
+// dr[i], i < rows, by the largest of the first `cols` entries, or, where these lie below 2^-400 of the largest of all n, by
+// that; entries of column j times dc[j] (dc may be null).
+__global__ void __launch_bounds__(256) row_scale_kernel(const double* __restrict__ K, int64_t ld, int n, int rows, int cols,
+                                                        const double* __restrict__ dc, double* __restrict__ dr) {
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (i >= rows) return;
+  const double2* row = reinterpret_cast<const double2*>(K + int64_t(i) * ld);
+  int m = kNoExp, all = kNoExp;
+  for (int j0 = 2 * lane; j0 < n; j0 += 256) {  // four loads of two entries in flight
+    double2 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = j0 + 64 * u < n ? row[j0 / 2 + 32 * u] : make_double2(0.0, 0.0);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int j = j0 + 64 * u + h;
+        if (j >= n) continue;
+        const int e = exponent_of(h ? v[u].y : v[u].x) + (dc ? exponent_of(dc[j]) - 1 : 0);
+        if (j < cols) m = max(m, e);
+        all = max(all, e);
+      }
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  all = __reduce_max_sync(0xffffffffu, all);
+  if (lane == 0) dr[i] = scale_by(m > all - 400 ? m : all);
+}
+
+// Column N + k (blockIdx.y == 0) or row N + k of K, by its entries in the first N rows (columns) with the scales of these,
+// beside kernel entries of up to 1: largest entry to 1 where it is below, geometric mean to 1 where that is above, and else
+// as it is.  Not by the largest throughout: a few nodes far from the others have kernel rows of 1e-10 and, scaled to 1,
+// monomials of 1e10; made 1, they leave those of all other nodes at 1e-10 and the polynomial wrong by 1.6e-6
+// (20 x 16 nodes, one facet far away; with the mean, 2.6e-12).
+__global__ void __launch_bounds__(256) monomial_scale_kernel(const double* __restrict__ K, int64_t ld, int N,
+                                                             double* __restrict__ dr, double* __restrict__ dc) {
+  __shared__ int sum_s, count_s, max_s;
+  const bool column = blockIdx.y == 0;
+  const int k = N + blockIdx.x;
+  if (threadIdx.x == 0) {
+    sum_s = count_s = 0;
+    max_s = -4000;
+  }
+  __syncthreads();
+  int sum = 0, count = 0, most = -4000;  // exponents: below 2,200 each
+  for (int i = threadIdx.x; i < N; i += blockDim.x) {
+    const double v = fabs(column ? K[int64_t(i) * ld + k] * dr[i] : K[int64_t(k) * ld + i] * dc[i]);
+    if (!(v > 0.0) || !isfinite(v)) continue;
+    int e;
+    frexp(v, &e);
+    sum += e;
+    ++count;
+    most = max(most, e);
+  }
+  atomicAdd(&sum_s, sum);
+  atomicAdd(&count_s, count);
+  atomicMax(&max_s, most);
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  const int e = count_s ? max(__double2int_rn(double(sum_s) / count_s), min(max_s, 0)) : 0;
+  (column ? dc : dr)[k] = ldexp(1.0, -e);
+}
+
+// Largest exponents of the columns of |K| diag(dr) over a chunk of the first `rows` rows per blockIdx.y, plus kExpBias, into
+// the low words of colmax, which must start at zero; column_scale_kernel then makes dc of them in place.
 constexpr int kColScaleChunks = 64;
-__global__ void col_max_kernel(const double* __restrict__ K, int64_t ld, int n, const double* __restrict__ dr,
-                               unsigned long long* __restrict__ colmax) {
+constexpr int kExpBias = 8192;
+__global__ void __launch_bounds__(256) column_exponents_kernel(const double* __restrict__ K, int64_t ld, int n, int rows,
+                                                               const double* __restrict__ dr, int2* __restrict__ colmax) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
-  const int rows = int(ceil_div(n, kColScaleChunks));
-  const int i0 = blockIdx.y * rows, i1 = min(n, i0 + rows);
-  double m = 0.0;
-  for (int i = i0; i < i1; ++i) m = fmax(m, fabs(K[int64_t(i) * ld + j]) * dr[i]);
-  if (m > 0.0) atomicMax(colmax + j, (unsigned long long)__double_as_longlong(m));
+  const int chunk = int(ceil_div(rows, kColScaleChunks));
+  const int i0 = blockIdx.y * chunk, i1 = min(rows, i0 + chunk);
+  int m = kNoExp;
+  for (int i = i0; i < i1; i += 8) {  // eight loads in flight
+    double v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) v[u] = i + u < i1 ? K[int64_t(i + u) * ld + j] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (i + u < i1) m = max(m, exponent_of(v[u]) + exponent_of(dr[i + u]) - 1);
+  }
+  if (m > kNoExp / 2) atomicMax(&colmax[j].x, m + kExpBias);
+}
+__global__ void column_scale_kernel(int n, double* __restrict__ dc) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= n) return;
+  const int m = reinterpret_cast<const int2*>(dc)[j].x;
+  dc[j] = m ? scale_by(m - kExpBias) : 1.0;
 }
 
 // dc_j = 2^-e with max_i |K_ij| dr_i in [2^(e-1), 2^e)  (dc holds the maxima' bits on entry)
@@ -99,23 +188,19 @@ __global__ void col_scale_kernel(int n, double* __restrict__ dc) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= n) return;
   const double m = __longlong_as_double((long long)reinterpret_cast<unsigned long long*>(dc)[j]);
-  int e = 0;
-  if (m > 0.0 && isfinite(m)) frexp(m, &e);
-  dc[j] = ldexp(1.0, -e);
+  dc[j] = pow2_scale(m);
 }
-
 
 // dr[i] = 2^-e with the row maximum (FP32 bit pattern in maxbits) in [2^(e-1), 2^e)
 __global__ void row_scale_bits_kernel(const unsigned* __restrict__ maxbits, int n, double* __restrict__ dr) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  const double m = double(__uint_as_float(maxbits[i]));
-  int e = 0;
-  if (m > 0.0 && isfinite(m)) frexp(m, &e);
-  dr[i] = ldexp(1.0, -e);
+  dr[i] = pow2_scale(double(__uint_as_float(maxbits[i])));
 }
 
-// Column maxima of |Khi| diag(dr) (the FP32 plane of an unscaled double-float K), as col_max_kernel.
+// Column maxima of |Khi| diag(dr) (the FP32 plane of an unscaled double-float K) over a chunk of rows per
+// blockIdx.y, combined with an integer atomicMax on the bit patterns (non-negative doubles order like their bits); colmax
+// must start at zero.
 __global__ void col_max_f32_kernel(const float* __restrict__ Khi, int64_t ld, int n, const double* __restrict__ dr,
                                    unsigned long long* __restrict__ colmax) {
   const int j = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1007,7 +1092,7 @@ int factor_launch(const SolveWs& w, int n, int precision, cudaStream_t s, bool p
   UPDES_CUDA_TRY(cudaMemsetAsync(w.state, 0, 4 * sizeof(int32_t), s));  // invalid until the factors are complete
   const int64_t total = int64_t(n) * w.ld;
   if (precision == UPDES_PREC_FP64) {
-    if (!planes_ready) {  // a fallback after the FP32 attempt: W was overwritten, K is rebuilt from its planes
+    if (!planes_ready) {
       join_df_kernel<<<unsigned(ceil_div(total, 256)), 256, 0, s>>>(w.Khi, w.Klo, w.W, total);
       UPDES_LAUNCH_CHECK();
     }
@@ -1113,14 +1198,28 @@ int assemble_stage(const updes_problem* p, const SolveWs& w, int n, int precisio
     }
   }
   if ((e = updes_assemble(p, w.W, w.ld, nullptr, 0, s))) return e;  // FP64 K, staged in the working buffer
-  row_scale_kernel<<<unsigned(ceil_div(int64_t(n) * 32, 256)), 256, 0, s>>>(w.W, w.ld, n, w.dr);
-  UPDES_LAUNCH_CHECK();
-  UPDES_CUDA_TRY(cudaMemsetAsync(w.dc, 0, size_t(n) * sizeof(double), s));
-  col_max_kernel<<<dim3(unsigned(ceil_div(n, 256)), kColScaleChunks), 256, 0, s>>>(
-      w.W, w.ld, n, w.dr, reinterpret_cast<unsigned long long*>(w.dc));
-  UPDES_LAUNCH_CHECK();
-  col_scale_kernel<<<unsigned(ceil_div(n, 256)), 256, 0, s>>>(n, w.dc);
-  UPDES_LAUNCH_CHECK();
+  // the mixed path by whole rows and columns, like its double-float assembly; the FP64 path over the kernel block first
+  const int first = precision == UPDES_PREC_FP64 ? p->N : n;
+  auto rows_by = [&](int rows, const double* dc) -> int {
+    row_scale_kernel<<<unsigned(ceil_div(int64_t(rows) * 32, 256)), 256, 0, s>>>(w.W, w.ld, n, rows, rows, dc, w.dr);
+    UPDES_LAUNCH_CHECK();
+    return UPDES_OK;
+  };
+  auto columns_by = [&](int rows) -> int {
+    UPDES_CUDA_TRY(cudaMemsetAsync(w.dc, 0, size_t(n) * sizeof(double), s));
+    column_exponents_kernel<<<dim3(unsigned(ceil_div(n, 256)), kColScaleChunks), 256, 0, s>>>(
+        w.W, w.ld, n, rows, w.dr, reinterpret_cast<int2*>(w.dc));
+    UPDES_LAUNCH_CHECK();
+    column_scale_kernel<<<unsigned(ceil_div(n, 256)), 256, 0, s>>>(n, w.dc);
+    UPDES_LAUNCH_CHECK();
+    return UPDES_OK;
+  };
+  if ((e = rows_by(first, nullptr)) || (e = columns_by(first))) return e;
+  if (first < n) {
+    monomial_scale_kernel<<<dim3(unsigned(n - first), 2), 256, 0, s>>>(w.W, w.ld, first, w.dr, w.dc);
+    UPDES_LAUNCH_CHECK();
+    if ((e = rows_by(n, w.dc)) || (e = columns_by(n))) return e;
+  }
   // the FP64 path factors the equilibrated FP64 K itself (written back in place), not the 48-bit sum of its
   // planes: on systems near the FP64 limit (r^5 at N = 10,000) the planes' rounding alone would be 32x the
   // FP64 rounding of K
@@ -1168,13 +1267,9 @@ int solve_stage(const updes_problem* p, const SolveWs& w, int n, const double* q
     if (info->converged || !o.fallback_fp64) break;
     precision = UPDES_PREC_FP64;
     info->fell_back = 1;
-    // the FP32 attempt overwrote the working matrix: K is assembled again in FP64 and scaled in place with the
-    // same powers of two, so the fallback factors the FP64 K (not the 48-bit sum of its planes); the planes,
-    // the residuals' operator, stay as they are
-    if ((e = updes_assemble(p, w.W, w.ld, nullptr, 0, s))) return e;
-    split_df_kernel<<<unsigned(ceil_div(int64_t(n) * w.ld, 256)), 256, 0, s>>>(w.W, w.ld, nullptr, nullptr, w.ld, n,
-                                                                               w.dr, w.dc, 1);
-    UPDES_LAUNCH_CHECK();
+    // the FP32 attempt overwrote the working matrix and scaled K as the mixed path does: assembled and scaled again
+    bool ready = false;
+    if ((e = assemble_stage(p, w, n, precision, info, s, &ready))) return e;
     if ((e = factor_stage(w, n, precision, info, s, true))) return e;
   }
   Timer t(s);
