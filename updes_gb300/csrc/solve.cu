@@ -76,8 +76,8 @@ __device__ __forceinline__ double pow2_scale(double m) {
 // Scaling of the FP64 factorisation.  Its digit products (gemm_tc64.cu) share one power of two along a row of L and a column
 // of U, so the entries that meet there have to be of one size.  In K = [[op Phi, op P], [P^T, 0]] of a domain of side S they
 // are not: Phi is S^(2a+1) beside the ones of P, and scaled by the whole row's and column's largest entry, the ones, it
-// stays so.  So the kernel block's rows and columns are scaled to their own maxima, each monomial's column and row to the
-// size that its entries then have beside these (monomial_scale_kernel), and only then whole rows and columns: whatever the
+// stays so.  So the kernel block's rows and columns are scaled to their own maxima, the polynomial ones to the
+// size that the constant then has beside these (polynomial_scale_kernel), and only then whole rows and columns: whatever the
 // side, a matrix like the unit square's.  r^3, 600 nodes, side 2^-10: nodal values wrong by 1.6e-7 with whole rows
 // and columns alone, by 4e-14 (as on the unit square) with this.
 
@@ -121,38 +121,30 @@ __global__ void __launch_bounds__(256) row_scale_kernel(const double* __restrict
   if (lane == 0) dr[i] = scale_by(m > all - 400 ? m : all);
 }
 
-// Column N + k (blockIdx.y == 0) or row N + k of K, by its entries in the first N rows (columns) with the scales of these,
-// beside kernel entries of up to 1: largest entry to 1 where it is below, geometric mean to 1 where that is above, and else
-// as it is.  Not by the largest throughout: a few nodes far from the others have kernel rows of 1e-10 and, scaled to 1,
-// monomials of 1e10; made 1, they leave those of all other nodes at 1e-10 and the polynomial wrong by 1.6e-6
-// (20 x 16 nodes, one facet far away; with the mean, 2.6e-12).
-__global__ void __launch_bounds__(256) monomial_scale_kernel(const double* __restrict__ K, int64_t ld, int N,
-                                                             double* __restrict__ dr, double* __restrict__ dc) {
-  __shared__ int sum_s, count_s, max_s;
-  const bool column = blockIdx.y == 0;
-  const int k = N + blockIdx.x;
-  if (threadIdx.x == 0) {
-    sum_s = count_s = 0;
-    max_s = -4000;
-  }
+// The polynomial columns (blockIdx.x == 0) or rows of K, all by one power of two: the constant's entries in the first N rows
+// (columns), with the scales of these, brought to a geometric mean of 1 where that is above, beside kernel entries of up to 1.
+// One factor for all, because monomials that are large among themselves (nodes far from the origin) are better left so:
+// 36 x 24 nodes around 100, Gaussian, 1.3e-11 with each at 1, 5.8e-13 with whole rows.  Not by the largest entry: a
+// few nodes far from the others have kernel rows of 1e-10 and, scaled to 1, a constant of 1e10; made 1, it leaves all
+// other nodes' at 1e-10 and the polynomial wrong by 1.6e-6 (20 x 16 nodes, one facet far away; with the mean, 2.6e-12).
+__global__ void __launch_bounds__(256) polynomial_scale_kernel(const double* __restrict__ K, int64_t ld, int N, int M,
+                                                               double* __restrict__ dr, double* __restrict__ dc) {
+  __shared__ int sum_s, count_s;
+  const bool columns = blockIdx.x == 0;
+  if (threadIdx.x == 0) sum_s = count_s = 0;
   __syncthreads();
-  int sum = 0, count = 0, most = -4000;  // exponents: below 2,200 each
+  int sum = 0, count = 0;  // of exponents: below 2,200 each
   for (int i = threadIdx.x; i < N; i += blockDim.x) {
-    const double v = fabs(column ? K[int64_t(i) * ld + k] * dr[i] : K[int64_t(k) * ld + i] * dc[i]);
-    if (!(v > 0.0) || !isfinite(v)) continue;
-    int e;
-    frexp(v, &e);
-    sum += e;
+    const int e = exponent_of(columns ? K[int64_t(i) * ld + N] : K[int64_t(N) * ld + i]);
+    if (e == kNoExp || e >= 1025) continue;
+    sum += e + exponent_of(columns ? dr[i] : dc[i]) - 1;
     ++count;
-    most = max(most, e);
   }
   atomicAdd(&sum_s, sum);
   atomicAdd(&count_s, count);
-  atomicMax(&max_s, most);
   __syncthreads();
-  if (threadIdx.x != 0) return;
-  const int e = count_s ? max(__double2int_rn(double(sum_s) / count_s), min(max_s, 0)) : 0;
-  (column ? dc : dr)[k] = ldexp(1.0, -e);
+  const int e = count_s ? max(__double2int_rn(double(sum_s) / count_s), 0) : 0;
+  if (threadIdx.x < M) (columns ? dc : dr)[N + threadIdx.x] = ldexp(1.0, -e);
 }
 
 // Largest exponents of the columns of |K| diag(dr) over a chunk of the first `rows` rows per blockIdx.y, plus kExpBias, into
@@ -1216,7 +1208,7 @@ int assemble_stage(const updes_problem* p, const SolveWs& w, int n, int precisio
   };
   if ((e = rows_by(first, nullptr)) || (e = columns_by(first))) return e;
   if (first < n) {
-    monomial_scale_kernel<<<dim3(unsigned(n - first), 2), 256, 0, s>>>(w.W, w.ld, first, w.dr, w.dc);
+    polynomial_scale_kernel<<<2, 256, 0, s>>>(w.W, w.ld, first, n - first, w.dr, w.dc);
     UPDES_LAUNCH_CHECK();
     if ((e = rows_by(n, w.dc)) || (e = columns_by(n))) return e;
   }
