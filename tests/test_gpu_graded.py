@@ -8,8 +8,8 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-def _nodes(nx, ny, side):
-    rng = np.random.default_rng(nx * ny)
+def _nodes(nx, ny, side, seed=None):
+    rng = np.random.default_rng(nx * ny if seed is None else seed)
     ids = np.arange(nx * ny)
     ii, jj = ids // ny, ids % ny
     X = np.stack([np.linspace(0.0, 1.0, nx)[ii], np.linspace(0.0, 1.0, ny)[jj]], axis=-1)
@@ -135,3 +135,52 @@ def test_far_nodes_do_not_spoil_the_scaling():
     sol = U.pde_solver(lap, lambda x, centers, rbf, fields: 0.0 * x[0], cloud, bcs, partial(U.gaussian, eps=12.0), 1,
                        options=U.SolverOptions(precision="fp64", reuse_factorization=False))
     assert np.max(np.abs(sol.vals - exact)) <= 3e-10
+
+
+@pytest.mark.parametrize("squeeze", [(0.001, 1.0), (0.01, 0.01)])
+def test_kernels_that_decouple_most_nodes(squeeze):
+    # Gaussians scaled to the finest spacing of an anisotropic (or half squeezed) cloud: K stays graded whatever its scaling,
+    # and the solution has to come out as FP64 multiply-adds give it.  LAPACK's lies within 2e-13 and 1e-11 of extended
+    # precision (four clouds each); 16 times what it gives here, and never less than 16 times 2e-14.
+    import scipy.linalg as sl
+    import updes_gb300 as U
+    from functools import partial
+    nx, ny, wide = 36, 24, np.longdouble
+    X = _nodes(nx, ny, 1.0, seed=0)
+    X = X * squeeze if squeeze[1] == 1.0 else np.where(X[:, :1] < 0.5, X * squeeze, X)
+    cloud = U.SquareCloud(Nx=nx, Ny=ny, coords=X, facet_types={f: "d" for f in ("South", "West", "North", "East")})
+    X = np.asarray(cloud.sorted_nodes)
+    N, Ni = cloud.N, cloud.Ni
+    d2 = ((X[:, None] - X[None]) ** 2).sum(-1)
+    eps = 0.8 / np.median(np.sqrt((d2 + 9.0 * np.eye(N)).min(1)))
+    low, span = X.min(0), X.max(0) - X.min(0)
+    x = ((X - low) / span).T
+    values = np.sin(2.0 * x[0]) * np.exp(x[1])
+    bcs = {f: values[np.asarray(cloud.facet_nodes[f])] for f in cloud.facet_types}
+    lap = lambda x, center, rbf, monomial, fields: U.nodal_laplacian(x, center, rbf, monomial)
+    rhs = lambda x: np.cos(3.0 * (x[0] - low[0]) / span[0] + (x[1] - low[1]) / span[1]) / np.max(span) ** 2
+    got = U.pde_solver(lap, lambda x, centers, rbf, fields: rhs(x), cloud, bcs, partial(U.gaussian, eps=eps), 1,
+                       options=U.SolverOptions(precision="fp64", reuse_factorization=False)).vals
+    # the same system in extended precision: K c = q with the kernels' own diagonal left out, A c at the nodes
+    Xw, e2 = X.astype(wide), wide(eps) ** 2
+    r2 = (Xw[:, None, 0] - Xw[None, :, 0]) ** 2 + (Xw[:, None, 1] - Xw[None, :, 1]) ** 2
+    phi = np.exp(-e2 * r2)
+    np.fill_diagonal(phi, 0.0)
+    P = np.concatenate([np.ones((N, 1), wide), Xw], axis=1)
+    A = np.concatenate([phi, P], axis=1)
+    K = np.concatenate([A, np.concatenate([P.T, np.zeros((3, 3), wide)], axis=1)])
+    K[:Ni, :N] = ((4.0 * e2 * e2 * r2 - 4.0 * e2) * phi)[:Ni]
+    K[:Ni, N:] = 0.0
+    q = np.concatenate([rhs(X[:Ni].T), values[Ni:], np.zeros(3)])
+    size = lambda m: 2.0 ** -np.frexp(m.astype(float))[1].astype(float)
+    r = size(np.abs(K).max(1))
+    c = size(np.abs(K * r[:, None]).max(0))
+    lu = sl.lu_factor((K * r[:, None] * c).astype(float))
+    y = sl.lu_solve(lu, r * q)
+    lapack = (A @ (c * y)).astype(float)
+    y = y.astype(wide)
+    for _ in range(4):
+        y = y + sl.lu_solve(lu, (r * (q - K @ (c * y))).astype(float))
+    want = (A @ (c * y)).astype(float)
+    error = lambda v: np.max(np.abs(v - want)) / np.max(np.abs(want))
+    assert error(got) <= 16.0 * max(error(lapack), 2e-14)

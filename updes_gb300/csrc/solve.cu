@@ -812,7 +812,8 @@ struct SolveWs {
   float* dinv128;  // the same for 128 x 128 blocks
   unsigned long long* xtag;  // tagged hand-off words of the 128-row triangular solves (2n)
   int32_t* piv;
-  int32_t* state;  // [0] n of the factored system, [1] precision of its factors, [2] 1 when valid
+  int32_t* state;  // [0] n of the factored system, [1] precision of its factors, [2] 1 when valid, [3] generation,
+                   // [4] 1 for FP64 factors made by multiply-adds instead of digit products
   int64_t ld;
 };
 
@@ -1076,19 +1077,27 @@ extern "C" int updes_solve_workspace(const updes_problem* p, const updes_solve_o
 
 namespace {
 
+constexpr int kStateInts = 5;
+
+// Backward error above which factors from digit products are not trusted (8,192 u): K is then factored again by FP64
+// multiply-adds, whatever its rows and columns look like.  The digits' own solutions of the kernels and clouds tried
+// lie at 2e-15 to 8e-14; where the scaled K is still graded (Gaussian kernels that decouple most of the nodes, 36 x 24 nodes on
+// 0.001 x 1: values wrong by 6.7e-12 instead of 6.6e-13) they lie at 1e-11 and above.
+constexpr double kDigitsBackwardError = 0x1p-40;
+
 // Factors of the equilibrated K (double-float planes) at `precision`; records the factored state.
 // planes_ready: the working copy already holds the equilibrated K, written by the assembly: for FP32 factors
 // the planes F32 and Wlo (double-float assembly), for FP64 factors the FP64 matrix W.
-int factor_launch(const SolveWs& w, int n, int precision, cudaStream_t s, bool planes_ready) {
+int factor_launch(const SolveWs& w, int n, int precision, cudaStream_t s, bool planes_ready, bool multiply_adds = false) {
   int e;
-  UPDES_CUDA_TRY(cudaMemsetAsync(w.state, 0, 4 * sizeof(int32_t), s));  // invalid until the factors are complete
+  UPDES_CUDA_TRY(cudaMemsetAsync(w.state, 0, kStateInts * sizeof(int32_t), s));  // invalid until the factors are complete
   const int64_t total = int64_t(n) * w.ld;
   if (precision == UPDES_PREC_FP64) {
     if (!planes_ready) {
       join_df_kernel<<<unsigned(ceil_div(total, 256)), 256, 0, s>>>(w.Khi, w.Klo, w.W, total);
       UPDES_LAUNCH_CHECK();
     }
-    e = factor_core(n, w.W, w.ld, precision, nullptr, w.ld, w.piv, w.lu, s, true);
+    e = factor_core(n, w.W, w.ld, precision, nullptr, w.ld, w.piv, w.lu, s, !multiply_adds);
   } else {
     if (!planes_ready) {
       UPDES_CUDA_TRY(cudaMemcpyAsync(w.F32, w.Khi, size_t(total) * 4, cudaMemcpyDeviceToDevice, s));
@@ -1102,34 +1111,37 @@ int factor_launch(const SolveWs& w, int n, int precision, cudaStream_t s, bool p
 }
 
 // Waits for what factor_launch issued, reports on it and marks the factors as complete.
-int factor_finish(const SolveWs& w, int n, int precision, updes_solve_info* info, cudaStream_t s, Timer& t) {
+int factor_finish(const SolveWs& w, int n, int precision, updes_solve_info* info, cudaStream_t s, Timer& t,
+                  bool multiply_adds = false) {
   int e;
   DeviceStatus h;
   if ((e = read_status(w.lu.st, s, &h))) return e;
   if (h.error) return h.error;
   info->lu_info = h.lu_info;
   info->t_factor_ms += t.stop();
-  // {n, precision, valid, generation}: the generation tells derived copies of these factors (the batched
+  // {n, precision, valid, generation, multiply_adds}: the generation tells derived copies of these factors (the batched
   // solves' double-float planes) that they are stale after a refactorisation
   static std::atomic<int32_t> generation{0};
-  const int32_t st4[4] = {n, precision, 1, generation.fetch_add(1) + 1};
-  UPDES_CUDA_TRY(cudaMemcpyAsync(w.state, st4, sizeof st4, cudaMemcpyHostToDevice, s));
+  const int32_t state[kStateInts] = {n, precision, 1, generation.fetch_add(1) + 1, multiply_adds};
+  UPDES_CUDA_TRY(cudaMemcpyAsync(w.state, state, sizeof state, cudaMemcpyHostToDevice, s));
   UPDES_CUDA_TRY(cudaStreamSynchronize(s));
   return UPDES_OK;
 }
 
-int factor_stage(const SolveWs& w, int n, int precision, updes_solve_info* info, cudaStream_t s, bool planes_ready) {
+int factor_stage(const SolveWs& w, int n, int precision, updes_solve_info* info, cudaStream_t s, bool planes_ready,
+                 bool multiply_adds = false) {
   Timer t(s);
-  if (int e = factor_launch(w, n, precision, s, planes_ready)) return e;
-  return factor_finish(w, n, precision, info, s, t);
+  if (int e = factor_launch(w, n, precision, s, planes_ready, multiply_adds)) return e;
+  return factor_finish(w, n, precision, info, s, t, multiply_adds);
 }
 
-int read_state(const SolveWs& w, int n, int* precision, cudaStream_t s) {
-  int32_t st3[3] = {0, 0, 0};
-  UPDES_CUDA_TRY(cudaMemcpyAsync(st3, w.state, sizeof st3, cudaMemcpyDeviceToHost, s));
+int read_state(const SolveWs& w, int n, int* precision, bool* multiply_adds, cudaStream_t s) {
+  int32_t state[kStateInts] = {};
+  UPDES_CUDA_TRY(cudaMemcpyAsync(state, w.state, sizeof state, cudaMemcpyDeviceToHost, s));
   UPDES_CUDA_TRY(cudaStreamSynchronize(s));
-  if (st3[2] != 1 || st3[0] != n) return UPDES_ERR_INVALID;
-  *precision = st3[1];
+  if (state[2] != 1 || state[0] != n) return UPDES_ERR_INVALID;
+  *precision = state[1];
+  *multiply_adds = state[4] != 0;
   return UPDES_OK;
 }
 
@@ -1230,8 +1242,9 @@ int solve_stage(const updes_problem* p, const SolveWs& w, int n, const double* q
                 cudaStream_t s) {
   const unsigned g = unsigned(ceil_div(n, 256));
   int precision, e;
-  if ((e = read_state(w, n, &precision, s))) return e;
-  for (int attempt = 0; attempt < 2; ++attempt) {
+  bool multiply_adds;
+  if ((e = read_state(w, n, &precision, &multiply_adds, s))) return e;
+  for (;;) {
     Timer t(s);
     if (qstride == 1) {
       rhs_kernel<<<g, 256, 0, s>>>(q, p->N, n, w.dr, w.bs);
@@ -1252,17 +1265,22 @@ int solve_stage(const updes_problem* p, const SolveWs& w, int n, const double* q
     if ((e = read_status(w.lu.st, s, &h))) return e;
     if (h.error) return h.error;
     info->t_refine_ms += t.stop();
-    if (precision == UPDES_PREC_FP64) {
+    const bool again = precision == UPDES_PREC_FP64 && !multiply_adds && !info->lu_info &&
+                       info->backward_error > kDigitsBackwardError;
+    if (precision == UPDES_PREC_FP64 && !again) {
       info->converged = 1;
       break;
     }
-    if (info->converged || !o.fallback_fp64) break;
+    if (precision == UPDES_PREC_FP32) {
+      if (info->converged || !o.fallback_fp64) break;
+      info->fell_back = 1;
+    }
     precision = UPDES_PREC_FP64;
-    info->fell_back = 1;
-    // the FP32 attempt overwrote the working matrix and scaled K as the mixed path does: assembled and scaled again
+    multiply_adds = again;
+    // the factors overwrote the working matrix, and the mixed path scales K in its own way: assembled and scaled again
     bool ready = false;
     if ((e = assemble_stage(p, w, n, precision, info, s, &ready))) return e;
-    if ((e = factor_stage(w, n, precision, info, s, true))) return e;
+    if ((e = factor_stage(w, n, precision, info, s, ready, multiply_adds))) return e;
   }
   Timer t(s);
   // the values of a mixed-precision solve in double-float (polyharmonic kernels; UPDES_DF_EVAL=0: FP64)
@@ -1564,23 +1582,30 @@ extern "C" int updes_solve_transpose(const updes_problem* p, const double* g, do
   if (!info) info = &dummy;
   std::memset(info, 0, sizeof *info);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  int precision = 0;
-  if (int e0 = read_state(w, n, &precision, s)) return e0;  // no factorisation of this system in the workspace
+  int precision = 0, e;
+  bool multiply_adds;
+  if ((e = read_state(w, n, &precision, &multiply_adds, s))) return e;  // no factorisation of this system in the workspace
   const unsigned gr = unsigned(ceil_div(n, 256));
   Timer t(s);
-  UPDES_CUDA_TRY(cudaMemsetAsync(w.lu.st, 0, sizeof(DeviceStatus), s));
-  // K^T lambda = g  <=>  Ks^T mu = dc .* g,  lambda = dr .* mu
-  UPDES_CUDA_TRY(cudaMemcpyAsync(w.bs, g, size_t(n) * 8, cudaMemcpyDeviceToDevice, s));
-  axpby_kernel<<<gr, 256, 0, s>>>(w.bs, 1.0, w.bs, 0.0, n, w.dc);
-  UPDES_LAUNCH_CHECK();
-  abs_kernel<<<gr, 256, 0, s>>>(w.bs, w.bsabs, n);
-  UPDES_LAUNCH_CHECK();
-  UPDES_CUDA_TRY(cudaMemcpyAsync(w.x, w.bs, size_t(n) * 8, cudaMemcpyDeviceToDevice, s));
-  int e;
-  if ((e = precond(w, n, precision, w.x, w.x, s, true))) return e;
-  updes_solve_opts oi = o;
-  if (precision == UPDES_PREC_FP64) oi.max_iters = 0;
-  if ((e = gmres(w, n, precision, oi, info, s, true))) return e;
+  for (;;) {
+    UPDES_CUDA_TRY(cudaMemsetAsync(w.lu.st, 0, sizeof(DeviceStatus), s));
+    // K^T lambda = g  <=>  Ks^T mu = dc .* g,  lambda = dr .* mu
+    UPDES_CUDA_TRY(cudaMemcpyAsync(w.bs, g, size_t(n) * 8, cudaMemcpyDeviceToDevice, s));
+    axpby_kernel<<<gr, 256, 0, s>>>(w.bs, 1.0, w.bs, 0.0, n, w.dc);
+    UPDES_LAUNCH_CHECK();
+    abs_kernel<<<gr, 256, 0, s>>>(w.bs, w.bsabs, n);
+    UPDES_LAUNCH_CHECK();
+    UPDES_CUDA_TRY(cudaMemcpyAsync(w.x, w.bs, size_t(n) * 8, cudaMemcpyDeviceToDevice, s));
+    if ((e = precond(w, n, precision, w.x, w.x, s, true))) return e;
+    updes_solve_opts oi = o;
+    if (precision == UPDES_PREC_FP64) oi.max_iters = 0;
+    if ((e = gmres(w, n, precision, oi, info, s, true))) return e;
+    if (precision != UPDES_PREC_FP64 || multiply_adds || info->backward_error <= kDigitsBackwardError) break;
+    multiply_adds = true;  // as in solve_stage
+    bool ready = false;
+    if ((e = assemble_stage(p, w, n, precision, info, s, &ready))) return e;
+    if ((e = factor_stage(w, n, precision, info, s, ready, multiply_adds))) return e;
+  }
   if (precision == UPDES_PREC_FP64) info->converged = 1;
   info->fell_back = precision == UPDES_PREC_FP64 && o.precision == UPDES_PREC_FP32;
   axpby_kernel<<<gr, 256, 0, s>>>(w.x, 1.0, w.x, 0.0, n, w.dr);
