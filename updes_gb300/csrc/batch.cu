@@ -60,10 +60,16 @@ __device__ __forceinline__ void split(double v, float& h, float& l) {
   l = float(v - double(h));
 }
 
-// Header of the batch workspace: {n, precision of the factors, valid, factor generation}
+// Header of the batch workspace: the system and the factors that it was prepared for.  N: of n = N + M; values: the
+// value matrix was prepared as well (not on local supports).
 struct BatchHeader {
-  int32_t n, precision, valid, generation;
+  int32_t n, precision, valid, generation, N, values;
 };
+// Whether a preparation is of the factors in the solve workspace (its state words).
+__device__ __forceinline__ bool describes(const BatchHeader* hdr, const int32_t* state, int n, int N) {
+  return state[0] == n && state[2] == 1 && hdr->n == n && hdr->N == N && hdr->valid == 1 && hdr->precision == state[1] &&
+         hdr->generation == state[3];
+}
 
 // A solved entry on its way to the blocks after it: two words, each with a tag in its high half (set: 1) and one FP32
 // half of the double-float value in its low half, each stored and loaded as one single-copy-atomic access.
@@ -93,15 +99,18 @@ __global__ void batch_residual_kernel(const double* __restrict__ Bs, const doubl
   Res[e] = Bs[e] - s;
 }
 
-// vals[i][c] = sum_p partial[p][i][c]; NaN if the header does not describe a preparation of an n x n system
+// vals[i][c] = sum_p partial[p][i][c]; NaN, and UPDES_ERR_INVALID in the status, if the header does not describe a
+// preparation of this system with its values
 __global__ void batch_values_kernel(const double* __restrict__ partial, int splits, int N, int n, int R,
-                                    double* __restrict__ vals, int64_t ldv, const BatchHeader* __restrict__ hdr) {
+                                    double* __restrict__ vals, int64_t ldv, const int32_t* __restrict__ state,
+                                    const BatchHeader* __restrict__ hdr, DeviceStatus* st) {
   const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const bool ok = describes(hdr, state, n, N) && hdr->values == 1;
+  if (!ok && e == 0) status_error(st, UPDES_ERR_INVALID);
   if (e >= int64_t(N) * R) return;
   const int64_t i = e / R, c = e % R;
   double s = 0.0;
   for (int p = 0; p < splits; ++p) s += partial[(int64_t(p) * N + i) * kMaxR + c];
-  const bool ok = hdr->n == n && hdr->valid == 1;
   vals[i * ldv + c] = ok ? s : __longlong_as_double(0x7ff8000000000000ll);
 }
 
@@ -113,8 +122,7 @@ __global__ void batch_rhs_kernel(const double* __restrict__ Q, int64_t ldq, int 
                                  const int32_t* __restrict__ state, const BatchHeader* __restrict__ hdr,
                                  DeviceStatus* st) {
   const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const bool ok = state[0] == n && state[2] == 1 && hdr->n == n && hdr->valid == 1 &&
-                  hdr->precision == state[1] && hdr->generation == state[3];
+  const bool ok = describes(hdr, state, n, N);
   if (!ok && e == 0) status_error(st, UPDES_ERR_INVALID);
   if (e >= int64_t(n) * R) return;
   const int i = int(e / R), c = int(e % R);
@@ -513,7 +521,7 @@ extern "C" int updes_batch_prepare(const updes_problem* p, void* workspace, size
       if ((e = value_rows(p, r0, rows, b.chunk, ld, s))) return e;
       if ((e = rhs64_matrix(b.chunk, nullptr, nullptr, ld, p->N, n, r0, rows, b.Vd, s))) return e;
     }
-  const BatchHeader hd{n, h[1], 1, h[3]};
+  const BatchHeader hd{n, h[1], 1, h[3], p->N, p->supports ? 0 : 1};
   UPDES_CUDA_TRY(cudaMemcpyAsync(b.hdr, &hd, sizeof hd, cudaMemcpyHostToDevice, s));
   UPDES_CUDA_TRY(cudaStreamSynchronize(s));
   return UPDES_OK;
@@ -577,7 +585,7 @@ extern "C" int updes_eval_values_prepared(const updes_problem* p, int32_t R, con
   const int splits = rhs64_splits(p->N, n);
   if ((e = rhs64_multiply(b.Vd, p->N, n, C, ldc, R, b.columns, b.partial, splits, st, s))) return e;
   batch_values_kernel<<<unsigned(ceil_div(int64_t(p->N) * R, 256)), 256, 0, s>>>(b.partial, splits, p->N, n, R, vals,
-                                                                               ldv, b.hdr);
+                                                                               ldv, state, b.hdr, st);
   UPDES_LAUNCH_CHECK();
   return UPDES_OK;
 }
