@@ -323,8 +323,8 @@ UPDES_API int updes_eval_values_batch(const updes_problem* p, int32_t R, const d
                                       int64_t ldv, void* stream);
 
 /*
- * The same values from what updes_batch_prepare derived (the value matrix [Phi P] as digits, multiplied on the
- * tensor cores): for callers that evaluate many blocks of one system, such as a time step after updes_solve_batch.
+ * The same values from what updes_batch_prepare derived (Phi as digits, multiplied on the tensor cores, P by FP64
+ * multiply-adds): for callers that evaluate many blocks of one system, such as a time step after updes_solve_batch.
  * workspace and batch_ws as there; a missing or stale preparation, or one of another system, gives NaN values and
  * UPDES_ERR_INVALID in the workspace's status word.  UPDES_ERR_UNSUPPORTED on local supports.
  */

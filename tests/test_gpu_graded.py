@@ -184,3 +184,34 @@ def test_kernels_that_decouple_most_nodes(squeeze):
     want = (A @ (c * y)).astype(float)
     error = lambda v: np.max(np.abs(v - want)) / np.max(np.abs(want))
     assert error(got) <= 16.0 * max(error(lapack), 2e-14)
+
+
+@pytest.mark.parametrize("side", [1.0, 2.0 ** -7, 2.0 ** -10])
+@pytest.mark.parametrize("nx,ny,a,degree", [(30, 20, 1, 1), (16, 16, 1, 2), (40, 13, 2, 2)])
+def test_time_step_values_on_a_small_domain(side, nx, ny, a, degree):
+    # vals = Phi C + P C: the kernel part from digits cut at 2^-56 of the largest entry of a row (column) in a block of 256
+    # columns (rows), twice 256 cuts of at most 2^-55 with the products left out; the sums and the polynomial part in FP64
+    import updes_gb300 as U
+    from functools import partial
+    from updes_gb300.multirhs import MultiRHSSolver
+    op = lambda x, center, rbf, monomial, fields=None: (U.nodal_value(x, center, rbf, monomial)
+                                                        - 0.01 * side ** 2 * U.nodal_laplacian(x, center, rbf, monomial))
+    cloud = U.SquareCloud(Nx=nx, Ny=ny, coords=_nodes(nx, ny, side),
+                          facet_types={f: "d" for f in ("South", "West", "North", "East")})
+    s = MultiRHSSolver(op, cloud, {f: np.zeros(len(cloud.facet_nodes[f])) for f in cloud.facet_types},
+                       partial(U.polyharmonic, a=a), degree)
+    X = np.asarray(cloud.sorted_nodes)
+    x = X.T / side
+    C, V = (t.cpu().numpy() for t in s.solve(np.stack([np.sin(3.0 * x[0]) * np.exp(x[1]), np.cos(x[0] + 2.0 * x[1])], axis=1)))
+    wide = np.longdouble
+    Xw = X.astype(wide)
+    phi = np.sqrt((Xw[:, None, 0] - Xw[None, :, 0]) ** 2 + (Xw[:, None, 1] - Xw[None, :, 1]) ** 2) ** (2 * a + 1)
+    powers = [(i - j, j) for i in range(degree + 1) for j in range(i + 1)]
+    P = np.stack([Xw[:, 0] ** i * Xw[:, 1] ** j for i, j in powers], axis=-1)
+    N = len(X)
+    want = (phi @ C[:N] + P @ C[N:]).astype(float)
+    bound = 16 * 2.0 ** -53 * (np.abs(phi) @ np.abs(C[:N]) + np.abs(P) @ np.abs(C[N:])).astype(float)
+    for k in range(0, N, 256):
+        bound += 512 * 2.0 ** -55 * np.outer(np.abs(phi[:, k:k + 256]).max(1), np.abs(C[k:min(k + 256, N)]).max(0)).astype(float)
+    wrong = np.abs(V - want) > bound
+    assert not wrong.any(), f"{int(wrong.sum())} values, by up to {np.max(np.abs(V - want) / bound):.1e} of the bound"

@@ -1047,25 +1047,24 @@ extern "C" int updes_eval_values_t(const updes_problem* p, const double* g, doub
   return UPDES_OK;
 }
 
-// Rows [r0, r0 + rows) of the value matrix [Phi P] (N x n, every node in a support), to out (rows x ld).
+// Rows [r0, r0 + rows) of the kernel part Phi of the value matrix (N x N, every node in a support), to out (rows x ld).
 namespace {
 template <int KIND>
 __global__ void __launch_bounds__(256) value_rows_kernel(updes_problem p, int r0, int rows, double* __restrict__ out,
                                                          int64_t ld) {
   const int ip = (KIND == UPDES_RBF_POLYHARMONIC) ? 2 * int(p.rbf_param) + 1 : int(p.rbf_param);
   const int j = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
-  if (i >= rows || j >= p.N + p.M) return;
+  if (i >= rows || j >= p.N) return;
   const int r = r0 + i;
   const double xi = p.nodes[2 * r], yi = p.nodes[2 * r + 1];
   double v = 0.0;
-  if (j >= p.N) v = monomial_terms(j - p.N, xi, yi).m;
-  else if (j != r || p.self_term) v = rbf_value<KIND>(xi - p.nodes[2 * j], yi - p.nodes[2 * j + 1], p.rbf_param, ip);
+  if (j != r || p.self_term) v = rbf_value<KIND>(xi - p.nodes[2 * j], yi - p.nodes[2 * j + 1], p.rbf_param, ip);
   out[int64_t(i) * ld + j] = v;
 }
 }  // namespace
 
 int value_rows(const updes_problem* p, int r0, int rows, double* out, int64_t ld, cudaStream_t s) {
-  const dim3 grid(unsigned(ceil_div(p->N + p->M, 256)), unsigned(rows));
+  const dim3 grid(unsigned(ceil_div(p->N, 256)), unsigned(rows));
   switch (p->rbf) {
     case UPDES_RBF_POLYHARMONIC: value_rows_kernel<UPDES_RBF_POLYHARMONIC><<<grid, 256, 0, s>>>(*p, r0, rows, out, ld); break;
     case UPDES_RBF_GAUSSIAN: value_rows_kernel<UPDES_RBF_GAUSSIAN><<<grid, 256, 0, s>>>(*p, r0, rows, out, ld); break;

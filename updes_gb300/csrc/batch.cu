@@ -8,7 +8,8 @@
 // applied in double-float arithmetic.  updes_batch_prepare derives once per factorisation what the calls read:
 //   * the inverses of the factors' 64 x 64 diagonal blocks and each block row times its inverse, as hi/lo FP32
 //     planes (about as accurate as an FP64 triangular solve, on the FP32 pipes);
-//   * the digits of Ks and of the value matrix [Phi P] for the tensor-core products (gemm_tc64.cu).
+//   * the digits of Ks and of the value matrix [Phi P], without the polynomial columns, for the tensor-core products
+//     (gemm_tc64.cu).
 //
 // Every double-float accumulation renormalises after each term (fast two-sum), so its error stays at
 // about 2^-48 of the running sum however many terms a thread adds.
@@ -19,6 +20,7 @@
 #include "common.cuh"
 #include "gemm_tc.cuh"
 #include "lu.cuh"
+#include "rbf.cuh"
 #include "stats.cuh"
 
 namespace {
@@ -88,20 +90,25 @@ __device__ __forceinline__ Word get_word(const Word* w) {  // past L1, so that a
 }
 __device__ __forceinline__ bool is_set(const Word& w) { return (w.hi >> 32) == 1 && (w.lo >> 32) == 1; }
 
-// Res = Bs - sum_p partial[p] (partials: splits x n x 64)
+// Res = Bs - sum_p partial[p] - K[:, N:] X[N:] (partials: splits x n x 64, the product with K's first N columns).  The
+// polynomial columns, and their coefficients, are of another size than the kernel's, with which they would share a digit
+// scale, and few: FP64 multiply-adds.
 __global__ void batch_residual_kernel(const double* __restrict__ Bs, const double* __restrict__ partial, int splits,
-                                      int n, int R, double* __restrict__ Res) {
+                                      int n, int N, int R, const float* __restrict__ Khi, const float* __restrict__ Klo,
+                                      int64_t ld, const double* __restrict__ X, double* __restrict__ Res) {
   const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (e >= int64_t(n) * R) return;
   const int64_t i = e / R, c = e % R;
   double s = 0.0;
   for (int p = 0; p < splits; ++p) s += partial[(int64_t(p) * n + i) * kMaxR + c];
+  for (int k = N; k < n; ++k) s = fma(double(Khi[i * ld + k]) + double(Klo[i * ld + k]), X[int64_t(k) * R + c], s);
   Res[e] = Bs[e] - s;
 }
 
-// vals[i][c] = sum_p partial[p][i][c]; NaN, and UPDES_ERR_INVALID in the status, if the header does not describe a
-// preparation of this system with its values
+// vals[i][c] = sum_p partial[p][i][c] + sum_k m_k(x_i) C[N + k][c]; NaN, and UPDES_ERR_INVALID in the status, if the header
+// does not describe a preparation of this system with its values
 __global__ void batch_values_kernel(const double* __restrict__ partial, int splits, int N, int n, int R,
+                                    const double* __restrict__ nodes, const double* __restrict__ C, int64_t ldc,
                                     double* __restrict__ vals, int64_t ldv, const int32_t* __restrict__ state,
                                     const BatchHeader* __restrict__ hdr, DeviceStatus* st) {
   const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -111,6 +118,8 @@ __global__ void batch_values_kernel(const double* __restrict__ partial, int spli
   const int64_t i = e / R, c = e % R;
   double s = 0.0;
   for (int p = 0; p < splits; ++p) s += partial[(int64_t(p) * N + i) * kMaxR + c];
+  const double x = nodes[2 * i], y = nodes[2 * i + 1];
+  for (int k = 0; k < n - N; ++k) s = fma(monomial_terms(k, x, y).m, C[int64_t(N + k) * ldc + c], s);
   vals[i * ldv + c] = ok ? s : __longlong_as_double(0x7ff8000000000000ll);
 }
 
@@ -514,12 +523,12 @@ extern "C" int updes_batch_prepare(const updes_problem* p, void* workspace, size
   UPDES_CUDA_TRY(cudaStreamSynchronize(s));
   if (h[0] != n || h[2] != 1) return UPDES_ERR_INVALID;  // no factorisation of this system in the workspace
   if ((e = h[1] == UPDES_PREC_FP64 ? prepare_factors(n, F64, ld, b, s) : prepare_factors(n, F32, ld, b, s))) return e;
-  if ((e = rhs64_matrix(nullptr, Khi, Klo, ld, n, n, 0, n, b.Kd, s))) return e;
+  if ((e = rhs64_matrix(nullptr, Khi, Klo, ld, n, p->N, 0, n, b.Kd, s))) return e;
   if (!p->supports)  // values on local supports have no batched form
     for (int r0 = 0; r0 < p->N; r0 += kChunk) {
       const int rows = std::min(kChunk, p->N - r0);
       if ((e = value_rows(p, r0, rows, b.chunk, ld, s))) return e;
-      if ((e = rhs64_matrix(b.chunk, nullptr, nullptr, ld, p->N, n, r0, rows, b.Vd, s))) return e;
+      if ((e = rhs64_matrix(b.chunk, nullptr, nullptr, ld, p->N, p->N, r0, rows, b.Vd, s))) return e;
     }
   const BatchHeader hd{n, h[1], 1, h[3], p->N, p->supports ? 0 : 1};
   UPDES_CUDA_TRY(cudaMemcpyAsync(b.hdr, &hd, sizeof hd, cudaMemcpyHostToDevice, s));
@@ -550,12 +559,12 @@ extern "C" int updes_solve_batch(const updes_problem* p, int32_t R, const double
   batch_rhs_kernel<<<g, 256, 0, s>>>(Q, ldq, p->N, n, R, dr, b.Bs, state, b.hdr, st);
   UPDES_LAUNCH_CHECK();
   if ((e = batch_precond(n, R, b, ld, piv, b.Bs, b.X, false, st, s))) return e;
-  const int splits = rhs64_splits(n, n);
+  const int splits = rhs64_splits(n, p->N);
   for (int it = 0; it < sweeps; ++it) {
     {
       StatScope sc(kStatGemv, s, 2.0 * n * n * R, 14.0 * n * double(n));
-      if ((e = rhs64_multiply(b.Kd, n, n, b.X, R, R, b.columns, b.partial, splits, st, s))) return e;
-      batch_residual_kernel<<<g, 256, 0, s>>>(b.Bs, b.partial, splits, n, R, b.D);
+      if ((e = rhs64_multiply(b.Kd, n, p->N, b.X, R, R, b.columns, b.partial, splits, st, s))) return e;
+      batch_residual_kernel<<<g, 256, 0, s>>>(b.Bs, b.partial, splits, n, p->N, R, Khi, Klo, ld, b.X, b.D);
       UPDES_LAUNCH_CHECK();
     }
     if ((e = batch_precond(n, R, b, ld, piv, b.D, b.X, true, st, s))) return e;
@@ -582,10 +591,10 @@ extern "C" int updes_eval_values_prepared(const updes_problem* p, int32_t R, con
   BatchWs b;
   batch_layout(n, static_cast<char*>(batch_ws), &b);
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const int splits = rhs64_splits(p->N, n);
-  if ((e = rhs64_multiply(b.Vd, p->N, n, C, ldc, R, b.columns, b.partial, splits, st, s))) return e;
-  batch_values_kernel<<<unsigned(ceil_div(int64_t(p->N) * R, 256)), 256, 0, s>>>(b.partial, splits, p->N, n, R, vals,
-                                                                               ldv, state, b.hdr, st);
+  const int splits = rhs64_splits(p->N, p->N);
+  if ((e = rhs64_multiply(b.Vd, p->N, p->N, C, ldc, R, b.columns, b.partial, splits, st, s))) return e;
+  batch_values_kernel<<<unsigned(ceil_div(int64_t(p->N) * R, 256)), 256, 0, s>>>(
+      b.partial, splits, p->N, n, R, p->nodes, C, ldc, vals, ldv, state, b.hdr, st);
   UPDES_LAUNCH_CHECK();
   return UPDES_OK;
 }
