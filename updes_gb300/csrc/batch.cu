@@ -30,6 +30,7 @@ constexpr int kMaxR = 64;    // right-hand sides per call
 constexpr int kCG = 8;       // right-hand sides per triangular-solve CTA
 constexpr int kLdt = kB + 8; // row stride of a staged tile: the 4 rows x 8 columns a warp reads at once fall in 32 banks
 constexpr int kChunk = 256;  // value rows staged at a time
+constexpr int kMaxM = 15;    // monomials of a system, at most (degree 4)
 
 __device__ __forceinline__ float2 sub2(float2 y, float2 x) { return __ffma2_rn(x, make_float2(-1.f, -1.f), y); }
 
@@ -90,25 +91,53 @@ __device__ __forceinline__ Word get_word(const Word* w) {  // past L1, so that a
 }
 __device__ __forceinline__ bool is_set(const Word& w) { return (w.hi >> 32) == 1 && (w.lo >> 32) == 1; }
 
-// Res = Bs - sum_p partial[p] - K[:, N:] X[N:] (partials: splits x n x 64, the product with K's first N columns).  The
-// polynomial columns, and their coefficients, are of another size than the kernel's, with which they would share a digit
-// scale, and few: FP64 multiply-adds.
+// The polynomial columns of K and of the value matrix, and their coefficients, are of another size than the kernel's, with
+// which they would share a digit scale, and few: FP64 multiply-adds.  KP (n x M) and VP (N x M), written while preparing
+// (from the planes and the nodes in each call they cost 20 us of a step's 4,700 at n = 6,403).
+__global__ void polynomial_columns_kernel(const float* __restrict__ Khi, const float* __restrict__ Klo, int64_t ld,
+                                          const double* __restrict__ nodes, int n, int N, double* __restrict__ KP,
+                                          double* __restrict__ VP) {
+  const int M = n - N, e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= n * M) return;
+  const int i = e / M, k = e % M;
+  KP[e] = double(Khi[int64_t(i) * ld + N + k]) + double(Klo[int64_t(i) * ld + N + k]);
+  if (i < N) VP[e] = monomial_terms(k, nodes[2 * i], nodes[2 * i + 1]).m;
+}
+
+// s + sum_k P[k] X[k ldx], k < M <= kMaxM, the loads in flight together
+__device__ __forceinline__ double add_polynomial(double s, const double* __restrict__ P, const double* __restrict__ X,
+                                                 int64_t ldx, int M) {
+  double p[kMaxM], x[kMaxM];
+#pragma unroll
+  for (int k = 0; k < kMaxM; ++k) {
+    if (k >= M) break;
+    p[k] = P[k];
+    x[k] = X[k * ldx];
+  }
+#pragma unroll
+  for (int k = 0; k < kMaxM; ++k) {
+    if (k >= M) break;
+    s = fma(p[k], x[k], s);
+  }
+  return s;
+}
+
+// Res = Bs - sum_p partial[p] - KP X[N:] (partials: splits x n x 64, the product with K's first N columns)
 __global__ void batch_residual_kernel(const double* __restrict__ Bs, const double* __restrict__ partial, int splits,
-                                      int n, int N, int R, const float* __restrict__ Khi, const float* __restrict__ Klo,
-                                      int64_t ld, const double* __restrict__ X, double* __restrict__ Res) {
+                                      int n, int N, int R, const double* __restrict__ KP, const double* __restrict__ X,
+                                      double* __restrict__ Res) {
   const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (e >= int64_t(n) * R) return;
   const int64_t i = e / R, c = e % R;
   double s = 0.0;
   for (int p = 0; p < splits; ++p) s += partial[(int64_t(p) * n + i) * kMaxR + c];
-  for (int k = N; k < n; ++k) s = fma(double(Khi[i * ld + k]) + double(Klo[i * ld + k]), X[int64_t(k) * R + c], s);
-  Res[e] = Bs[e] - s;
+  Res[e] = Bs[e] - add_polynomial(s, KP + i * (n - N), X + int64_t(N) * R + c, R, n - N);
 }
 
-// vals[i][c] = sum_p partial[p][i][c] + sum_k m_k(x_i) C[N + k][c]; NaN, and UPDES_ERR_INVALID in the status, if the header
+// vals[i][c] = sum_p partial[p][i][c] + sum_k VP[i][k] C[N + k][c]; NaN, and UPDES_ERR_INVALID in the status, if the header
 // does not describe a preparation of this system with its values
 __global__ void batch_values_kernel(const double* __restrict__ partial, int splits, int N, int n, int R,
-                                    const double* __restrict__ nodes, const double* __restrict__ C, int64_t ldc,
+                                    const double* __restrict__ VP, const double* __restrict__ C, int64_t ldc,
                                     double* __restrict__ vals, int64_t ldv, const int32_t* __restrict__ state,
                                     const BatchHeader* __restrict__ hdr, DeviceStatus* st) {
   const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -118,8 +147,7 @@ __global__ void batch_values_kernel(const double* __restrict__ partial, int spli
   const int64_t i = e / R, c = e % R;
   double s = 0.0;
   for (int p = 0; p < splits; ++p) s += partial[(int64_t(p) * N + i) * kMaxR + c];
-  const double x = nodes[2 * i], y = nodes[2 * i + 1];
-  for (int k = 0; k < n - N; ++k) s = fma(monomial_terms(k, x, y).m, C[int64_t(N + k) * ldc + c], s);
+  s = add_polynomial(s, VP + i * (n - N), C + int64_t(N) * ldc + c, ldc, n - N);
   vals[i * ldv + c] = ok ? s : __longlong_as_double(0x7ff8000000000000ll);
 }
 
@@ -402,7 +430,7 @@ __global__ void __launch_bounds__(kTriThreads) batch_tri_kernel(const float* __r
 struct BatchWs {
   BatchHeader* hdr;
   float *Gh, *Gl, *tilesL, *tilesU;  // premultiplied factors, inverted diagonal blocks
-  double *invL, *invU, *Bs, *X, *D, *partial, *chunk;
+  double *invL, *invU, *Bs, *X, *D, *partial, *chunk, *KP, *VP;
   Word* words;  // tickets (the first word), then the words of both solves
   void *Kd, *Vd, *columns;  // digits of Ks, of the value matrix, of a multiplied block
 };
@@ -431,6 +459,8 @@ size_t batch_layout(int n, char* base, BatchWs* w) {
   b.words = reinterpret_cast<Word*>(take((1 + 2 * size_t(n) * kMaxR) * sizeof(Word)));
   b.partial = reinterpret_cast<double*>(take(kRhs64MaxSplits * v));
   b.chunk = reinterpret_cast<double*>(take(size_t(kChunk) * ld * sizeof(double)));
+  b.KP = reinterpret_cast<double*>(take(size_t(n) * kMaxM * sizeof(double)));
+  b.VP = reinterpret_cast<double*>(take(size_t(n) * kMaxM * sizeof(double)));
   b.Kd = take(rhs64_matrix_bytes(n, n));
   b.Vd = take(rhs64_matrix_bytes(n, n));
   b.columns = take(rhs64_columns_bytes(n));
@@ -524,6 +554,9 @@ extern "C" int updes_batch_prepare(const updes_problem* p, void* workspace, size
   if (h[0] != n || h[2] != 1) return UPDES_ERR_INVALID;  // no factorisation of this system in the workspace
   if ((e = h[1] == UPDES_PREC_FP64 ? prepare_factors(n, F64, ld, b, s) : prepare_factors(n, F32, ld, b, s))) return e;
   if ((e = rhs64_matrix(nullptr, Khi, Klo, ld, n, p->N, 0, n, b.Kd, s))) return e;
+  polynomial_columns_kernel<<<unsigned(ceil_div(int64_t(n) * p->M, 256)), 256, 0, s>>>(Khi, Klo, ld, p->nodes, n, p->N, b.KP,
+                                                                                     b.VP);
+  UPDES_LAUNCH_CHECK();
   if (!p->supports)  // values on local supports have no batched form
     for (int r0 = 0; r0 < p->N; r0 += kChunk) {
       const int rows = std::min(kChunk, p->N - r0);
@@ -564,7 +597,7 @@ extern "C" int updes_solve_batch(const updes_problem* p, int32_t R, const double
     {
       StatScope sc(kStatGemv, s, 2.0 * n * n * R, 14.0 * n * double(n));
       if ((e = rhs64_multiply(b.Kd, n, p->N, b.X, R, R, b.columns, b.partial, splits, st, s))) return e;
-      batch_residual_kernel<<<g, 256, 0, s>>>(b.Bs, b.partial, splits, n, p->N, R, Khi, Klo, ld, b.X, b.D);
+      batch_residual_kernel<<<g, 256, 0, s>>>(b.Bs, b.partial, splits, n, p->N, R, b.KP, b.X, b.D);
       UPDES_LAUNCH_CHECK();
     }
     if ((e = batch_precond(n, R, b, ld, piv, b.D, b.X, true, st, s))) return e;
@@ -594,7 +627,7 @@ extern "C" int updes_eval_values_prepared(const updes_problem* p, int32_t R, con
   const int splits = rhs64_splits(p->N, p->N);
   if ((e = rhs64_multiply(b.Vd, p->N, p->N, C, ldc, R, b.columns, b.partial, splits, st, s))) return e;
   batch_values_kernel<<<unsigned(ceil_div(int64_t(p->N) * R, 256)), 256, 0, s>>>(
-      b.partial, splits, p->N, n, R, p->nodes, C, ldc, vals, ldv, state, b.hdr, st);
+      b.partial, splits, p->N, n, R, b.VP, C, ldc, vals, ldv, state, b.hdr, st);
   UPDES_LAUNCH_CHECK();
   return UPDES_OK;
 }
