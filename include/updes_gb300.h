@@ -293,11 +293,11 @@ UPDES_API int updes_solve_factored(const updes_problem* p, int32_t nrhs, const d
  * Batched right-hand sides with a fixed number of refinement sweeps.  R <= 64
  * columns of the row-major N x R block Q (ldq) are solved together against the
  * factors that updes_factor left in `workspace`: X = M^-1 Q, then `sweeps`
- * times X += M^-1 (Q - K X), with the residual and the triangular solves in
- * double-float arithmetic; coeffs (n x R, ldc) receives X.  FP64 factors
- * (precision UPDES_PREC_FP64) give M^-1 the accuracy of an FP64 solve, so one
- * sweep reaches FP64 quality; FP32 factors converge only as fast as classical
- * refinement on them allows.
+ * times X += M^-1 (Q - K X), with the triangular solves in double-float
+ * arithmetic and the residual from exact products of digits; coeffs (n x R,
+ * ldc) receives X.  With FP64 factors (precision UPDES_PREC_FP64) one sweep
+ * reaches FP64 quality, and they get one whatever `sweeps` says; FP32 factors
+ * converge only as fast as classical refinement on them allows.
  * updes_batch_prepare (once per factorisation; synchronises) derives the
  * batch's copy of the factors, and the digits of K and of the value matrix.  updes_solve_batch then only launches kernels on
  * `stream`: no synchronisation and no host reads, so a time step built from it

@@ -69,3 +69,27 @@ def test_a_preparation_on_local_supports_has_no_values():
     assert local.dp.c.support_width > 0 and full.dp.c.support_width == 0
     V, status = _values(full.dp, local.ws, local.bws)
     assert torch.isnan(V).all() and status == _lib.ERR_INVALID
+
+
+@pytest.mark.parametrize("nx,ny,a,degree,substitution", [(30, 20, 1, 1, 1.2e-12), (40, 35, 2, 2, 8.0e-11), (24, 24, 3, 2, 5.2e-10)])
+@pytest.mark.parametrize("R", [1, 9])
+def test_triangles_are_solved_as_accurately_as_by_substitution(nx, ny, a, degree, substitution, R):
+    # Values without a refinement sweep asked for, against the refined ones.  A substitution in 48-bit arithmetic leaves
+    # 1.2e-12, 8e-11 and 5.2e-10 of the largest value (emulated on a CPU for r^3, r^5 and r^7); 32 times that.
+    from functools import partial
+    rng = np.random.default_rng(0)
+    ids = np.arange(nx * ny)
+    ii, jj = ids // ny, ids % ny
+    coords = np.stack([np.linspace(0.0, 1.0, nx)[ii], np.linspace(0.0, 1.0, ny)[jj]], axis=-1)
+    inner = (ii > 0) & (ii < nx - 1) & (jj > 0) & (jj < ny - 1)
+    coords[inner] += rng.uniform(-0.2, 0.2, size=(nx * ny, 2))[inner] * min(1.0 / (nx - 1), 1.0 / (ny - 1))
+    cloud = U.SquareCloud(Nx=nx, Ny=ny, coords=coords, facet_types=FACETS)
+    lap = lambda x, center, rbf, monomial, fields=None: U.nodal_laplacian(x, center, rbf, monomial)
+    s = MultiRHSSolver(lap, cloud, {f: np.zeros(len(cloud.facet_nodes[f])) for f in FACETS},
+                       partial(U.polyharmonic, a=a), degree, sweeps=0)
+    x = np.asarray(cloud.sorted_nodes).T
+    Q = np.stack([np.sin((3.0 + k) * x[0]) * np.cosh(x[1]) for k in range(R)], axis=1)
+    plain = s.solve(Q)[1].cpu().numpy()
+    s.sweeps = 4
+    want = s.solve(Q)[1].cpu().numpy()
+    assert np.max(np.abs(plain - want)) <= 32 * substitution * np.max(np.abs(want))

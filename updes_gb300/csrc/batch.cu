@@ -6,13 +6,13 @@
 //   X = M^-1 Bs;  repeat `sweeps` times:  X += M^-1 (Bs - Ks X)
 // with Ks the equilibrated K (the exact sum of the solve workspace's double-float planes) and M^-1 the LU factors
 // applied in double-float arithmetic.  updes_batch_prepare derives once per factorisation what the calls read:
-//   * the inverses of the factors' 64 x 64 diagonal blocks and each block row times its inverse, as hi/lo FP32
-//     planes (about as accurate as an FP64 triangular solve, on the FP32 pipes);
+//   * the inverses of the factors' 64 x 64 diagonal blocks and each block row times its inverse (or, for an ill-conditioned
+//     block, as it is), as hi/lo FP32 planes: a solve leaves residuals of about 2^-48, on the FP32 pipes;
 //   * the digits of Ks and of the value matrix [Phi P], without the polynomial columns, for the tensor-core products
 //     (gemm_tc64.cu).
 //
-// Every double-float accumulation renormalises after each term (fast two-sum), so its error stays at
-// about 2^-48 of the running sum however many terms a thread adds.
+// A thread's double-float sums are renormalised every eight terms, so their error stays at about 2^-46 of the running sum
+// however many terms it adds.
 #include <algorithm>
 #include <atomic>
 #include <cstring>
@@ -31,6 +31,7 @@ constexpr int kCG = 8;       // right-hand sides per triangular-solve CTA
 constexpr int kLdt = kB + 8; // row stride of a staged tile: the 4 rows x 8 columns a warp reads at once fall in 32 banks
 constexpr int kChunk = 256;  // value rows staged at a time
 constexpr int kMaxM = 15;    // monomials of a system, at most (degree 4)
+constexpr int kMaxBlocks = 1024;  // block rows; a factorisation has at most 800 (n <= 51,200)
 
 __device__ __forceinline__ float2 sub2(float2 y, float2 x) { return __ffma2_rn(x, make_float2(-1.f, -1.f), y); }
 
@@ -125,7 +126,8 @@ __device__ __forceinline__ double add_polynomial(double s, const double* __restr
 // Res = Bs - sum_p partial[p] - KP X[N:] (partials: splits x n x 64, the product with K's first N columns)
 __global__ void batch_residual_kernel(const double* __restrict__ Bs, const double* __restrict__ partial, int splits,
                                       int n, int N, int R, const double* __restrict__ KP, const double* __restrict__ X,
-                                      double* __restrict__ Res) {
+                                      double* __restrict__ Res, const int32_t* __restrict__ skip) {
+  if (skip && *skip) return;
   const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (e >= int64_t(n) * R) return;
   const int64_t i = e / R, c = e % R;
@@ -175,21 +177,40 @@ __global__ void batch_unscale_kernel(const double* __restrict__ X, const double*
   out[int64_t(i) * ldo + c] = dc[i] * X[e];
 }
 
-// Inverses of the diagonal blocks of a triangular factor F (LOWER: unit lower), 64 x 64 each, and their hi/lo planes
-// (tiles[blk] = {hi, lo}).  Rows and columns beyond n count as the identity.
+// A block row is solved with its diagonal block's inverse I_b either before or after its sum: x_b = I_b y_b + sum G x with
+// G = -I_b T (a hand-off costs one product), or, where |I_b| |T_bb| has a row sum above kPremultiplied, x_b = I_b r with
+// r = y_b - sum T x and one step of refinement, x_b += I_b (r - T_bb x_b) (three products more).  The first rounds
+// I_b y_b and the products before they cancel, which leaves residuals of up to that row sum times 2^-48 (a substitution:
+// 2^-48), and a refinement sweep brings those down only while they are small: r^7 with 576 nodes has row sums of 5e5, and
+// its values were wrong by 8e-5 without a sweep, 5e-10 with one (by substitution 5e-10 and 3e-11).  Below the limit one sweep
+// leaves what it leaves after a substitution (r^3, r^5, r^7 and multiquadrics of 600 to 3,000 nodes), so a solve
+// on FP64 factors has at least one.  At a limit of 256 the steps of 6,403 multiquadrics took
+// 10 % longer, at 4,096 0.5 %, here 0.1 %.
+constexpr double kPremultiplied = 16384.0;
+
+// Three pairs of 64 x 64 hi/lo planes a diagonal block: what the right-hand side is multiplied by (I_b, or the identity),
+// and for the second form I_b and -T_bb.
+constexpr int kTilePlanes = 6;
+
+// Inverses of the diagonal blocks of a triangular factor F (LOWER: unit lower), 64 x 64 each, their planes (see above) and
+// which form their rows take (after[blk] = 1: the second).  Rows and columns beyond n count as the identity.
 struct InverseSmem {
   double T[kB][kB + 1], I[kB][kB + 1];
 };
 
 template <typename TF, bool LOWER>
 __global__ void __launch_bounds__(256) tri_inverse_kernel(const TF* __restrict__ F, int64_t ldf, int n,
-                                                          double* __restrict__ inv, float* __restrict__ tiles) {
+                                                          double* __restrict__ inv, float* __restrict__ tiles,
+                                                          int32_t* __restrict__ after) {
   extern __shared__ double inv_smem[];
   InverseSmem& sm = *reinterpret_cast<InverseSmem*>(inv_smem);
+  __shared__ double row_sum[kB];
   const int blk = blockIdx.x, r0 = blk * kB, tid = threadIdx.x;
   for (int e = tid; e < kB * kB; e += blockDim.x) {
     const int i = e >> 6, j = e & 63;
-    sm.T[i][j] = (r0 + i < n && r0 + j < n) ? double(F[int64_t(r0 + i) * ldf + r0 + j]) : (i == j ? 1.0 : 0.0);
+    double t = (r0 + i < n && r0 + j < n) ? double(F[int64_t(r0 + i) * ldf + r0 + j]) : (i == j ? 1.0 : 0.0);
+    if (LOWER ? j >= i : j < i) t = LOWER && i == j ? 1.0 : 0.0;  // the triangle alone
+    sm.T[i][j] = t;
   }
   __syncthreads();
   if (tid < kB) {  // a column of the inverse by substitution
@@ -207,27 +228,55 @@ __global__ void __launch_bounds__(256) tri_inverse_kernel(const TF* __restrict__
     }
   }
   __syncthreads();
-  float* out = tiles + int64_t(blk) * 2 * kB * kB;
+  if (tid < kB) {
+    double t = 0.0;
+    for (int k = 0; k < kB; ++k) t += fabs(sm.T[tid][k]);
+    row_sum[tid] = t;
+  }
+  __syncthreads();
+  bool large = false;
+  if (tid < kB) {
+    double t = 0.0;
+    for (int k = 0; k < kB; ++k) t = fma(fabs(sm.I[tid][k]), row_sum[k], t);  // of |I_b| |T_bb|
+    large = !(t <= kPremultiplied);
+  }
+  const bool second = __syncthreads_or(large);
+  if (tid == 0) after[blk] = second;
+  float* out = tiles + int64_t(blk) * kTilePlanes * kB * kB;
   for (int e = tid; e < kB * kB; e += blockDim.x) {
-    const double x = sm.I[e >> 6][e & 63];
+    const int i = e >> 6, j = e & 63;
+    const double x = sm.I[i][j];
     inv[int64_t(blk) * kB * kB + e] = x;
-    split(x, out[e], out[kB * kB + e]);
+    split(second ? (i == j ? 1.0 : 0.0) : x, out[e], out[kB * kB + e]);
+    if (!second) continue;
+    split(x, out[2 * kB * kB + e], out[3 * kB * kB + e]);
+    split(-sm.T[i][j], out[4 * kB * kB + e], out[5 * kB * kB + e]);
   }
 }
 
-// G = -I_b T for every block T of block row b beside the diagonal (below it in L, above it in U), as hi/lo planes in
-// the place of T; a CTA a block, the lower triangle's inverses in invL, the upper's in invU.
+// G = -I_b T, or -T for the rows of the second form, for every block T of block row b beside the diagonal (below it in L,
+// above it in U), as hi/lo planes in the place of T; a CTA a block, the lower triangle's inverses in invL, the upper's in invU.
 template <typename TF>
 __global__ void __launch_bounds__(256) tri_premultiply_kernel(const TF* __restrict__ F, int64_t ldf, int n,
                                                               const double* __restrict__ invL,
-                                                              const double* __restrict__ invU, float* __restrict__ Gh,
-                                                              float* __restrict__ Gl) {
+                                                              const double* __restrict__ invU,
+                                                              const int32_t* __restrict__ afterL,
+                                                              const int32_t* __restrict__ afterU,
+                                                              float* __restrict__ Gh, float* __restrict__ Gl) {
   extern __shared__ double inv_smem[];
   InverseSmem& sm = *reinterpret_cast<InverseSmem*>(inv_smem);
   const int b = blockIdx.y, q = blockIdx.x, tid = threadIdx.x;
   if (b == q) return;
   const double* inv = (q < b ? invL : invU) + int64_t(b) * kB * kB;
   const int r0 = b * kB, c0 = q * kB;
+  if ((q < b ? afterL : afterU)[b]) {
+    for (int e = tid; e < kB * kB; e += blockDim.x) {
+      const int r = r0 + (e >> 6), c = c0 + (e & 63);
+      if (r < n && c < ldf)
+        split(c < n ? -double(F[int64_t(r) * ldf + c]) : 0.0, Gh[int64_t(r) * ldf + c], Gl[int64_t(r) * ldf + c]);
+    }
+    return;
+  }
   for (int e = tid; e < kB * kB; e += blockDim.x) {
     const int i = e >> 6, j = e & 63;
     sm.I[i][j] = inv[e];
@@ -259,11 +308,12 @@ __global__ void __launch_bounds__(256) tri_premultiply_kernel(const TF* __restri
 // Triangular solve of n x R right-hand sides (LOWER: unit lower, forward; else upper, backward).
 // One CTA per (64-row block, group of 8 right-hand sides), taken in ticket order.  Block b is
 //   x_b = I_b y_b + sum_q G_bq x_q,   G_bq = -I_b T_bq,
-// with I_b the inverted diagonal block: what is left to do when x_{b-1} arrives is one 64 x 64 product and one
-// hand-off (a substitution inside each block and hand-offs through counters and fences made the chain 32 us a block).
+// with I_b the inverted diagonal block (or, by after[b], the second form above): what is left to do when x_{b-1} arrives is
+// one 64 x 64 product and one hand-off (a substitution inside each block and hand-offs through counters and fences made the
+// chain 32 us a block).
 // Tiles are staged by cp.async one ahead, and the words of a block are read one tile ahead of their use, so blocks
 // solved long ago cost no waiting.
-// Bound by the FP32 pipes for many columns (15 packed instructions per two double-float multiply-adds, which issue every
+// Bound by the FP32 pipes for many columns (12 packed instructions per two double-float multiply-adds, which issue every
 // other cycle: 64 columns of n = 6,406 take 0.96 ms a triangle), by the chain for few (8
 // columns: 0.45 ms, 4.4 us a block).
 // A thread owns rows rg + 16 u (u < 4), the columns 2 cg and 2 cg + 1, and every eighth term of the inner sum.
@@ -274,34 +324,27 @@ struct TriSmem {
   float Xh[2][kB][kCG], Xl[2][kB][kCG];
 };
 
-template <bool LOWER>
-__global__ void __launch_bounds__(kTriThreads) batch_tri_kernel(const float* __restrict__ Gh,
-                                                                const float* __restrict__ Gl, int64_t ldg,
-                                                                const float* __restrict__ tiles, int n, int R,
-                                                                const double* __restrict__ Bin,
-                                                                const int32_t* __restrict__ perm, const Word* win,
-                                                                Word* wout, double* Y, int accumulate, int* ticket,
-                                                                DeviceStatus* st) {
-  extern __shared__ float4 tri_smem[];
-  TriSmem& sm = *reinterpret_cast<TriSmem*>(tri_smem);
-  __shared__ int s_tk;
+// One (block row, column group).  The second form has code of its own, out of line: a block runs its code once, on the chain,
+// and the form's instructions between those of the first cost that 0.2 us a block, taken or not.
+template <bool LOWER, bool SECOND>
+__device__ __noinline__ void tri_block(TriSmem& sm, int t, int cbase, const float* __restrict__ Gh,
+                                          const float* __restrict__ Gl, int64_t ldg, const float* __restrict__ tiles, int n,
+                                          int R, const double* __restrict__ Bin, const int32_t* __restrict__ perm,
+                                          const Word* win, Word* wout, double* Y, int accumulate, DeviceStatus* st) {
   const int tid = threadIdx.x;
   const int ks = tid & (kKs - 1), rg = (tid >> 3) & 15, cg = tid >> 7;
-  const int G = int(ceil_div(R, kCG)), nblk = int(ceil_div(n, kB));
-  if (tid == 0) s_tk = atomicAdd(ticket, 1);
-  __syncthreads();
-  const int t = s_tk / G, cbase = (s_tk % G) * kCG;
-  if (t >= nblk) return;
+  const int nblk = int(ceil_div(n, kB));
   const int blk = LOWER ? t : nblk - 1 - t, r0 = blk * kB;
   auto block_at = [&](int q) { return LOWER ? q : nblk - 1 - q; };  // the q-th block to be solved
 
-  // item 0 is the inverse times the right-hand side, item i > 0 the product with the (i-1)-th solved block
+  // item 0 is the inverse (or the identity) times the right-hand side, item i, 1 <= i <= t, the product with the (i-1)-th
+  // solved block; items t + 1 .. t + 3 are those of the second form: I_b r, -T_bb x, I_b times what is left
   auto stage = [&](int i) {
     const float *hi, *lo;
     int64_t ld;
     int rows = kB, cols = kB;
-    if (i == 0) {
-      hi = tiles + int64_t(blk) * 2 * kB * kB;
+    if (i == 0 || (SECOND && i > t)) {
+      hi = tiles + (int64_t(blk) * kTilePlanes + (i == 0 ? 0 : i == t + 2 ? 4 : 2)) * kB * kB;
       lo = hi + kB * kB;
       ld = kB;
     } else {
@@ -347,6 +390,52 @@ __global__ void __launch_bounds__(kTriThreads) batch_tri_kernel(const float* __r
   float2 ah[4], al[4];
 #pragma unroll
   for (int u = 0; u < 4; ++u) ah[u] = al[u] = make_float2(0.f, 0.f);
+  // The sum over the eight threads of a row: each exchange also halves what a thread keeps, down to one row of a pair
+  // of columns in two threads, so that thread ks ends with row rg + 16 (ks & 3), column 2 cg + (ks >> 2), in (h, l).
+  auto reduce = [&](float& h, float& l) {
+#pragma unroll
+    for (int u = 0; u < 4; u += 2) {  // lanes that differ in bit 0 split rows u, u + 1
+      const bool up = ks & 1;
+      const float2 sh = up ? ah[u] : ah[u + 1], sl = up ? al[u] : al[u + 1];
+      float2 kh = up ? ah[u + 1] : ah[u], kl = up ? al[u + 1] : al[u];
+      df_add(__shfl_xor_sync(0xffffffffu, sh.x, 1), __shfl_xor_sync(0xffffffffu, sl.x, 1), kh.x, kl.x);
+      df_add(__shfl_xor_sync(0xffffffffu, sh.y, 1), __shfl_xor_sync(0xffffffffu, sl.y, 1), kh.y, kl.y);
+      ah[u] = kh;
+      al[u] = kl;
+    }
+    float2 rh, rl;
+    {
+      const bool up = ks & 2;
+      const float2 sh = up ? ah[0] : ah[2], sl = up ? al[0] : al[2];
+      rh = up ? ah[2] : ah[0];
+      rl = up ? al[2] : al[0];
+      df_add(__shfl_xor_sync(0xffffffffu, sh.x, 2), __shfl_xor_sync(0xffffffffu, sl.x, 2), rh.x, rl.x);
+      df_add(__shfl_xor_sync(0xffffffffu, sh.y, 2), __shfl_xor_sync(0xffffffffu, sl.y, 2), rh.y, rl.y);
+    }
+    const bool up = ks & 4;
+    h = up ? rh.y : rh.x;
+    l = up ? rl.y : rl.x;
+    df_add(__shfl_xor_sync(0xffffffffu, up ? rh.x : rh.y, 4), __shfl_xor_sync(0xffffffffu, up ? rl.x : rl.y, 4), h, l);
+  };
+  // ah, al += the staged item times its 64 x 8 block
+  auto multiply = [&](int b) {
+#pragma unroll
+    for (int k = 0; k < kB / kKs; ++k) {
+      const int kk = kKs * k + ks;
+      const float2 xh = *reinterpret_cast<const float2*>(&sm.Xh[b][kk][2 * cg]);
+      const float2 xn = *reinterpret_cast<const float2*>(&sm.Xn[b][kk][2 * cg]);
+      const float2 xl = *reinterpret_cast<const float2*>(&sm.Xl[b][kk][2 * cg]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        df_mac2(sm.F[b][0][rg + 16 * u][kk], sm.F[b][1][rg + 16 * u][kk], xh, xn, xl, ah[u], al[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {  // eight terms on: renormalised
+      const float2 s = __fadd2_rn(ah[u], al[u]);
+      al[u] = sub2(al[u], sub2(s, ah[u]));
+      ah[u] = s;
+    }
+  };
   for (int i = 0; i <= t; ++i) {
     const int b = i & 1;
     if (i > 0) {
@@ -370,52 +459,37 @@ __global__ void __launch_bounds__(kTriThreads) batch_tri_kernel(const float* __r
       stage(i + 1);
       pre = fetch(i + 1);
     }
-#pragma unroll
-    for (int k = 0; k < kB / kKs; ++k) {
-      const int kk = kKs * k + ks;
-      const float2 xh = *reinterpret_cast<const float2*>(&sm.Xh[b][kk][2 * cg]);
-      const float2 xn = *reinterpret_cast<const float2*>(&sm.Xn[b][kk][2 * cg]);
-      const float2 xl = *reinterpret_cast<const float2*>(&sm.Xl[b][kk][2 * cg]);
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        df_mac2(sm.F[b][0][rg + 16 * u][kk], sm.F[b][1][rg + 16 * u][kk], xh, xn, xl, ah[u], al[u]);
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {  // eight terms on: renormalised
-      const float2 s = __fadd2_rn(ah[u], al[u]);
-      al[u] = sub2(al[u], sub2(s, ah[u]));
-      ah[u] = s;
-    }
+    multiply(b);
   }
-  // The sum over the eight threads of a row: each exchange also halves what a thread keeps, down to one row of a pair
-  // of columns in two threads, so that thread ks ends with row rg + 16 (ks & 3), column 2 cg + (ks >> 2).
-#pragma unroll
-  for (int u = 0; u < 4; u += 2) {  // lanes that differ in bit 0 split rows u, u + 1
-    const bool up = ks & 1;
-    const float2 sh = up ? ah[u] : ah[u + 1], sl = up ? al[u] : al[u + 1];
-    float2 kh = up ? ah[u + 1] : ah[u], kl = up ? al[u + 1] : al[u];
-    df_add(__shfl_xor_sync(0xffffffffu, sh.x, 1), __shfl_xor_sync(0xffffffffu, sl.x, 1), kh.x, kl.x);
-    df_add(__shfl_xor_sync(0xffffffffu, sh.y, 1), __shfl_xor_sync(0xffffffffu, sl.y, 1), kh.y, kl.y);
-    ah[u] = kh;
-    al[u] = kl;
-  }
-  float2 rh, rl;
-  {
-    const bool up = ks & 2;
-    const float2 sh = up ? ah[0] : ah[2], sl = up ? al[0] : al[2];
-    rh = up ? ah[2] : ah[0];
-    rl = up ? al[2] : al[0];
-    df_add(__shfl_xor_sync(0xffffffffu, sh.x, 2), __shfl_xor_sync(0xffffffffu, sl.x, 2), rh.x, rl.x);
-    df_add(__shfl_xor_sync(0xffffffffu, sh.y, 2), __shfl_xor_sync(0xffffffffu, sl.y, 2), rh.y, rl.y);
-  }
+  const int own_row = rg + 16 * (ks & 3), own_col = 2 * cg + (ks >> 2);
   float h, l;
-  {
-    const bool up = ks & 4;
-    h = up ? rh.y : rh.x;
-    l = up ? rl.y : rl.x;
-    df_add(__shfl_xor_sync(0xffffffffu, up ? rh.x : rh.y, 4), __shfl_xor_sync(0xffffffffu, up ? rl.x : rl.y, 4), h, l);
+  reduce(h, l);
+  if constexpr (SECOND) {  // (h, l) is r; x = I_b r, x += I_b (r - T_bb x)
+    const float rh = h, rl = l;
+    float xh = 0.f, xl = 0.f;
+    stage(t + 1);
+    for (int i = t + 1; i <= t + 3; ++i) {
+      const int b = i & 1;
+      if (i == t + 2) {
+        xh = h;
+        xl = l;
+      } else if (i == t + 3) {
+        df_add(rh, rl, h, l);
+      }
+      sm.Xh[b][own_row][own_col] = h;
+      sm.Xn[b][own_row][own_col] = -h;
+      sm.Xl[b][own_row][own_col] = l;
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
+      if (i < t + 3) stage(i + 1);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) ah[u] = al[u] = make_float2(0.f, 0.f);
+      multiply(b);
+      reduce(h, l);
+    }
+    df_add(xh, xl, h, l);
   }
-  const int own = r0 + rg + 16 * (ks & 3), c = cbase + 2 * cg + (ks >> 2);
+  const int own = r0 + own_row, c = cbase + own_col;
   if (own < n && c < R) {
     const int64_t at = int64_t(own) * R + c;
     put_word(wout + at, h, l);
@@ -426,11 +500,38 @@ __global__ void __launch_bounds__(kTriThreads) batch_tri_kernel(const float* __r
   }
 }
 
+template <bool LOWER>
+__global__ void __launch_bounds__(kTriThreads) batch_tri_kernel(const float* __restrict__ Gh,
+                                                                const float* __restrict__ Gl, int64_t ldg,
+                                                                const float* __restrict__ tiles,
+                                                                const int32_t* __restrict__ after, int n, int R,
+                                                                const double* __restrict__ Bin,
+                                                                const int32_t* __restrict__ perm, const Word* win,
+                                                                Word* wout, double* Y, int accumulate, int* ticket,
+                                                                DeviceStatus* st, const int32_t* __restrict__ skip) {
+  extern __shared__ float4 tri_smem[];
+  TriSmem& sm = *reinterpret_cast<TriSmem*>(tri_smem);
+  __shared__ int s_tk;
+  if (skip && *skip) return;
+  const int G = int(ceil_div(R, kCG)), nblk = int(ceil_div(n, kB));
+  __shared__ uint8_t s_after[kMaxBlocks];
+  if (threadIdx.x == 0) s_tk = atomicAdd(ticket, 1);
+  for (int i = threadIdx.x; i < nblk; i += kTriThreads) s_after[i] = uint8_t(after[i]);  // beside the ticket's latency
+  __syncthreads();
+  const int t = s_tk / G, cbase = (s_tk % G) * kCG;
+  if (t >= nblk) return;
+  if (s_after[LOWER ? t : nblk - 1 - t])
+    tri_block<LOWER, true>(sm, t, cbase, Gh, Gl, ldg, tiles, n, R, Bin, perm, win, wout, Y, accumulate, st);
+  else
+    tri_block<LOWER, false>(sm, t, cbase, Gh, Gl, ldg, tiles, n, R, Bin, perm, win, wout, Y, accumulate, st);
+}
+
 // ---------------------------------------------------------------------------
 struct BatchWs {
   BatchHeader* hdr;
   float *Gh, *Gl, *tilesL, *tilesU;  // premultiplied factors, inverted diagonal blocks
   double *invL, *invU, *Bs, *X, *D, *partial, *chunk, *KP, *VP;
+  int32_t *afterL, *afterU;  // which block rows take the second form
   Word* words;  // tickets (the first word), then the words of both solves
   void *Kd, *Vd, *columns;  // digits of Ks, of the value matrix, of a multiplied block
 };
@@ -449,8 +550,10 @@ size_t batch_layout(int n, char* base, BatchWs* w) {
   b.hdr = reinterpret_cast<BatchHeader*>(take(sizeof(BatchHeader)));
   b.Gh = reinterpret_cast<float*>(take(size_t(n) * ld * sizeof(float)));
   b.Gl = reinterpret_cast<float*>(take(size_t(n) * ld * sizeof(float)));
-  b.tilesL = reinterpret_cast<float*>(take(nblk * 2 * kB * kB * sizeof(float)));
-  b.tilesU = reinterpret_cast<float*>(take(nblk * 2 * kB * kB * sizeof(float)));
+  b.tilesL = reinterpret_cast<float*>(take(nblk * kTilePlanes * kB * kB * sizeof(float)));
+  b.tilesU = reinterpret_cast<float*>(take(nblk * kTilePlanes * kB * kB * sizeof(float)));
+  b.afterL = reinterpret_cast<int32_t*>(take(nblk * sizeof(int32_t)));
+  b.afterU = reinterpret_cast<int32_t*>(take(nblk * sizeof(int32_t)));
   b.invL = reinterpret_cast<double*>(take(nblk * kB * kB * sizeof(double)));
   b.invU = reinterpret_cast<double*>(take(nblk * kB * kB * sizeof(double)));
   b.Bs = reinterpret_cast<double*>(take(v));
@@ -498,28 +601,29 @@ namespace {
 template <typename TF>
 int prepare_factors(int n, const TF* F, int64_t ld, const BatchWs& b, cudaStream_t s) {
   const unsigned nblk = unsigned(ceil_div(n, kB));
-  tri_inverse_kernel<TF, true><<<nblk, 256, sizeof(InverseSmem), s>>>(F, ld, n, b.invL, b.tilesL);
+  tri_inverse_kernel<TF, true><<<nblk, 256, sizeof(InverseSmem), s>>>(F, ld, n, b.invL, b.tilesL, b.afterL);
   UPDES_LAUNCH_CHECK();
-  tri_inverse_kernel<TF, false><<<nblk, 256, sizeof(InverseSmem), s>>>(F, ld, n, b.invU, b.tilesU);
+  tri_inverse_kernel<TF, false><<<nblk, 256, sizeof(InverseSmem), s>>>(F, ld, n, b.invU, b.tilesU, b.afterU);
   UPDES_LAUNCH_CHECK();
-  tri_premultiply_kernel<TF><<<dim3(nblk, nblk), 256, sizeof(InverseSmem), s>>>(F, ld, n, b.invL, b.invU, b.Gh, b.Gl);
+  tri_premultiply_kernel<TF><<<dim3(nblk, nblk), 256, sizeof(InverseSmem), s>>>(F, ld, n, b.invL, b.invU, b.afterL,
+                                                                                 b.afterU, b.Gh, b.Gl);
   UPDES_LAUNCH_CHECK();
   return UPDES_OK;
 }
 
 // Y (+)= M^-1 B for n x R blocks (permute, L, U).
 int batch_precond(int n, int R, const BatchWs& b, int64_t ld, const int32_t* piv, const double* B, double* Y,
-                  bool accumulate, DeviceStatus* st, cudaStream_t s) {
+                  bool accumulate, DeviceStatus* st, cudaStream_t s, const int32_t* skip = nullptr) {
   const unsigned grid = unsigned(ceil_div(n, kB) * ceil_div(R, kCG));
   StatScope sc(kStatTrsv, s, 2.0 * n * n * R, double(n) * n * 8.0);
   int* tickets = reinterpret_cast<int*>(b.words);
   Word *wL = b.words + 1, *wU = wL + size_t(n) * R;
   UPDES_CUDA_TRY(cudaMemsetAsync(b.words, 0, (1 + 2 * size_t(n) * R) * sizeof(Word), s));
-  batch_tri_kernel<true><<<grid, kTriThreads, sizeof(TriSmem), s>>>(b.Gh, b.Gl, ld, b.tilesL, n, R, B, piv + n, nullptr, wL,
-                                                            nullptr, 0, tickets, st);
+  batch_tri_kernel<true><<<grid, kTriThreads, sizeof(TriSmem), s>>>(b.Gh, b.Gl, ld, b.tilesL, b.afterL, n, R, B, piv + n, nullptr, wL,
+                                                            nullptr, 0, tickets, st, skip);
   UPDES_LAUNCH_CHECK();
-  batch_tri_kernel<false><<<grid, kTriThreads, sizeof(TriSmem), s>>>(b.Gh, b.Gl, ld, b.tilesU, n, R, nullptr, nullptr, wL, wU, Y,
-                                                             accumulate, tickets + 1, st);
+  batch_tri_kernel<false><<<grid, kTriThreads, sizeof(TriSmem), s>>>(b.Gh, b.Gl, ld, b.tilesU, b.afterU, n, R, nullptr, nullptr, wL, wU, Y,
+                                                             accumulate, tickets + 1, st, skip);
   UPDES_LAUNCH_CHECK();
   return UPDES_OK;
 }
@@ -536,6 +640,7 @@ extern "C" int updes_batch_prepare(const updes_problem* p, void* workspace, size
                                    size_t batch_ws_bytes, void* stream) {
   if (!p || !batch_ws) return UPDES_ERR_INVALID;
   const int n = p->N + p->M;
+  if (ceil_div(n, kB) > kMaxBlocks) return UPDES_ERR_UNSUPPORTED;
   if (batch_ws_bytes < batch_layout(n, nullptr, nullptr)) return UPDES_ERR_WORKSPACE;
   const float *Khi, *Klo, *F32;
   const double *F64, *dr, *dc;
@@ -575,6 +680,7 @@ extern "C" int updes_solve_batch(const updes_problem* p, int32_t R, const double
   if (!p || R <= 0 || R > kMaxR || !Q || !coeffs || ldq < R || ldc < R || sweeps < 0 || !batch_ws)
     return UPDES_ERR_INVALID;
   const int n = p->N + p->M;
+  if (ceil_div(n, kB) > kMaxBlocks) return UPDES_ERR_UNSUPPORTED;
   if (batch_ws_bytes < batch_layout(n, nullptr, nullptr)) return UPDES_ERR_WORKSPACE;
   const float *Khi, *Klo, *F32;
   const double *F64, *dr, *dc;
@@ -593,14 +699,18 @@ extern "C" int updes_solve_batch(const updes_problem* p, int32_t R, const double
   UPDES_LAUNCH_CHECK();
   if ((e = batch_precond(n, R, b, ld, piv, b.Bs, b.X, false, st, s))) return e;
   const int splits = rhs64_splits(n, p->N);
-  for (int it = 0; it < sweeps; ++it) {
+  // FP64 factors (precision 0 in the header) get a sweep in any case, see kPremultiplied; the kernels read which they are
+  static_assert(UPDES_PREC_FP64 == 0, "skip");
+  const int32_t* skip = sweeps == 0 ? &b.hdr->precision : nullptr;
+  for (int it = 0; it < std::max(sweeps, 1); ++it) {
     {
       StatScope sc(kStatGemv, s, 2.0 * n * n * R, 14.0 * n * double(n));
-      if ((e = rhs64_multiply(b.Kd, n, p->N, b.X, R, R, b.columns, b.partial, splits, st, s))) return e;
-      batch_residual_kernel<<<g, 256, 0, s>>>(b.Bs, b.partial, splits, n, p->N, R, b.KP, b.X, b.D);
+      if ((e = rhs64_multiply(b.Kd, n, p->N, b.X, R, R, b.columns, b.partial, splits, st, s, skip)))
+        return e;
+      batch_residual_kernel<<<g, 256, 0, s>>>(b.Bs, b.partial, splits, n, p->N, R, b.KP, b.X, b.D, skip);
       UPDES_LAUNCH_CHECK();
     }
-    if ((e = batch_precond(n, R, b, ld, piv, b.D, b.X, true, st, s))) return e;
+    if ((e = batch_precond(n, R, b, ld, piv, b.D, b.X, true, st, s, skip))) return e;
   }
   batch_unscale_kernel<<<g, 256, 0, s>>>(b.X, dc, n, R, coeffs, ldc);
   UPDES_LAUNCH_CHECK();

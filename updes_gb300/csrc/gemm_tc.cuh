@@ -29,6 +29,7 @@ int ozaki64_update(double* C, int64_t ldc, const double* A, int64_t lda, const d
 // of rows [r0, r0 + rows) into `matrix` (rhs64_matrix_bytes(m, n) bytes), from FP64 rows (A, lda) or, with A null,
 // from the sum of two FP32 planes.  rhs64_multiply leaves the product as `splits` partial sums, each m x 64 (row
 // stride 64), to be added in order; `columns`: scratch of rhs64_columns_bytes(n).  rhs64_setup before a capture.
+// skip (device, may be null): nothing is done when it holds something other than 0.
 constexpr int kRhs64MaxSplits = 16;
 size_t rhs64_matrix_bytes(int m, int n);
 size_t rhs64_columns_bytes(int n);
@@ -37,4 +38,4 @@ int rhs64_setup();
 int rhs64_matrix(const double* A, const float* hi, const float* lo, int64_t lda, int m, int n, int r0, int rows,
                  void* matrix, cudaStream_t s);
 int rhs64_multiply(const void* matrix, int m, int n, const double* X, int64_t ldx, int R, void* columns,
-                   double* partial, int splits, DeviceStatus* st, cudaStream_t s);
+                   double* partial, int splits, DeviceStatus* st, cudaStream_t s, const int32_t* skip = nullptr);

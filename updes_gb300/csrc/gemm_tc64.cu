@@ -456,7 +456,8 @@ constexpr int kBlockK = 256;
 __global__ void __launch_bounds__(kThreads, 1)
     rhs64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const int* __restrict__ Ae, const int* __restrict__ Be, double* __restrict__ partial, int m, int nkb,
-                 int splits, DeviceStatus* st) {
+                 int splits, DeviceStatus* st, const int32_t* __restrict__ skip) {
+  if (skip && *skip) return;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ Ctrl ctl;
@@ -619,7 +620,8 @@ __global__ void __launch_bounds__(256) matrix_digits_kernel(const double* __rest
 // Digits of X (n x R, ldx) as 64 columns (those from R on zero): a block per (k block, 8 columns), a warp a column.
 __global__ void __launch_bounds__(256) columns_digits_kernel(const double* __restrict__ X, int64_t ldx, int n, int R,
                                                              int nkb, uint16_t* __restrict__ Bd,
-                                                             int* __restrict__ Be) {
+                                                             int* __restrict__ Be, const int32_t* __restrict__ skip) {
+  if (skip && *skip) return;
   __shared__ double t[kBlockK][9];
   const int kb = blockIdx.x, c0 = blockIdx.y * 8;
   for (int e = threadIdx.x; e < kBlockK * 8; e += blockDim.x) {
@@ -752,18 +754,18 @@ int rhs64_setup() {
 }
 
 int rhs64_multiply(const void* matrix, int m, int n, const double* X, int64_t ldx, int R, void* columns,
-                   double* partial, int splits, DeviceStatus* st, cudaStream_t s) {
+                   double* partial, int splits, DeviceStatus* st, cudaStream_t s, const int32_t* skip) {
   const int nkb = k_blocks(n);
   const MatrixDigits a = matrix_view(const_cast<void*>(matrix), m, n), b = matrix_view(columns, TN, n);
   CUtensorMap mapA, mapB;
   if (int e = make_map(&mapA, a.d, m, nkb * kBlockK, TM)) return e;
   if (int e = make_map(&mapB, b.d, TN, nkb * kBlockK, TN)) return e;
   if (int e = rhs64_setup()) return e;
-  columns_digits_kernel<<<dim3(unsigned(nkb), TN / 8), 256, 0, s>>>(X, ldx, n, R, nkb, b.d, b.e);
+  columns_digits_kernel<<<dim3(unsigned(nkb), TN / 8), 256, 0, s>>>(X, ldx, n, R, nkb, b.d, b.e, skip);
   UPDES_LAUNCH_CHECK();
   const int items = int(ceil_div(m, TM)) * splits;
   rhs64_kernel<<<std::min(items, num_sms_cached()), kThreads, kStages * kStageBytes + 1024, s>>>(
-      mapA, mapB, a.e, b.e, partial, m, nkb, splits, st);
+      mapA, mapB, a.e, b.e, partial, m, nkb, splits, st, skip);
   UPDES_LAUNCH_CHECK();
   return UPDES_OK;
 }

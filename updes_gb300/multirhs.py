@@ -32,8 +32,8 @@ class MultiRHSSolver:
     ``boundary_conditions`` fixes the boundary values used by ``implicit_steps``
     (the same for every column); ``solve`` takes complete right-hand sides.
     ``sweeps`` is the number of refinement sweeps after the first solve.  With the default FP64
-    factors one sweep brings every column to FP64 accuracy; FP32 factors (``precision="fp32"``)
-    contract only as fast as their conditioning allows and need more.
+    factors one sweep brings every column to FP64 accuracy, and there is always one; FP32 factors
+    (``precision="fp32"``) contract only as fast as their conditioning allows and need more.
     """
 
     def __init__(self, diff_operator, cloud, boundary_conditions, rbf, max_degree, diff_args=None, options=None,
