@@ -46,7 +46,9 @@ inline int smem_opt_in(const void* func, int bytes, std::atomic<unsigned long lo
 // Launch of a kernel; with `early` (its predecessor on the stream is a kernel of this library) its CTAs may be placed as soon as
 // every CTA of the predecessor has called allow_next() (or has left) and the SMs have room, and wait in wait_previous()
 // until the predecessor is complete and its writes are visible.  Every CTA of a kernel launched like this calls
-// wait_previous() before it touches memory, so a kernel that is complete implies all before it.  A waiting CTA holds its
+// wait_previous() before it touches memory, so a kernel that is complete implies all before it.  Such a kernel is alive while
+// its predecessor writes, so it reads what that may write by plain or __ldcg loads only: no __ldg, no const __restrict__
+// (both allow the non-coherent path, which wants the data constant for the kernel's whole life).  A waiting CTA holds its
 // place on the SM: beside a second stream only kernels of few CTAs are launched early (with all of them the mixed LU at
 // n = 22,506 took 149 ms, with none 111, with its short chain's 108; at n = 600, on one stream, 1.13 with all, 1.21 with none).
 template <class... P, class... A>

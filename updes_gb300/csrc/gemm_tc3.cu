@@ -140,7 +140,7 @@ __device__ __forceinline__ void mma_steps(uint32_t d, uint64_t a0, uint64_t b0, 
 // ---- digit pre-pass ------------------------------------------------------------------------------------
 // A (m x K, lda) -> Ad (see digit_at) and As[r] = 2^(e-8), one warp per row; bx is the block's index among the row
 // part's blocks.
-__device__ __forceinline__ void digits_rows(int bx, const float* __restrict__ A, int64_t lda, int m, int K, int Kp,
+__device__ __forceinline__ void digits_rows(int bx, const float* A, int64_t lda, int m, int K, int Kp,
                                             __half* __restrict__ Ad, float* __restrict__ As) {
   const int64_t r = (int64_t(bx) * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
@@ -174,7 +174,7 @@ __device__ __forceinline__ void digits_rows(int bx, const float* __restrict__ A,
 }
 
 // B (K x nc, ldb) -> Bd (transposed, in tiles of TN columns) and Bs[c]; a CTA per 32 columns.
-__device__ __forceinline__ void digits_cols(int bx, const float* __restrict__ B, int64_t ldb, int nc, int K, int Kp, int TN,
+__device__ __forceinline__ void digits_cols(int bx, const float* B, int64_t ldb, int nc, int K, int Kp, int TN,
                                             __half* __restrict__ Bd, float* __restrict__ Bs) {
   __shared__ float t[kMaxK][33];
   const int c0 = bx * 32;
@@ -207,8 +207,7 @@ __device__ __forceinline__ void digits_cols(int bx, const float* __restrict__ B,
 
 // Both digit passes of one update in a single launch: blocks [0, row_blocks) take the rows of A, the others the
 // column tiles of B.
-__global__ void __launch_bounds__(256) digits_kernel(const float* __restrict__ A, int64_t lda, int m,
-                                                     const float* __restrict__ B, int64_t ldb, int nc, int K, int Kp,
+__global__ void __launch_bounds__(256) digits_kernel(const float* A, int64_t lda, int m, const float* B, int64_t ldb, int nc, int K, int Kp,
                                                      int TN, int row_blocks, __half* __restrict__ Ad, float* __restrict__ As,
                                                      __half* __restrict__ Bd, float* __restrict__ Bs) {
   const int b = int(blockIdx.x);
@@ -251,13 +250,14 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
 template <int TN>
 __global__ void __launch_bounds__(kThreads, 1)
     ozaki3_kernel(const __grid_constant__ CUtensorMap tmCh, const __grid_constant__ CUtensorMap tmCl,
-                  const __half* __restrict__ Ad, const __half* __restrict__ Bd, const float* __restrict__ As, const float* __restrict__ Bs, int m, int nc, int Kp,
+                  const __half* Ad, const __half* Bd, const float* As, const float* Bs, int m, int nc, int Kp,
                   DeviceStatus* st) {
   using C = Cfg<TN>;
   constexpr int kStages = C::kStages, kBTile = C::kBTile, kStageBytes = C::kStageBytes, kCols = C::kCols;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   __shared__ Ctrl ctl;
+  __shared__ __align__(16) float s_scales[kEpiWarps][kCols];  // of a warp's columns of B
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int tiles_n = int(ceil_div(nc, TN)), tiles_m = int(ceil_div(m, TM));
   const int ntiles = tiles_n * tiles_m;
@@ -384,6 +384,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint8_t* bufh = smem + kStages * kStageBytes + ew * 2 * kCBox;
     uint8_t* bufl = bufh + kCBox;
     uint64_t* cbar = &ctl.cfull[ew];
+    float* scales = s_scales[ew];
     const uint32_t lane_base = (uint32_t(q * 32) << 16) + uint32_t(h * kCols);
     int loads = 0, waited = 0;  // pieces of C requested / taken over
     // the warp's pieces of C, 32 columns each, in the order in which it takes them: (tile, slice), those inside C only
@@ -408,7 +409,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int t = blockIdx.x; t < ntiles; t += gridDim.x, ++tl) {
       const int r0 = (t / tiles_n) * TM + q * 32, c0 = (t % tiles_n) * TN + h * kCols;
       const uint32_t ph = uint32_t(tl) & 1u;
-      const float sa = r0 + lane < m ? -__ldg(As + r0 + lane) : 0.f;
+      const float sa = r0 + lane < m ? -__ldcg(As + r0 + lane) : 0.f;
+      // the columns' scales, for every lane (those of columns beyond nc are scratch bytes of no effect: the store leaves
+      // these columns out)
+      __syncwarp();
+#pragma unroll
+      for (int u = lane; u < kCols; u += 32) scales[u] = __ldcg(Bs + c0 + u);
       float2 gh[kCols / 2], gl[kCols / 2];  // the row's sums over the warp's columns, as column pairs
       // every wait ends in a warp vote, so a warp always leaves together (tcgen05.ld needs all 32 lanes)
       if (!__all_sync(0xffffffffu, mbar_wait(&ctl.hi_done, ph, abort_flag))) {
@@ -453,9 +459,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
       for (int sl = 0; sl < kCols / 32; ++sl) {
         if (!ok || !piece_in(t, sl)) continue;
-        // the columns' scales, the same for every lane (those of columns beyond nc are scratch bytes of no effect: the
-        // store leaves these columns out)
-        const float4* sb = reinterpret_cast<const float4*>(Bs + c0 + sl * 32);
+        const float4* sb = reinterpret_cast<const float4*>(scales + sl * 32);
         ok = __all_sync(0xffffffffu, mbar_wait(cbar, uint32_t(waited) & 1u, abort_flag));
         if (!ok) {
           if (lane == 0) give_up(45);
@@ -468,7 +472,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
           const int off = ((c ^ (lane & 7)) << 4);
-          const float4 sb4 = __ldg(sb + c);
+          const float4 sb4 = sb[c];
           const float4 hv = *reinterpret_cast<float4*>(hrow + off), lv = *reinterpret_cast<float4*>(lrow + off);
           float2 hx[2] = {make_float2(hv.x, hv.y), make_float2(hv.z, hv.w)};
           float2 lx[2] = {make_float2(lv.x, lv.y), make_float2(lv.z, lv.w)};

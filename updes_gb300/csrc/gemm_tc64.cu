@@ -149,7 +149,7 @@ __device__ __forceinline__ void write_digits(const double* v, int emax, uint16_t
 }
 
 // A (m x K, lda) -> Ad[p][r][k] and Ae[r]; 8 consecutive k a lane, `span` lanes (a power of two >= Kp / 8) a row.
-__device__ __forceinline__ void digits_rows(int bx, const double* __restrict__ A, int64_t lda, int m, int K, int Kp,
+__device__ __forceinline__ void digits_rows(int bx, const double* A, int64_t lda, int m, int K, int Kp,
                                             int span, uint16_t* __restrict__ Ad, int* __restrict__ Ae) {
   const int64_t t = int64_t(bx) * blockDim.x + threadIdx.x;
   const int r = int(t / span), q = int(t % span), k0 = q * 8;
@@ -169,7 +169,7 @@ __device__ __forceinline__ void digits_rows(int bx, const double* __restrict__ A
 
 // B (K x nc, ldb) -> Bd[p][c][k] and Be[c]; a lane a column, a warp 32 consecutive k, Kp / 32 warps a group of 32
 // columns, 8 / (Kp / 32) groups a block.
-__device__ __forceinline__ void digits_cols(int bx, const double* __restrict__ B, int64_t ldb, int nc, int K, int Kp,
+__device__ __forceinline__ void digits_cols(int bx, const double* B, int64_t ldb, int nc, int K, int Kp,
                                             uint16_t* __restrict__ Bd, int* __restrict__ Be) {
   __shared__ int s_max[8][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -196,8 +196,7 @@ __device__ __forceinline__ void digits_cols(int bx, const double* __restrict__ B
 }
 
 // Both digit passes of an update in one launch: blocks [0, row_blocks) take rows of A, the others columns of B.
-__global__ void __launch_bounds__(256) digits64_kernel(const double* __restrict__ A, int64_t lda, int m,
-                                                       const double* __restrict__ B, int64_t ldb, int nc, int K,
+__global__ void __launch_bounds__(256) digits64_kernel(const double* A, int64_t lda, int m, const double* B, int64_t ldb, int nc, int K,
                                                        int Kp, int span, int row_blocks, uint16_t* __restrict__ Ad,
                                                        int* __restrict__ Ae, uint16_t* __restrict__ Bd,
                                                        int* __restrict__ Be) {
@@ -296,7 +295,7 @@ __device__ __forceinline__ uint32_t read_sums(uint32_t taddr, long long* v) {
 
 __global__ void __launch_bounds__(kThreads, 1)
     ozaki64_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                   const int* __restrict__ Ae, const int* __restrict__ Be, double* __restrict__ C, int64_t ldc, int m,
+                   const int* Ae, const int* Be, double* C, int64_t ldc, int m,
                    int nc, int Kp, DeviceStatus* st) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -405,7 +404,8 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll 1
       for (int half = 0; half < 2; ++half) {
         const int c = c0 + half * kCols + lane;
-        const int eb = c < nc ? __ldg(Be + c) : 0;
+        const int eb = c < nc ? __ldcg(Be + c) : 0;
+        const int er = r0 + ew * 16 + (lane & 15), ea = er < m ? __ldcg(Ae + er) : 0;  // row i's in lane i
         double* cp = C + int64_t(r0 + ew * 16) * ldc + c;
         double old[16];
 #pragma unroll
@@ -418,9 +418,9 @@ __global__ void __launch_bounds__(kThreads, 1)
         epilogue_barrier();
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          const int r = r0 + ew * 16 + i;
+          const int r = r0 + ew * 16 + i, e = __shfl_sync(0xffffffffu, ea, i);
           if (c < nc && r < m && !*abort_flag)
-            __stcs(cp + int64_t(i) * ldc, add_scaled<-1>(old[i], sV[ew * 16 + i][lane], __ldg(Ae + r), eb));
+            __stcs(cp + int64_t(i) * ldc, add_scaled<-1>(old[i], sV[ew * 16 + i][lane], e, eb));
         }
         if (half == 0) epilogue_barrier();
       }

@@ -239,7 +239,7 @@ constexpr int kSwapMapStride = 512;
 struct MapRows {
   int dst[128], src[128];
 };
-__device__ __forceinline__ int read_map(MapRows& m, const int32_t* __restrict__ map) {
+__device__ __forceinline__ int read_map(MapRows& m, const int32_t* map) {
   for (int t = threadIdx.x; t < 128; t += blockDim.x) {
     m.dst[t] = map[1 + t];
     m.src[t] = map[129 + t];
@@ -345,7 +345,7 @@ __device__ __forceinline__ void solve_df64(const float (*L)[65], float (*Xh)[LD]
 
 template <int COLS>
 __global__ void __launch_bounds__(4 * COLS) trsm_df64_kernel(float* Whi, float* Wlo, int64_t ld, int k, TrsmDfCols cols,
-                                                             const int32_t* __restrict__ map) {
+                                                             const int32_t* map) {
   extern __shared__ float4 trsm_df_smem[];
   TrsmDfSmem<COLS>& sm = *reinterpret_cast<TrsmDfSmem<COLS>*>(trsm_df_smem);
   const int tid = threadIdx.x, lane = tid & 31;
@@ -432,7 +432,7 @@ struct BlockRowSmem {
   float B[192][65];  // the block of L below the diagonal block
 };
 
-__global__ void __launch_bounds__(256) block_row_df_kernel(float* Whi, const float* __restrict__ Wlo, int64_t ld, int k0,
+__global__ void __launch_bounds__(256) block_row_df_kernel(float* Whi, const float* Wlo, int64_t ld, int k0,
                                                            int64_t c0, int64_t c1) {
   extern __shared__ float4 block_row_smem[];
   BlockRowSmem& sm = *reinterpret_cast<BlockRowSmem*>(block_row_smem);
@@ -548,7 +548,7 @@ struct Trsm64Smem {
 
 template <int NBK>
 __global__ void __launch_bounds__(128) trsm64_kernel(double* W, int64_t ld, int k, int w, int64_t c0, int64_t c1,
-                                                     const int32_t* __restrict__ map, int64_t left, int64_t left_end,
+                                                     const int32_t* map, int64_t left, int64_t left_end,
                                                      int left_ctas) {
   extern __shared__ double trsm64_smem[];
   Trsm64Smem<NBK>& sm = *reinterpret_cast<Trsm64Smem<NBK>*>(trsm64_smem);
