@@ -230,9 +230,13 @@ class _Batch:
 
     def run(self, idx, precisions, widths, max_sweeps, ctas):
         """Solve the systems ``idx`` (host indices into the batch) in one call; returns the status."""
-        return self.end(self.begin(idx, precisions, widths, max_sweeps, ctas))
+        workspace = _Workspace(self.dps[0].device)
+        try:
+            return self.end(self.begin(idx, precisions, widths, max_sweeps, ctas, workspace))
+        finally:
+            workspace.give_back()
 
-    def begin(self, idx, precisions, widths, max_sweeps, ctas):
+    def begin(self, idx, precisions, widths, max_sweeps, ctas, workspace):
         """Issue the solves of the systems ``idx`` without waiting for them; the result goes to ``end``."""
         torch, lib = self.torch, _lib.load()
         c = len(idx)
@@ -244,7 +248,7 @@ class _Batch:
         nbytes, tbytes = ctypes.c_size_t(), ctypes.c_size_t()
         _lib.check(lib.updes_solve_batched_workspace(probs, c, int(ctas), ctypes.byref(nbytes)),
                    "updes_solve_batched_workspace")
-        ws = _workspace(nbytes.value, self.dps[0].device)
+        ws = workspace.of(nbytes.value)
         _lib.check(lib.updes_solve_batched_tables(c, ctypes.byref(tbytes)), "updes_solve_batched_tables")
         tables = torch.empty(tbytes.value, dtype=torch.uint8, device=self.dps[0].device)
         stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
@@ -269,14 +273,24 @@ class _Batch:
 _WS: dict = {}
 
 
-def _workspace(nbytes, device):
-    torch = _torch()
-    buf = _WS.get(device.index)
-    if buf is None or buf.numel() < nbytes:
-        _WS.pop(device.index, None)
-        buf = torch.empty(int(nbytes), dtype=torch.uint8, device=device)
-        _WS[device.index] = buf
-    return buf
+class _Workspace:
+    """Scratch of one batch, out of the cache (one buffer per device) until ``give_back``: while parts of the batch run, the
+    callers' functions may call ``pde_solver_batched`` themselves, on any stream.  The parts run one after another on one
+    stream and share it."""
+
+    def __init__(self, device):
+        self.device, self.buffer = device, _WS.pop(device.index, None)
+
+    def of(self, nbytes):
+        if self.buffer is None or self.buffer.numel() < nbytes:
+            self.buffer = _torch().empty(int(nbytes), dtype=_torch().uint8, device=self.device)
+        return self.buffer
+
+    def give_back(self):
+        old = _WS.get(self.device.index)
+        if self.buffer is not None and (old is None or old.numel() < self.buffer.numel()):
+            _WS[self.device.index] = self.buffer
+        self.buffer = None
 
 
 def free_workspace():
@@ -368,6 +382,7 @@ def pde_solver_batched(systems, options=None, precision="auto", max_sweeps=4, ct
     parts = []  # (first system, batch, precisions, widths, what begin returned, events around it)
     prepare_s = 0.0
     st = _lib.OK
+    workspace = _Workspace(torch.device("cuda", torch.cuda.current_device()))
     try:
         for first, last in _parts([s["cloud"].N for s in systems]):
             t0 = time.perf_counter()
@@ -378,13 +393,14 @@ def pde_solver_batched(systems, options=None, precision="auto", max_sweeps=4, ct
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record()
             parts.append((first, batch, precs, widths, batch.begin(list(range(batch.count)), precs, widths, max_sweeps,
-                                                                   ctas), (e0, e1)))
+                                                                   ctas, workspace), (e0, e1)))
             e1.record()
     finally:
         for _, batch, _, _, begun, _ in parts:
             one = batch.end(begun)
             if st == _lib.OK or (st == _lib.ERR_SINGULAR and one != _lib.OK):
                 st = one
+        workspace.give_back()
     used = ["fp64" if code[nm] == _lib.PREC_FP64 else "fp32" for nm in names]
     relaunched, relaunch_ms, widths_all = 0, 0.0, []
     for first, batch, precs, widths, _, _ in parts:
