@@ -352,8 +352,8 @@ UPDES_API int updes_solve_many(const updes_problem* problems, int32_t count, con
 
 /*
  * Many independent systems in one call of at most two launches.  With
- * `ctas` = 0, systems that would hold one SM for longer than the average SM's
- * share of the batch are solved by thread-block clusters of eight CTAs on a
+ * `ctas` = 0, the systems of at least the size that updes_solve_batched_plan
+ * gives are solved by thread-block clusters of eight CTAs on a
  * second stream, which `stream` waits for; the others, and with `ctas` > 0
  * all of them, by `ctas` single CTAs (0 = one per SM).  Both take systems
  * from device work queues, largest first; a CTA or a cluster
@@ -391,6 +391,11 @@ UPDES_API int updes_solve_batched(const updes_problem* problems, int32_t count, 
  * after updes_solve_batched_end, whatever that returns.  tables: device memory of updes_solve_batched_tables bytes
  * that the batch has to itself until then; the workspace may be given to further batches on the same stream. */
 UPDES_API int updes_solve_batched_tables(int32_t count, size_t* bytes);
+/* How a batch of systems of n[i] unknowns is split with `ctas` = 0: those of at least *from unknowns go to clusters (INT32_MAX:
+ * none), and the launch should take about *ms (FP32).  On a device of `sms` SMs that holds `teams` clusters of eight CTAs;
+ * sms = 0: the current device. */
+UPDES_API int updes_solve_batched_plan(const int32_t* n, int32_t count, int32_t sms, int32_t teams, int32_t* from,
+                                       double* ms);
 UPDES_API int updes_solve_batched_begin(const updes_problem* problems, int32_t count, const double* const* q,
                                         double* const* coeffs, double* const* vals, const int32_t* precision,
                                         const int32_t* panel_width, int32_t max_sweeps, int32_t ctas, void* workspace,

@@ -124,6 +124,8 @@ SIGNATURES = {
     "updes_solve_batched_workspace": (ctypes.c_int, [ctypes.POINTER(Problem), _i32, _i32, ctypes.POINTER(_sz)]),
     "updes_solve_batched": (ctypes.c_int, [ctypes.POINTER(Problem), _i32, _vp, _vp, _vp, _vp, _vp, _i32, _i32,
                                            ctypes.POINTER(SolveInfo), _vp, _sz, _vp]),
+    "updes_solve_batched_plan": (ctypes.c_int, [_vp, _i32, _i32, _i32, ctypes.POINTER(_i32),
+                                                ctypes.POINTER(ctypes.c_double)]),
     "updes_solve_batched_tables": (ctypes.c_int, [_i32, ctypes.POINTER(_sz)]),
     "updes_solve_batched_begin": (ctypes.c_int, [ctypes.POINTER(Problem), _i32, _vp, _vp, _vp, _vp, _vp, _i32, _i32,
                                                  _vp, _sz, _vp, _sz, _vp, ctypes.POINTER(_vp)]),

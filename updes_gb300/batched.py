@@ -2,9 +2,8 @@
 
 The reference solves each system with its own ``pde_solver`` call (updes/operators.py:559-618).
 ``pde_solver_batched`` prepares every system on the host exactly as ``pde_solver`` does (operator capture,
-boundary rows, right-hand side) and hands them all to ``updes_solve_batched``: systems that would hold one SM for
-longer than the average SM's share of the batch are solved by thread-block clusters of eight CTAs, the others by
-single CTAs beside them.  Either takes systems from a device work queue, largest first, and runs each one's assembly,
+boundary rows, right-hand side) and hands them all to ``updes_solve_batched``: where the launch would wait for a few
+large systems they are solved by thread-block clusters of eight CTAs, the others by single CTAs beside them.  Either takes systems from a device work queue, largest first, and runs each one's assembly,
 LU, refinement and values by itself.
 A batch of 128 systems or more is prepared and launched in up to four parts: the host works on a part while the GPU
 solves those before it.

@@ -21,11 +21,14 @@
 // The scratch of a CTA or cluster (its slice of the workspace) holds K, the working matrix and A for the largest
 // system.  Every wait is a CTA or cluster barrier (the CTAs of a cluster run at the same time), so nothing can hang.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstring>
+#include <functional>
 #include <memory>
 #include <new>
 #include <numeric>
+#include <queue>
 #include <vector>
 
 #include "common.cuh"
@@ -902,22 +905,81 @@ int sm_count() {
 
 std::atomic<unsigned long long> g_batched_smem_done[2];
 
-// Who solves what, from the sizes alone.  A system that would keep one SM busy for longer than the average SM's share of
-// the batch (costs as n^3) is solved by clusters: with one CTA a system the launch lasts as long as its largest one (256
-// clouds of up to 2,025 nodes: 376 ms; so split 118, at half the limit 135, at twice 154).  A cluster takes n = 2,031
-// from 353 to 49 ms, n = 790 from 30 to 8.6, n = 406 from 7.3 to 3.6, n = 202 only from 2.2 to 1.7, and below that
-// nothing; two rounds of clusters (17 systems) take 18.8 ms against 37.6 at n = 790, 7.2 against 8.4 at 406 and 3.6
-// against 3.5 at 202.  So systems of fewer than 384 unknowns always take one CTA each, as those within the share do, on
-// the SMs that no cluster holds and then on those that are done.  With a CTA count given by the caller every system
-// takes one CTA.
+// Who solves what, from the sizes alone: the systems of at least some size by clusters, the others by one CTA each on the SMs
+// that no cluster holds and then on those that are done, with the size that gives the shortest launch by the times below.
+// A cluster shortens one system (n = 2,031 from 353 to 49 ms, n = 790 from 30 to 8.6) but its eight SMs do less together,
+// so it pays where a launch would wait for a few large systems and not where the SMs are full: 256 clouds of up to
+// 2,025 nodes 376 ms with one CTA a system, 118 with clusters for the large ones; 152 systems of 784 nodes 30 ms with
+// one CTA each, 84 on clusters (a rule by the average SM's share of n^3 took those: 127 of them 77 ms instead of 45). Below 384
+// unknowns a cluster gains nothing.  With a CTA count given by the caller every system takes one CTA.
 constexpr int kCoopMinN = 384;
+
+// Milliseconds of a system on one CTA (batches of 64 and one at a time) and on a cluster, FP32; FP64 takes up to 2.3 times as
+// long on either.
+constexpr struct { double n, single, cluster; } kSystemMs[] = {
+    {64, 0.55, 1.2}, {100, 0.9, 1.5}, {200, 2.1, 2.1}, {400, 7.0, 3.45}, {787, 29.5, 8.5},
+    {1603, 172, 29.8}, {2028, 350, 48.9}, {3028, 1180, 125}, {4096, 3300, 280}};
+
+double system_ms(int n, bool cluster) {
+  const int last = int(sizeof kSystemMs / sizeof kSystemMs[0]) - 1;
+  int i = 1;
+  while (i < last && n > kSystemMs[i].n) ++i;
+  const auto &a = kSystemMs[i - 1], &b = kSystemMs[i];
+  const double x = (std::log(std::max(n, 1)) - std::log(a.n)) / (std::log(b.n) - std::log(a.n));
+  const double ya = cluster ? a.cluster : a.single, yb = cluster ? b.cluster : b.single;
+  return std::exp(std::log(ya) + x * (std::log(yb) - std::log(ya)));
+}
+
+// The launch of systems of sizes n (falling), those up to index `coop` on clusters: each goes to the first that is free.
+double launch_ms(const std::vector<int>& n, size_t coop, int sms, int teams) {
+  std::priority_queue<double, std::vector<double>, std::greater<double>> team, sm;
+  const int held = int(std::min<size_t>(coop, size_t(teams)));
+  for (int i = 0; i < held; ++i) team.push(0.0);
+  double end = 0.0;
+  for (size_t i = 0; i < coop; ++i) {
+    const double t = team.top() + system_ms(n[i], true);
+    team.pop();
+    team.push(t);
+    end = std::max(end, t);
+  }
+  for (int i = 0; i < sms - held * kMaxC; ++i) sm.push(0.0);
+  for (; !team.empty(); team.pop())
+    for (int i = 0; i < kMaxC; ++i) sm.push(team.top());
+  for (size_t i = coop; i < n.size(); ++i) {
+    const double t = sm.top() + system_ms(n[i], false);
+    sm.pop();
+    sm.push(t);
+    end = std::max(end, t);
+  }
+  return end;
+}
+
+// The size from which systems go to clusters (INT_MAX: none) and the launch's time.  At most 24 sizes are tried.
+int cluster_from(std::vector<int> n, int sms, int teams, double* ms) {
+  std::sort(n.begin(), n.end(), std::greater<int>());
+  *ms = launch_ms(n, 0, sms, 0);
+  int from = INT_MAX;
+  if (teams <= 0 || sms < teams * kMaxC) return from;
+  std::vector<size_t> ends;  // behind the last system of each size
+  for (size_t i = 0; i < n.size() && n[i] >= kCoopMinN; ++i)
+    if (i + 1 == n.size() || n[i + 1] != n[i]) ends.push_back(i + 1);
+  const size_t step = (ends.size() + 23) / 24;
+  for (size_t k = 0; k < ends.size(); k += step) {
+    const double t = launch_ms(n, ends[k], sms, teams);
+    if (t < 0.98 * *ms) {
+      *ms = t;
+      from = n[ends[k] - 1];
+    }
+  }
+  return from;
+}
 
 struct Split {
   int n_coop = 0, n_single = 0;      // largest size of either kind
   int coop = 0, single = 0;          // systems
   int teams = 0, ctas = 0;           // clusters; CTAs for the others
-  double limit = 0.0;                // n^3 above which a system is solved by a cluster
-  bool by_cluster(int n) const { return n >= kCoopMinN && double(n) * n * n > limit; }
+  int from = INT_MAX;                // size from which a system is solved by a cluster
+  bool by_cluster(int n) const { return n >= from; }
   size_t coop_slice() const { return coop ? slice_bytes_for(n_coop) : 0; }
   size_t single_slice() const { return single ? slice_bytes_for(n_single) : 0; }
   size_t slices() const { return coop_slice() * size_t(teams) + single_slice() * size_t(ctas); }
@@ -951,13 +1013,12 @@ int max_teams() {
 Split split_batch(const updes_problem* problems, int32_t count, int32_t ctas) {
   Split s;
   const int sms = sm_count(), teams = ctas > 0 ? 0 : max_teams();
-  auto cost = [&](int32_t i) {
-    const double n = double(problems[i].N) + problems[i].M;
-    return n * n * n;
-  };
-  double total = 0.0;
-  for (int32_t i = 0; i < count; ++i) total += cost(i);
-  s.limit = teams > 0 ? total / std::max(sms, 1) : INFINITY;
+  if (teams > 0) {
+    std::vector<int> n(count);
+    for (int32_t i = 0; i < count; ++i) n[i] = problems[i].N + problems[i].M;
+    double ms;
+    s.from = cluster_from(std::move(n), sms, teams, &ms);
+  }
   for (int32_t i = 0; i < count; ++i) {
     const int n = problems[i].N + problems[i].M;
     if (s.by_cluster(n)) {
@@ -980,6 +1041,20 @@ size_t tables_bytes_for(int32_t count) {
   return align256(size_t(count) * (sizeof(BatchSys) + sizeof(BatchOut) + 4)) + 1024;
 }
 }  // namespace
+
+extern "C" int updes_solve_batched_plan(const int32_t* n, int32_t count, int32_t sms, int32_t teams, int32_t* from,
+                                        double* ms) {
+  if (!n || count <= 0 || sms < 0 || teams < 0 || !from || !ms) return UPDES_ERR_INVALID;
+  for (int32_t i = 0; i < count; ++i)
+    if (n[i] <= 0 || n[i] > kMaxBatchN) return UPDES_ERR_UNSUPPORTED;
+  if (sms == 0) {
+    sms = sm_count();
+    teams = max_teams();
+    if (sms <= 0) return UPDES_ERR_CUDA;
+  }
+  *from = cluster_from(std::vector<int>(n, n + count), sms, teams, ms);
+  return UPDES_OK;
+}
 
 extern "C" int updes_solve_batched_tables(int32_t count, size_t* bytes) {
   if (count <= 0 || !bytes) return UPDES_ERR_INVALID;
