@@ -5,8 +5,8 @@ The reference solves each system with its own ``pde_solver`` call (updes/operato
 boundary rows, right-hand side) and hands them all to ``updes_solve_batched``: where the launch would wait for a few
 large systems they are solved by thread-block clusters of eight CTAs, the others by single CTAs beside them.  Either takes systems from a device work queue, largest first, and runs each one's assembly,
 LU, refinement and values by itself.
-A batch of 128 systems or more is prepared and launched in up to four parts: the host works on a part while the GPU
-solves those before it.
+A batch of 128 systems or more may be prepared and launched in up to four parts: the host works on a part while the GPU
+solves those before it, where that finishes earlier than one launch of all.
 
 Precision per system:
 
@@ -326,9 +326,9 @@ def _tune_widths(batch, precisions, tuner, max_sweeps):
 
 
 def _parts(sizes):
-    """The consecutive parts [first, last) in which a batch is prepared and launched, so that the host prepares a part while
+    """The consecutive pieces [first, last) in which a batch is prepared, so that the host can prepare a piece while
     the GPU solves those before it (256 clouds: 240 ms of preparation, most of it the callers' functions, beside 118 ms
-    of solves): one part below 128 systems, where a part would not fill the GPU; else four with about 30, 30, 25 and 15 %
+    of solves): one below 128 systems, where a part would not fill the GPU; else four with about 30, 30, 25 and 15 %
     of the nodes, the last one small because nothing runs beside its solves."""
     if len(sizes) < 128:
         return [(0, len(sizes))]
@@ -343,7 +343,35 @@ def _parts(sizes):
     return parts
 
 
-def _prepare_part(systems, opts):
+def _finish(ready, later, host, now, gpu, solve):
+    """When the batch is done, at best, and whether ``ready`` should be launched now for it: the systems [first, last) of
+    ``ready`` are prepared, ``later`` are the pieces still to be prepared in ``host`` seconds each, the GPU is free at ``gpu``
+    and ``solve(piece)`` are the seconds of a launch.  A piece that waits is launched with the next."""
+    if not later:
+        return max(now, gpu) + solve(ready), True
+    launch = _finish(later[0], later[1:], host[1:], now + host[0], max(now, gpu) + solve(ready), solve)[0]
+    wait = _finish((ready[0], later[0][1]), later[1:], host[1:], now + host[0], gpu, solve)[0]
+    return min(launch, wait), launch <= wait + 0.01 * (wait - now)  # what is launched is done with, if the rest is as good
+
+
+def _launch_seconds(sizes, precisions, ctas):
+    """The estimated duration of one launch of systems of ``sizes`` unknowns, as a function of a piece [first, last).  FP64
+    takes up to 2.3 times as long."""
+    known = {}
+
+    def solve(piece):
+        if piece not in known:
+            n = sizes[piece[0]:piece[1]]
+            start, ms = ctypes.c_int32(), ctypes.c_double()
+            _lib.check(_lib.load().updes_solve_batched_plan((ctypes.c_int32 * len(n))(*n), len(n), int(ctas), 0,
+                                                            ctypes.byref(start), ctypes.byref(ms)), "updes_solve_batched_plan")
+            fp64 = sum(p == "fp64" for p in precisions[piece[0]:piece[1]]) / len(n)
+            known[piece] = ms.value * 1e-3 * (1.0 + 1.3 * fp64)
+        return known[piece]
+    return solve
+
+
+def _prepare_systems(systems, opts):
     prepared = []
     for sysd in systems:
         bcs = boundary_conditions_func_to_arr(sysd["boundary_conditions"], sysd["cloud"])
@@ -352,8 +380,7 @@ def _prepare_part(systems, opts):
     for sysd in systems:
         if getattr(sysd["cloud"], "sorted_local_supports", None) is not None:
             raise _lib.UpdesError(_lib.ERR_UNSUPPORTED, "updes_solve_batched (local supports)")
-    return _Batch([s["cloud"] for s in systems], [s["rbf"] for s in systems], [s["max_degree"] for s in systems],
-                  prepared, opts.self_term)
+    return prepared
 
 
 def pde_solver_batched(systems, options=None, precision="auto", max_sweeps=4, ctas=0, tuner="default"):
@@ -371,8 +398,8 @@ def pde_solver_batched(systems, options=None, precision="auto", max_sweeps=4, ct
     systems = list(systems)
     if not systems:
         return []
-    for sysd in systems:
-        n = sysd["cloud"].N + compute_nb_monomials(sysd["max_degree"])
+    sizes = [sysd["cloud"].N + compute_nb_monomials(sysd["max_degree"]) for sysd in systems]
+    for n in sizes:
         if n > MAX_N:
             raise ValueError(f"system of n = {n} unknowns exceeds the batched solver's limit of {MAX_N}")
     names = list(precision) if isinstance(precision, (list, tuple)) else [precision] * len(systems)
@@ -383,17 +410,30 @@ def pde_solver_batched(systems, options=None, precision="auto", max_sweeps=4, ct
     st = _lib.OK
     workspace = _Workspace(torch.device("cuda", torch.cuda.current_device()))
     try:
-        for first, last in _parts([s["cloud"].N for s in systems]):
+        pieces = _parts([s["cloud"].N for s in systems])
+        solve = _launch_seconds(sizes, names, ctas)
+        first, prepared, gpu_free = 0, [], 0.0
+        for k, (begin, last) in enumerate(pieces):
             t0 = time.perf_counter()
-            batch = _prepare_part(systems[first:last], opts)
+            prepared += _prepare_systems(systems[begin:last], opts)
+            now = time.perf_counter()
+            prepare_s += now - t0
+            host = [prepare_s * sum(sizes[a:b]) / sum(sizes[:last]) for a, b in pieces[k + 1:]]
+            if not _finish((first, last), pieces[k + 1:], host, now, gpu_free, solve)[1]:
+                continue
+            part = systems[first:last]
+            batch = _Batch([s["cloud"] for s in part], [s["rbf"] for s in part], [s["max_degree"] for s in part], prepared,
+                           opts.self_term)
             precs = [code[p] for p in names[first:last]]
-            prepare_s += time.perf_counter() - t0
+            prepare_s += time.perf_counter() - now
+            gpu_free = max(now, gpu_free) + solve((first, last))
             widths = _tune_widths(batch, precs, tuner, max_sweeps) if tuner is not None else [16] * batch.count
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
             e0.record()
             parts.append((first, batch, precs, widths, batch.begin(list(range(batch.count)), precs, widths, max_sweeps,
                                                                    ctas, workspace), (e0, e1)))
             e1.record()
+            first, prepared = last, []
     finally:
         for _, batch, _, _, begun, _ in parts:
             one = batch.end(begun)
