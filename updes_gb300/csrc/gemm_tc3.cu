@@ -76,16 +76,6 @@ __host__ __device__ constexpr uint32_t idesc(int n) {
   return (1u << 4) | (uint32_t(n >> 3) << 17) | (uint32_t(TM >> 4) << 24);
 }
 
-// tcgen05 shared-memory matrix descriptor: K-major, 64B swizzle, 8-row groups 512 B apart.
-__device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
-  uint64_t d = uint64_t((saddr & 0x3FFFFu) >> 4);
-  d |= uint64_t(1) << 16;
-  d |= uint64_t(512 >> 4) << 32;
-  d |= uint64_t(1) << 46;
-  d |= uint64_t(4) << 61;
-  return d;
-}
-
 __device__ __forceinline__ float pow2f(int e) { return __int_as_float((e + 127) << 23); }
 
 __device__ __forceinline__ int exp_of(float mx) {
@@ -226,18 +216,6 @@ struct Ctrl {
   uint32_t tmem;
   int abort_flag;
 };
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
 
 // A contiguous copy into shared memory that completes on an mbarrier (16-byte aligned, a multiple of 16 bytes).
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint64_t* bar, uint64_t policy) {
