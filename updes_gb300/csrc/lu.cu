@@ -422,9 +422,9 @@ __global__ void __launch_bounds__(4 * COLS) trsm_df64_kernel(float* Whi, float* 
 // number of columns, in which the next block cannot begin; here it is the CTA's own chain, about 45 us, up to the columns that fill
 // the SMs once.
 constexpr int kRowCols = 16;
-// Up to this many columns: n = 2,873 5.59 ms a factorisation against 6.19, 5,000 10.8 against 11.6, 10,006 27.6 against
-// 28.3 (with the launches from 4,096 columns on 27.7, never 27.7), 22,506 107.1 against 107.8 (never: 110.8), because many
-// columns are bound by the FP32 pipes here and by the tensor cores there.
+// Up to this many columns, because many columns are bound by the FP32 pipes here and by the tensor cores there.  A
+// factorisation with this limit and with the launches for any number of columns: n = 2,873 5.59 and 6.19 ms, 5,000 10.8 and
+// 11.6, 10,006 27.6 and 28.3 (limit 4,096: 27.7, none: 27.7), 22,506 107.1 and 107.8 (no limit: 110.8).
 constexpr int kFusedRowCols = 8192;
 struct BlockRowSmem {
   float Xh[256][kRowCols + 1], Xl[256][kRowCols + 1];
@@ -1017,7 +1017,7 @@ int launch_panel(void* W, const float* Wlo, int64_t ldw, TF* F, int64_t ldf, int
   return UPDES_OK;
 }
 
-constexpr int kOuterNb = 4 * kLuNb;   // 256: width of the big exact trailing updates
+constexpr int kOuterNb = 4 * kLuNb;   // 256: width of the big trailing updates
 constexpr int kSwapMapInts = kSwapMapStride;  // one panel's swap map (257 ints used): 2 KB per slot
 constexpr int kLookaheadMinN = 1024;  // smaller factorisations run their steps in order on one stream
 constexpr int kLookaheadCtas = kMaxPanelCtas;  // SMs kept for the look-ahead block beside the trailing update
@@ -1043,7 +1043,7 @@ void add_swap_job(SwapJobs& j, int64_t& maxc, float* plane, int64_t c0, int64_t 
 
 // Mixed LU of the double-float matrix (Whi, Wlo) with FP32 factors overwriting Whi.  Blocks of 256 columns:
 // each block's 64-wide panels are factored with their own updates, then the block row of U is solved and the
-// trailing matrix updated by the exact tensor-core update with K = 256.
+// trailing matrix updated on the tensor cores with K = 256.
 //
 // Look-ahead (n >= kLookaheadMinN): the trailing update after block j is split into the next block's 256
 // columns, done first, and the rest.  The next block is then factored on a second stream on kLookaheadCtas

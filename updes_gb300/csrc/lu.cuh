@@ -12,14 +12,14 @@ int lu_factor_64(int n, double* W, int64_t ld, int32_t* piv, void* ws, size_t ws
                  cudaStream_t s, bool use_digits);
 
 // The panel W[k:n, k:k+w] (w <= 64) factored in place on one thread-block cluster (panel.cu): interchanges to
-// piv[k..k+w) and their net permutation to swap_map (257 ints, may be null).  UPDES_ERR_UNSUPPORTED when its rows do
-// not fit the cluster's shared memory.  after_kernel: launched early, as by launch_next.
+// piv[k..k+w) and their net permutation to swap_map (257 ints, may be null).  UPDES_ERR_UNSUPPORTED when a thread
+// would have more rows than its registers hold.  after_kernel: launched early, as by launch_next.
 int panel_cluster(float* W, int64_t ld, int n, int k, int w, int32_t* piv, int32_t* swap_map, DeviceStatus* st,
                   cudaStream_t s, bool after_kernel);
 int panel_cluster(double* W, int64_t ld, int n, int k, int w, int32_t* piv, int32_t* swap_map, DeviceStatus* st,
                   cudaStream_t s, bool after_kernel);
 
-// mode: 0 = L, 1 = U, 2 = U^T, 3 = L^T (x overwritten in place); sync_ws: ceil(n/64)+1 ints.
+// mode: 0 = L, 1 = U, 2 = U^T, 3 = L^T (x overwritten in place); sync_ws: ceil(n/64)+2 ints.
 // dinv (FP32 factors only, may be null): inverted diagonal blocks from diag_inverse, applied as matvecs
 // instead of the substitution inside each block.
 // xh, xl (n FP32 each, may be null): scratch planes that carry solved blocks in double-float between CTAs
@@ -40,7 +40,8 @@ size_t diag_inverse128_bytes(int n);
 int diag_inverse128(int n, const float* F, int64_t ldf, const float* dinv64, float* dinv128, cudaStream_t s);
 
 // Mixed LU on a double-float working matrix (Whi, Wlo FP32 planes): factors in FP32 (overwriting Whi),
-// every trailing update formed exactly on the tensor cores and accumulated in double-float.
+// every trailing update formed from digit products on the tensor cores (to 2^-27 of |L||U| in the worst case, 2^-33 and
+// better as a rule, see gemm_tc3.cu) and accumulated in double-float.
 size_t lu_df_workspace_bytes(int n);
 int lu_factor_df(int n, float* Whi, float* Wlo, int64_t ld, int32_t* piv, void* ws, size_t ws_bytes, DeviceStatus* st,
                  cudaStream_t s);
