@@ -9,15 +9,18 @@
 // exact but for d2's rounding to 11 bits, at most 2^-33 of the row's maximum.  The products go to three FP32
 // tensor-memory accumulators by their size: g0 = d0 e0, g1 = d0 e1 + d1 e0, g2 = d0 e2 + d1 e1 + d2 e0 + d1 e2 + d2 e1.
 // The 256 products d0 e0 add up to an integer of at most 2^24: the tensor cores add no rounding to g0.  g1 is a multiple
-// of 2^-12, exact up to 2^12; at its largest, 2^16 (every entry of both operands near its maximum, with the same
-// remainder), a step drops at most 2^-8, 2^-32 of that sum's g0.  g2 is rounded below 2^-16 of its 2^8.  d2 e2 (2^-26,
+// of 2^-12, exact up to 2^12.  It gets there only where the remainders behind the leading digits are alike over a row and a
+// column: up to 2^16, where each of its 32 instructions drops 2^-8, 2^-32 of that sum's g0 (constant rows and columns lost
+// all but 2^-26 of |A||B|).  Such rows and columns have their leading digits rounded at spread places instead
+// (spread_place).  g2 is rounded below 2^-16 of its 2^8.  d2 e2 (2^-26,
 // 2^-42 of the largest product) is left out: 8 products.  The epilogue forms g0 + g1 + g2 as a double-float with
 // error-free transformations (FP32 ALU: GB300's FP64 rate is low) and subtracts it from C, once per tile.
 // Measured against 64 bits, relative to |A||B|, K = 256, and beside it three 9-bit integer digits under a scale per 64 of
 // K: normal entries 2^-37.8 (2^-29.1), columns graded by 2^-16 2^-32.8 (2^-27.6), cosines falling as 1/k 2^-33.1
 // (2^-27.6), entries spread over 2^20 2^-29.6 (2^-23.9), within a factor of 4 2^-40.4 (2^-40.2), constant rows and columns
-// 2^-29.1 (2^-36.4).  As a preconditioner the factors are the better for it: 7-8 iterations at n = 22,506 for 9-11.  The small
-// entries of a graded block matter to the Schur complement: with d1 cut at 2^-8 (g1 always exact) it took 14-25.
+// 2^-32 (2^-36.4), 2^-10 of variation over a row 2^-31.  As a preconditioner the factors are the better for it: 7-8 iterations
+// at n = 22,506 for 9-11.
+// The small entries of a graded block matter to the Schur complement: with d1 cut at 2^-8 (g1 always exact) it took 14-25.
 //
 // What bounds it.  The previous form (tiles of 128 x 64, 8 products, a fold of four accumulators per 64 of K) moved 2.6 MB
 // through shared memory for a 128 x 128 x 256 piece and took 25,600 clocks.  So the tiles are 128 x 128, the digit planes
@@ -99,12 +102,33 @@ __device__ __forceinline__ void fast_two_sum2(float2 a, float2 b, float2& s, flo
   e = sub2(b, sub2(s, a));
 }
 
-// The digits of one FP32 value under `scale` (|v * scale| <= 256): every step is exact but the last conversion.
-__device__ __forceinline__ void split3(float v, float scale, float (&d)[kDigits]) {
+// A row or column in whose runs of 64 steps the remainders behind the leading digits add up to more than this in all (in
+// units of that digit, with the entries' signs; without a pattern 7 +- 3) hardly varies: its d1 are alike, and sums with
+// another such one outgrow g1's 24 bits.  Its leading digits are rounded at places spread over the steps instead, which
+// lets the remainders cancel and takes d2 a bit.
+constexpr int kAlike = 24 << 12;  // in units of 2^-12
+__device__ __forceinline__ int remainder_of(float v, float scale) {
+  const float x = fabsf(__fmul_rn(v, scale));
+  return __float2int_rn(__fmul_rn(__fsub_rn(x, rintf(x)), 4096.f));
+}
+// The warp's largest of numbers that are not negative.
+__device__ __forceinline__ float warp_max(float v) {
+  return __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(v)));
+}
+// The k-th place, between -1/2 and 1/2: the fraction of k times the golden ratio, spread evenly over any run of steps and,
+// unlike the bits of k in reverse, over every other or every third step too, where signs may alternate.
+__device__ __forceinline__ float spread_place(int k) {
+  return float(int(unsigned(k) * 0x9E3779B9u)) * 0x1p-32f;
+}
+
+// The digits of one FP32 value under `scale` (|v * scale| < 256), the leading one rounded with `place` added: every step is
+// exact but the last conversion.
+__device__ __forceinline__ void split3(float v, float scale, float place, float (&d)[kDigits]) {
   const float x = __fmul_rn(v, scale);
-  d[0] = rintf(x);
+  d[0] = copysignf(rintf(__fadd_rn(fabsf(x), place)), x);
   const float y = __fmul_rn(__fsub_rn(x, d[0]), 4096.f);
-  const float i1 = rintf(y);  // |i1| <= 2048: 11 bits and a sign, exact in FP16
+  // |y| <= 2048, or 4096 with a place: 11 bits and a sign, exact in FP16 (beyond 2048 the even ones)
+  const float i1 = __half2float(__float2half_rn(rintf(y)));
   d[1] = __fmul_rn(i1, 0x1p-12f);
   d[2] = __fmul_rn(__fsub_rn(y, i1), 0x1p-12f);
 }
@@ -145,17 +169,22 @@ __device__ __forceinline__ void digits_rows(int bx, const float* A, int64_t lda,
       v[u][w] = k < K ? A[r * lda + k] : 0.f;
       mx = fmaxf(mx, fabsf(v[u][w]));
     }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+  mx = warp_max(mx);
   const int e = exp_of(mx);
   if (lane == 0) As[r] = pow2f(e - 8);
   const float scale = pow2f(8 - e);
+  int left = 0;
+#pragma unroll
+  for (int u = 0; u < kMaxK / 64; ++u)
+    left += abs(__reduce_add_sync(0xffffffffu, remainder_of(v[u][0], scale) + remainder_of(v[u][1], scale)));
+  const bool alike = left > kAlike;
 #pragma unroll
   for (int u = 0; u < kMaxK / 64; ++u) {
     if (u * 64 >= Kp) break;
+    const int k = u * 64 + 2 * lane;
     float da[kDigits], db[kDigits];
-    split3(v[u][0], scale, da);
-    split3(v[u][1], scale, db);
+    split3(v[u][0], scale, alike ? spread_place(k) : 0.f, da);
+    split3(v[u][1], scale, alike ? spread_place(k + 1) : 0.f, db);
 #pragma unroll
     for (int p = 0; p < kDigits; ++p)
       *reinterpret_cast<__half2*>(Ad + digit_at(r / TM, int(r % TM), p, u * 64 + 2 * lane, Kp / TK, TM)) =
@@ -178,15 +207,18 @@ __device__ __forceinline__ void digits_cols(int bx, const float* B, int64_t ldb,
     if (gc >= nc) continue;
     float mx = 0.f;
     for (int k = lane; k < Kp; k += 32) mx = fmaxf(mx, fabsf(t[k][c]));
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    mx = warp_max(mx);
     const int e = exp_of(mx);
     if (lane == 0) Bs[gc] = pow2f(e - 8);
     const float scale = pow2f(8 - e);
+    int left = 0;
+    for (int k = lane; k < Kp; k += 64)
+      left += abs(__reduce_add_sync(0xffffffffu, remainder_of(t[k][c], scale) + remainder_of(t[k + 32][c], scale)));
+    const bool alike = left > kAlike;
     for (int k = 2 * lane; k < Kp; k += 64) {
       float da[kDigits], db[kDigits];
-      split3(t[k][c], scale, da);
-      split3(t[k + 1][c], scale, db);
+      split3(t[k][c], scale, alike ? spread_place(k) : 0.f, da);
+      split3(t[k + 1][c], scale, alike ? spread_place(k + 1) : 0.f, db);
 #pragma unroll
       for (int p = 0; p < kDigits; ++p)
         *reinterpret_cast<__half2*>(Bd + digit_at(gc / TN, int(gc % TN), p, k, Kp / TK, TN)) =

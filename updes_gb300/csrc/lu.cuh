@@ -40,8 +40,8 @@ size_t diag_inverse128_bytes(int n);
 int diag_inverse128(int n, const float* F, int64_t ldf, const float* dinv64, float* dinv128, cudaStream_t s);
 
 // Mixed LU on a double-float working matrix (Whi, Wlo FP32 planes): factors in FP32 (overwriting Whi),
-// every trailing update formed from digit products on the tensor cores (to 2^-27 of |L||U| in the worst case, 2^-33 and
-// better as a rule, see gemm_tc3.cu) and accumulated in double-float.
+// every trailing update formed from digit products on the tensor cores (to 2^-31 of |L||U| where its entries are of one size,
+// see gemm_tc3.cu) and accumulated in double-float.
 size_t lu_df_workspace_bytes(int n);
 int lu_factor_df(int n, float* Whi, float* Wlo, int64_t ld, int32_t* piv, void* ws, size_t ws_bytes, DeviceStatus* st,
                  cudaStream_t s);
