@@ -152,6 +152,27 @@ __device__ __forceinline__ void mma_steps(uint32_t d, uint64_t a0, uint64_t b0, 
 }
 
 // ---- digit pre-pass ------------------------------------------------------------------------------------
+// The digits of row r of tile t (`rows` rows a tile): v[u][w] is the entry k = 64 u + 2 lane + w.
+__device__ __forceinline__ void write_digits(const float (&v)[kMaxK / 64][2], float scale, int lane, int Kp, int64_t t, int r,
+                                             int rows, __half* __restrict__ out) {
+  int left = 0;
+#pragma unroll
+  for (int u = 0; u < kMaxK / 64; ++u)
+    left += abs(__reduce_add_sync(0xffffffffu, remainder_of(v[u][0], scale) + remainder_of(v[u][1], scale)));
+  const bool alike = left > kAlike;
+#pragma unroll
+  for (int u = 0; u < kMaxK / 64; ++u) {
+    if (u * 64 >= Kp) break;
+    const int k = u * 64 + 2 * lane;
+    float da[kDigits], db[kDigits];
+    split3(v[u][0], scale, alike ? spread_place(k) : 0.f, da);
+    split3(v[u][1], scale, alike ? spread_place(k + 1) : 0.f, db);
+#pragma unroll
+    for (int p = 0; p < kDigits; ++p)
+      *reinterpret_cast<__half2*>(out + digit_at(t, r, p, k, Kp / TK, rows)) = __floats2half2_rn(da[p], db[p]);
+  }
+}
+
 // A (m x K, lda) -> Ad (see digit_at) and As[r] = 2^(e-8), one warp per row; bx is the block's index among the row
 // part's blocks.
 __device__ __forceinline__ void digits_rows(int bx, const float* A, int64_t lda, int m, int K, int Kp,
@@ -172,24 +193,7 @@ __device__ __forceinline__ void digits_rows(int bx, const float* A, int64_t lda,
   mx = warp_max(mx);
   const int e = exp_of(mx);
   if (lane == 0) As[r] = pow2f(e - 8);
-  const float scale = pow2f(8 - e);
-  int left = 0;
-#pragma unroll
-  for (int u = 0; u < kMaxK / 64; ++u)
-    left += abs(__reduce_add_sync(0xffffffffu, remainder_of(v[u][0], scale) + remainder_of(v[u][1], scale)));
-  const bool alike = left > kAlike;
-#pragma unroll
-  for (int u = 0; u < kMaxK / 64; ++u) {
-    if (u * 64 >= Kp) break;
-    const int k = u * 64 + 2 * lane;
-    float da[kDigits], db[kDigits];
-    split3(v[u][0], scale, alike ? spread_place(k) : 0.f, da);
-    split3(v[u][1], scale, alike ? spread_place(k + 1) : 0.f, db);
-#pragma unroll
-    for (int p = 0; p < kDigits; ++p)
-      *reinterpret_cast<__half2*>(Ad + digit_at(r / TM, int(r % TM), p, u * 64 + 2 * lane, Kp / TK, TM)) =
-          __floats2half2_rn(da[p], db[p]);
-  }
+  write_digits(v, pow2f(8 - e), lane, Kp, r / TM, int(r % TM), TM, Ad);
 }
 
 // B (K x nc, ldb) -> Bd (transposed, in tiles of TN columns) and Bs[c]; a CTA per 32 columns.
@@ -205,25 +209,19 @@ __device__ __forceinline__ void digits_cols(int bx, const float* B, int64_t ldb,
   for (int c = warp; c < 32; c += blockDim.x / 32) {
     const int64_t gc = c0 + c;
     if (gc >= nc) continue;
+    float v[kMaxK / 64][2];
     float mx = 0.f;
-    for (int k = lane; k < Kp; k += 32) mx = fmaxf(mx, fabsf(t[k][c]));
+#pragma unroll
+    for (int u = 0; u < kMaxK / 64; ++u)
+#pragma unroll
+      for (int w = 0; w < 2; ++w) {
+        v[u][w] = u * 64 < Kp ? t[u * 64 + 2 * lane + w][c] : 0.f;
+        mx = fmaxf(mx, fabsf(v[u][w]));
+      }
     mx = warp_max(mx);
     const int e = exp_of(mx);
     if (lane == 0) Bs[gc] = pow2f(e - 8);
-    const float scale = pow2f(8 - e);
-    int left = 0;
-    for (int k = lane; k < Kp; k += 64)
-      left += abs(__reduce_add_sync(0xffffffffu, remainder_of(t[k][c], scale) + remainder_of(t[k + 32][c], scale)));
-    const bool alike = left > kAlike;
-    for (int k = 2 * lane; k < Kp; k += 64) {
-      float da[kDigits], db[kDigits];
-      split3(t[k][c], scale, alike ? spread_place(k) : 0.f, da);
-      split3(t[k + 1][c], scale, alike ? spread_place(k + 1) : 0.f, db);
-#pragma unroll
-      for (int p = 0; p < kDigits; ++p)
-        *reinterpret_cast<__half2*>(Bd + digit_at(gc / TN, int(gc % TN), p, k, Kp / TK, TN)) =
-            __floats2half2_rn(da[p], db[p]);
-    }
+    write_digits(v, pow2f(8 - e), lane, Kp, gc / TN, int(gc % TN), TN, Bd);
   }
 }
 
