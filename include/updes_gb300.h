@@ -168,6 +168,8 @@ UPDES_API int updes_lu_workspace(int32_t n, int32_t precision, size_t* bytes);
  * FP64 and may be A itself (in-place); with UPDES_PREC_FP32, F is FP32 and
  * receives L and U rounded to FP32 while every Schur-complement update is
  * accumulated in FP64 in A (FP32 factors of an FP64-accurate elimination).
+ * FP64 updates are chains of FP64 multiply-adds, for a matrix of any scaling
+ * (updes_solve and updes_factor, which scale theirs, use the tensor cores).
  * piv: device, 2n ints: [0, n) the interchanges (row k swapped with piv[k] at
  * step k, LAPACK getrf convention, 0-based), [n, 2n) the resulting row
  * permutation (row i of P A is row piv[n + i] of A).
@@ -250,6 +252,10 @@ UPDES_API int updes_solve_workspace(const updes_problem* p, const updes_solve_op
  * Assemble, factor and solve K c = [q; 0], then vals = [Phi P] c.
  * q: device, N (interior rhs then boundary values in sorted order);
  * coeffs: device, n; vals: device, N (may be NULL).
+ * FP64 factors come from digit products on the tensor cores; a solution of
+ * theirs (here, in updes_solve_factored and in updes_solve_transpose) with a
+ * backward error above 2^-40 is computed again from factors made by FP64
+ * multiply-adds, which then replace them in the workspace.
  * Replaces pde_solver's assemble_B → lineax QR → core_compute_coefficients
  * sequence (updes/operators.py:602-618).
  */
