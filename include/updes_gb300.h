@@ -254,8 +254,9 @@ UPDES_API int updes_solve_workspace(const updes_problem* p, const updes_solve_op
  * coeffs: device, n; vals: device, N (may be NULL).
  * FP64 factors come from digit products on the tensor cores; a solution of
  * theirs (here, in updes_solve_factored and in updes_solve_transpose) with a
- * backward error above 2^-40 is computed again from factors made by FP64
- * multiply-adds, which then replace them in the workspace.
+ * backward error above 2^-43 and a residual above 128 u |L||U||x| is computed
+ * again from factors made by FP64 multiply-adds, which then replace them in
+ * the workspace.
  * Replaces pde_solver's assemble_B → lineax QR → core_compute_coefficients
  * sequence (updes/operators.py:602-618).
  */

@@ -215,3 +215,67 @@ def test_time_step_values_on_a_small_domain(side, nx, ny, a, degree):
         bound += 512 * 2.0 ** -55 * np.outer(np.abs(phi[:, k:k + 256]).max(1), np.abs(C[k:min(k + 256, N)]).max(0)).astype(float)
     wrong = np.abs(V - want) > bound
     assert not wrong.any(), f"{int(wrong.sum())} values, by up to {np.max(np.abs(V - want) / bound):.1e} of the bound"
+
+
+@pytest.mark.parametrize("index", [12, 24, 36])
+def test_flat_kernels_are_not_factored_again(index):
+    # a Gaussian that is singular to working precision: a large backward error (FP64 multiply-adds: 1e-10 as well) that no
+    # factors can lower, so as many panels as r^3 takes on the same cloud
+    from functools import partial
+    import updes_gb300 as U
+    from updes_gb300 import _lib, operators, workloads
+    system = workloads.uneven_clouds(index + 1)[index]
+
+    def panels(rbf):
+        _lib.stats_reset(timing=True)
+        U.pde_solver(**dict(system, rbf=rbf), options=U.SolverOptions(precision="fp64", reuse_factorization=False))
+        count = _lib.stats_read()["by_class"]["panel"]["count"]
+        _lib.stats_reset()
+        return count, operators.LAST_INFO["backward_error"]
+
+    (once, small), (count, large) = panels(partial(U.polyharmonic, a=1)), panels(system["rbf"])
+    assert small < 2.0 ** -46 and large > 2.0 ** -40
+    assert count == once > 0
+
+
+def test_quintic_kernel_on_two_spacings():
+    # r^5 with half of the nodes at 0.03 of the others' spacing, a backward error hardly above the usual: the values as FP64
+    # multiply-adds give them.  LAPACK's lie 1.2e-7 from extended precision; 16 times what it gives here.
+    import scipy.linalg as sl
+    import updes_gb300 as U
+    from functools import partial
+    nx, ny, wide = 22, 16, np.longdouble
+    X = _nodes(nx, ny, 1.0, seed=0)
+    X = np.where(X[:, :1] < 0.5, X * 0.03, X)
+    cloud = U.SquareCloud(Nx=nx, Ny=ny, coords=X, facet_types={f: "d" for f in ("South", "West", "North", "East")})
+    X = np.asarray(cloud.sorted_nodes)
+    N, Ni = cloud.N, cloud.Ni
+    low, span = X.min(0), X.max(0) - X.min(0)
+    x = ((X - low) / span).T
+    values = np.sin(2.0 * x[0]) * np.exp(x[1])
+    bcs = {f: values[np.asarray(cloud.facet_nodes[f])] for f in cloud.facet_types}
+    lap = lambda x, center, rbf, monomial, fields: U.nodal_laplacian(x, center, rbf, monomial)
+    rhs = lambda x: np.cos(3.0 * (x[0] - low[0]) / span[0] + (x[1] - low[1]) / span[1]) / np.max(span) ** 2
+    got = U.pde_solver(lap, lambda x, centers, rbf, fields: rhs(x), cloud, bcs, partial(U.polyharmonic, a=2), 2,
+                       options=U.SolverOptions(precision="fp64", reuse_factorization=False)).vals
+    Xw = X.astype(wide)
+    r2 = ((Xw[:, None] - Xw[None]) ** 2).sum(-1)
+    x, y = Xw.T
+    P = np.stack([np.ones(N, wide), x, y, x * x, x * y, y * y], axis=1)
+    A = np.concatenate([np.sqrt(r2) * r2 * r2, P], axis=1)
+    K = np.concatenate([A, np.concatenate([P.T, np.zeros((6, 6), wide)], axis=1)])
+    K[:Ni, :N] = (25.0 * np.sqrt(r2) * r2)[:Ni]
+    K[:Ni, N:] = np.array([0, 0, 0, 2, 0, 2], wide)
+    q = np.concatenate([rhs(X[:Ni].T), values[Ni:], np.zeros(6)])
+    size = lambda m: 2.0 ** -np.frexp(m.astype(float))[1].astype(float)
+    r = size(np.abs(K).max(1))
+    c = size(np.abs(K * r[:, None]).max(0))
+    lu = sl.lu_factor((K * r[:, None] * c).astype(float))
+    y = sl.lu_solve(lu, r * q)
+    lapack = (A @ (c * y)).astype(float)
+    y = y.astype(wide)
+    for _ in range(8):
+        y = y + sl.lu_solve(lu, (r * (q - K @ (c * y))).astype(float))
+    want = (A @ (c * y)).astype(float)
+    error = lambda v: np.max(np.abs(v - want)) / np.max(np.abs(want))
+    assert error(got) <= 16.0 * error(lapack)

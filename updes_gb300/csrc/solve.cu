@@ -1077,13 +1077,93 @@ extern "C" int updes_solve_workspace(const updes_problem* p, const updes_solve_o
 
 namespace {
 
+// out = |T| |v| for one triangle T of the factors in F (row-major), L with its unit diagonal: by rows, a warp each, or
+// transposed, a block for 32 columns.  from: v_i is v[from[i]].  With r, also *worst, the largest |r_i| / out_i, r_i being
+// r[to[i]] (an order of non-negative doubles is that of their bits).  Bound by the one read of the triangle; it runs only on
+// solutions whose backward error is large already.
+template <bool TRANS>
+__global__ void __launch_bounds__(256) abs_triangle_kernel(const double* __restrict__ F, int64_t ld, int n, bool lower,
+                                                           const double* __restrict__ v, const int32_t* __restrict__ from,
+                                                           double* __restrict__ out, const double* __restrict__ r,
+                                                           const int32_t* __restrict__ to, unsigned long long* worst) {
+  __shared__ double part[8][32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int i = TRANS ? blockIdx.x * 32 + lane : blockIdx.x * 8 + wid;  // of out
+  auto at = [&](int j) { return fabs(v[from ? from[j] : j]); };
+  double sum = 0.0;
+  if (i < n) {
+    // the entries off the diagonal are before it in L's rows and U's columns, behind it in U's rows and L's columns
+    const bool before = lower != TRANS;
+    const int j0 = before ? 0 : i + 1, j1 = before ? i : n;
+    const int64_t step = TRANS ? ld : 1;
+    const double* f = F + (TRANS ? int64_t(i) : int64_t(i) * ld);
+    for (int j = j0 + (TRANS ? wid : lane); j < j1; j += TRANS ? 8 : 32) sum = fma(fabs(f[j * step]), at(j), sum);
+  }
+  if (TRANS) {
+    part[wid][lane] = sum;
+    __syncthreads();
+    if (wid != 0) return;
+    for (int q = 1; q < 8; ++q) sum += part[q][lane];
+  } else {
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    if (lane != 0) return;
+  }
+  if (i >= n) return;
+  sum = fma(lower ? 1.0 : fabs(F[int64_t(i) * ld + i]), at(i), sum);
+  out[i] = sum;
+  if (r) {
+    const double a = fabs(r[to ? to[i] : i]);
+    atomicMax(worst, static_cast<unsigned long long>(__double_as_longlong(a != 0.0 ? a / sum : 0.0)));
+  }
+}
+
+// *worst = max_i |r_i| / (P^T |L| |U| |x|)_i (trans: (|U^T| |L^T| P |x|)_i) for the FP64 factors and the residual r and
+// solution x that gmres left: what multiply-adds keep below a small multiple of u, however K is graded.
+int residual_by_factors(const SolveWs& w, int n, bool trans, double* worst, cudaStream_t s) {
+  const int32_t* perm = w.piv + n;
+  unsigned long long* dev = reinterpret_cast<unsigned long long*>(w.h);
+  UPDES_CUDA_TRY(cudaMemsetAsync(dev, 0, sizeof *dev, s));
+  const unsigned rows = unsigned(ceil_div(n, 8)), columns = unsigned(ceil_div(n, 32));
+  if (trans) {
+    abs_triangle_kernel<true><<<columns, 256, 0, s>>>(w.W, w.ld, n, true, w.x, perm, w.z, nullptr, nullptr, nullptr);
+    UPDES_LAUNCH_CHECK();
+    abs_triangle_kernel<true><<<columns, 256, 0, s>>>(w.W, w.ld, n, false, w.z, nullptr, w.wv, w.r, nullptr, dev);
+  } else {
+    abs_triangle_kernel<false><<<rows, 256, 0, s>>>(w.W, w.ld, n, false, w.x, nullptr, w.z, nullptr, nullptr, nullptr);
+    UPDES_LAUNCH_CHECK();
+    abs_triangle_kernel<false><<<rows, 256, 0, s>>>(w.W, w.ld, n, true, w.z, nullptr, w.wv, w.r, perm, dev);
+  }
+  UPDES_LAUNCH_CHECK();
+  UPDES_CUDA_TRY(cudaMemcpyAsync(worst, dev, sizeof *worst, cudaMemcpyDeviceToHost, s));
+  UPDES_CUDA_TRY(cudaStreamSynchronize(s));
+  return UPDES_OK;
+}
+
 constexpr int kStateInts = 5;
 
-// Backward error above which factors from digit products are not trusted (8,192 u): K is then factored again by FP64
-// multiply-adds, whatever its rows and columns look like.  The digits' own solutions of the kernels and clouds tried
-// lie at 2e-15 to 8e-14; where the scaled K is still graded (Gaussian kernels that decouple most of the nodes, 36 x 24 nodes on
-// 0.001 x 1: values wrong by 6.7e-12 instead of 6.6e-13) they lie at 1e-11 and above.
-constexpr double kDigitsBackwardError = 0x1p-40;
+// When factors from digit products are not trusted: K is then factored again by FP64 multiply-adds, whatever its rows and
+// columns look like.  Where the scaled K is still graded (Gaussian kernels that decouple most of the nodes, two clusters of
+// very different spacing) the digits can lose what multiply-adds keep: 22 x 16 nodes, one half squeezed to 0.03,
+// values wrong by 1e-2 instead of 1.3e-14 (Gaussian), by 2.2e-6 instead of 1.4e-7 (r^5).  The backward error is then above
+// 1,024 u, 1.7e-13 and more (the kernels and clouds in use: 2e-15 to 1.1e-13).  But a flat Gaussian, singular to working
+// precision, leaves it there too, whatever the factors are made of, so the residual is also compared with what the factors'
+// own size lets multiply-adds leave.  In u: 158 flat Gaussians 2 to 25 from digits, 3 to 23 from multiply-adds; graded
+// kernels 82 to 1e13 (260 and above where the values suffer) and 15 to 69, of which the 48-bit planes of K and x in the
+// residual are up to 64.  512 uneven clouds, half of them flat Gaussians, eight streams: 1.87 s by the backward error alone,
+// 1.27 with both, as without any check.
+constexpr double kDigitsBackwardError = 0x1p-43;
+constexpr double kDigitsResidual = 128 * 0x1p-53;
+
+// Whether the digits' factors have to be made again, after gmres left x and r.
+int digits_failed(const SolveWs& w, int n, bool trans, const updes_solve_info& info, bool* failed, cudaStream_t s) {
+  *failed = false;
+  if (!(info.backward_error > kDigitsBackwardError)) return UPDES_OK;
+  double worst = 0.0;
+  if (int e = residual_by_factors(w, n, trans, &worst, s)) return e;
+  *failed = !(worst <= kDigitsResidual);
+  if (trace_on()) std::fprintf(stderr, "[updes solve n=%d] residual of the factors' size: %.1f u\n", n, worst * 0x1p53);
+  return UPDES_OK;
+}
 
 // Factors of the equilibrated K (double-float planes) at `precision`; records the factored state.
 // planes_ready: the working copy already holds the equilibrated K, written by the assembly: for FP32 factors
@@ -1265,8 +1345,8 @@ int solve_stage(const updes_problem* p, const SolveWs& w, int n, const double* q
     if ((e = read_status(w.lu.st, s, &h))) return e;
     if (h.error) return h.error;
     info->t_refine_ms += t.stop();
-    const bool again = precision == UPDES_PREC_FP64 && !multiply_adds && !info->lu_info &&
-                       info->backward_error > kDigitsBackwardError;
+    bool again = precision == UPDES_PREC_FP64 && !multiply_adds && !info->lu_info;
+    if (again && (e = digits_failed(w, n, false, *info, &again, s))) return e;
     if (precision == UPDES_PREC_FP64 && !again) {
       info->converged = 1;
       break;
@@ -1600,8 +1680,9 @@ extern "C" int updes_solve_transpose(const updes_problem* p, const double* g, do
     updes_solve_opts oi = o;
     if (precision == UPDES_PREC_FP64) oi.max_iters = 0;
     if ((e = gmres(w, n, precision, oi, info, s, true))) return e;
-    if (precision != UPDES_PREC_FP64 || multiply_adds || info->backward_error <= kDigitsBackwardError) break;
-    multiply_adds = true;  // as in solve_stage
+    if (precision != UPDES_PREC_FP64 || multiply_adds) break;
+    if ((e = digits_failed(w, n, true, *info, &multiply_adds, s))) return e;
+    if (!multiply_adds) break;
     bool ready = false;
     if ((e = assemble_stage(p, w, n, precision, info, s, &ready))) return e;
     if ((e = factor_stage(w, n, precision, info, s, ready, multiply_adds))) return e;
